@@ -244,14 +244,15 @@ int32_t mcrt_set_timing(mcrt_executor* executor, int32_t enabled);
 int32_t mcrt_set_capacity(mcrt_executor* executor, int32_t paths);
 
 /* The traversal kernel variants compiled into the library: up to `max`
- * (threads per block, shared-memory short-stack entries per thread) pairs,
- * and *count = how many there are. Variant 0, (128, 4), is the default. No
+ * (threads per block, stack entries) pairs, and *count = how many there are.
+ * Variant 0, (128, 4), is the default. The walk's stack is in local memory,
+ * so the second number names a pair but no longer changes its kernels. No
  * counterpart in the reference (its traversal is one JavaScript loop). */
 int32_t mcrt_traversal_variants(int32_t max, int32_t* blocks, int32_t* stacks, int32_t* count);
 
 /* Chooses the closest-hit and shadow traversal kernels of an executor by
- * block size and short-stack depth (one of mcrt_traversal_variants); the
- * autotuner sets it. Results do not depend on the choice. */
+ * a pair of mcrt_traversal_variants (its block size decides); the autotuner
+ * sets it. Results do not depend on the choice. */
 int32_t mcrt_set_traversal(mcrt_executor* executor, int32_t block, int32_t stack);
 
 int32_t mcrt_get_stats(mcrt_executor* executor, mcrt_stats* out);

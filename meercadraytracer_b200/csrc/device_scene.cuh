@@ -1,9 +1,14 @@
 // Device-resident scene: the layout of a compiled scene in HBM.
 //
 //  nodes   64 B per inner BVH node: both children's boxes and references, so
-//          one inner-node visit is one aligned 64 B fetch (4 x 128-bit loads).
-//  tris    48 B per triangle: the three vertices (for the watertight test)
-//          plus flags / culled side and the material index in the w lanes.
+//          one inner-node visit is one aligned 64 B fetch. A row per axis
+//          holds (left min, right min | left max, right max): register pairs
+//          that sm_100a's two-wide float instructions take as they are loaded.
+//  tris    48 B per triangle: a row per axis of the three vertices (v0, v1 |
+//          v2, flag word). The watertight test permutes the axes by loading
+//          the rows in the ray's order instead of selecting components, so
+//          the flag word stands in every row.
+//  tri_mats  material index per triangle, read once per hit.
 //  attrs   64 B per triangle: vertex normals and uvs, read once per hit.
 //  tangents, colors: per triangle, only where a normal map / vertex colours
 //          are used.
@@ -24,13 +29,11 @@ constexpr int kStackMax = kMaxDepth + 4;
 constexpr int kMaxPassThrough = 64;  // tracer.ts:30
 constexpr int kMaxLights = 63;       // shadow slots: one per light plus the environment estimate
 
-// Child reference of an inner node: count == 0 -> inner node index in `ref`;
-// count > 0 -> leaf covering triangles [ref, ref + count); count < 0 -> absent.
+// Child references: >= 0 an inner node's index, < 0 a leaf whose first
+// triangle is ~ref.
 struct alignas(16) DNode {
-  float4 lxy;   // left  min.x, max.x, min.y, max.y
-  float4 rxy;   // right min.x, max.x, min.y, max.y
-  float4 lrz;   // left  min.z, max.z, right min.z, max.z
-  int4 kids;    // left ref, right ref, left count, right count
+  float4 x, y, z;  // per axis: left min, right min, left max, right max
+  int4 kids;       // left ref, right ref, left count, right count
 };
 
 struct alignas(16) DMaterial {
@@ -83,6 +86,7 @@ struct DFog {
 struct DScene {
   const DNode* nodes;
   const float4* tris;
+  const int* tri_mats;
   const float4* attrs;
   const float4* tangents;
   const float4* colors;  // 3 per triangle, or null
@@ -103,9 +107,9 @@ struct DScene {
   DFog fog;
 };
 
-// Per-triangle packed word in tris[3k].w: flags (bits 0-7), culled side (bits 8-15).
-MCRT_D int tri_flags(float w) { return __float_as_int(w) & 0xff; }
-MCRT_D int tri_side(float w) { return (__float_as_int(w) >> 8) & 0xff; }
+// Per-triangle flag word: flags (bits 0-7), culled side (bits 8-15), last of its leaf (bit 16).
+MCRT_D int tri_flags(int word) { return word & 0xff; }
+MCRT_D int tri_side(int word) { return (word >> 8) & 0xff; }
 
 // ----------------------------------------------------------------- textures
 // wrap, src/textures.ts:229-236.

@@ -62,23 +62,21 @@ int32_t guard(F&& f) {
 }
 
 // ------------------------------------------------------------ conversions
-// tris: v0, v1 = v0 + e1, v2 = v0 + e2 (sums in double, rounded once), with
-// flags | side << 8 and the material index in the w lanes.
+// tris: rows per axis of v0, v1 = v0 + e1, v2 = v0 + e2 (sums in double,
+// rounded once) with flags | side << 8 in every row; tri_mats: materials.
 __global__ void k_pack_tris(const float* __restrict__ t9, const uint32_t* __restrict__ mats,
                             const uint8_t* __restrict__ flags, const uint8_t* __restrict__ sides, int n,
-                            float4* __restrict__ out) {
+                            float4* __restrict__ out, int* __restrict__ mats_out) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const float* t = t9 + 9 * static_cast<size_t>(k);
-  float v1[3], v2[3];
+  const float word = __int_as_float(static_cast<int>(flags[k]) | (static_cast<int>(sides[k]) << 8));
   for (int a = 0; a < 3; a++) {
-    v1[a] = static_cast<float>(static_cast<double>(t[a]) + static_cast<double>(t[3 + a]));
-    v2[a] = static_cast<float>(static_cast<double>(t[a]) + static_cast<double>(t[6 + a]));
+    const float v1 = static_cast<float>(static_cast<double>(t[a]) + static_cast<double>(t[3 + a]));
+    const float v2 = static_cast<float>(static_cast<double>(t[a]) + static_cast<double>(t[6 + a]));
+    out[3 * static_cast<size_t>(k) + a] = make_float4(t[a], v1, v2, word);
   }
-  const int word = static_cast<int>(flags[k]) | (static_cast<int>(sides[k]) << 8);
-  out[3 * static_cast<size_t>(k)] = make_float4(t[0], t[1], t[2], __int_as_float(word));
-  out[3 * static_cast<size_t>(k) + 1] = make_float4(v1[0], v1[1], v1[2], __int_as_float(static_cast<int>(mats[k])));
-  out[3 * static_cast<size_t>(k) + 2] = make_float4(v2[0], v2[1], v2[2], 0.0f);
+  mats_out[k] = static_cast<int>(mats[k]);
 }
 
 // attrs: the 9 normal floats then the 6 uv floats of a triangle, padded to 16.
@@ -107,9 +105,9 @@ __global__ void k_pack_nodes(const float* __restrict__ bounds, const int* __rest
   const float* bl = bounds + 6 * static_cast<size_t>(l);
   const float* br = bounds + 6 * static_cast<size_t>(r);
   DNode d;
-  d.lxy = make_float4(bl[0], bl[3], bl[1], bl[4]);
-  d.rxy = make_float4(br[0], br[3], br[1], br[4]);
-  d.lrz = make_float4(bl[2], bl[5], br[2], br[5]);
+  d.x = make_float4(bl[0], br[0], bl[3], br[3]);
+  d.y = make_float4(bl[1], br[1], bl[4], br[4]);
+  d.z = make_float4(bl[2], br[2], bl[5], br[5]);
   // Child references: an inner node's index, or ~first for a leaf.
   const int lc = nodes[3 * l + 1], rc = nodes[3 * r + 1];
   d.kids = make_int4(lc > 0 ? ~nodes[3 * l] : index[l], rc > 0 ? ~nodes[3 * r] : index[r], lc, rc);
@@ -124,7 +122,8 @@ __global__ void k_mark_leaf_ends(const int* __restrict__ nodes, int m, float4* _
   const int first = nodes[3 * i], count = nodes[3 * i + 1];
   if (count <= 0) return;
   float4* t = tris + 3 * static_cast<size_t>(first + count - 1);
-  t->w = __int_as_float(__float_as_int(t->w) | kLeafEnd);
+  const float word = __int_as_float(__float_as_int(t->w) | kLeafEnd);
+  for (int a = 0; a < 3; a++) t[a].w = word;
 }
 
 int blocks(long long n, int b) { return static_cast<int>((n + b - 1) / b); }
@@ -165,12 +164,12 @@ class DevBuf {
 };
 
 struct GeometryGpu {
-  DevBuf nodes, tris, attrs, tangents, colors;
+  DevBuf nodes, tris, tri_mats, attrs, tangents, colors;
   int tri_count = 0, root_count = 0, node_count = 0;
   float eps = 1e-7f;
   int64_t max_material = -1;
   bool has_colors = false;
-  size_t bytes() const { return nodes.size() + tris.size() + attrs.size() + tangents.size() + colors.size(); }
+  size_t bytes() const { return nodes.size() + tris.size() + tri_mats.size() + attrs.size() + tangents.size() + colors.size(); }
 };
 
 struct TextureGpu {
@@ -262,6 +261,7 @@ DScene make_scene(mcrt_executor* ex) {
   DScene s{};
   s.nodes = ex->geo.nodes.as<DNode>();
   s.tris = ex->geo.tris.as<float4>();
+  s.tri_mats = ex->geo.tri_mats.as<int>();
   s.attrs = ex->geo.attrs.as<float4>();
   s.tangents = ex->geo.tangents.as<float4>();
   s.colors = ex->geo.has_colors ? ex->geo.colors.as<float4>() : nullptr;
@@ -572,8 +572,9 @@ int32_t mcrt_send_geometry(mcrt_executor* ex, int32_t version, const mcrt_geomet
       flags.upload(g->flags, n, s);
       sides.upload(g->sides, n, s);
       G.tris.ensure(sizeof(float4) * 3 * n);
+      G.tri_mats.ensure(sizeof(int) * n);
       k_pack_tris<<<blocks(n, 256), 256, 0, s>>>(t9.as<float>(), mats.as<uint32_t>(), flags.as<uint8_t>(),
-                                                 sides.as<uint8_t>(), n, G.tris.as<float4>());
+                                                 sides.as<uint8_t>(), n, G.tris.as<float4>(), G.tri_mats.as<int>());
       nrm.upload(g->normals, sizeof(float) * 9 * n, s);
       uvs.upload(g->uvs, sizeof(float) * 6 * n, s);
       G.attrs.ensure(sizeof(float) * 16 * n);
@@ -1097,7 +1098,9 @@ int32_t mcrt_compile_instances(mcrt_executor* ex, int32_t version, int32_t count
     G.has_colors = false;
     if (n > 0) {
       G.tris.ensure(sizeof(float4) * 3 * n);
-      k_pack_tris<<<blocks(n, 256), 256, 0, s>>>(g.triangles, g.materials, g.flags, g.sides, n, G.tris.as<float4>());
+      G.tri_mats.ensure(sizeof(int) * n);
+      k_pack_tris<<<blocks(n, 256), 256, 0, s>>>(g.triangles, g.materials, g.flags, g.sides, n, G.tris.as<float4>(),
+                                                 G.tri_mats.as<int>());
       G.attrs.ensure(sizeof(float) * 16 * n);
       k_pack_attrs<<<blocks(n, 256), 256, 0, s>>>(g.normals, g.uvs, n, G.attrs.as<float>());
       G.tangents.ensure(sizeof(float) * 4 * n);

@@ -51,16 +51,13 @@ MCRT_D unsigned int queue_append(unsigned int* counter) {
 }
 
 // ------------------------------------------------------------------- walks
-// The traversal every query kernel runs (traverse_persistent): B threads per
-// block, S shared-memory stack entries per thread, warps refilled once REFILL
-// lanes are idle.
-template <int REFILL, int B, int S, class Q>
+// The traversal every query kernel runs (traverse_persistent), warps refilled
+// once REFILL lanes are idle.
+template <int REFILL, class Q>
 MCRT_D void walk(const DScene& sc, Q& q, int n, unsigned* counter, unsigned& status) {
-  __shared__ int stack[S * B];
-  TravStackT<S> st;
-  st.smem = stack + threadIdx.x;
-  st.stride = B;
-  st.sp = 0;
+  int below[kStackMax + 2];
+  TravStack st;
+  st.init(below);
   traverse_persistent<REFILL>(sc, q, n, counter, st, status);
 }
 
@@ -176,13 +173,17 @@ struct ExtendQuery {
   }
   MCRT_D const TravRay& ray() const { return cs.r; }
   MCRT_D float t_max() const { return cs.tmax; }
-  MCRT_D bool leaf(int first) { return cs.leaf(sc, first); }
+  MCRT_D int side(int word) const { return cs.cull_side(word); }
+  MCRT_D HitAction hit(int k, const TriHit& h, int) {
+    cs.take(k, h);
+    return kGoOn;
+  }
+  MCRT_D bool resume() { return true; }
   MCRT_D void finish() {
-    const ClosestHit& h = cs.h;
-    const unsigned word = h.tri >= 0 ? ((h.front ? 0x80000000u : 0u) | static_cast<unsigned>(h.tri + 1)) : 0u;
-    ps.hit[pid] = make_float4(h.t, h.u, h.v, __uint_as_float(word));
+    ps.hit[pid] = make_float4(cs.t(), cs.u, cs.v, __uint_as_float(cs.hit));
     if (hist) {
-      const int c = h.tri >= 0 ? material_class(sc, h.material) : 0;
+      const int tri = cs.triangle();
+      const int c = tri >= 0 ? material_class(sc, __ldg(sc.tri_mats + tri)) : 0;
       ps.cls[qi] = static_cast<uint8_t>(c);
       atomicAdd(hist + c, 1u);
     }
@@ -207,25 +208,27 @@ struct ClassHistogram {
   }
 };
 
-// B threads per block, S short-stack entries per thread (a traversal variant).
-// 1280 / B blocks per SM: the register cap (48) costs a few bytes of spills
-// and buys a ninth more resident warps than the unconstrained 56 registers.
-template <int B, int S>
-__global__ void __launch_bounds__(B, 1280 / B) k_extend(DScene sc, PathState ps, const int* __restrict__ queue, int n,
+// B threads per block.
+// 1024 / B blocks per SM: 64 registers, no spills (56 with 20 bytes of spills
+// measured 1-2 % slower on incoherent rays, 72 no faster).
+template <int B>
+__global__ void __launch_bounds__(B, 1024 / B) k_extend(DScene sc, PathState ps, const int* __restrict__ queue, int n,
                                               Counters* cnt, unsigned int* bins) {
   __shared__ unsigned int hist[kShadeClasses];
   ClassHistogram ch{bins, hist};
   unsigned status = 0;
   ExtendQuery q{sc, ps, queue, 0, {}, ch.begin(), 0};
-  walk<kRefillClosest, B, S>(sc, q, n, &cnt->fetch, status);
+  walk<kRefillClosest>(sc, q, n, &cnt->fetch, status);
   if (status) atomicOr(&cnt->status, status);
   ch.end();
 }
 
 // The same over a queue of coherent rays (the camera rays), warp by warp
 // (traverse_packet); B / 32 warp stacks of kStackMax entries in shared memory.
+// 1152 / B blocks per SM: 56 registers (12 bytes of spills) were 1 % faster
+// on the 1080p frame than 64.
 template <int B>
-__global__ void __launch_bounds__(B) k_extend_packet(DScene sc, PathState ps, const int* __restrict__ queue, int n,
+__global__ void __launch_bounds__(B, 1152 / B) k_extend_packet(DScene sc, PathState ps, const int* __restrict__ queue, int n,
                                                      Counters* cnt, unsigned int* bins) {
   __shared__ int2 stack[(B / 32) * kStackMax];
   __shared__ unsigned int hist[kShadeClasses];
@@ -247,7 +250,7 @@ MCRT_D int shade_class(const DScene& sc, const PathState& ps, int pid) {
   const unsigned word = __float_as_uint(__ldg(reinterpret_cast<const float*>(ps.hit + pid) + 3));
   const int tri = static_cast<int>(word & 0x7fffffffu) - 1;
   if (tri < 0) return 0;
-  return material_class(sc, __float_as_int(__ldg(&sc.tris[3 * static_cast<size_t>(tri) + 1].w)));
+  return material_class(sc, __ldg(sc.tri_mats + tri));
 }
 
 // Places the block's tile [first, first + blockDim.x) of the queue: ranks
@@ -446,10 +449,10 @@ MCRT_D void shade_path(const DScene& sc, const FrameParams& fp, const PathState&
     T.z *= expf(-m4.z * t);
   }
   V3 va, vb, vc;
-  float4 tw0, tw1;
-  load_tri(sc, tri, va, vb, vc, tw0, tw1);
-  const DMaterial& mat = sc.materials[__float_as_int(tw1.w)];
-  const int tflags = tri_flags(tw0.w);
+  int tword, tmat;
+  load_tri(sc, tri, va, vb, vc, tword, tmat);
+  const DMaterial& mat = sc.materials[tmat];
+  const int tflags = tri_flags(tword);
   const V3 o = V3{o4.x, o4.y, o4.z};
   const V3 p = o + d * t;
   const float w1 = h4.y, w2 = h4.z, w0 = 1.0f - w1 - w2;
@@ -823,64 +826,77 @@ __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSM) k_shade(DScene sc, 
 // ------------------------------------------------------------------ shadow
 // transmittance / attenuateShadow, tracer.ts:529-594, for one shadow ray: the
 // any-hit walk stops at an opaque triangle or when almost no light is left.
+// A hit on a triangle that is not opaque pauses the query: its material is
+// looked up outside the walk's inner loops (resume), whose registers those
+// lookups would otherwise have spilled at every node, and the walk goes on
+// with the rest of the leaf.
 struct ShadowQuery {
   const DScene& sc;
   const PathState& ps;
   int capacity;
   unsigned* status;
-  int pid, slot;
+  // In local memory: the distances of the see-through hits so far, then the
+  // transmittance (3), the depth inside volumes (3) and the hit that paused
+  // the query (4). An array of the kernel's: indexed at run time inside this
+  // struct it would put the ray in local memory too.
+  float* seen;
+  int entry;  // this query's entry of the shadow queue
+  int nseen;  // distances in the list
   bool cast_only, blocked;
   float max_t;
   TravRay r;
-  V3 w, shadow, depth;
-  int nseen;
-  float seen[kShadowSeen];
+  MCRT_D const float4* record() const { return ps.shadow_queue + 3 * static_cast<size_t>(entry); }
   MCRT_D void load(int i) {
-    const float4* e = ps.shadow_queue + 3 * static_cast<size_t>(i);
-    const float4 e0 = e[0], e1 = e[1], e2 = e[2];
-    pid = __float_as_int(e1.w);
-    const int tag = __float_as_int(e2.w);
-    slot = tag & 0xffff;
-    cast_only = (tag & 0x10000) != 0;
-    max_t = e0.w;
-    r = make_trav_ray(V3{e0.x, e0.y, e0.z}, V3{e1.x, e1.y, e1.z});
-    w = V3{e2.x, e2.y, e2.z};
-    shadow = V3{1.0f, 1.0f, 1.0f};
-    depth = V3{0.0f, 0.0f, 0.0f};
+    entry = i;
+    load_ray();
+    cast_only = (__float_as_int(record()[2].w) & 0x10000) != 0;
     nseen = 0;
     blocked = false;
   }
+  MCRT_D void load_ray() {
+    const float4* e = record();
+    const float4 e0 = e[0], e1 = e[1];
+    max_t = e0.w;
+    r = make_trav_ray(V3{e0.x, e0.y, e0.z}, V3{e1.x, e1.y, e1.z});
+  }
   MCRT_D const TravRay& ray() const { return r; }
   MCRT_D float t_max() const { return max_t; }
-  MCRT_D bool leaf(int first) {
-    for (int k = first; k < sc.tri_count; k++) {
-      V3 a, b, c;
-      float4 w0, w1;
-      load_tri(sc, k, a, b, c, w0, w1);
-      const bool last = leaf_end(w0.w);
-      TriHit th;
-      if (intersect_triangle(r, a, b, c, max_t, 2, th) && visit(k, th, w0, w1)) return false;
-      if (last) break;
-    }
-    return true;
-  }
-  // One hit of the visitor; true once the ray is blocked.
-  MCRT_D bool visit(int k, const TriHit& th, float4 w0, float4 w1) {
-    const int fl = tri_flags(w0.w);
-    if (cast_only && (fl & 2) == 0) return false;
+  MCRT_D int side(int) const { return 2; }
+  MCRT_D HitAction hit(int k, const TriHit& h, int word) {
+    const int fl = tri_flags(word);
+    if (cast_only && (fl & 2) == 0) return kGoOn;
     if (fl & 1) {
       blocked = true;
-      return true;
+      return kStop;
     }
-    const DMaterial& mat = sc.materials[__float_as_int(w1.w)];
+    float* at = seen + kShadowSeen + 6;
+    at[0] = h.t;
+    at[1] = h.u;
+    at[2] = h.v;
+    at[3] = __int_as_float(k | (h.front ? static_cast<int>(0x80000000u) : 0));
+    return kPause;
+  }
+  // The visitor's answer to the hit that paused the query; false once the
+  // ray is blocked. The ray is read again afterwards rather than kept.
+  MCRT_D bool resume() {
+    const float* at = seen + kShadowSeen + 6;
+    const float t = at[0], u = at[1], v = at[2];
+    const int tag = __float_as_int(at[3]);
+    see_through(tag & 0x7fffffff, t, u, v, tag < 0);
+    if (blocked) return false;
+    load_ray();
+    return true;
+  }
+  MCRT_D void see_through(int k, float t, float u, float v, bool front) {
+    const DMaterial& mat = sc.materials[__ldg(sc.tri_mats + k)];
     float alpha = mat.opacity;
     V3 col = V3{mat.color[0], mat.color[1], mat.color[2]};
     if (mat.map >= 0 || mat.alpha_map >= 0) {
       const float4* at = sc.attrs + 4 * static_cast<size_t>(k);
       const float4 a2 = __ldg(at + 2), a3 = __ldg(at + 3);
-      const float ww0 = 1.0f - th.u - th.v;
-      const float tu = a2.y * ww0 + a2.w * th.u + a3.y * th.v;
-      const float tv = a2.z * ww0 + a3.x * th.u + a3.z * th.v;
+      const float ww0 = 1.0f - u - v;
+      const float tu = a2.y * ww0 + a2.w * u + a3.y * v;
+      const float tv = a2.z * ww0 + a3.x * u + a3.z * v;
       if (mat.map >= 0) {
         const float4 tx = sample_texture(sc, mat.map, tu, tv);
         alpha *= tx.w;
@@ -888,50 +904,69 @@ struct ShadowQuery {
       }
       if (mat.alpha_map >= 0) alpha *= sample_texture(sc, mat.alpha_map, tu, tv).y;
     }
-    if (mat.alpha_test > 0.0f && alpha < mat.alpha_test) return false;
+    if (mat.alpha_test > 0.0f && alpha < mat.alpha_test) return;
     if (!mat.transparent) alpha = 1.0f;
     bool dup = false;
-    for (int i = 0; i < nseen; i++) dup |= fabsf(seen[i] - th.t) <= sc.eps;
-    if (dup) return false;
+    for (int i = 0; i < nseen; i++) dup |= fabsf(seen[i] - t) <= sc.eps;
+    if (dup) return;
+    float* shadow = seen + kShadowSeen;
+    float* depth = shadow + 3;
+    if (nseen == 0) {
+      for (int i = 0; i < 3; i++) {
+        shadow[i] = 1.0f;
+        depth[i] = 0.0f;
+      }
+    }
     if (nseen < kShadowSeen) {
-      seen[nseen++] = th.t;
+      seen[nseen++] = t;
     } else {
       *status |= kStatusShadowListOverflow;
     }
     if (mat.thickness > 0.0f) {
-      const float sgn = th.front ? -th.t : th.t;
-      depth = depth + V3{mat.attenuation[0], mat.attenuation[1], mat.attenuation[2]} * sgn;
+      const float sgn = front ? -t : t;
+      const V3 d = V3{depth[0], depth[1], depth[2]} + V3{mat.attenuation[0], mat.attenuation[1], mat.attenuation[2]} * sgn;
+      depth[0] = d.x;
+      depth[1] = d.y;
+      depth[2] = d.z;
     }
     const float open = 1.0f - alpha;
     const float through = mat.transmission;
-    shadow = shadow * (V3{open, open, open} + col * (alpha * through));
-    if (shadow.x + shadow.y + shadow.z < 1e-4f) {
-      blocked = true;
-      return true;
-    }
-    return false;
+    const V3 s = V3{shadow[0], shadow[1], shadow[2]} * (V3{open, open, open} + col * (alpha * through));
+    shadow[0] = s.x;
+    shadow[1] = s.y;
+    shadow[2] = s.z;
+    if (s.x + s.y + s.z < 1e-4f) blocked = true;
   }
   MCRT_D void finish() {
+    const float4* e = record();
+    const float4 e2 = e[2];
     V3 result = V3{0.0f, 0.0f, 0.0f};
     if (!blocked) {
-      V3 s = shadow;
-      if (depth.x > 0.0f) s.x *= expf(-depth.x);
-      if (depth.y > 0.0f) s.y *= expf(-depth.y);
-      if (depth.z > 0.0f) s.z *= expf(-depth.z);
-      if (s.x + s.y + s.z > 0.0f) result = w * s;
+      result = V3{e2.x, e2.y, e2.z};
+      if (nseen > 0) {
+        V3 s = V3{seen[kShadowSeen], seen[kShadowSeen + 1], seen[kShadowSeen + 2]};
+        const V3 depth = V3{seen[kShadowSeen + 3], seen[kShadowSeen + 4], seen[kShadowSeen + 5]};
+        if (depth.x > 0.0f) s.x *= expf(-depth.x);
+        if (depth.y > 0.0f) s.y *= expf(-depth.y);
+        if (depth.z > 0.0f) s.z *= expf(-depth.z);
+        result = s.x + s.y + s.z > 0.0f ? result * s : V3{0.0f, 0.0f, 0.0f};
+      }
     }
-    ps.slots[static_cast<size_t>(slot) * capacity + pid] = make_float4(result.x, result.y, result.z, 0.0f);
+    const int slot = __float_as_int(e2.w) & 0xffff;
+    ps.slots[static_cast<size_t>(slot) * capacity + __float_as_int(e[1].w)] =
+        make_float4(result.x, result.y, result.z, 0.0f);
   }
 };
 
-// 1152 / B blocks per SM: at 128 threads a cap of 56 registers (about 30 bytes
-// of spills) keeps nine blocks resident instead of eight, 0.7 % faster; a cap
-// of 48 spills in the walk itself and measured 40 % slower.
-template <int B, int S>
-__global__ void __launch_bounds__(B, 1152 / B) k_shadow(DScene sc, PathState ps, int n, int capacity, Counters* cnt) {
+// 1024 / B blocks per SM: 64 registers; the see-through lookups between the
+// walk's loops spill 44 bytes (72 registers: no spills, no faster; 56: 1-2 %
+// slower).
+template <int B>
+__global__ void __launch_bounds__(B, 1024 / B) k_shadow(DScene sc, PathState ps, int n, int capacity, Counters* cnt) {
   unsigned status = 0;
-  ShadowQuery q{sc, ps, capacity, &status};
-  walk<kRefillShadow, B, S>(sc, q, n, &cnt->fetch_shadow, status);
+  float seen[kShadowSeen + 10];
+  ShadowQuery q{sc, ps, capacity, &status, seen};
+  walk<kRefillShadow>(sc, q, n, &cnt->fetch_shadow, status);
   if (status) atomicOr(&cnt->status, status);
 }
 
@@ -1056,10 +1091,16 @@ struct RayQuery {
   }
   MCRT_D const TravRay& ray() const { return cs.r; }
   MCRT_D float t_max() const { return cs.tmax; }
-  MCRT_D bool leaf(int first) { return cs.leaf(sc, first); }
+  MCRT_D int side(int word) const { return cs.cull_side(word); }
+  MCRT_D HitAction hit(int k, const TriHit& h, int) {
+    cs.take(k, h);
+    return kGoOn;
+  }
+  MCRT_D bool resume() { return true; }
   MCRT_D void finish() {
-    hits[i] = make_int4(cs.h.tri, __float_as_int(cs.h.t), __float_as_int(cs.h.u),
-                        (cs.h.front ? 1 : 0) | (min(cs.tests, 0xffffff) << 8));
+    // A miss counts as a front face, as the walk starts.
+    hits[i] = make_int4(cs.triangle(), __float_as_int(cs.t()), __float_as_int(cs.u),
+                        cs.hit == 0u || (cs.hit >> 31) != 0u ? 1 : 0);
   }
 };
 
@@ -1067,7 +1108,7 @@ __global__ void __launch_bounds__(kBlock) k_trace_rays(DScene sc, const float4* 
                                                        int4* __restrict__ hits, unsigned* fetch) {
   unsigned status = 0;
   RayQuery q{sc, rays, cull, hits, 0, {}};
-  walk<kRefill, kBlock, kShort>(sc, q, n, fetch, status);
+  walk<kRefill>(sc, q, n, fetch, status);
   if (status) atomicOr(fetch + 1, status);
 }
 
@@ -1088,17 +1129,12 @@ struct CountQuery {
   }
   MCRT_D const TravRay& ray() const { return r; }
   MCRT_D float t_max() const { return limit; }
-  MCRT_D bool leaf(int first) {
-    for (int k = first; k < sc.tri_count; k++) {
-      V3 a, b, c;
-      float4 w0, w1;
-      load_tri(sc, k, a, b, c, w0, w1);
-      TriHit th;
-      if (intersect_triangle(r, a, b, c, limit, 2, th)) hits++;
-      if (leaf_end(w0.w)) break;
-    }
-    return true;
+  MCRT_D int side(int) const { return 2; }
+  MCRT_D HitAction hit(int, const TriHit&, int) {
+    hits++;
+    return kGoOn;
   }
+  MCRT_D bool resume() { return true; }
   MCRT_D void finish() { counts[i] = hits; }
 };
 
@@ -1106,7 +1142,7 @@ __global__ void __launch_bounds__(kBlock) k_count_hits(DScene sc, const float4* 
                                                        int* __restrict__ counts, unsigned* fetch) {
   unsigned status = 0;
   CountQuery q{sc, rays, counts, 0, 0, 0.0f, {}};
-  walk<kRefill, kBlock, kShort>(sc, q, n, fetch, status);
+  walk<kRefill>(sc, q, n, fetch, status);
   if (status) atomicOr(fetch + 1, status);
 }
 
@@ -1265,8 +1301,11 @@ int persistent_blocks(K kernel, long long n, int block = kBlock) {
   return static_cast<int>(std::min<long long>(blocks_for(n, block), limit));
 }
 
-// The traversal kernels compiled for each variant (block size, short-stack
-// depth); the autotuner picks one per scene and workload.
+// The traversal kernels of each variant, by block size; the autotuner picks one
+// per scene and workload. A pair's second number, once the depth of a
+// shared-memory short stack, is kept for the callers that name pairs by it:
+// the walk's stack is in local memory, so pairs of one block size share their
+// kernels.
 using ExtendFn = void (*)(DScene, PathState, const int*, int, Counters*, unsigned int*);
 using ShadowFn = void (*)(DScene, PathState, int, int, Counters*);
 
@@ -1276,7 +1315,7 @@ struct PlainVariant {
   ShadowFn shadow;
 };
 
-#define MCRT_PLAIN_VARIANT(B, S) PlainVariant{B, S, k_extend<B, S>, k_shadow<B, S>}
+#define MCRT_PLAIN_VARIANT(B, S) PlainVariant{B, S, k_extend<B>, k_shadow<B>}
 const PlainVariant kPlainVariants[] = {
     MCRT_PLAIN_VARIANT(128, 4), MCRT_PLAIN_VARIANT(128, 8), MCRT_PLAIN_VARIANT(64, 16),
     MCRT_PLAIN_VARIANT(128, 16), MCRT_PLAIN_VARIANT(256, 8), MCRT_PLAIN_VARIANT(256, 16),
@@ -1526,15 +1565,15 @@ __global__ void __launch_bounds__(kBlock) k_batch_raygen(const BatchTables* __re
   }
 }
 
-template <int B, int S>
-__global__ void __launch_bounds__(B, 1280 / B) k_batch_extend(DScene sc, int s, BatchTables* t, PathState ps,
+template <int B>
+__global__ void __launch_bounds__(B, 1024 / B) k_batch_extend(DScene sc, int s, BatchTables* t, PathState ps,
                                                     BatchCounters* bc) {
   SceneQueues* sq = &t->scenes[s];
   const int n = static_cast<int>(sq->count);
   if (n == 0) return;
   unsigned status = 0;
   ExtendQuery q{sc, ps, ps.queue[t->iteration & 1] + sq->base, 0, {}, nullptr, 0};
-  walk<kRefillClosest, B, S>(sc, q, n, &sq->fetch, status);
+  walk<kRefillClosest>(sc, q, n, &sq->fetch, status);
   if (status) atomicOr(&bc->status, status);
 }
 
@@ -1566,8 +1605,8 @@ __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSM) k_batch_shade(DScen
   }
 }
 
-template <int B, int S>
-__global__ void __launch_bounds__(B, 1152 / B) k_batch_shadow(DScene sc, int s, BatchTables* t, PathState ps, int capacity,
+template <int B>
+__global__ void __launch_bounds__(B, 1024 / B) k_batch_shadow(DScene sc, int s, BatchTables* t, PathState ps, int capacity,
                                                     int slots, BatchCounters* bc) {
   SceneQueues* sq = &t->scenes[s];
   const int n = static_cast<int>(sq->shadow_count);
@@ -1575,8 +1614,9 @@ __global__ void __launch_bounds__(B, 1152 / B) k_batch_shadow(DScene sc, int s, 
   unsigned status = 0;
   PathState pq = ps;
   pq.shadow_queue += 3ull * sq->base * static_cast<unsigned>(slots);
-  ShadowQuery q{sc, pq, capacity, &status};
-  walk<kRefillShadow, B, S>(sc, q, n, &sq->fetch_shadow, status);
+  float seen[kShadowSeen + 10];
+  ShadowQuery q{sc, pq, capacity, &status, seen};
+  walk<kRefillShadow>(sc, q, n, &sq->fetch_shadow, status);
   if (status) atomicOr(&bc->status, status);
 }
 
@@ -1733,7 +1773,7 @@ struct BatchVariant {
 };
 
 // The same variants, in the same order, as kPlainVariants.
-#define MCRT_BATCH_VARIANT(B, S) BatchVariant{B, S, k_batch_extend<B, S>, k_batch_shadow<B, S>}
+#define MCRT_BATCH_VARIANT(B, S) BatchVariant{B, S, k_batch_extend<B>, k_batch_shadow<B>}
 const BatchVariant kBatchVariants[] = {
     MCRT_BATCH_VARIANT(128, 4), MCRT_BATCH_VARIANT(128, 8), MCRT_BATCH_VARIANT(64, 16),
     MCRT_BATCH_VARIANT(128, 16), MCRT_BATCH_VARIANT(256, 8), MCRT_BATCH_VARIANT(256, 16),

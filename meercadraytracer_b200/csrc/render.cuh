@@ -201,8 +201,8 @@ struct BatchGrids {
 cudaError_t batch_grids(BatchGrids* g, int variant, int capacity);
 
 // Traversal variants: the closest-hit and shadow kernels compiled for several
-// (threads per block, shared-memory short-stack entries per thread) pairs.
-// Variant 0 is the default (128, 16).
+// block sizes, named by (threads per block, stack entries) pairs; the second
+// number no longer changes the kernels. Variant 0 is the default, (128, 4).
 int traversal_variant_count();
 void traversal_variant_info(int variant, int* block, int* stack);
 int find_traversal_variant(int block, int stack);  // -1 when not compiled
