@@ -58,7 +58,7 @@ MCRT_D void walk(const DScene& sc, Q& q, int n, unsigned* counter, unsigned& sta
   int below[kStackMax + 2];
   TravStack st;
   st.init(below);
-  traverse_persistent<REFILL>(sc, q, n, counter, st, status);
+  traverse_persistent<REFILL>(sc, q, n, query_lanes(n), counter, st, status);
 }
 
 // ---------------------------------------------------------------- mapping
@@ -1301,6 +1301,14 @@ int persistent_blocks(K kernel, long long n, int block = kBlock) {
   return static_cast<int>(std::min<long long>(blocks_for(n, block), limit));
 }
 
+// Blocks of a per-lane walk (traverse_persistent) over n queries: down to one
+// query per warp (query_lanes).
+template <class K>
+int walk_blocks(K kernel, long long n, int block = kBlock) {
+  const int limit = resident_limit(reinterpret_cast<const void*>(kernel), block);
+  return static_cast<int>(std::min<long long>(blocks_for(n, block / 32), limit));
+}
+
 // The traversal kernels of each variant, by block size; the autotuner picks one
 // per scene and workload. A pair's second number, once the depth of a
 // shared-memory short stack, is kept for the callers that name pairs by it:
@@ -1421,7 +1429,7 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
         k_extend_packet<kBlock><<<persistent_blocks(k_extend_packet<kBlock>, n), kBlock, 0, stream>>>(
             scene, ps, ps.queue[cur], n, cnt, class_bins);
       } else {
-        tv.extend<<<persistent_blocks(tv.extend, n, tv.block), tv.block, 0, stream>>>(scene, ps, ps.queue[cur], n,
+        tv.extend<<<walk_blocks(tv.extend, n, tv.block), tv.block, 0, stream>>>(scene, ps, ps.queue[cur], n,
                                                                                       cnt, class_bins);
       }
       tm.stop(st.ms_extend, st.n_extend);
@@ -1452,7 +1460,7 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
       if (n_shadow > 0) {
         cudaMemsetAsync(&cnt->fetch_shadow, 0, sizeof(unsigned int), sh);
         tm.start();
-        tv.shadow<<<persistent_blocks(tv.shadow, n_shadow, tv.block), tv.block, 0, sh>>>(scene, ps, n_shadow, cap,
+        tv.shadow<<<walk_blocks(tv.shadow, n_shadow, tv.block), tv.block, 0, sh>>>(scene, ps, n_shadow, cap,
                                                                                          cnt);
         tm.stop(st.ms_shadow, st.n_shadow);
         st.any_rays += n_shadow;
@@ -1501,7 +1509,7 @@ cudaError_t primary_hits(const DScene& scene, FrameParams fp, PathBuffers& buffe
   k_raygen<<<blocks_for(n, kBlock), kBlock, 0, stream>>>(fp, ps, n);
   cudaMemsetAsync(&buffers.counters()->fetch, 0, sizeof(unsigned int), stream);
   const PlainVariant& tv = plain_variant(0);
-  tv.extend<<<persistent_blocks(tv.extend, n, tv.block), tv.block, 0, stream>>>(scene, ps, ps.queue[0], n,
+  tv.extend<<<walk_blocks(tv.extend, n, tv.block), tv.block, 0, stream>>>(scene, ps, ps.queue[0], n,
                                                                                   buffers.counters(), nullptr);
   return cudaGetLastError();
 }
@@ -1523,7 +1531,7 @@ cudaError_t launch_trace_rays(const DScene& scene, const float4* rays, int count
                               unsigned* fetch, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   cudaMemsetAsync(fetch, 0, sizeof(unsigned), s);
-  k_trace_rays<<<persistent_blocks(k_trace_rays, count), kBlock, 0, s>>>(scene, rays, count, cull, hits, fetch);
+  k_trace_rays<<<walk_blocks(k_trace_rays, count), kBlock, 0, s>>>(scene, rays, count, cull, hits, fetch);
   return cudaGetLastError();
 }
 
@@ -1531,7 +1539,7 @@ cudaError_t launch_count_hits(const DScene& scene, const float4* rays, int count
                               cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   cudaMemsetAsync(fetch, 0, sizeof(unsigned), s);
-  k_count_hits<<<persistent_blocks(k_count_hits, count), kBlock, 0, s>>>(scene, rays, count, counts, fetch);
+  k_count_hits<<<walk_blocks(k_count_hits, count), kBlock, 0, s>>>(scene, rays, count, counts, fetch);
   return cudaGetLastError();
 }
 
