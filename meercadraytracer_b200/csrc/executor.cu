@@ -90,17 +90,20 @@ __global__ void k_pack_attrs(const float* __restrict__ normals, const float* __r
   o[15] = 0.0f;
 }
 
-__global__ void k_inner_flags(const int* __restrict__ nodes, int m, int* __restrict__ flags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m) flags[i] = nodes[3 * i + 1] == 0 ? 1 : 0;
+// One DNode per inner node of the reference layout (first, count, axis with
+// children at first and first + 1), numbered by `index`; without one the tree
+// is numbered breadth first, as the device builder's, where the k-th inner
+// node's children are nodes 1 + 2k and 2 + 2k.
+__device__ __forceinline__ int inner_index(const int* nodes, const int* index, int i) {
+  return index ? index[i] : (nodes[3 * i] - 1) >> 1;
 }
 
-// One DNode per inner node of the reference layout (first, count, axis with
-// children at first and first + 1), numbered in order by `index`.
 __global__ void k_pack_nodes(const float* __restrict__ bounds, const int* __restrict__ nodes,
                              const int* __restrict__ index, int m, DNode* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m || nodes[3 * i + 1] != 0 || index[i] < 0) return;  // a leaf, or unreachable from the root
+  if (i >= m || nodes[3 * i + 1] != 0) return;  // a leaf
+  const int at = inner_index(nodes, index, i);
+  if (at < 0) return;  // unreachable from the root
   const int l = nodes[3 * i], r = l + 1;
   const float* bl = bounds + 6 * static_cast<size_t>(l);
   const float* br = bounds + 6 * static_cast<size_t>(r);
@@ -110,8 +113,9 @@ __global__ void k_pack_nodes(const float* __restrict__ bounds, const int* __rest
   d.z = make_float4(bl[2], br[2], bl[5], br[5]);
   // Child references: an inner node's index, or ~first for a leaf.
   const int lc = nodes[3 * l + 1], rc = nodes[3 * r + 1];
-  d.kids = make_int4(lc > 0 ? ~nodes[3 * l] : index[l], rc > 0 ? ~nodes[3 * r] : index[r], lc, rc);
-  out[index[i]] = d;
+  d.kids = make_int4(lc > 0 ? ~nodes[3 * l] : inner_index(nodes, index, l),
+                     rc > 0 ? ~nodes[3 * r] : inner_index(nodes, index, r), lc, rc);
+  out[at] = d;
 }
 
 // Flags the last triangle of every leaf (kLeafEnd), which ends the leaf's
@@ -207,7 +211,6 @@ struct mcrt_executor {
   RenderStats stats;
   double ms_total = 0;
   DevBuf sum, image, list_x, list_y, out_tile, rays, hits, scratch;
-  DevBuf pack_flag, pack_index, pack_temp;  // node packing of device-compiled geometry, kept across rebuilds
   DevBuf dfg_buf, srgb_lut;
   cudaTextureObject_t dfg_tex = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1108,20 +1111,11 @@ int32_t mcrt_compile_instances(mcrt_executor* ex, int32_t version, int32_t count
                  "copy");
       k_mark_leaf_ends<<<blocks(m, 256), 256, 0, s>>>(g.nodes, m, G.tris.as<float4>());
       if (G.root_count == 0) {
-        // A full binary tree of m nodes has (m - 1) / 2 inner nodes; buffers
-        // are sized for the most any build of n triangles can make, so a
+        // A full binary tree of m nodes has (m - 1) / 2 inner nodes; the buffer
+        // is sized for the most any build of n triangles can make, so a
         // rebuild every frame allocates (and synchronises) nothing.
-        DevBuf& flag = ex->pack_flag;
-        DevBuf& index = ex->pack_index;
-        DevBuf& temp = ex->pack_temp;
-        const size_t m_cap = 2 * static_cast<size_t>(n);
-        flag.ensure(sizeof(int) * m_cap);
-        index.ensure(sizeof(int) * m_cap);
-        k_inner_flags<<<blocks(m, 256), 256, 0, s>>>(g.nodes, m, flag.as<int>());
-        temp.ensure(sizeof(int) * exclusive_scan_scratch());
-        exclusive_scan(flag.as<int>(), index.as<int>(), m, temp.as<int>(), s);
         G.nodes.ensure(sizeof(DNode) * std::max(n - 1, 1));
-        k_pack_nodes<<<blocks(m, 256), 256, 0, s>>>(g.bounds, g.nodes, index.as<int>(), m, G.nodes.as<DNode>());
+        k_pack_nodes<<<blocks(m, 256), 256, 0, s>>>(g.bounds, g.nodes, nullptr, m, G.nodes.as<DNode>());
         cuda_check(cudaGetLastError(), "BVH conversion");
         cuda_check(cudaStreamSynchronize(s), "geometry pack");
       }

@@ -1,13 +1,12 @@
 // GPU binned-SAH BVH build and geometry compile (src/bvh.ts:16-178,
 // src/compile.ts:359-432).
 //
-// The build runs level by level, one thread block per node being split. It
-// makes exactly the reference's decisions: per-triangle bounds and centroids
-// are computed in double and rounded to float as the reference's Float32Array
-// stores do; bins, areas and SAH costs are computed in double; this file is
-// compiled without fused multiply-add contraction so every double operation
-// rounds as JavaScript's does. Hence every node splits the same set of
-// triangles as the reference, with the same 16 bins, leaves of at most 4
+// The build makes exactly the reference's decisions: per-triangle bounds and
+// centroids are computed in double and rounded to float as the reference's
+// Float32Array stores do; bins, areas and SAH costs are computed in double;
+// this file is compiled without fused multiply-add contraction so every double
+// operation rounds as JavaScript's does. Hence every node splits the same set
+// of triangles as the reference, with the same 16 bins, leaves of at most 4
 // (SAH leaves up to 16) and depth at most 100. Only the numbering of nodes
 // (breadth first here) and the order of triangles inside a leaf may differ;
 // partitions here are stable.
@@ -19,7 +18,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <initializer_list>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -36,19 +34,10 @@ static_assert(kBins <= kMaxBins, "the default bin count must fit the bin arrays"
 constexpr int kMaxLeaf = 4;    // bvh.ts:4
 constexpr int kBuildDepth = 100;  // bvh.ts:5
 constexpr int kBuildBlock = 256;
-// A node of at least kWideMin triangles is binned and partitioned by several
-// blocks, kSegment triangles each; the results are combined with exact
-// (order independent) atomics, so the decisions equal a single block's.
-constexpr int kWideMin = 1 << 15;
-constexpr int kSegment = 1 << 13;
-// A node of at most kWarpMax triangles is split by one warp (8 per block):
-// a whole block per node left most threads idle at the deep levels (512
-// measured 5 % faster than 128 on an 83.9M-triangle build, 2048 no faster).
-constexpr int kWarpMax = 512;
-constexpr int kWarpsPerBlock = kBuildBlock / 32;
 // A node of at most kTinyMax triangles is split by half a warp, one triangle
-// per lane: its bins are never materialised (see k_split_tiny).
+// per lane: its bins are never materialised (see sub_split_tiny).
 constexpr int kTinyMax = 16;
+constexpr int kWideMin = 1 << 15;  // see BuildCtl::slot_depth
 
 void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
@@ -73,10 +62,6 @@ struct DevArray {
   }
 };
 
-struct Slot {
-  int node, first, count, depth;
-};
-
 // A resident mesh of instanced geometry.
 struct DMeshRef {
   const float* pos;
@@ -96,45 +81,6 @@ struct DInstance {
   uint32_t material;
 };
 
-// mode: -1 leaf, 0 split at `bin` of `axis` (binned with lo and scale), 1
-// split the run in half.
-struct Split {
-  int mode, axis, bin, nleft;
-  double lo, scale;
-};
-
-// Accumulators of one wide node: bounds (node min xyz, -max xyz, centroid
-// min xyz, -max xyz, all min-reduced), then bin counts and boxes.
-struct WideAcc {
-  float box[12];
-  int cnt[3][kMaxBins];
-  float bb[3][kMaxBins][6];
-  unsigned done;
-};
-
-// Per level: blocks of each slot, where its blocks start, its wide index.
-struct LevelPlan {
-  const int* nb;     // blocks per slot
-  const int* boff;   // first block of each slot
-  const int* wid;    // index into the wide accumulators (valid when nb > 1)
-  int active;        // slots
-};
-
-// Float min / max through integer atomics (exact, order independent).
-__device__ __forceinline__ void atomic_min_f(float* a, float v) {
-  if (__float_as_int(v) >= 0) {
-    atomicMin(reinterpret_cast<int*>(a), __float_as_int(v));
-  } else {
-    atomicMax(reinterpret_cast<unsigned*>(a), __float_as_uint(v));
-  }
-}
-__device__ __forceinline__ void atomic_max_f(float* a, float v) {
-  if (__float_as_int(v) >= 0) {
-    atomicMax(reinterpret_cast<int*>(a), __float_as_int(v));
-  } else {
-    atomicMin(reinterpret_cast<unsigned*>(a), __float_as_uint(v));
-  }
-}
 __device__ __forceinline__ void atomic_min_d(double* a, double v) {
   long long b = __double_as_longlong(v);
   if (b >= 0) {
@@ -181,213 +127,272 @@ __host__ __device__ inline double js_hypot3(double a, double b, double c) {
   return sqrt(sum) * mx;
 }
 
-// Per-triangle box and centroid, bvh.ts:22-33.
-__global__ void k_prepare(const float* __restrict__ tris, int n, float4* __restrict__ bmin, float4* __restrict__ bmax,
-                          float4* __restrict__ cent, uint32_t* __restrict__ order) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float* o = tris + 9 * static_cast<size_t>(i);
-  double lo[3], hi[3];
-  for (int a = 0; a < 3; a++) {
-    const double v0 = o[a], v1 = v0 + static_cast<double>(o[3 + a]), v2 = v0 + static_cast<double>(o[6 + a]);
-    lo[a] = fmin(v0, fmin(v1, v2));
-    hi[a] = fmax(v0, fmax(v1, v2));
-  }
-  bmin[i] = make_float4(static_cast<float>(lo[0]), static_cast<float>(lo[1]), static_cast<float>(lo[2]), 0.0f);
-  bmax[i] = make_float4(static_cast<float>(hi[0]), static_cast<float>(hi[1]), static_cast<float>(hi[2]), 0.0f);
-  cent[i] = make_float4(static_cast<float>((lo[0] + hi[0]) * 0.5), static_cast<float>((lo[1] + hi[1]) * 0.5),
-                        static_cast<float>((lo[2] + hi[2]) * 0.5), 0.0f);
-  order[i] = i;
+// ------------------------------------------------------------------ build
+// Two phases. Nodes of more than kSub triangles are split level by level,
+// each level by two launches over segments of the level's triangles: k_bin
+// bins a segment (several blocks of one node through exact atomics), and the
+// last block of a node takes the split and queues the children; k_part moves
+// the segment's triangles to their sides and gathers the children's bounds on
+// the way. Counts, queues and offsets stay on the device, so the host only
+// enqueues launches. Nodes of at most kSub triangles are then finished, all
+// the way down, by one warp each in shared memory (k_subtrees).
+//
+// Triangles travel as what the build reads of them (box, centroid, index: 40
+// bytes) instead of through an index array, so every pass streams.
+//
+// Numbering. The reference layout here is breadth first: the k-th inner node
+// in (depth, first) order has its children at 1 + 2k and 2 + 2k. Nodes are
+// found in no such order, so each inner node sets a bit at [depth][first], and
+// a prefix count over the bits gives every k (k_rank_*, k_emit).
+//
+// Leaves tile the triangles, and the boundary before each leaf but the first
+// is the split of exactly one inner node: both kinds of node are kept at such
+// a position until they are numbered.
+constexpr int kSub = 256;          // triangles of a subtree that one warp finishes
+constexpr int kSegMax = 4096;      // most triangles of a level kernel's segment (a multiple of kBuildBlock)
+constexpr int kSegMin = 512;
+constexpr unsigned kRootTag = 0xffffffffu;
+constexpr int kLevels = kBuildDepth + 1;
+constexpr int kRankGroup = 8;      // bitmap words per stored prefix
+
+// Floats ordered as integers (min and max by integer atomics and reductions).
+__device__ __forceinline__ int ordered(float f) {
+  const int i = __float_as_int(f);
+  return i ^ ((i >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float unordered(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+
+// A triangle on its way through the build.
+struct Prims {
+  float4* a;  // box min xyz, box max x
+  float4* b;  // box max yz, centroid xy
+  float2* c;  // centroid z, triangle index
+};
+
+// A node of the level phase. box: node min xyz, max xyz, centroid min xyz,
+// max xyz, as ordered integers. tag: twice the parent's first triangle, plus 1
+// for a right child.
+struct Node {
+  int first, count, depth;
+  unsigned tag;
+  int seg0, nseg, acc;
+  unsigned done;
+  int box[12];
+  int mode, axis, bin, nleft;  // the split: 0 binned, 1 the run in half
+  double lo, scale;
+  int child[2];  // index in the next level, or -1: a subtree
+};
+
+struct Subtree {
+  int first, count, depth;
+  unsigned tag;
+  int parity;  // which buffer holds its triangles
+};
+
+// Bins of a node that several blocks share.
+struct Acc {
+  int cnt[3][kMaxBins];
+  int bb[3][kMaxBins][6];
+};
+
+struct LevelCtl {
+  int nodes, segs, accs;
+};
+
+struct BuildCtl {
+  LevelCtl level[kLevels + 1];
+  int subtrees, next_subtree;
+  int inner_depth;   // deepest inner node, -1 for none
+  int slot_depth;    // deepest node that is not a leaf its parent's split already decided
+  int inner_nodes;   // set by k_rank_write
+};
+
+struct BuildState {
+  BuildCtl* ctl;
+  Prims prims[2];
+  Node* nodes[2];
+  int* segs[2];        // node of each segment
+  int* seg_left;       // triangles going left in the node's segments before this one
+  int* seg_cum;        // [segment][axis][bin]: triangles in bins <= bin
+  Acc* acc[2];
+  Subtree* subtrees;
+  // Nodes by position, until they are numbered.
+  float4 *inner_a, *inner_b, *leaf_a, *leaf_b;  // box min xyz, max x | max yz, first or count, depth (| axis << 8)
+  unsigned *inner_t, *leaf_t;                   // tags
+  unsigned* leaf_bits;                          // leaf starts
+  unsigned* depth_bits;                         // [depth][first]: inner nodes
+  int* rank;                                    // inner nodes before each group of kRankGroup words
+  uint32_t* order;
+  int n, words, seg, bins;                      // words: 32-bit words of one bitmap row
+};
+
+__device__ __forceinline__ void set_bit(unsigned* bits, size_t i) { atomicOr(bits + (i >> 5), 1u << (i & 31)); }
+
+__device__ __forceinline__ void put_inner(const BuildState& st, int mid, const float* box, int first, int depth,
+                                          int axis, unsigned tag) {
+  st.inner_a[mid] = make_float4(box[0], box[1], box[2], box[3]);
+  st.inner_b[mid] = make_float4(box[4], box[5], __int_as_float(first), __int_as_float(depth | (axis << 8)));
+  st.inner_t[mid] = tag;
+  set_bit(st.depth_bits, static_cast<size_t>(depth) * st.words * 32 + first);
 }
 
-__device__ __forceinline__ float comp4(float4 v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
-
-__device__ __forceinline__ int bin_of(float c, double lo, double scale, int bins) {
-  return static_cast<int>(fmin(static_cast<double>(bins - 1), floor((static_cast<double>(c) - lo) * scale)));
+__device__ __forceinline__ void put_leaf(const BuildState& st, int first, const float* box, int count, int depth,
+                                         unsigned tag) {
+  st.leaf_a[first] = make_float4(box[0], box[1], box[2], box[3]);
+  st.leaf_b[first] = make_float4(box[4], box[5], __int_as_float(count), __int_as_float(depth));
+  st.leaf_t[first] = tag;
 }
 
-// The slot whose blocks include block b: the last j with boff[j] <= b.
-__device__ __forceinline__ int slot_of_block(const LevelPlan& lp, int b) {
-  int lo = 0, hi = lp.active - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (lp.boff[mid] <= b) {
-      lo = mid;
-    } else {
-      hi = mid - 1;
-    }
-  }
-  return lo;
+__device__ __forceinline__ void add_prim(float* m, float4 a, float4 b, float cz) {
+  m[0] = fminf(m[0], a.x); m[1] = fminf(m[1], a.y); m[2] = fminf(m[2], a.z);
+  m[3] = fmaxf(m[3], a.w); m[4] = fmaxf(m[4], b.x); m[5] = fmaxf(m[5], b.y);
+  m[6] = fminf(m[6], b.z); m[7] = fminf(m[7], b.w); m[8] = fminf(m[8], cz);
+  m[9] = fmaxf(m[9], b.z); m[10] = fmaxf(m[10], b.w); m[11] = fmaxf(m[11], cz);
 }
 
-// Blocks of each slot (0 for a warp- or half-warp-sized node), its wide,
-// small (one warp) and tiny (half a warp) flags.
-__global__ void k_level_plan(const Slot* __restrict__ slots, int active, int* __restrict__ nb,
-                             int* __restrict__ wide, int* __restrict__ small, int* __restrict__ tiny) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= active) return;
-  const int c = slots[j].count;
-  const int w = c >= kWideMin ? 1 : 0;
-  const int ti = c <= kTinyMax ? 1 : 0;
-  const int sm = !ti && c <= kWarpMax ? 1 : 0;
-  nb[j] = w ? (c + kSegment - 1) / kSegment : (sm || ti ? 0 : 1);
-  wide[j] = w;
-  small[j] = sm;
-  tiny[j] = ti;
+__device__ __forceinline__ bool is_max(int i) { return (i >= 3 && i < 6) || i >= 9; }
+
+__device__ __forceinline__ void clear_box(float* m) {
+#pragma unroll
+  for (int i = 0; i < 12; i++) m[i] = is_max(i) ? -INFINITY : INFINITY;
 }
 
-__global__ void k_level_totals(const int* __restrict__ nb, const int* __restrict__ boff,
-                               const int* __restrict__ wide, const int* __restrict__ wid,
-                               const int* __restrict__ small, const int* __restrict__ spos,
-                               const int* __restrict__ tiny, const int* __restrict__ tpos, int active,
-                               int* __restrict__ out) {
-  out[0] = boff[active - 1] + nb[active - 1];
-  out[1] = wid[active - 1] + wide[active - 1];
-  out[2] = spos[active - 1] + small[active - 1];
-  out[3] = tpos[active - 1] + tiny[active - 1];
+// A box's bounds over the warp (every lane gets them), as ordered integers.
+__device__ __forceinline__ int warp_bound(float v, bool max) {
+  const int o = ordered(v);
+  return max ? __reduce_max_sync(0xffffffffu, o) : __reduce_min_sync(0xffffffffu, o);
 }
 
-// The warp-sized slots of a level, listed, then the half-warp-sized ones
-// (from totals[2] on).
-__global__ void k_small_list(const int* __restrict__ small, const int* __restrict__ spos,
-                             const int* __restrict__ tiny, const int* __restrict__ tpos, int active,
-                             const int* __restrict__ totals, int* __restrict__ list) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= active) return;
-  if (small[j]) list[spos[j]] = j;
-  if (tiny[j]) list[totals[2] + tpos[j]] = j;
-}
-
-__global__ void k_wide_init(WideAcc* __restrict__ acc, int count) {
-  const int i = blockIdx.x;
-  if (i >= count) return;
-  WideAcc& a = acc[i];
-  for (int k = threadIdx.x; k < 12; k += blockDim.x) a.box[k] = INFINITY;
-  for (int k = threadIdx.x; k < 3 * kMaxBins; k += blockDim.x) {
-    const int ax = k / kMaxBins, b = k % kMaxBins;
-    a.cnt[ax][b] = 0;
-    for (int q = 0; q < 3; q++) {
-      a.bb[ax][b][q] = INFINITY;
-      a.bb[ax][b][3 + q] = -INFINITY;
-    }
-  }
-  if (threadIdx.x == 0) a.done = 0;
-}
-
-// The 12 bounds of triangles order[first, end) reduced over the block into out[12].
-__device__ void block_bounds(const uint32_t* __restrict__ order, int first, int end, const float4* __restrict__ bmin,
-                             const float4* __restrict__ bmax, const float4* __restrict__ cent, float* out) {
-  __shared__ float red[kBuildBlock / 32][12];
-  const int tid = threadIdx.x;
+// Per-triangle box and centroid, bvh.ts:22-33, and the root's bounds.
+__global__ void __launch_bounds__(kBuildBlock) k_prepare(const float* __restrict__ tris, BuildState st) {
+  __shared__ int red[12];
+  if (threadIdx.x < 12) red[threadIdx.x] = ordered(is_max(threadIdx.x) ? -INFINITY : INFINITY);
+  __syncthreads();
   float m[12];
-  for (int i = 0; i < 12; i++) m[i] = INFINITY;
-  for (int k = first + tid; k < end; k += kBuildBlock) {
-    const uint32_t t = order[k];
-    const float4 a = bmin[t], b = bmax[t], c = cent[t];
-    m[0] = fminf(m[0], a.x); m[1] = fminf(m[1], a.y); m[2] = fminf(m[2], a.z);
-    m[3] = fminf(m[3], -b.x); m[4] = fminf(m[4], -b.y); m[5] = fminf(m[5], -b.z);
-    m[6] = fminf(m[6], c.x); m[7] = fminf(m[7], c.y); m[8] = fminf(m[8], c.z);
-    m[9] = fminf(m[9], -c.x); m[10] = fminf(m[10], -c.y); m[11] = fminf(m[11], -c.z);
+  clear_box(m);
+  const Prims p = st.prims[0];
+  for (int i = blockIdx.x * kBuildBlock + threadIdx.x; i < st.n; i += gridDim.x * kBuildBlock) {
+    const float* o = tris + 9 * static_cast<size_t>(i);
+    double lo[3], hi[3];
+    for (int a = 0; a < 3; a++) {
+      const double v0 = o[a], v1 = v0 + static_cast<double>(o[3 + a]), v2 = v0 + static_cast<double>(o[6 + a]);
+      lo[a] = fmin(v0, fmin(v1, v2));
+      hi[a] = fmax(v0, fmax(v1, v2));
+    }
+    const float4 a4 = make_float4(static_cast<float>(lo[0]), static_cast<float>(lo[1]), static_cast<float>(lo[2]),
+                                  static_cast<float>(hi[0]));
+    const float4 b4 = make_float4(static_cast<float>(hi[1]), static_cast<float>(hi[2]),
+                                  static_cast<float>((lo[0] + hi[0]) * 0.5), static_cast<float>((lo[1] + hi[1]) * 0.5));
+    const float cz = static_cast<float>((lo[2] + hi[2]) * 0.5);
+    p.a[i] = a4;
+    p.b[i] = b4;
+    p.c[i] = make_float2(cz, __int_as_float(i));
+    add_prim(m, a4, b4, cz);
   }
-  for (int off = 16; off > 0; off >>= 1)
-    for (int i = 0; i < 12; i++) m[i] = fminf(m[i], __shfl_xor_sync(0xffffffffu, m[i], off));
-  if ((tid & 31) == 0)
-    for (int i = 0; i < 12; i++) red[tid >> 5][i] = m[i];
-  __syncthreads();
-  if (tid < 12) {
-    float v = INFINITY;
-    for (int w = 0; w < kBuildBlock / 32; w++) v = fminf(v, red[w][tid]);
-    out[tid] = v;
-  }
-  __syncthreads();
-}
-
-// Partial bounds of each wide node, one segment per block.
-__global__ void __launch_bounds__(kBuildBlock) k_bounds(LevelPlan lp, const Slot* __restrict__ slots,
-                                                        const uint32_t* __restrict__ order,
-                                                        const float4* __restrict__ bmin,
-                                                        const float4* __restrict__ bmax,
-                                                        const float4* __restrict__ cent, WideAcc* __restrict__ acc) {
-  __shared__ int sj;
-  if (threadIdx.x == 0) sj = slot_of_block(lp, blockIdx.x);
-  __syncthreads();
-  const int j = sj;
-  if (lp.nb[j] <= 1) return;
-  const Slot s = slots[j];
-  const int seg = blockIdx.x - lp.boff[j];
-  const int first = s.first + seg * kSegment;
-  const int end = min(s.first + s.count, first + kSegment);
-  __shared__ float part[12];
-  block_bounds(order, first, end, bmin, bmax, cent, part);
-  if (threadIdx.x < 12) atomic_min_f(&acc[lp.wid[j]].box[threadIdx.x], part[threadIdx.x]);
-}
-
-// The choice of a node (bvh.ts:137-163) from its cheapest split candidate
-// (best_axis < 0: none): a SAH leaf, the binned split with `nleft` triangles
-// on the left, or the median split when the bins put everything on one side.
-__device__ void commit_choice(const Slot& s, const float* nb, double best_cost, int best_axis, int best_split,
-                              int nleft, const double* lo, const double* scale, int j, int* nodes, Split* split,
-                              int* is_split, bool wide, int* live_out) {
-  Split d{1, 0, 0, s.count >> 1, 0.0, 0.0};
-  bool leaf = false;
-  if (best_axis >= 0) {
-    const double parent_area = area(nb[0], nb[1], nb[2], -static_cast<double>(nb[3]), -static_cast<double>(nb[4]),
-                                     -static_cast<double>(nb[5]));
-    const double split_cost = 1 + (1 * best_cost) / fmax(parent_area, 1e-30);
-    if (split_cost >= 1.0 * s.count && s.count <= 16) {
-      leaf = true;
-    } else {
-      d = Split{0, best_axis, best_split, nleft, lo[best_axis], scale[best_axis]};
-      if (nleft == 0 || nleft == s.count) d = Split{1, best_axis, 0, s.count >> 1, 0.0, 0.0};
+  for (int i = 0; i < 12; i++) {
+    const int v = warp_bound(m[i], is_max(i));
+    if ((threadIdx.x & 31) == 0) {
+      if (is_max(i)) {
+        atomicMax(&red[i], v);
+      } else {
+        atomicMin(&red[i], v);
+      }
     }
   }
-  if (leaf) {
-    int* nd = nodes + 3 * static_cast<size_t>(s.node);
-    nd[0] = s.first; nd[1] = s.count; nd[2] = 0;
-    split[j] = Split{-1, 0, 0, 0, 0.0, 0.0};
-    is_split[j] = 0;
-    live_out[j] = 0;
-  } else {
-    split[j] = d;
-    is_split[j] = 1;
-    // Children that will be leaves whatever the next level decides (few
-    // enough triangles, or at the depth limit) are finished by this node's
-    // scatter when one block partitions it; only the others go on.
-    const bool last = s.depth + 1 >= kBuildDepth;
-    const int small = wide ? 0 : (last || d.nleft <= kMaxLeaf ? 1 : 0) + (last || s.count - d.nleft <= kMaxLeaf ? 1 : 0);
-    live_out[j] = 2 - small;
+  __syncthreads();
+  if (threadIdx.x < 12 && st.ctl->level[0].nodes > 0) {
+    int* box = st.nodes[0][0].box;
+    if (is_max(threadIdx.x)) {
+      atomicMax(box + threadIdx.x, red[threadIdx.x]);
+    } else {
+      atomicMin(box + threadIdx.x, red[threadIdx.x]);
+    }
   }
 }
 
-// The SAH sweeps (bvh.ts:110-134) and the choice (bvh.ts:137-163) of one
-// node from its bins, on one thread. nb: the node's 12 bounds as block_bounds
-// gives them; lo / scale / live: the binning of each axis.
-__device__ void decide(const Slot& s, const float* nb, const int (*cnt)[kMaxBins], const float (*bbox)[kMaxBins][6],
-                       const double* lo, const double* scale, const bool* live, int bins, int j, int* nodes,
-                       Split* split, int* is_split, bool wide, int* live_out) {
-  // Called by the 32 lanes of one warp, lane i holding bin i. The right
-  // sweep's unions and counts are suffix scans, the left sweep's prefix
-  // scans (min, max and sums are exact in any order, and the areas and costs
-  // are the same expressions, so every candidate cost equals the one-thread
-  // sweep's); the first minimum in (axis, split) order wins, as there. The
-  // unions are taken on the float bin bounds and widened to double for the
-  // areas: min and max commute with the exact float-to-double conversion, so
-  // the values are the reference's, for half the shuffles.
+// Math.min(bins - 1, Math.floor((c - lo) * scale)), bvh.ts:98: the product is
+// never negative, so truncation is the floor; a NaN goes to the last bin.
+__device__ __forceinline__ int bin_of(float c, double lo, double scale, int bins) {
+  const double v = (static_cast<double>(c) - lo) * scale;
+  return v < static_cast<double>(bins - 1) ? static_cast<int>(v) : bins - 1;
+}
+
+// Queues a node of the next level (the whole block; the node's index is the
+// same in every thread).
+__device__ void start_node(const BuildState& st, int level, int j, int first, int count, int depth, unsigned tag,
+                           int seg0, int nseg, int acc) {
+  Node& d = st.nodes[level & 1][j];
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    d.first = first;
+    d.count = count;
+    d.depth = depth;
+    d.tag = tag;
+    d.seg0 = seg0;
+    d.nseg = nseg;
+    d.acc = acc;
+    d.done = 0;
+  }
+  if (tid < 12) d.box[tid] = ordered(is_max(tid) ? -INFINITY : INFINITY);
+  for (int i = tid; i < nseg; i += blockDim.x) st.segs[level & 1][seg0 + i] = j;
+  if (acc >= 0) {
+    Acc& a = st.acc[level & 1][acc];
+    for (int i = tid; i < 3 * kMaxBins; i += blockDim.x) {
+      (&a.cnt[0][0])[i] = 0;
+      for (int q = 0; q < 6; q++) (&a.bb[0][0][0])[6 * i + q] = ordered(q < 3 ? INFINITY : -INFINITY);
+    }
+  }
+}
+
+// The root: a node of level 0, or a subtree of its own. One block; the
+// control block is zeroed before it.
+__global__ void __launch_bounds__(kBuildBlock) k_root(BuildState st) {
+  if (st.n <= kSub) {
+    if (threadIdx.x == 0) {
+      st.subtrees[0] = Subtree{0, st.n, 0, kRootTag, 0};
+      st.ctl->subtrees = 1;
+    }
+  } else {
+    const int nseg = (st.n + st.seg - 1) / st.seg;
+    if (threadIdx.x == 0) st.ctl->level[0] = LevelCtl{1, nseg, 1};
+    start_node(st, 0, 0, 0, st.n, 0, kRootTag, 0, nseg, nseg > 1 ? 0 : -1);
+  }
+  if (threadIdx.x == 0) st.ctl->inner_depth = -1;
+}
+
+// The cheapest split of a node's bins (bvh.ts:110-134), on one warp, lane i
+// holding bin i: the right sweep's unions and counts are suffix scans, the
+// left sweep's prefix scans (min, max and sums are exact in any order, and the
+// areas and costs are the same expressions, so every candidate cost equals the
+// one-thread sweep's); the first minimum in (axis, split) order wins, as
+// there. The unions are taken on the float bin bounds and widened to double
+// for the areas: min and max commute with the exact float-to-double
+// conversion, so the values are the reference's, for half the shuffles. The
+// result is the same in every lane.
+struct Choice {
+  double cost;
+  int axis, split, nleft;  // axis < 0: no candidate
+};
+
+__device__ Choice best_split(const int (*cnt)[kMaxBins], const int (*bbox)[kMaxBins][6], const bool* live, int bins) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  double best_cost = INFINITY;
-  int best_axis = -1, best_split = -1;
+  Choice best{INFINITY, -1, -1, 0};
   for (int a = 0; a < 3; a++) {
     if (!live[a]) continue;
     const bool in = lane < bins;
-    const float* o = bbox[a][lane < kMaxBins ? lane : 0];
-    int c = in ? cnt[a][lane] : 0;
-    float b0 = in ? o[0] : INFINITY, b1 = in ? o[1] : INFINITY, b2 = in ? o[2] : INFINITY;
-    float b3 = in ? o[3] : -INFINITY, b4 = in ? o[4] : -INFINITY, b5 = in ? o[5] : -INFINITY;
+    const int* o = bbox[a][lane < kMaxBins ? lane : 0];
+    const int c = in ? cnt[a][lane] : 0;
+    const float b0 = in ? unordered(o[0]) : INFINITY, b1 = in ? unordered(o[1]) : INFINITY;
+    const float b2 = in ? unordered(o[2]) : INFINITY, b3 = in ? unordered(o[3]) : -INFINITY;
+    const float b4 = in ? unordered(o[4]) : -INFINITY, b5 = in ? unordered(o[5]) : -INFINITY;
     // Suffix: bins [lane, bins).
     int rc = c;
     float r0 = b0, r1 = b1, r2 = b2, r3 = b3, r4 = b4, r5 = b5;
-    for (int off = 1; off < 32; off <<= 1) {
+    // Prefix: bins [0, lane].
+    int lc = c;
+    float l0 = b0, l1 = b1, l2 = b2, l3 = b3, l4 = b4, l5 = b5;
+    for (int off = 1; off < bins; off <<= 1) {
       const int oc = __shfl_down_sync(full, rc, off);
       const float o0 = __shfl_down_sync(full, r0, off), o1 = __shfl_down_sync(full, r1, off);
       const float o2 = __shfl_down_sync(full, r2, off), o3 = __shfl_down_sync(full, r3, off);
@@ -397,22 +402,17 @@ __device__ void decide(const Slot& s, const float* nb, const int (*cnt)[kMaxBins
         r0 = fminf(r0, o0); r1 = fminf(r1, o1); r2 = fminf(r2, o2);
         r3 = fmaxf(r3, o3); r4 = fmaxf(r4, o4); r5 = fmaxf(r5, o5);
       }
-    }
-    const double right_area = rc > 0 ? area(r0, r1, r2, r3, r4, r5) : 0;
-    // Prefix: bins [0, lane].
-    int lc = c;
-    float l0 = b0, l1 = b1, l2 = b2, l3 = b3, l4 = b4, l5 = b5;
-    for (int off = 1; off < 32; off <<= 1) {
-      const int oc = __shfl_up_sync(full, lc, off);
-      const float o0 = __shfl_up_sync(full, l0, off), o1 = __shfl_up_sync(full, l1, off);
-      const float o2 = __shfl_up_sync(full, l2, off), o3 = __shfl_up_sync(full, l3, off);
-      const float o4 = __shfl_up_sync(full, l4, off), o5 = __shfl_up_sync(full, l5, off);
+      const int pc = __shfl_up_sync(full, lc, off);
+      const float p0 = __shfl_up_sync(full, l0, off), p1 = __shfl_up_sync(full, l1, off);
+      const float p2 = __shfl_up_sync(full, l2, off), p3 = __shfl_up_sync(full, l3, off);
+      const float p4 = __shfl_up_sync(full, l4, off), p5 = __shfl_up_sync(full, l5, off);
       if (lane >= off) {
-        lc += oc;
-        l0 = fminf(l0, o0); l1 = fminf(l1, o1); l2 = fminf(l2, o2);
-        l3 = fmaxf(l3, o3); l4 = fmaxf(l4, o4); l5 = fmaxf(l5, o5);
+        lc += pc;
+        l0 = fminf(l0, p0); l1 = fminf(l1, p1); l2 = fminf(l2, p2);
+        l3 = fmaxf(l3, p3); l4 = fmaxf(l4, p4); l5 = fmaxf(l5, p5);
       }
     }
+    const double right_area = rc > 0 ? area(r0, r1, r2, r3, r4, r5) : 0;
     // Split after bin `lane`: the left union with the right union from lane + 1.
     const int rc2 = __shfl_down_sync(full, rc, 1);
     const double ra2 = __shfl_down_sync(full, right_area, 1);
@@ -421,228 +421,419 @@ __device__ void decide(const Slot& s, const float* nb, const int (*cnt)[kMaxBins
       cost = lc * area(l0, l1, l2, l3, l4, l5) + rc2 * ra2;
       if (isnan(cost)) cost = INFINITY;
     }
-    int at = lane;
+    int at = lane, atl = lc;
     for (int off = 16; off > 0; off >>= 1) {
       const double oc = __shfl_xor_sync(full, cost, off);
       const int oi = __shfl_xor_sync(full, at, off);
+      const int ol = __shfl_xor_sync(full, atl, off);
       if (oc < cost || (oc == cost && oi < at)) {
         cost = oc;
         at = oi;
+        atl = ol;
       }
     }
-    if (cost < best_cost) {
-      best_cost = cost;
-      best_axis = a;
-      best_split = at;
-    }
+    if (cost < best.cost) best = Choice{cost, a, at, atl};
   }
-  if (lane != 0) return;
-  int nleft = 0;
-  if (best_axis >= 0)
-    for (int i = 0; i <= best_split; i++) nleft += cnt[best_axis][i];
-  commit_choice(s, nb, best_cost, best_axis, best_split, nleft, lo, scale, j, nodes, split, is_split, wide, live_out);
+  return best;
 }
 
-// Bounds, leaf test, binning and SAH choice of every node of a level
-// (bvh.ts:55-144). A node of one block is handled by that block alone; the
-// blocks of a wide node bin their segments into the node's accumulators
-// (k_bounds has reduced its bounds) and the last block to finish decides.
-__global__ void __launch_bounds__(kBuildBlock) k_split(LevelPlan lp, const Slot* __restrict__ slots,
-                                                       const uint32_t* __restrict__ order,
-                                                       const float4* __restrict__ bmin, const float4* __restrict__ bmax,
-                                                       const float4* __restrict__ cent, float* __restrict__ bounds,
-                                                       int* __restrict__ nodes, Split* __restrict__ split,
-                                                       int* __restrict__ is_split, WideAcc* __restrict__ acc,
-                                                       int bins, int* __restrict__ live_children) {
-  __shared__ int sj;
-  __shared__ float nb[12];  // node min xyz, -max xyz, centroid min xyz, -max xyz
+// The choice (bvh.ts:137-163): mode -1 a SAH leaf, 0 the binned split, 1 the
+// run in half (no candidate, or the bins put everything on one side).
+__device__ __forceinline__ int choose(const Choice& c, const float* box, int count, int& axis, int& nleft) {
+  axis = max(c.axis, 0);
+  nleft = count >> 1;
+  if (c.axis < 0) return 1;
+  const double parent_area = area(box[0], box[1], box[2], box[3], box[4], box[5]);
+  const double split_cost = 1 + (1 * c.cost) / fmax(parent_area, 1e-30);
+  if (split_cost >= 1.0 * count && count <= 16) return -1;
+  if (c.nleft == 0 || c.nleft == count) return 1;
+  nleft = c.nleft;
+  return 0;
+}
+
+__device__ __forceinline__ void binning(const float* cmin, const float* cmax, int bins, double* lo, double* scale,
+                                        bool* live) {
+  for (int a = 0; a < 3; a++) {
+    lo[a] = cmin[a];
+    const double extent = static_cast<double>(cmax[a]) - lo[a];
+    live[a] = extent > 0;
+    scale[a] = live[a] ? bins / extent : 0.0;
+  }
+}
+
+__device__ __forceinline__ void bin_prim(int* cnt, int* bb, const int* v) {
+  atomicAdd(cnt, 1);
+  atomicMin(bb, v[0]); atomicMin(bb + 1, v[1]); atomicMin(bb + 2, v[2]);
+  atomicMax(bb + 3, v[3]); atomicMax(bb + 4, v[4]); atomicMax(bb + 5, v[5]);
+}
+
+// One segment of a level (see above). What bounds it: shared-memory atomics,
+// seven per triangle and axis. A warp whose triangles all fall into one bin of
+// an axis (neighbours in the model, at the upper levels) reduces them first
+// and adds once.
+__global__ void __launch_bounds__(kBuildBlock) k_bin(int level, BuildState st) {
+  using Scan = cub::BlockScan<int, kBuildBlock>;
+  __shared__ typename Scan::TempStorage scan_tmp;
   __shared__ int cnt[3][kMaxBins];
-  __shared__ float bbox[3][kMaxBins][6];
-  __shared__ int last;
-  const int tid = threadIdx.x;
-  if (tid == 0) sj = slot_of_block(lp, blockIdx.x);
-  __syncthreads();
-  const int j = sj;
-  const Slot s = slots[j];
-  const int blocks = lp.nb[j];
-  const bool wide = blocks > 1;
-  const int seg = blockIdx.x - lp.boff[j];
-  WideAcc* wa = wide ? acc + lp.wid[j] : nullptr;
-  if (wide) {
-    if (tid < 12) nb[tid] = __ldcg(&wa->box[tid]);
+  __shared__ int bbox[3][kMaxBins][6];
+  __shared__ int s_flag, s_child[2], s_seg0[2], s_acc[2], s_mode, s_axis, s_bin, s_nleft;
+  const unsigned full = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int bins = st.bins, total = st.ctl->level[level].segs;
+  const Prims p = st.prims[level & 1];
+  for (int s = blockIdx.x; s < total; s += gridDim.x) {
+    __syncthreads();  // the last segment's shared values are no longer read
+    const int j = st.segs[level & 1][s];
+    Node& nd = st.nodes[level & 1][j];
+    const int nfirst = nd.first, ncount = nd.count, nseg = nd.nseg, seg = s - nd.seg0, depth = nd.depth;
+    for (int i = tid; i < 3 * kMaxBins; i += kBuildBlock) {
+      (&cnt[0][0])[i] = 0;
+      for (int q = 0; q < 6; q++) (&bbox[0][0][0])[6 * i + q] = ordered(q < 3 ? INFINITY : -INFINITY);
+    }
+    float box[12];
+    for (int i = 0; i < 12; i++) box[i] = unordered(nd.box[i]);
+    double lo[3], scale[3];
+    bool live[3];
+    binning(box + 6, box + 9, bins, lo, scale, live);
     __syncthreads();
-  } else {
-    block_bounds(order, s.first, s.first + s.count, bmin, bmax, cent, nb);
-  }
-  if (tid == 0 && seg == 0) {
-    float* bo = bounds + 6 * static_cast<size_t>(s.node);
-    bo[0] = nb[0]; bo[1] = nb[1]; bo[2] = nb[2];
-    bo[3] = -nb[3]; bo[4] = -nb[4]; bo[5] = -nb[5];
-  }
-  if (s.count <= kMaxLeaf || s.depth >= kBuildDepth) {
-    if (tid == 0 && seg == 0) {
-      int* nd = nodes + 3 * static_cast<size_t>(s.node);
-      nd[0] = s.first; nd[1] = s.count; nd[2] = 0;
-      split[j] = Split{-1, 0, 0, 0, 0.0, 0.0};
-      is_split[j] = 0;
-      live_children[j] = 0;
-    }
-    return;
-  }
-  for (int i = tid; i < 3 * kMaxBins; i += kBuildBlock) {
-    const int a = i / kMaxBins, b = i % kMaxBins;
-    cnt[a][b] = 0;
-    for (int q = 0; q < 3; q++) {
-      bbox[a][b][q] = INFINITY;
-      bbox[a][b][3 + q] = -INFINITY;
-    }
-  }
-  // Bin the centroids along every axis with extent (bvh.ts:89-109).
-  const double cmin[3] = {nb[6], nb[7], nb[8]};
-  const double cmax[3] = {-nb[9], -nb[10], -nb[11]};
-  double lo[3], scale[3];
-  bool live[3];
-  for (int a = 0; a < 3; a++) {
-    lo[a] = cmin[a];
-    const double extent = cmax[a] - lo[a];
-    live[a] = extent > 0;
-    scale[a] = live[a] ? bins / extent : 0.0;
-  }
-  __syncthreads();
-  const int first = wide ? s.first + seg * kSegment : s.first;
-  const int end = wide ? min(s.first + s.count, first + kSegment) : s.first + s.count;
-  for (int k = first + tid; k < end; k += kBuildBlock) {
-    const uint32_t t = order[k];
-    const float4 a4 = bmin[t], b4 = bmax[t], c4 = cent[t];
-    for (int a = 0; a < 3; a++) {
-      if (!live[a]) continue;
-      const int b = bin_of(comp4(c4, a), lo[a], scale[a], bins);
-      atomicAdd(&cnt[a][b], 1);
-      atomic_min_f(&bbox[a][b][0], a4.x);
-      atomic_min_f(&bbox[a][b][1], a4.y);
-      atomic_min_f(&bbox[a][b][2], a4.z);
-      atomic_max_f(&bbox[a][b][3], b4.x);
-      atomic_max_f(&bbox[a][b][4], b4.y);
-      atomic_max_f(&bbox[a][b][5], b4.z);
-    }
-  }
-  __syncthreads();
-  if (wide) {
-    // Fold this segment's bins into the node's, then let the last block decide.
-    for (int i = tid; i < 3 * bins; i += kBuildBlock) {
-      const int a = i / bins, b = i % bins;
-      if (!live[a] || cnt[a][b] == 0) continue;
-      atomicAdd(&wa->cnt[a][b], cnt[a][b]);
-      for (int q = 0; q < 3; q++) {
-        atomic_min_f(&wa->bb[a][b][q], bbox[a][b][q]);
-        atomic_max_f(&wa->bb[a][b][3 + q], bbox[a][b][3 + q]);
+    const int first = nfirst + seg * st.seg, end = min(nfirst + ncount, first + st.seg);
+    for (int base = first; base < end; base += kBuildBlock) {
+      const int k = base + tid;
+      const bool valid = k < end;
+      float4 a4 = make_float4(INFINITY, INFINITY, INFINITY, -INFINITY);
+      float4 b4 = make_float4(-INFINITY, -INFINITY, 0.0f, 0.0f);
+      float cz = 0.0f;
+      if (valid) {
+        a4 = p.a[k];
+        b4 = p.b[k];
+        cz = p.c[k].x;
+      }
+      const int v[6] = {ordered(a4.x), ordered(a4.y), ordered(a4.z), ordered(a4.w), ordered(b4.x), ordered(b4.y)};
+      const float c3[3] = {b4.z, b4.w, cz};
+      const int here = __popc(__ballot_sync(full, valid));
+      if (here == 0) continue;
+      int w[6];
+      bool reduced = false;
+      for (int a = 0; a < 3; a++) {
+        if (!live[a]) continue;
+        const int b = valid ? bin_of(c3[a], lo[a], scale[a], bins) : 0;
+        const int b0 = __shfl_sync(full, b, 0);  // lane 0 is valid when any is
+        if (__all_sync(full, !valid || b == b0)) {
+          if (!reduced) {
+            for (int q = 0; q < 6; q++)
+              w[q] = q < 3 ? __reduce_min_sync(full, v[q]) : __reduce_max_sync(full, v[q]);
+            reduced = true;
+          }
+          if (lane == 0) {
+            bin_prim(&cnt[a][b0], bbox[a][b0], w);
+            if (here > 1) atomicAdd(&cnt[a][b0], here - 1);
+          }
+        } else if (valid) {
+          bin_prim(&cnt[a][b], bbox[a][b], v);
+        }
       }
     }
-    __threadfence();
     __syncthreads();
-    if (tid == 0) last = atomicAdd(&wa->done, 1u) == static_cast<unsigned>(blocks - 1) ? 1 : 0;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int i = tid; i < 3 * bins; i += kBuildBlock) {
-      const int a = i / bins, b = i % bins;
-      cnt[a][b] = __ldcg(&wa->cnt[a][b]);
-      for (int q = 0; q < 6; q++) bbox[a][b][q] = __ldcg(&wa->bb[a][b][q]);
+    if (nseg > 1) {
+      // This segment's cumulative counts, and its bins folded into the node's.
+      Acc& acc = st.acc[level & 1][nd.acc];
+      if (tid < 96) {
+        const int a = tid >> 5;
+        int c = cnt[a][lane];
+        for (int off = 1; off < 32; off <<= 1) {
+          const int o = __shfl_up_sync(full, c, off);
+          if (lane >= off) c += o;
+        }
+        st.seg_cum[(static_cast<size_t>(s) * 3 + a) * kMaxBins + lane] = c;
+      }
+      for (int i = tid; i < 3 * bins; i += kBuildBlock) {
+        const int a = i / bins, b = i - a * bins;
+        if (!live[a] || cnt[a][b] == 0) continue;
+        atomicAdd(&acc.cnt[a][b], cnt[a][b]);
+        for (int q = 0; q < 3; q++) {
+          atomicMin(&acc.bb[a][b][q], bbox[a][b][q]);
+          atomicMax(&acc.bb[a][b][3 + q], bbox[a][b][3 + q]);
+        }
+      }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_flag = atomicAdd(&nd.done, 1u) == static_cast<unsigned>(nseg - 1) ? 1 : 0;
+      __syncthreads();
+      if (!s_flag) continue;
+      __threadfence();
+      for (int i = tid; i < 3 * kMaxBins; i += kBuildBlock) {
+        (&cnt[0][0])[i] = __ldcg(&acc.cnt[0][0] + i);
+        for (int q = 0; q < 6; q++) (&bbox[0][0][0])[6 * i + q] = __ldcg(&acc.bb[0][0][0] + 6 * i + q);
+      }
+      __syncthreads();
+    }
+    if (tid < 32) {
+      const Choice c = best_split(cnt, bbox, live, bins);
+      if (lane == 0) {
+        int axis, nleft;
+        const int mode = choose(c, box, ncount, axis, nleft);  // never a leaf: more than kSub triangles
+        nd.mode = s_mode = mode;
+        nd.axis = s_axis = axis;
+        nd.bin = s_bin = c.split;
+        nd.nleft = s_nleft = nleft;
+        nd.lo = lo[axis];
+        nd.scale = scale[axis];
+        put_inner(st, nfirst + nleft, box, nfirst, depth, axis, nd.tag);
+        atomicMax(&st.ctl->inner_depth, depth);
+        const int kids[2] = {nleft, ncount - nleft};
+        const bool last = depth + 1 >= kBuildDepth;
+        int deepest = depth;
+        for (int q = 0; q < 2; q++) {
+          s_child[q] = -1;
+          s_acc[q] = -1;
+          if (kids[q] > kSub && !last) {
+            const int ns = (kids[q] + st.seg - 1) / st.seg;
+            LevelCtl& next = st.ctl->level[level + 1];
+            s_child[q] = atomicAdd(&next.nodes, 1);
+            s_seg0[q] = atomicAdd(&next.segs, ns);
+            if (ns > 1) s_acc[q] = atomicAdd(&next.accs, 1);
+          } else {
+            const int t = atomicAdd(&st.ctl->subtrees, 1);
+            st.subtrees[t] = Subtree{nfirst + (q ? nleft : 0), kids[q], depth + 1,
+                                     2u * static_cast<unsigned>(nfirst) + q, (level + 1) & 1};
+            // A wide node's small children were nodes of the next level.
+            if (ncount >= kWideMin) deepest = depth + 1;
+          }
+          nd.child[q] = s_child[q];
+        }
+        atomicMax(&st.ctl->slot_depth, deepest);
+      }
     }
     __syncthreads();
+    for (int q = 0; q < 2; q++) {
+      if (s_child[q] < 0) continue;
+      const int kc = q ? ncount - s_nleft : s_nleft;
+      start_node(st, level + 1, s_child[q], nfirst + (q ? s_nleft : 0), kc, depth + 1,
+                 2u * static_cast<unsigned>(nfirst) + q, s_seg0[q], (kc + st.seg - 1) / st.seg, s_acc[q]);
+    }
+    // Triangles going left before each of the node's segments.
+    const int seg0 = s - seg;
+    int running = 0;
+    for (int base = 0; base < nseg; base += kBuildBlock) {
+      const int i = base + tid;
+      int left = 0;
+      if (i < nseg && nseg > 1) {
+        left = s_mode == 0 ? __ldcg(&st.seg_cum[(static_cast<size_t>(seg0 + i) * 3 + s_axis) * kMaxBins + s_bin])
+                           : max(0, min(s_nleft - i * st.seg, min(st.seg, ncount - i * st.seg)));
+      }
+      int pre = 0, sum = 0;
+      Scan(scan_tmp).ExclusiveSum(left, pre, sum);
+      if (i < nseg) st.seg_left[seg0 + i] = running + pre;
+      running += sum;
+      __syncthreads();
+    }
   }
-  if (tid < 32) decide(s, nb, cnt, bbox, lo, scale, live, bins, j, nodes, split, is_split, wide, live_children);
 }
 
-// k_split for warp-sized nodes: one warp per node, 8 per block, with the
-// node's bounds reduced over shuffles and its bins in the warp's own shared
-// memory; the same decisions as a block would take.
-__global__ void __launch_bounds__(kBuildBlock) k_split_small(const int* __restrict__ list, int count,
-                                                             const Slot* __restrict__ slots,
-                                                             const uint32_t* __restrict__ order,
-                                                             const float4* __restrict__ bmin,
-                                                             const float4* __restrict__ bmax,
-                                                             const float4* __restrict__ cent,
-                                                             float* __restrict__ bounds, int* __restrict__ nodes,
-                                                             Split* __restrict__ split, int* __restrict__ is_split,
-                                                             int bins, int* __restrict__ live_children) {
-  __shared__ int cnt_s[kWarpsPerBlock][3][kMaxBins];
-  __shared__ float bbox_s[kWarpsPerBlock][3][kMaxBins][6];
+// The stable partition of one segment (bvh.ts:145-171): each warp takes an
+// eighth of it, counts its lefts, and moves its triangles to the places its
+// predecessors leave. What bounds it: DRAM (40 bytes read and written).
+__global__ void __launch_bounds__(kBuildBlock) k_part(int level, BuildState st) {
+  constexpr int kWarps = kBuildBlock / 32;
+  __shared__ int s_lefts[kWarps];
+  __shared__ int s_box[2][12];
   const unsigned full = 0xffffffffu;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k = blockIdx.x * kWarpsPerBlock + w;
-  if (k >= count) return;  // the whole warp
-  const int j = list[k];
-  const Slot s = slots[j];
-  float nb[12];
-  for (int i = 0; i < 12; i++) nb[i] = INFINITY;
-  for (int q = s.first + lane; q < s.first + s.count; q += 32) {
-    const uint32_t t = order[q];
-    const float4 a = bmin[t], b = bmax[t], c = cent[t];
-    nb[0] = fminf(nb[0], a.x); nb[1] = fminf(nb[1], a.y); nb[2] = fminf(nb[2], a.z);
-    nb[3] = fminf(nb[3], -b.x); nb[4] = fminf(nb[4], -b.y); nb[5] = fminf(nb[5], -b.z);
-    nb[6] = fminf(nb[6], c.x); nb[7] = fminf(nb[7], c.y); nb[8] = fminf(nb[8], c.z);
-    nb[9] = fminf(nb[9], -c.x); nb[10] = fminf(nb[10], -c.y); nb[11] = fminf(nb[11], -c.z);
-  }
-  for (int off = 16; off > 0; off >>= 1)
-    for (int i = 0; i < 12; i++) nb[i] = fminf(nb[i], __shfl_xor_sync(full, nb[i], off));
-  if (lane == 0) {
-    float* bo = bounds + 6 * static_cast<size_t>(s.node);
-    bo[0] = nb[0]; bo[1] = nb[1]; bo[2] = nb[2];
-    bo[3] = -nb[3]; bo[4] = -nb[4]; bo[5] = -nb[5];
-  }
-  if (s.count <= kMaxLeaf || s.depth >= kBuildDepth) {
-    if (lane == 0) {
-      int* nd = nodes + 3 * static_cast<size_t>(s.node);
-      nd[0] = s.first; nd[1] = s.count; nd[2] = 0;
-      split[j] = Split{-1, 0, 0, 0, 0.0, 0.0};
-      is_split[j] = 0;
-      live_children[j] = 0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int total = st.ctl->level[level].segs;
+  const Prims p = st.prims[level & 1], o = st.prims[(level + 1) & 1];
+  for (int s = blockIdx.x; s < total; s += gridDim.x) {
+    __syncthreads();
+    const Node& nd = st.nodes[level & 1][st.segs[level & 1][s]];
+    const int nfirst = nd.first, seg = s - nd.seg0, nleft = nd.nleft, mode = nd.mode, axis = nd.axis, bin = nd.bin;
+    const double lo = nd.lo, scale = nd.scale;
+    const int child[2] = {nd.child[0], nd.child[1]};
+    const int first = nfirst + seg * st.seg, end = min(nfirst + nd.count, first + st.seg);
+    if (tid < 24) (&s_box[0][0])[tid] = ordered(is_max(tid % 12) ? -INFINITY : INFINITY);
+    const int rounds = (end - first + kBuildBlock - 1) / kBuildBlock;  // an equal share for every warp
+    const int from = first + warp * 32 * rounds;
+    unsigned mine = 0;  // lane r: the warp's round r, lanes going left
+    for (int r = 0; r < rounds; r++) {
+      const int k = from + 32 * r + lane;
+      bool f = false;
+      if (k < end) {
+        if (mode == 0) {
+          const float c = axis == 2 ? p.c[k].x : (axis == 0 ? p.b[k].z : p.b[k].w);
+          f = bin_of(c, lo, scale, st.bins) <= bin;
+        } else {
+          f = k - nfirst < nleft;
+        }
+      }
+      const unsigned b = __ballot_sync(full, f);
+      if (lane == r) mine = b;
     }
-    return;
+    const int lefts = __reduce_add_sync(full, static_cast<unsigned>(__popc(mine)));
+    if (lane == 0) s_lefts[warp] = lefts;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; w++) before += s_lefts[w];
+    int lpos = nfirst + st.seg_left[s] + before;
+    int rpos = nfirst + nleft + (from - nfirst) - (st.seg_left[s] + before);
+    float ml[12], mr[12];
+    clear_box(ml);
+    clear_box(mr);
+    for (int r = 0; r < rounds; r++) {
+      const int k = from + 32 * r + lane;
+      const unsigned b = __shfl_sync(full, mine, r);
+      if (k < end) {
+        const float4 a4 = p.a[k], b4 = p.b[k];
+        const float2 c2 = p.c[k];
+        const int pre = __popc(b & ((1u << lane) - 1u));
+        const bool f = (b >> lane) & 1u;
+        const int dst = f ? lpos + pre : rpos + (lane - pre);
+        o.a[dst] = a4;
+        o.b[dst] = b4;
+        o.c[dst] = c2;
+        if (f) {
+          add_prim(ml, a4, b4, c2.x);
+        } else {
+          add_prim(mr, a4, b4, c2.x);
+        }
+      }
+      lpos += __popc(b);
+      rpos += max(0, min(32, end - (from + 32 * r))) - __popc(b);
+    }
+    for (int q = 0; q < 2; q++) {
+      if (child[q] < 0) continue;  // a subtree takes its own bounds
+      for (int i = 0; i < 12; i++) {
+        const int v = warp_bound(q ? mr[i] : ml[i], is_max(i));
+        if (lane == 0) {
+          if (is_max(i)) {
+            atomicMax(&s_box[q][i], v);
+          } else {
+            atomicMin(&s_box[q][i], v);
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < 24) {
+      const int q = tid / 12, i = tid - 12 * q;
+      if (child[q] >= 0) {
+        int* box = st.nodes[(level + 1) & 1][child[q]].box;
+        if (is_max(i)) {
+          atomicMax(box + i, s_box[q][i]);
+        } else {
+          atomicMin(box + i, s_box[q][i]);
+        }
+      }
+    }
   }
-  int (*cnt)[kMaxBins] = cnt_s[w];
-  float (*bbox)[kMaxBins][6] = bbox_s[w];
+}
+
+// ---- subtrees
+
+// Shared memory of a warp that finishes a subtree.
+struct SubWarp {
+  float pr[9][kSub];      // box min xyz, max xyz, centroid xyz
+  unsigned leaf[kSub];    // by position: count | depth << 9 | parent's first << 16 | right << 24, 0 for none
+  int cnt[3][kMaxBins];
+  int bbox[3][kMaxBins][6];
+  uint2 todo[kSub / (kTinyMax + 1) + 2];       // nodes of more than kTinyMax triangles
+  uint2 tiny[kSub / (kMaxLeaf + 1) + 2];       // smaller ones
+  uint8_t ord[kSub];      // the triangles' order
+};
+constexpr int kSubWarps = 2;
+
+// A subtree's node: x = first | count << 16; y = depth | parent's first << 8 |
+// right << 16 | root << 17 (positions within the subtree).
+__device__ __forceinline__ uint2 sub_node(int first, int count, int depth, int pfirst, int side) {
+  return make_uint2(first | (count << 16), depth | (pfirst << 8) | (side << 16));
+}
+__device__ __forceinline__ unsigned sub_tag(const Subtree& t, uint2 e) {
+  if (e.y >> 17) return t.tag;
+  return 2u * static_cast<unsigned>(t.first + ((e.y >> 8) & 0xff)) + ((e.y >> 16) & 1u);
+}
+
+// After a split: a child is a leaf, or waits in one of the two lists.
+__device__ __forceinline__ void sub_child(SubWarp& w, int first, int count, int depth, int pfirst, int side,
+                                          int& ntodo, int& ntiny, bool write) {
+  const bool leaf = count <= kMaxLeaf || depth >= kBuildDepth;
+  if (leaf) {
+    if (write) w.leaf[first] = count | (depth << 9) | (pfirst << 16) | (side << 24);
+  } else if (count <= kTinyMax) {
+    if (write) w.tiny[ntiny] = sub_node(first, count, depth, pfirst, side);
+    ntiny++;
+  } else {
+    if (write) w.todo[ntodo] = sub_node(first, count, depth, pfirst, side);
+    ntodo++;
+  }
+}
+
+// One node of more than kTinyMax triangles, by the whole warp: its bounds, its
+// bins in shared memory, the split and the partition.
+__device__ void sub_split(const BuildState& st, const Subtree& t, SubWarp& w, uint2 e, int& ntodo, int& ntiny) {
+  constexpr int kRounds = kSub / 32;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int f = e.x & 0xffff, n = e.x >> 16, depth = e.y & 0xff;
+  int id[kRounds];
+  float m[12];
+  clear_box(m);
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    id[r] = -1;
+    if (32 * r + lane < n) {
+      id[r] = w.ord[f + 32 * r + lane];
+      for (int q = 0; q < 3; q++) {
+        m[q] = fminf(m[q], w.pr[q][id[r]]);
+        m[3 + q] = fmaxf(m[3 + q], w.pr[3 + q][id[r]]);
+        m[6 + q] = fminf(m[6 + q], w.pr[6 + q][id[r]]);
+        m[9 + q] = fmaxf(m[9 + q], w.pr[6 + q][id[r]]);
+      }
+    }
+  }
+  float box[12];
+#pragma unroll
+  for (int i = 0; i < 12; i++) box[i] = unordered(warp_bound(m[i], is_max(i)));
   for (int i = lane; i < 3 * kMaxBins; i += 32) {
-    const int a = i / kMaxBins, b = i % kMaxBins;
-    cnt[a][b] = 0;
-    for (int q = 0; q < 3; q++) {
-      bbox[a][b][q] = INFINITY;
-      bbox[a][b][3 + q] = -INFINITY;
-    }
+    (&w.cnt[0][0])[i] = 0;
+    for (int q = 0; q < 6; q++) (&w.bbox[0][0][0])[6 * i + q] = ordered(q < 3 ? INFINITY : -INFINITY);
   }
-  const double cmin[3] = {nb[6], nb[7], nb[8]};
-  const double cmax[3] = {-nb[9], -nb[10], -nb[11]};
   double lo[3], scale[3];
   bool live[3];
-  for (int a = 0; a < 3; a++) {
-    lo[a] = cmin[a];
-    const double extent = cmax[a] - lo[a];
-    live[a] = extent > 0;
-    scale[a] = live[a] ? bins / extent : 0.0;
-  }
+  binning(box + 6, box + 9, st.bins, lo, scale, live);
   __syncwarp();
-  for (int q = s.first + lane; q < s.first + s.count; q += 32) {
-    const uint32_t t = order[q];
-    const float4 a4 = bmin[t], b4 = bmax[t], c4 = cent[t];
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    if (id[r] < 0) continue;
+    int v[6];
+    for (int q = 0; q < 6; q++) v[q] = ordered(w.pr[q][id[r]]);
     for (int a = 0; a < 3; a++) {
       if (!live[a]) continue;
-      const int b = bin_of(comp4(c4, a), lo[a], scale[a], bins);
-      atomicAdd(&cnt[a][b], 1);
-      atomic_min_f(&bbox[a][b][0], a4.x);
-      atomic_min_f(&bbox[a][b][1], a4.y);
-      atomic_min_f(&bbox[a][b][2], a4.z);
-      atomic_max_f(&bbox[a][b][3], b4.x);
-      atomic_max_f(&bbox[a][b][4], b4.y);
-      atomic_max_f(&bbox[a][b][5], b4.z);
+      const int b = bin_of(w.pr[6 + a][id[r]], lo[a], scale[a], st.bins);
+      bin_prim(&w.cnt[a][b], w.bbox[a][b], v);
     }
   }
   __syncwarp();
-  decide(s, nb, cnt, bbox, lo, scale, live, bins, j, nodes, split, is_split, false, live_children);
+  const Choice c = best_split(w.cnt, w.bbox, live, st.bins);
+  int axis, nleft;
+  const int mode = choose(c, box, n, axis, nleft);  // never a leaf: more than 16 triangles
+  if (lane == 0) put_inner(st, t.first + f + nleft, box, t.first + f, depth, axis, sub_tag(t, e));
+  int lpos = f, rpos = f + nleft;
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    if (32 * r >= n) break;
+    const bool valid = id[r] >= 0;
+    const bool left = valid && (mode == 0 ? bin_of(w.pr[6 + axis][id[r]], lo[axis], scale[axis], st.bins) <= c.split
+                                          : 32 * r + lane < nleft);
+    const unsigned b = __ballot_sync(full, left);
+    const int pre = __popc(b & ((1u << lane) - 1u));
+    if (valid) w.ord[left ? lpos + pre : rpos + (lane - pre)] = static_cast<uint8_t>(id[r]);
+    lpos += __popc(b);
+    rpos += min(32, n - 32 * r) - __popc(b);
+  }
+  sub_child(w, f, nleft, depth + 1, f, 0, ntodo, ntiny, lane == 0);
+  sub_child(w, f + nleft, n - nleft, depth + 1, f, 1, ntodo, ntiny, lane == 0);
+  __syncwarp();
 }
 
-// k_split for nodes of at most kTinyMax triangles: half a warp per node, one
-// triangle per lane, so two nodes per warp. Per axis the lanes sort their
+// Two nodes of at most kTinyMax triangles, half a warp each, one triangle per
+// lane; `valid`: this half holds one. No bins: per axis the lanes sort their
 // triangles by bin (a bitonic network on bin * 16 + lane), then prefix and
 // suffix unions over the sorted order give, at the last triangle of each
 // occupied bin b, the left set {bins <= b} and the right set {bins > b} of the
@@ -651,70 +842,37 @@ __global__ void __launch_bounds__(kBuildBlock) k_split_small(const int* __restri
 // the first or from the last occupied bin leave a side empty, so the first
 // minimum over these candidates in (axis, split) order is the binned sweep's:
 // the same costs from the same float unions, the same choice.
-__global__ void __launch_bounds__(kBuildBlock) k_split_tiny(const int* __restrict__ list, int count,
-                                                            const Slot* __restrict__ slots,
-                                                            const uint32_t* __restrict__ order,
-                                                            const float4* __restrict__ bmin,
-                                                            const float4* __restrict__ bmax,
-                                                            const float4* __restrict__ cent,
-                                                            float* __restrict__ bounds, int* __restrict__ nodes,
-                                                            Split* __restrict__ split, int* __restrict__ is_split,
-                                                            int bins, int* __restrict__ live_children) {
+__device__ void sub_split_tiny(const BuildState& st, const Subtree& t, SubWarp& w, uint2 e, bool valid, int& ntodo,
+                               int& ntiny, int& deep) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, i = lane & 15;
-  const int pair = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (2 * pair >= count) return;  // the whole warp
-  const int k = 2 * pair + (lane >> 4);
-  const bool valid = k < count;  // this half holds a node (every lane still shuffles)
-  const int j = valid ? list[k] : 0;
-  const Slot s = valid ? slots[j] : Slot{0, 0, 0, 0};
-  const int n = s.count;
+  const int f = e.x & 0xffff, n = valid ? e.x >> 16 : 0, depth = e.y & 0xff;
   const bool has = i < n;
+  const int id = has ? w.ord[f + i] : 0;
+  float p[9];
+#pragma unroll
+  for (int q = 0; q < 9; q++) p[q] = has ? w.pr[q][id] : (q >= 3 && q < 6 ? -INFINITY : INFINITY);
   float m[12];
-  for (int q = 0; q < 12; q++) m[q] = INFINITY;
-  float4 a4 = make_float4(INFINITY, INFINITY, INFINITY, 0.0f), b4 = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
-  float4 c4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  if (has) {
-    const uint32_t t = order[s.first + i];
-    a4 = bmin[t];
-    b4 = bmax[t];
-    c4 = cent[t];
-    m[0] = a4.x; m[1] = a4.y; m[2] = a4.z;
-    m[3] = -b4.x; m[4] = -b4.y; m[5] = -b4.z;
-    m[6] = c4.x; m[7] = c4.y; m[8] = c4.z;
-    m[9] = -c4.x; m[10] = -c4.y; m[11] = -c4.z;
-  }
-  for (int off = 8; off > 0; off >>= 1)
-    for (int q = 0; q < 12; q++) m[q] = fminf(m[q], __shfl_xor_sync(full, m[q], off, 16));
-  const bool leafy = n <= kMaxLeaf || s.depth >= kBuildDepth;
-  if (valid && i == 0) {
-    float* bo = bounds + 6 * static_cast<size_t>(s.node);
-    bo[0] = m[0]; bo[1] = m[1]; bo[2] = m[2];
-    bo[3] = -m[3]; bo[4] = -m[4]; bo[5] = -m[5];
-    if (leafy) {
-      int* nd = nodes + 3 * static_cast<size_t>(s.node);
-      nd[0] = s.first; nd[1] = s.count; nd[2] = 0;
-      split[j] = Split{-1, 0, 0, 0, 0.0, 0.0};
-      is_split[j] = 0;
-      live_children[j] = 0;
-    }
-  }
-  const bool work = valid && !leafy;
+#pragma unroll
+  for (int q = 0; q < 9; q++) m[q] = q >= 3 && q < 6 ? fmaxf(p[q], -INFINITY) : fminf(p[q], INFINITY);  // no NaN
+#pragma unroll
+  for (int q = 0; q < 3; q++) m[9 + q] = has ? fmaxf(p[6 + q], -INFINITY) : -INFINITY;
+  const unsigned half = lane < 16 ? 0x0000ffffu : 0xffff0000u;
+  float box[12];
+#pragma unroll
+  for (int q = 0; q < 12; q++)
+    box[q] = unordered(is_max(q) ? __reduce_max_sync(half, ordered(m[q])) : __reduce_min_sync(half, ordered(m[q])));
   double lo[3], scale[3];
   bool live[3];
-  for (int a = 0; a < 3; a++) {
-    lo[a] = m[6 + a];
-    const double extent = -static_cast<double>(m[9 + a]) - lo[a];
-    live[a] = work && extent > 0;
-    scale[a] = live[a] ? bins / extent : 0.0;
-  }
-  double best_cost = INFINITY;
-  int best_axis = -1, best_split = -1, best_nleft = 0;
+  binning(box + 6, box + 9, st.bins, lo, scale, live);
+  Choice best{INFINITY, -1, -1, 0};
   for (int a = 0; a < 3; a++) {
     // Sort the half's triangles by bin; lanes without one sort last.
-    const int bin = (has && live[a]) ? bin_of(comp4(c4, a), lo[a], scale[a], bins) : kMaxBins;
+    const int bin = (has && live[a]) ? bin_of(p[6 + a], lo[a], scale[a], st.bins) : kMaxBins;
     int key = (bin << 4) | i;
+#pragma unroll
     for (int kk = 2; kk <= 16; kk <<= 1) {
+#pragma unroll
       for (int jj = kk >> 1; jj > 0; jj >>= 1) {
         const int other = __shfl_xor_sync(full, key, jj, 16);
         const bool keep_min = ((i & jj) == 0) == ((i & kk) == 0);
@@ -722,10 +880,11 @@ __global__ void __launch_bounds__(kBuildBlock) k_split_tiny(const int* __restric
       }
     }
     const int src = key & 15, sb = key >> 4;
-    float l0 = __shfl_sync(full, a4.x, src, 16), l1 = __shfl_sync(full, a4.y, src, 16);
-    float l2 = __shfl_sync(full, a4.z, src, 16), l3 = __shfl_sync(full, b4.x, src, 16);
-    float l4 = __shfl_sync(full, b4.y, src, 16), l5 = __shfl_sync(full, b4.z, src, 16);
+    float l0 = __shfl_sync(full, p[0], src, 16), l1 = __shfl_sync(full, p[1], src, 16);
+    float l2 = __shfl_sync(full, p[2], src, 16), l3 = __shfl_sync(full, p[3], src, 16);
+    float l4 = __shfl_sync(full, p[4], src, 16), l5 = __shfl_sync(full, p[5], src, 16);
     float r0 = l0, r1 = l1, r2 = l2, r3 = l3, r4 = l4, r5 = l5;
+#pragma unroll
     for (int off = 1; off < 16; off <<= 1) {
       const float o0 = __shfl_up_sync(full, l0, off, 16), o1 = __shfl_up_sync(full, l1, off, 16);
       const float o2 = __shfl_up_sync(full, l2, off, 16), o3 = __shfl_up_sync(full, l3, off, 16);
@@ -753,6 +912,7 @@ __global__ void __launch_bounds__(kBuildBlock) k_split_tiny(const int* __restric
       if (isnan(cost)) cost = INFINITY;
     }
     int at = sb, atl = lc;
+#pragma unroll
     for (int off = 8; off > 0; off >>= 1) {
       const double oc = __shfl_xor_sync(full, cost, off, 16);
       const int oi = __shfl_xor_sync(full, at, off, 16);
@@ -763,202 +923,238 @@ __global__ void __launch_bounds__(kBuildBlock) k_split_tiny(const int* __restric
         atl = ol;
       }
     }
-    if (cost < best_cost) {
-      best_cost = cost;
-      best_axis = a;
-      best_split = at;
-      best_nleft = atl;
+    if (cost < best.cost) best = Choice{cost, a, at, atl};
+  }
+  int axis, nleft;
+  const int mode = choose(best, box, n, axis, nleft);
+  bool left = false;
+  if (has && mode >= 0) {
+    const float c = axis == 0 ? p[6] : (axis == 1 ? p[7] : p[8]);
+    const double l = axis == 0 ? lo[0] : (axis == 1 ? lo[1] : lo[2]);
+    const double sc = axis == 0 ? scale[0] : (axis == 1 ? scale[1] : scale[2]);
+    left = mode == 0 ? bin_of(c, l, sc, st.bins) <= best.split : i < nleft;
+  }
+  const unsigned b = __ballot_sync(full, left) >> (lane & 16);
+  const int pre = __popc(b & ((1u << i) - 1u));
+  if (has && mode >= 0) w.ord[f + (left ? pre : nleft + (i - pre))] = static_cast<uint8_t>(id);
+  if (valid && i == 0) {
+    if (mode < 0) {
+      w.leaf[f] = n | (depth << 9) | (((e.y >> 8) & 0xff) << 16) | (((e.y >> 16) & 1u) << 24);
+    } else {
+      put_inner(st, t.first + f + nleft, box, t.first + f, depth, axis, sub_tag(t, e));
     }
   }
-  if (work && i == 0)
-    commit_choice(s, m, best_cost, best_axis, best_split, best_nleft, lo, scale, j, nodes, split, is_split, false,
-                  live_children);
+  // Both halves' children into the lists, in the same order in every lane.
+  for (int h = 0; h < 2; h++) {
+    const int hm = __shfl_sync(full, mode, 16 * h), hn = __shfl_sync(full, n, 16 * h);
+    const int hf = __shfl_sync(full, f, 16 * h), hl = __shfl_sync(full, nleft, 16 * h);
+    const int hd = __shfl_sync(full, depth, 16 * h);
+    if (hn == 0) continue;
+    deep = max(deep, hm >= 0 ? hd : -1);
+    if (hm < 0) continue;
+    sub_child(w, hf, hl, hd + 1, hf, 0, ntodo, ntiny, lane == 0);
+    sub_child(w, hf + hl, hn - hl, hd + 1, hf, 1, ntodo, ntiny, lane == 0);
+  }
+  __syncwarp();
 }
 
-// The first triangle of a block's share of its node, and the end.
-__device__ __forceinline__ void block_range(const Slot& s, bool wide, int seg, int& first, int& end) {
-  first = wide ? s.first + seg * kSegment : s.first;
-  end = wide ? min(s.first + s.count, first + kSegment) : s.first + s.count;
-}
-
-__device__ __forceinline__ int goes_left(const Split& d, const Slot& s, int k, const float4* __restrict__ cent,
-                                         const uint32_t* __restrict__ order, int bins) {
-  return d.mode == 0 ? (bin_of(comp4(cent[order[k]], d.axis), d.lo, d.scale, bins) <= d.bin ? 1 : 0)
-                     : (k - s.first < d.nleft ? 1 : 0);
-}
-
-// After a split node's partition: its node entry, and its children either
-// queued for the next level (at live_pos[j]) or, when they must be leaves (at
-// most 4 triangles, or at the depth limit; never for a wide parent), finished
-// here: bounds (bvh.ts:55-72 on their triangles), node, and their triangles
-// in both order buffers, since no later level copies them across.
-__device__ void place_children(const Slot& s, const Split& d, bool wide, int j, const int* __restrict__ rank,
-                               int child_base, int* __restrict__ nodes, Slot* __restrict__ next,
-                               const int* __restrict__ live_pos, const uint32_t* order_out, uint32_t* order_keep,
-                               const float4* __restrict__ bmin, const float4* __restrict__ bmax,
-                               float* __restrict__ bounds) {
-  const int left = child_base + 2 * rank[j];
-  int* nd = nodes + 3 * static_cast<size_t>(s.node);
-  nd[0] = left; nd[1] = 0; nd[2] = d.axis;
-  const Slot kids[2] = {Slot{left, s.first, d.nleft, s.depth + 1},
-                        Slot{left + 1, s.first + d.nleft, s.count - d.nleft, s.depth + 1}};
-  int at = live_pos[j];
-  for (int c = 0; c < 2; c++) {
-    const Slot& k = kids[c];
-    const bool small = !wide && (k.count <= kMaxLeaf || k.depth >= kBuildDepth);
-    if (!small) {
-      next[at++] = k;
+// Finishes subtrees, one warp each, from a queue: a depth-first walk over its
+// larger nodes, then pairs of tiny ones, then its leaves and the order of its
+// triangles. What bounds it: issue slots (shuffles and shared-memory atomics);
+// nothing but the triangles in and the nodes out touches DRAM.
+__global__ void __launch_bounds__(32 * kSubWarps) k_subtrees(BuildState st) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  SubWarp& w = reinterpret_cast<SubWarp*>(smem)[threadIdx.x >> 5];
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int count = st.ctl->subtrees;
+  int inner_deep = -1, slot_deep = 0;
+  for (;;) {
+    int s = 0;
+    if (lane == 0) s = atomicAdd(&st.ctl->next_subtree, 1);
+    s = __shfl_sync(full, s, 0);
+    if (s >= count) break;
+    const Subtree t = st.subtrees[s];
+    const Prims p = st.prims[t.parity];
+    const int n = t.count;
+    const bool leaf = n <= kMaxLeaf || t.depth >= kBuildDepth;
+    if (leaf) {  // at the depth limit of any size
+      float m[12];
+      clear_box(m);
+      for (int k = lane; k < n; k += 32) {
+        const float4 a4 = p.a[t.first + k], b4 = p.b[t.first + k];
+        const float2 c2 = p.c[t.first + k];
+        add_prim(m, a4, b4, c2.x);
+        st.order[t.first + k] = __float_as_int(c2.y);
+      }
+      float box[6];
+      for (int q = 0; q < 6; q++) box[q] = unordered(warp_bound(m[q], is_max(q)));
+      if (lane == 0) {
+        put_leaf(st, t.first, box, n, t.depth, t.tag);
+        set_bit(st.leaf_bits, t.first);
+      }
       continue;
     }
-    float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    for (int q = k.first; q < k.first + k.count; q++) {
-      const uint32_t t = order_out[q];
-      order_keep[q] = t;
-      const float4 a = bmin[t], b = bmax[t];
-      m[0] = fminf(m[0], a.x); m[1] = fminf(m[1], a.y); m[2] = fminf(m[2], a.z);
-      m[3] = fmaxf(m[3], b.x); m[4] = fmaxf(m[4], b.y); m[5] = fmaxf(m[5], b.z);
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) {
+      const float4 a4 = p.a[t.first + k], b4 = p.b[t.first + k];
+      const float2 c2 = p.c[t.first + k];
+      w.pr[0][k] = a4.x; w.pr[1][k] = a4.y; w.pr[2][k] = a4.z;
+      w.pr[3][k] = a4.w; w.pr[4][k] = b4.x; w.pr[5][k] = b4.y;
+      w.pr[6][k] = b4.z; w.pr[7][k] = b4.w; w.pr[8][k] = c2.x;
+      w.leaf[k] = 0;
+      w.ord[k] = static_cast<uint8_t>(k);
     }
-    float* bo = bounds + 6 * static_cast<size_t>(k.node);
-    for (int a = 0; a < 6; a++) bo[a] = m[a];
-    int* kn = nodes + 3 * static_cast<size_t>(k.node);
-    kn[0] = k.first; kn[1] = k.count; kn[2] = 0;
+    const uint2 root = make_uint2(n << 16, t.depth | (1u << 17));
+    int ntodo = 0, ntiny = 0;
+    if (n > kTinyMax) {
+      if (lane == 0) w.todo[0] = root;
+      ntodo = 1;
+    } else {
+      if (lane == 0) w.tiny[0] = root;
+      ntiny = 1;
+    }
+    __syncwarp();
+    while (ntodo > 0) {
+      const uint2 e = w.todo[--ntodo];
+      inner_deep = max(inner_deep, static_cast<int>(e.y & 0xff));
+      __syncwarp();
+      sub_split(st, t, w, e, ntodo, ntiny);
+    }
+    while (ntiny > 0) {
+      const int take = min(ntiny, 2);
+      ntiny -= take;
+      const bool valid = (lane >> 4) < take;
+      const uint2 e = valid ? w.tiny[ntiny + (lane >> 4)] : make_uint2(0, 0);
+      __syncwarp();
+      sub_split_tiny(st, t, w, e, valid, ntodo, ntiny, inner_deep);
+    }
+    for (int base = 0; base < n; base += 32) {
+      const int k = base + lane;
+      const unsigned info = k < n ? w.leaf[k] : 0u;
+      if (info) {
+        float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        const int c = info & 0x1ff, depth = (info >> 9) & 0x7f;
+        for (int q = 0; q < c; q++) {
+          const int id = w.ord[k + q];
+          for (int a = 0; a < 3; a++) {
+            m[a] = fminf(m[a], w.pr[a][id]);
+            m[3 + a] = fmaxf(m[3 + a], w.pr[3 + a][id]);
+          }
+        }
+        // The root itself can be a leaf (the SAH's choice): then it keeps its tag.
+        const unsigned tag = c == n ? t.tag : 2u * static_cast<unsigned>(t.first + ((info >> 16) & 0xff)) + (info >> 24);
+        put_leaf(st, t.first + k, m, c, depth, tag);
+        if (c > kMaxLeaf && depth < kBuildDepth) slot_deep = max(slot_deep, depth);
+      }
+      if (k < n) st.order[t.first + k] = __float_as_int(p.c[t.first + w.ord[k]].y);
+      const unsigned starts = __ballot_sync(full, info != 0u);
+      if (lane == 0) {
+        const int at = t.first + base, sh = at & 31;
+        if (starts << sh) atomicOr(st.leaf_bits + (at >> 5), starts << sh);
+        if (sh && (starts >> (32 - sh))) atomicOr(st.leaf_bits + (at >> 5) + 1, starts >> (32 - sh));
+      }
+    }
+    __syncwarp();
+  }
+  slot_deep = __reduce_max_sync(full, slot_deep);
+  if (lane == 0) {
+    if (inner_deep >= 0) atomicMax(&st.ctl->inner_depth, inner_deep);
+    atomicMax(&st.ctl->slot_depth, max(slot_deep, inner_deep));
   }
 }
 
-// Triangles going left in each block's segment of a wide split node; 0 for
-// every other block.
-__global__ void __launch_bounds__(kBuildBlock) k_count_left(LevelPlan lp, const Slot* __restrict__ slots,
-                                                            const Split* __restrict__ split,
-                                                            const uint32_t* __restrict__ order,
-                                                            const float4* __restrict__ cent, int bins,
-                                                            int* __restrict__ blk_left) {
-  __shared__ int sj;
-  __shared__ int part[kBuildBlock / 32];
-  const int tid = threadIdx.x;
-  if (tid == 0) sj = slot_of_block(lp, blockIdx.x);
-  __syncthreads();
-  const int j = sj;
-  const Split d = split[j];
-  if (lp.nb[j] <= 1 || d.mode < 0) {
-    if (tid == 0) blk_left[blockIdx.x] = 0;
-    return;
-  }
-  const Slot s = slots[j];
-  int first, end;
-  block_range(s, true, blockIdx.x - lp.boff[j], first, end);
-  int c = 0;
-  for (int k = first + tid; k < end; k += kBuildBlock) c += goes_left(d, s, k, cent, order, bins);
-  for (int off = 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
-  if ((tid & 31) == 0) part[tid >> 5] = c;
-  __syncthreads();
-  if (tid == 0) {
-    int t = 0;
-    for (int w = 0; w < kBuildBlock / 32; w++) t += part[w];
-    blk_left[blockIdx.x] = t;
-  }
+// ---- numbering
+constexpr int kScanBlocks = 4 * 148;
+constexpr int kScanThreads = 256;
+
+__device__ __forceinline__ void scan_segment(long long n, long long& lo, long long& hi) {
+  const long long seg = (n + kScanBlocks - 1) / kScanBlocks;
+  lo = min(n, static_cast<long long>(blockIdx.x) * seg);
+  hi = min(n, lo + seg);
 }
 
-// Stable partition of each split node's run and its two children
-// (bvh.ts:145-171); leaves copy their run unchanged. A wide node's blocks
-// place their segments after the lefts and rights of the blocks before them
-// (blk_pre: exclusive sums of k_count_left over all blocks).
-__global__ void __launch_bounds__(kBuildBlock) k_scatter(LevelPlan lp, const Slot* __restrict__ slots,
-                                                         const Split* __restrict__ split,
-                                                         const int* __restrict__ rank, int child_base,
-                                                         const uint32_t* order,
-                                                         uint32_t* __restrict__ order_out,
-                                                         const float4* __restrict__ cent, int* __restrict__ nodes,
-                                                         Slot* __restrict__ next, const int* __restrict__ blk_pre,
-                                                         int bins, const int* __restrict__ live_pos,
-                                                         uint32_t* order_keep, const float4* __restrict__ bmin,
-                                                         const float4* __restrict__ bmax, float* __restrict__ bounds) {
-  using Scan = cub::BlockScan<int, kBuildBlock>;
-  __shared__ typename Scan::TempStorage scan_tmp;
-  __shared__ int sj;
-  const int tid = threadIdx.x;
-  if (tid == 0) sj = slot_of_block(lp, blockIdx.x);
+__device__ __forceinline__ long long rank_groups(const BuildState& st) {
+  return (static_cast<long long>(st.ctl->inner_depth + 1) * st.words + kRankGroup - 1) / kRankGroup;
+}
+
+__device__ __forceinline__ int group_bits(const unsigned* bits, long long g) {
+  const uint4* w = reinterpret_cast<const uint4*>(bits + kRankGroup * g);
+  const uint4 x = w[0], y = w[1];
+  return __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w) + __popc(y.x) + __popc(y.y) + __popc(y.z) + __popc(y.w);
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_rank_sums(BuildState st, int* __restrict__ sums) {
+  using Reduce = cub::BlockReduce<int, kScanThreads>;
+  __shared__ typename Reduce::TempStorage tmp;
+  long long lo, hi;
+  scan_segment(rank_groups(st), lo, hi);
+  int v = 0;
+  for (long long g = lo + threadIdx.x; g < hi; g += kScanThreads) v += group_bits(st.depth_bits, g);
+  const int total = Reduce(tmp).Sum(v);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_rank_write(BuildState st, const int* __restrict__ sums) {
+  using Reduce = cub::BlockReduce<int, kScanThreads>;
+  using Scan = cub::BlockScan<int, kScanThreads>;
+  __shared__ union {
+    typename Reduce::TempStorage reduce;
+    typename Scan::TempStorage scan;
+  } tmp;
+  __shared__ int base;
+  long long lo, hi;
+  scan_segment(rank_groups(st), lo, hi);
+  int before = 0;
+  for (int b = static_cast<int>(threadIdx.x); b < static_cast<int>(blockIdx.x); b += kScanThreads) before += sums[b];
+  const int offset = Reduce(tmp.reduce).Sum(before);
+  if (threadIdx.x == 0) base = offset;
   __syncthreads();
-  const int j = sj;
-  const Slot s = slots[j];
-  const Split d = split[j];
-  const bool wide = lp.nb[j] > 1;
-  const int seg = blockIdx.x - lp.boff[j];
-  int first, end;
-  block_range(s, wide, seg, first, end);
-  if (d.mode < 0) {
-    for (int k = first + tid; k < end; k += kBuildBlock) order_out[k] = order[k];
-    return;
-  }
-  int left_off = wide ? blk_pre[blockIdx.x] - blk_pre[lp.boff[j]] : 0;
-  int right_off = (first - s.first) - left_off;
-  for (int base = first; base < end; base += kBuildBlock) {
-    const int k = base + tid;
-    int f = 0;
-    uint32_t t = 0;
-    if (k < end) {
-      t = order[k];
-      f = goes_left(d, s, k, cent, order, bins);
-    }
-    int pre = 0, total = 0;
-    Scan(scan_tmp).ExclusiveSum(f, pre, total);
-    if (k < end) {
-      const int dst = f ? s.first + left_off + pre : s.first + d.nleft + right_off + (tid - pre);
-      order_out[dst] = t;
-    }
-    const int in_chunk = min(kBuildBlock, end - base);
-    left_off += total;
-    right_off += in_chunk - total;
+  int running = base;
+  if (blockIdx.x == kScanBlocks - 1 && threadIdx.x == 0) st.ctl->inner_nodes = running + sums[kScanBlocks - 1];
+  for (long long tile = lo; tile < hi; tile += kScanThreads) {
+    const long long g = tile + threadIdx.x;
+    const int v = g < hi ? group_bits(st.depth_bits, g) : 0;
+    int ex = 0, total = 0;
+    Scan(tmp.scan).ExclusiveSum(v, ex, total);
+    if (g < hi) st.rank[g] = running + ex;
+    running += total;
     __syncthreads();
   }
-  if (seg != 0) return;
-  if (!wide) __syncthreads();  // this block's order_out writes are visible to thread 0
-  if (tid == 0)
-    place_children(s, d, wide, j, rank, child_base, nodes, next, live_pos, order_out, order_keep, bmin, bmax, bounds);
 }
 
-// k_scatter for warp-sized nodes: one warp per node, a stable partition by
-// ballots over 32-triangle chunks.
-__global__ void __launch_bounds__(kBuildBlock) k_scatter_small(
-    const int* __restrict__ list, int count, const Slot* __restrict__ slots, const Split* __restrict__ split,
-    const int* __restrict__ rank, int child_base, const uint32_t* order, uint32_t* __restrict__ order_out,
-    const float4* __restrict__ cent, int* __restrict__ nodes, Slot* __restrict__ next, int bins,
-    const int* __restrict__ live_pos, uint32_t* order_keep, const float4* __restrict__ bmin,
-    const float4* __restrict__ bmax, float* __restrict__ bounds) {
-  const unsigned full = 0xffffffffu;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k = blockIdx.x * kWarpsPerBlock + w;
-  if (k >= count) return;  // the whole warp
-  const int j = list[k];
-  const Slot s = slots[j];
-  const Split d = split[j];
-  const int end = s.first + s.count;
-  if (d.mode < 0) {
-    for (int q = s.first + lane; q < end; q += 32) order_out[q] = order[q];
-    return;
-  }
-  int left_off = 0, right_off = 0;
-  for (int base = s.first; base < end; base += 32) {
-    const int q = base + lane;
-    int f = 0;
-    uint32_t t = 0;
-    if (q < end) {
-      t = order[q];
-      f = goes_left(d, s, q, cent, order, bins);
-    }
-    const unsigned ballot = __ballot_sync(full, f);
-    const int pre = __popc(ballot & ((1u << lane) - 1u));
-    const int total = __popc(ballot);
-    if (q < end) {
-      const int dst = f ? s.first + left_off + pre : s.first + d.nleft + right_off + (lane - pre);
-      order_out[dst] = t;
-    }
-    left_off += total;
-    right_off += min(32, end - base) - total;
-  }
-  __syncwarp();  // the warp's order_out writes are visible to lane 0
-  if (lane == 0)
-    place_children(s, d, false, j, rank, child_base, nodes, next, live_pos, order_out, order_keep, bmin, bmax,
-                   bounds);
+// Inner nodes before the one at [depth][first], breadth first.
+__device__ __forceinline__ int inner_rank(const BuildState& st, int depth, int first) {
+  const long long word = static_cast<long long>(depth) * st.words + (first >> 5);
+  const long long g = word / kRankGroup;
+  int r = st.rank[g];
+  for (long long q = g * kRankGroup; q < word; q++) r += __popc(st.depth_bits[q]);
+  return r + __popc(st.depth_bits[word] & ((1u << (first & 31)) - 1u));
+}
+
+__device__ __forceinline__ int node_index(const BuildState& st, unsigned tag, int depth) {
+  return tag == kRootTag ? 0 : 1 + 2 * inner_rank(st, depth - 1, static_cast<int>(tag >> 1)) + static_cast<int>(tag & 1u);
+}
+
+__device__ __forceinline__ void write_node(int i, float4 a, float4 b, int x, int y, int z, float* __restrict__ bounds,
+                                           int* __restrict__ nodes) {
+  float* bo = bounds + 6 * static_cast<size_t>(i);
+  bo[0] = a.x; bo[1] = a.y; bo[2] = a.z;
+  bo[3] = a.w; bo[4] = b.x; bo[5] = b.y;
+  int* nd = nodes + 3 * static_cast<size_t>(i);
+  nd[0] = x; nd[1] = y; nd[2] = z;
+}
+
+// The leaf that starts at each position, and the inner node that splits there.
+__global__ void __launch_bounds__(256) k_emit(BuildState st, float* __restrict__ bounds, int* __restrict__ nodes) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= st.n || !((st.leaf_bits[k >> 5] >> (k & 31)) & 1u)) return;
+  const float4 la = st.leaf_a[k], lb = st.leaf_b[k];
+  write_node(node_index(st, st.leaf_t[k], __float_as_int(lb.w)), la, lb, k, __float_as_int(lb.z), 0, bounds, nodes);
+  if (k == 0) return;
+  const float4 a = st.inner_a[k], b = st.inner_b[k];
+  const int first = __float_as_int(b.z), depth = __float_as_int(b.w) & 0xff, axis = __float_as_int(b.w) >> 8;
+  write_node(node_index(st, st.inner_t[k], depth), a, b, 1 + 2 * inner_rank(st, depth, first), 0, axis, bounds, nodes);
 }
 
 // ---- compile (src/compile.ts:336-343 and 359-432)
@@ -1182,107 +1378,23 @@ __global__ void k_reorder_f32(const uint32_t* __restrict__ order, int n, const f
   sides_out[i] = sides[s];
 }
 
-// Exclusive prefix sums of up to kScanMax int arrays of the same length n, in
-// two launches over a fixed grid of kScanBlocks blocks, each owning one
-// contiguous segment of every array: k_scan_sums adds up each block's
-// segments; k_scan_write gives each block the sums of the blocks before it
-// and scans its segments tile by tile. Integer sums are exact in any order,
-// so the results are those of a sequential scan.
-constexpr int kScanMax = 4;
-constexpr int kScanBlocks = 4 * 148;
-constexpr int kScanThreads = 256;
-
-struct ScanArrays {
-  const int* in[kScanMax];
-  int* out[kScanMax];
-  int count;
-};
-
-__device__ __forceinline__ void scan_segment(int n, int& lo, int& hi) {
-  const int seg = (n + kScanBlocks - 1) / kScanBlocks;
-  lo = min(n, static_cast<int>(blockIdx.x) * seg);
-  hi = min(n, lo + seg);
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_sums(ScanArrays a, int n, int* __restrict__ sums) {
-  using Reduce = cub::BlockReduce<int, kScanThreads>;
-  __shared__ typename Reduce::TempStorage tmp;
-  int lo, hi;
-  scan_segment(n, lo, hi);
-  for (int k = 0; k < a.count; k++) {
-    int v = 0;
-    for (int i = lo + static_cast<int>(threadIdx.x); i < hi; i += kScanThreads) v += a.in[k][i];
-    const int total = Reduce(tmp).Sum(v);
-    if (threadIdx.x == 0) sums[k * kScanBlocks + blockIdx.x] = total;
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_write(ScanArrays a, int n, const int* __restrict__ sums) {
-  using Reduce = cub::BlockReduce<int, kScanThreads>;
-  using Scan = cub::BlockScan<int, kScanThreads>;
-  __shared__ union {
-    typename Reduce::TempStorage reduce;
-    typename Scan::TempStorage scan;
-  } tmp;
-  __shared__ int base;
-  int lo, hi;
-  scan_segment(n, lo, hi);
-  for (int k = 0; k < a.count; k++) {
-    int before = 0;
-    for (int b = static_cast<int>(threadIdx.x); b < static_cast<int>(blockIdx.x); b += kScanThreads)
-      before += sums[k * kScanBlocks + b];
-    const int offset = Reduce(tmp.reduce).Sum(before);
-    if (threadIdx.x == 0) base = offset;
-    __syncthreads();
-    int running = base;
-    for (int tile = lo; tile < hi; tile += kScanThreads) {
-      const int i = tile + static_cast<int>(threadIdx.x);
-      const int v = i < hi ? a.in[k][i] : 0;
-      int ex = 0, total = 0;
-      Scan(tmp.scan).ExclusiveSum(v, ex, total);
-      if (i < hi) a.out[k][i] = running + ex;
-      running += total;
-      __syncthreads();
-    }
-    __syncthreads();  // every thread has read `base` before the next array rewrites it
-  }
-}
-
-// Exclusive sums of in[k] into out[k] (k < count <= kScanMax), each of length
-// n; `sums` holds kScanMax * kScanBlocks ints.
-void scan_arrays(std::initializer_list<const int*> in, std::initializer_list<int*> out, int n, int* sums,
-                 cudaStream_t s) {
-  ScanArrays a{};
-  a.count = static_cast<int>(in.size());
-  if (a.count > kScanMax || out.size() != in.size()) throw std::runtime_error("scan_arrays: bad array count");
-  int k = 0;
-  for (const int* p : in) a.in[k++] = p;
-  k = 0;
-  for (int* p : out) a.out[k++] = p;
-  if (n <= 0) return;
-  k_scan_sums<<<kScanBlocks, kScanThreads, 0, s>>>(a, n, sums);
-  k_scan_write<<<kScanBlocks, kScanThreads, 0, s>>>(a, n, sums);
-}
-
 }  // namespace
 
-void exclusive_scan(const int* in, int* out, int n, int* sums, cudaStream_t s) {
-  scan_arrays({in}, {out}, n, sums, s);
-}
-
-int exclusive_scan_scratch() { return kScanMax * kScanBlocks; }
+constexpr int kBuildGrid = 4 * 148;  // blocks of one wave of the level kernels
 
 struct BuildBuffers {
-  DevArray<float4> bmin, bmax, cent;
-  DevArray<uint32_t> order_tmp;
-  DevArray<Slot> slots[2];
-  DevArray<Split> split;
-  DevArray<int> is_split, rank;
-  DevArray<int> nb, boff, wide, wid, blk_left, blk_pre, totals, live, live_pos, small, spos, tiny, tpos, slist;
-  DevArray<WideAcc> acc;
-  DevArray<int> scan_sums;  // per-block sums of the level plan's prefix sums (scan_arrays)
-  DevArray<int> host_pair;
+  // build
+  DevArray<BuildCtl> ctl;
+  DevArray<float4> prim_a[2], prim_b[2];
+  DevArray<float2> prim_c[2];
+  DevArray<Node> level_nodes[2];
+  DevArray<int> segs[2], seg_left, seg_cum;
+  DevArray<Acc> acc[2];
+  DevArray<Subtree> subtrees;
+  DevArray<float4> inner_a, inner_b, leaf_a, leaf_b;
+  DevArray<unsigned> inner_t, leaf_t, leaf_bits, depth_bits;
+  DevArray<int> rank, scan_sums;
+  size_t dirty_words = 0;  // words of depth_bits that the last build may have set
   // compile
   DevArray<double> p, nrm, uv, colors, box;
   DevArray<uint8_t> has_color, flags, sides, flags_out, sides_out;
@@ -1308,96 +1420,86 @@ int SceneBuilder::build_device(const float* d_tris, int n, float* d_bounds, int*
   if (n <= 0) return 0;
   if (bins < 2 || bins > kMaxBins) throw std::runtime_error("bin count out of range");
   BuildBuffers& B = *b_;
-  float4* bmin = B.bmin.ensure(n);
-  float4* bmax = B.bmax.ensure(n);
-  float4* cent = B.cent.ensure(n);
-  uint32_t* tmp = B.order_tmp.ensure(n);
-  const int max_slots = std::max(1, n);
-  // Blocks of a level: one per node, plus the extra segments of wide nodes.
-  const int max_blocks = max_slots + n / kSegment + 1;
-  Slot* slots[2] = {B.slots[0].ensure(max_slots), B.slots[1].ensure(max_slots)};
-  Split* split = B.split.ensure(max_slots);
-  int* is_split = B.is_split.ensure(max_slots);
-  int* rank = B.rank.ensure(max_slots);
-  int* live = B.live.ensure(max_slots);
-  int* live_pos = B.live_pos.ensure(max_slots);
-  int* small = B.small.ensure(max_slots);
-  int* spos = B.spos.ensure(max_slots);
-  int* tiny = B.tiny.ensure(max_slots);
-  int* tpos = B.tpos.ensure(max_slots);
-  int* slist = B.slist.ensure(max_slots);
-  int* nbk = B.nb.ensure(max_slots);
-  int* boff = B.boff.ensure(max_slots);
-  int* wide = B.wide.ensure(max_slots);
-  int* wid = B.wid.ensure(max_slots);
-  int* blk_left = B.blk_left.ensure(max_blocks);
-  int* blk_pre = B.blk_pre.ensure(max_blocks);
-  int* totals = B.totals.ensure(4);
-  WideAcc* acc = B.acc.ensure(n / kWideMin + 1);
-  k_prepare<<<blocks_of(n, 256), 256, 0, s>>>(d_tris, n, bmin, bmax, cent, d_order);
-  Slot root{0, 0, n, 0};
-  check(cudaMemcpyAsync(slots[0], &root, sizeof(Slot), cudaMemcpyHostToDevice, s), "upload");
-  int* scan_sums = B.scan_sums.ensure(kScanMax * kScanBlocks);
-  int active = 1, total = 1, cur = 0;
-  uint32_t* order_a = d_order;
-  uint32_t* order_b = tmp;
-  int pair[2], tot[4], lives[2];
-  while (active > 0) {
-    k_level_plan<<<blocks_of(active, 256), 256, 0, s>>>(slots[cur], active, nbk, wide, small, tiny);
-    scan_arrays({nbk, wide, small, tiny}, {boff, wid, spos, tpos}, active, scan_sums, s);
-    k_level_totals<<<1, 1, 0, s>>>(nbk, boff, wide, wid, small, spos, tiny, tpos, active, totals);
-    k_small_list<<<blocks_of(active, 256), 256, 0, s>>>(small, spos, tiny, tpos, active, totals, slist);
-    check(cudaMemcpyAsync(tot, totals, sizeof(tot), cudaMemcpyDeviceToHost, s), "download");
-    check(cudaStreamSynchronize(s), "BVH level plan");
-    const int nblocks = tot[0], nwide = tot[1], nsmall = tot[2], ntiny = tot[3];
-    const int small_blocks = blocks_of(nsmall, kWarpsPerBlock);
-    // Both lists share k_scatter_small, one warp per node.
-    const int scatter_blocks = blocks_of(nsmall + ntiny, kWarpsPerBlock);
-    const LevelPlan lp{nbk, boff, wid, active};
-    if (nwide > 0) {
-      k_wide_init<<<nwide, 128, 0, s>>>(acc, nwide);
-      k_bounds<<<nblocks, kBuildBlock, 0, s>>>(lp, slots[cur], order_a, bmin, bmax, cent, acc);
-    }
-    if (nblocks > 0)
-      k_split<<<nblocks, kBuildBlock, 0, s>>>(lp, slots[cur], order_a, bmin, bmax, cent, d_bounds, d_nodes, split,
-                                              is_split, acc, bins, live);
-    if (nsmall > 0)
-      k_split_small<<<small_blocks, kBuildBlock, 0, s>>>(slist, nsmall, slots[cur], order_a, bmin, bmax, cent,
-                                                         d_bounds, d_nodes, split, is_split, bins, live);
-    if (ntiny > 0)
-      k_split_tiny<<<blocks_of(ntiny, 2 * kWarpsPerBlock), kBuildBlock, 0, s>>>(
-          slist + nsmall, ntiny, slots[cur], order_a, bmin, bmax, cent, d_bounds, d_nodes, split, is_split, bins, live);
-    scan_arrays({is_split, live}, {rank, live_pos}, active, scan_sums, s);
-    check(cudaMemcpyAsync(&pair[0], rank + active - 1, sizeof(int), cudaMemcpyDeviceToHost, s), "download");
-    check(cudaMemcpyAsync(&pair[1], is_split + active - 1, sizeof(int), cudaMemcpyDeviceToHost, s), "download");
-    check(cudaMemcpyAsync(&lives[0], live_pos + active - 1, sizeof(int), cudaMemcpyDeviceToHost, s), "download");
-    check(cudaMemcpyAsync(&lives[1], live + active - 1, sizeof(int), cudaMemcpyDeviceToHost, s), "download");
-    if (nwide > 0) {
-      k_count_left<<<nblocks, kBuildBlock, 0, s>>>(lp, slots[cur], split, order_a, cent, bins, blk_left);
-      scan_arrays({blk_left}, {blk_pre}, nblocks, scan_sums, s);
-    }
-    if (nblocks > 0)
-      k_scatter<<<nblocks, kBuildBlock, 0, s>>>(lp, slots[cur], split, rank, total, order_a, order_b, cent, d_nodes,
-                                                slots[cur ^ 1], blk_pre, bins, live_pos, order_a, bmin, bmax,
-                                                d_bounds);
-    if (nsmall + ntiny > 0)
-      k_scatter_small<<<scatter_blocks, kBuildBlock, 0, s>>>(slist, nsmall + ntiny, slots[cur], split, rank, total, order_a,
-                                                           order_b, cent, d_nodes, slots[cur ^ 1], bins, live_pos,
-                                                           order_a, bmin, bmax, d_bounds);
-    check(cudaStreamSynchronize(s), "BVH level");
-    const int splits = pair[0] + pair[1];
-    std::swap(order_a, order_b);
-    total += 2 * splits;
-    active = lives[0] + lives[1];
-    cur ^= 1;
-    last_levels_++;
+  const size_t N = static_cast<size_t>(n);
+  BuildState st{};
+  st.n = n;
+  st.words = (n + 31) / 32;
+  st.bins = bins;
+  // Segments of a level kernel: two waves of blocks over the whole input, so
+  // that a small build's upper levels have blocks for every SM.
+  const int per_block = (n + 2 * kBuildGrid - 1) / (2 * kBuildGrid);
+  st.seg = std::max(kSegMin, std::min(kSegMax, (per_block + kBuildBlock - 1) / kBuildBlock * kBuildBlock));
+  // The most nodes of more than kSub triangles that a level can hold, and
+  // their segments; every split of one makes at most one more subtree.
+  const size_t max_nodes = N / (kSub + 1) + 1;
+  const size_t max_segs = N / st.seg + max_nodes;
+  const size_t max_subtrees = std::min(N, max_nodes * kBuildDepth + 1);
+  const size_t rows = static_cast<size_t>(kBuildDepth) * st.words;
+  st.ctl = B.ctl.ensure(1);
+  for (int i = 0; i < 2; i++) {
+    st.prims[i] = Prims{B.prim_a[i].ensure(N), B.prim_b[i].ensure(N), B.prim_c[i].ensure(N)};
+    st.nodes[i] = B.level_nodes[i].ensure(max_nodes);
+    st.segs[i] = B.segs[i].ensure(max_segs);
+    st.acc[i] = B.acc[i].ensure(N / st.seg + 1);
   }
-  if (order_a != d_order) {
-    check(cudaMemcpyAsync(d_order, order_a, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s), "copy");
+  st.seg_left = B.seg_left.ensure(max_segs);
+  st.seg_cum = B.seg_cum.ensure(max_segs * 3 * kMaxBins);
+  st.subtrees = B.subtrees.ensure(max_subtrees);
+  st.inner_a = B.inner_a.ensure(N);
+  st.inner_b = B.inner_b.ensure(N);
+  st.leaf_a = B.leaf_a.ensure(N);
+  st.leaf_b = B.leaf_b.ensure(N);
+  st.inner_t = B.inner_t.ensure(N);
+  st.leaf_t = B.leaf_t.ensure(N);
+  st.leaf_bits = B.leaf_bits.ensure(st.words + 1);
+  const size_t had = B.depth_bits.n;
+  st.depth_bits = B.depth_bits.ensure(rows + kRankGroup);
+  if (B.depth_bits.n != had) B.dirty_words = B.depth_bits.n;
+  st.rank = B.rank.ensure(rows / kRankGroup + 2);
+  int* sums = B.scan_sums.ensure(kScanBlocks);
+  st.order = d_order;
+  check(cudaMemsetAsync(st.ctl, 0, sizeof(BuildCtl), s), "memset");
+  check(cudaMemsetAsync(st.leaf_bits, 0, sizeof(unsigned) * (st.words + 1), s), "memset");
+  check(cudaMemsetAsync(st.depth_bits, 0, sizeof(unsigned) * B.dirty_words, s), "memset");
+  B.dirty_words = B.depth_bits.n;  // until this build's depth is known
+  k_root<<<1, kBuildBlock, 0, s>>>(st);
+  k_prepare<<<std::min(blocks_of(n, kBuildBlock), 2 * kBuildGrid), kBuildBlock, 0, s>>>(d_tris, st);
+  const size_t smem = sizeof(SubWarp) * kSubWarps;
+  check(cudaFuncSetAttribute(k_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+        "shared memory");
+  // The levels, a few more than a balanced tree has, and the rest of the
+  // build behind them; whether that was all is read back once, at the end.
+  BuildCtl ctl;
+  int levels = 0, want = 0;
+  if (n > kSub) {
+    while ((static_cast<long long>(kSub) << want) < n) want++;
+    want += 4;
   }
-  check(cudaGetLastError(), "BVH build");
-  check(cudaStreamSynchronize(s), "BVH build");
-  return total;
+  for (;;) {
+    want = std::min(want, kBuildDepth);
+    for (; levels < want; levels++) {
+      const long long most = static_cast<long long>(N / st.seg) +
+                             std::min<long long>(max_nodes, levels < 30 ? 1ll << levels : max_nodes);
+      const int grid = static_cast<int>(std::min<long long>(most, 2 * kBuildGrid));
+      k_bin<<<grid, kBuildBlock, 0, s>>>(levels, st);
+      k_part<<<grid, kBuildBlock, 0, s>>>(levels, st);
+    }
+    k_subtrees<<<static_cast<int>(std::min<size_t>((max_subtrees + kSubWarps - 1) / kSubWarps, 2 * kBuildGrid)),
+                 32 * kSubWarps, smem, s>>>(st);
+    k_rank_sums<<<kScanBlocks, kScanThreads, 0, s>>>(st, sums);
+    k_rank_write<<<kScanBlocks, kScanThreads, 0, s>>>(st, sums);
+    k_emit<<<blocks_of(n, 256), 256, 0, s>>>(st, d_bounds, d_nodes);
+    check(cudaGetLastError(), "BVH build");
+    check(cudaMemcpyAsync(&ctl, st.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, s), "download");
+    check(cudaStreamSynchronize(s), "BVH build");
+    if (levels >= kBuildDepth || ctl.level[levels].segs == 0) break;
+    // A tree with deeper large nodes: more levels, then the subtrees they made.
+    check(cudaMemcpyAsync(&st.ctl->next_subtree, &ctl.subtrees, sizeof(int), cudaMemcpyHostToDevice, s), "upload");
+    want = levels + 8;
+  }
+  B.dirty_words = static_cast<size_t>(ctl.inner_depth + 1) * st.words;
+  last_levels_ = ctl.slot_depth + 1;
+  return 1 + 2 * ctl.inner_nodes;
 }
 
 void SceneBuilder::upload_meshes(int count, const MeshInput* meshes, cudaStream_t s) {
@@ -1555,13 +1657,18 @@ void SceneBuilder::compile_instances(int count, const InstanceInput* inst, int b
 
 size_t SceneBuilder::device_bytes() const {
   const BuildBuffers& B = *b_;
-  size_t t = B.bmin.n * 16 * 3 + B.order_tmp.n * 4 + (B.slots[0].n + B.slots[1].n) * sizeof(Slot) +
-             B.split.n * sizeof(Split) + (B.is_split.n + B.rank.n + B.nb.n + B.boff.n + B.wide.n + B.wid.n) * 4 +
-             (B.blk_left.n + B.blk_pre.n) * 4 + B.acc.n * sizeof(WideAcc) + B.scan_sums.n * 4 + B.p.n * 8 + B.nrm.n * 8 +
+  size_t t = B.p.n * 8 + B.nrm.n * 8 +
              B.uv.n * 8 + B.colors.n * 8 + B.tris.n * 4 + B.tris_out.n * 4 + B.nrm_out.n * 4 + B.uv_out.n * 4 +
              B.col_out.n * 4 + B.tan_out.n * 4 + B.bounds.n * 4 + B.nodes.n * 4 + B.mats.n * 4 + B.mats_out.n * 4 +
              B.order.n * 4 + B.flags.n + B.sides.n + B.flags_out.n + B.sides_out.n + B.has_color.n +
-             B.flat_nrm.n * 4 + B.flat_uv.n * 4 + B.inst.n * sizeof(DInstance);
+             B.flat_nrm.n * 4 + B.flat_uv.n * 4 + B.inst.n * sizeof(DInstance) + B.ctl.n * sizeof(BuildCtl) +
+             (B.inner_a.n + B.inner_b.n + B.leaf_a.n + B.leaf_b.n) * 16 + (B.inner_t.n + B.leaf_t.n) * 4 +
+             (B.leaf_bits.n + B.depth_bits.n + B.rank.n + B.scan_sums.n + B.seg_left.n + B.seg_cum.n) * 4 +
+             B.subtrees.n * sizeof(Subtree);
+  for (int i = 0; i < 2; i++) {
+    t += (B.prim_a[i].n + B.prim_b[i].n) * 16 + B.prim_c[i].n * 8 + B.level_nodes[i].n * sizeof(Node) +
+         B.segs[i].n * 4 + B.acc[i].n * sizeof(Acc);
+  }
   for (const auto& a : B.mesh_pos) t += a.n * 4;
   for (const auto& a : B.mesh_nrm) t += a.n * 4;
   for (const auto& a : B.mesh_uv) t += a.n * 4;
