@@ -108,6 +108,7 @@ struct DScene {
 };
 
 // Per-triangle flag word: flags (bits 0-7), culled side (bits 8-15), last of its leaf (bit 16).
+constexpr int kLeafEnd = 1 << 16;
 MCRT_D int tri_flags(int word) { return word & 0xff; }
 MCRT_D int tri_side(int word) { return (word >> 8) & 0xff; }
 

@@ -1088,9 +1088,15 @@ int32_t mcrt_compile_instances(mcrt_executor* ex, int32_t version, int32_t count
     ex->have_geometry = false;
     DeviceGeometry g{};
     float times[3] = {0, 0, 0};
-    ex->builder.compile_instances(count, in.data(), bins, ex->stream, &g, times);
-    // Make it resident as mcrt_send_geometry does, from device memory.
+    // The triangles are written where the renders read them.
     GeometryGpu& G = ex->geo;
+    const size_t T = static_cast<size_t>(total);
+    const PackedGeometry packed{static_cast<float4*>(G.tris.ensure(sizeof(float4) * 3 * T)),
+                                static_cast<int*>(G.tri_mats.ensure(sizeof(int) * T)),
+                                static_cast<float4*>(G.attrs.ensure(sizeof(float4) * 4 * T)),
+                                static_cast<float4*>(G.tangents.ensure(sizeof(float4) * T))};
+    ex->builder.compile_instances(count, in.data(), bins, ex->stream, packed, out != nullptr, &g, times);
+    // Make it resident as mcrt_send_geometry does, from device memory.
     cudaStream_t s = ex->stream;
     const int n = g.n, m = g.node_count;
     G.tri_count = n;
@@ -1100,16 +1106,6 @@ int32_t mcrt_compile_instances(mcrt_executor* ex, int32_t version, int32_t count
     G.max_material = n > 0 ? max_material : -1;
     G.has_colors = false;
     if (n > 0) {
-      G.tris.ensure(sizeof(float4) * 3 * n);
-      G.tri_mats.ensure(sizeof(int) * n);
-      k_pack_tris<<<blocks(n, 256), 256, 0, s>>>(g.triangles, g.materials, g.flags, g.sides, n, G.tris.as<float4>(),
-                                                 G.tri_mats.as<int>());
-      G.attrs.ensure(sizeof(float) * 16 * n);
-      k_pack_attrs<<<blocks(n, 256), 256, 0, s>>>(g.normals, g.uvs, n, G.attrs.as<float>());
-      G.tangents.ensure(sizeof(float) * 4 * n);
-      cuda_check(cudaMemcpyAsync(G.tangents.as<float>(), g.tangents, sizeof(float) * 4 * n, cudaMemcpyDeviceToDevice, s),
-                 "copy");
-      k_mark_leaf_ends<<<blocks(m, 256), 256, 0, s>>>(g.nodes, m, G.tris.as<float4>());
       if (G.root_count == 0) {
         // A full binary tree of m nodes has (m - 1) / 2 inner nodes; the buffer
         // is sized for the most any build of n triangles can make, so a

@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "device_scene.cuh"
 #include "scene_build.cuh"
 
 namespace mcrt {
@@ -72,11 +73,10 @@ struct DMeshRef {
 };
 
 // An instance on the device: its world matrix, normal matrix (filled by
-// k_instance_matrices), first output triangle and per-triangle words.
+// k_instance_matrices) and per-triangle words.
 struct DInstance {
   double world[16];
   double nm[9];
-  long long tri_base;
   int mesh, mirror, flags, side, flat;
   uint32_t material;
 };
@@ -263,32 +263,31 @@ __device__ __forceinline__ int warp_bound(float v, bool max) {
   return max ? __reduce_max_sync(0xffffffffu, o) : __reduce_min_sync(0xffffffffu, o);
 }
 
-// Per-triangle box and centroid, bvh.ts:22-33, and the root's bounds.
-__global__ void __launch_bounds__(kBuildBlock) k_prepare(const float* __restrict__ tris, BuildState st) {
+// A triangle's box and centroid (bvh.ts:22-33) into place i, and into the
+// thread's bounds.
+__device__ __forceinline__ void put_prim(const Prims& p, int i, const float* o, float* m) {
+  double lo[3], hi[3];
+  for (int a = 0; a < 3; a++) {
+    const double v0 = o[a], v1 = v0 + static_cast<double>(o[3 + a]), v2 = v0 + static_cast<double>(o[6 + a]);
+    lo[a] = fmin(v0, fmin(v1, v2));
+    hi[a] = fmax(v0, fmax(v1, v2));
+  }
+  const float4 a4 = make_float4(static_cast<float>(lo[0]), static_cast<float>(lo[1]), static_cast<float>(lo[2]),
+                                static_cast<float>(hi[0]));
+  const float4 b4 = make_float4(static_cast<float>(hi[1]), static_cast<float>(hi[2]),
+                                static_cast<float>((lo[0] + hi[0]) * 0.5), static_cast<float>((lo[1] + hi[1]) * 0.5));
+  const float cz = static_cast<float>((lo[2] + hi[2]) * 0.5);
+  p.a[i] = a4;
+  p.b[i] = b4;
+  p.c[i] = make_float2(cz, __int_as_float(i));
+  add_prim(m, a4, b4, cz);
+}
+
+// The block's bounds into the root's.
+__device__ __forceinline__ void put_root_bounds(const BuildState& st, const float* m) {
   __shared__ int red[12];
   if (threadIdx.x < 12) red[threadIdx.x] = ordered(is_max(threadIdx.x) ? -INFINITY : INFINITY);
   __syncthreads();
-  float m[12];
-  clear_box(m);
-  const Prims p = st.prims[0];
-  for (int i = blockIdx.x * kBuildBlock + threadIdx.x; i < st.n; i += gridDim.x * kBuildBlock) {
-    const float* o = tris + 9 * static_cast<size_t>(i);
-    double lo[3], hi[3];
-    for (int a = 0; a < 3; a++) {
-      const double v0 = o[a], v1 = v0 + static_cast<double>(o[3 + a]), v2 = v0 + static_cast<double>(o[6 + a]);
-      lo[a] = fmin(v0, fmin(v1, v2));
-      hi[a] = fmax(v0, fmax(v1, v2));
-    }
-    const float4 a4 = make_float4(static_cast<float>(lo[0]), static_cast<float>(lo[1]), static_cast<float>(lo[2]),
-                                  static_cast<float>(hi[0]));
-    const float4 b4 = make_float4(static_cast<float>(hi[1]), static_cast<float>(hi[2]),
-                                  static_cast<float>((lo[0] + hi[0]) * 0.5), static_cast<float>((lo[1] + hi[1]) * 0.5));
-    const float cz = static_cast<float>((lo[2] + hi[2]) * 0.5);
-    p.a[i] = a4;
-    p.b[i] = b4;
-    p.c[i] = make_float2(cz, __int_as_float(i));
-    add_prim(m, a4, b4, cz);
-  }
   for (int i = 0; i < 12; i++) {
     const int v = warp_bound(m[i], is_max(i));
     if ((threadIdx.x & 31) == 0) {
@@ -308,6 +307,15 @@ __global__ void __launch_bounds__(kBuildBlock) k_prepare(const float* __restrict
       atomicMin(box + threadIdx.x, red[threadIdx.x]);
     }
   }
+}
+
+// Every triangle of `tris` (v0, e1, e2) into the build, and the root's bounds.
+__global__ void __launch_bounds__(kBuildBlock) k_prepare(const float* __restrict__ tris, BuildState st) {
+  float m[12];
+  clear_box(m);
+  for (int i = blockIdx.x * kBuildBlock + threadIdx.x; i < st.n; i += gridDim.x * kBuildBlock)
+    put_prim(st.prims[0], i, tris + 9 * static_cast<size_t>(i), m);
+  put_root_bounds(st, m);
 }
 
 // Math.min(bins - 1, Math.floor((c - lo) * scale)), bvh.ts:98: the product is
@@ -1202,14 +1210,11 @@ __global__ void k_reorder(const uint32_t* __restrict__ order, int n, const float
   sides_out[i] = sides[s];
 }
 
-// writeTangent (compile.ts:406-432) and the vertex bounding box (compile.ts:378-385).
-__global__ void k_tangents(const float* __restrict__ tris, const float* __restrict__ uvs, int n,
-                           float* __restrict__ tangents, double* __restrict__ box) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// The vertex bounding box of a grid's threads (compile.ts:378-385): each block
+// reduces its own, then one atomic per bound.
+struct VertexBox {
   double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  if (i < n) {
-    const float* o = tris + 9 * static_cast<size_t>(i);
-    const float* u6 = uvs + 6 * static_cast<size_t>(i);
+  __device__ __forceinline__ void add(const float* o) {
     for (int v = 0; v < 3; v++) {
       for (int a = 0; a < 3; a++) {
         const double x = static_cast<double>(o[a]) + (v == 1 ? o[3 + a] : v == 2 ? o[6 + a] : 0.0f);
@@ -1217,45 +1222,71 @@ __global__ void k_tangents(const float* __restrict__ tris, const float* __restri
         hi[a] = fmax(hi[a], x);
       }
     }
-    const double e1x = o[3], e1y = o[4], e1z = o[5], e2x = o[6], e2y = o[7], e2z = o[8];
-    const double du1 = static_cast<double>(u6[2]) - u6[0], dv1 = static_cast<double>(u6[3]) - u6[1];
-    const double du2 = static_cast<double>(u6[4]) - u6[0], dv2 = static_cast<double>(u6[5]) - u6[1];
-    const double nx = e1y * e2z - e1z * e2y, ny = e1z * e2x - e1x * e2z, nz = e1x * e2y - e1y * e2x;
-    const double d = du1 * dv2 - du2 * dv1;
-    double tx, ty, tz, sign = 1;
-    if (fabs(d) > 1e-20) {
-      const double r = 1 / d;
-      tx = (e1x * dv2 - e2x * dv1) * r;
-      ty = (e1y * dv2 - e2y * dv1) * r;
-      tz = (e1z * dv2 - e2z * dv1) * r;
-      const double bx = (e2x * du1 - e1x * du2) * r, by = (e2y * du1 - e1y * du2) * r, bz = (e2z * du1 - e1z * du2) * r;
-      const double cx = ny * tz - nz * ty, cy = nz * tx - nx * tz, cz = nx * ty - ny * tx;
-      sign = cx * bx + cy * by + cz * bz < 0 ? -1 : 1;
-    } else if (fabs(nx) < 0.9 * js_hypot3(nx, ny, nz)) {
-      tx = 0; ty = -nz; tz = ny;
-    } else {
-      tx = nz; ty = 0; tz = -nx;
-    }
-    double length = js_hypot3(tx, ty, tz);
-    if (length == 0 || isnan(length)) length = 1;
-    float* t = tangents + 4 * static_cast<size_t>(i);
-    t[0] = static_cast<float>(tx / length);
-    t[1] = static_cast<float>(ty / length);
-    t[2] = static_cast<float>(tz / length);
-    t[3] = static_cast<float>(sign);
   }
-  for (int off = 16; off > 0; off >>= 1) {
-    for (int a = 0; a < 3; a++) {
-      lo[a] = fmin(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-      hi[a] = fmax(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+  __device__ __forceinline__ void reduce(double* box) {
+    __shared__ double red[kBuildBlock / 32][6];
+    for (int off = 16; off > 0; off >>= 1) {
+      for (int a = 0; a < 3; a++) {
+        lo[a] = fmin(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
+        hi[a] = fmax(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+      }
+    }
+    if ((threadIdx.x & 31) == 0) {
+      for (int a = 0; a < 3; a++) {
+        red[threadIdx.x >> 5][a] = lo[a];
+        red[threadIdx.x >> 5][3 + a] = hi[a];
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+      double v = red[0][threadIdx.x];
+      for (int w = 1; w < kBuildBlock / 32; w++)
+        v = threadIdx.x < 3 ? fmin(v, red[w][threadIdx.x]) : fmax(v, red[w][threadIdx.x]);
+      if (threadIdx.x < 3) {
+        atomic_min_d(box + threadIdx.x, v);
+      } else {
+        atomic_max_d(box + threadIdx.x, v);
+      }
     }
   }
-  if ((threadIdx.x & 31) == 0 && i - static_cast<int>(threadIdx.x & 31) < n) {
-    for (int a = 0; a < 3; a++) {
-      atomic_min_d(box + a, lo[a]);
-      atomic_max_d(box + 3 + a, hi[a]);
-    }
+};
+
+// writeTangent (compile.ts:406-432) of a triangle (v0, e1, e2) with its uvs.
+__device__ float4 tangent_of(const float* o, const float* u6) {
+  const double e1x = o[3], e1y = o[4], e1z = o[5], e2x = o[6], e2y = o[7], e2z = o[8];
+  const double du1 = static_cast<double>(u6[2]) - u6[0], dv1 = static_cast<double>(u6[3]) - u6[1];
+  const double du2 = static_cast<double>(u6[4]) - u6[0], dv2 = static_cast<double>(u6[5]) - u6[1];
+  const double nx = e1y * e2z - e1z * e2y, ny = e1z * e2x - e1x * e2z, nz = e1x * e2y - e1y * e2x;
+  const double d = du1 * dv2 - du2 * dv1;
+  double tx, ty, tz, sign = 1;
+  if (fabs(d) > 1e-20) {
+    const double r = 1 / d;
+    tx = (e1x * dv2 - e2x * dv1) * r;
+    ty = (e1y * dv2 - e2y * dv1) * r;
+    tz = (e1z * dv2 - e2z * dv1) * r;
+    const double bx = (e2x * du1 - e1x * du2) * r, by = (e2y * du1 - e1y * du2) * r, bz = (e2z * du1 - e1z * du2) * r;
+    const double cx = ny * tz - nz * ty, cy = nz * tx - nx * tz, cz = nx * ty - ny * tx;
+    sign = cx * bx + cy * by + cz * bz < 0 ? -1 : 1;
+  } else if (fabs(nx) < 0.9 * js_hypot3(nx, ny, nz)) {
+    tx = 0; ty = -nz; tz = ny;
+  } else {
+    tx = nz; ty = 0; tz = -nx;
   }
+  double length = js_hypot3(tx, ty, tz);
+  if (length == 0 || isnan(length)) length = 1;
+  return make_float4(static_cast<float>(tx / length), static_cast<float>(ty / length), static_cast<float>(tz / length),
+                     static_cast<float>(sign));
+}
+
+__global__ void __launch_bounds__(kBuildBlock) k_tangents(const float* __restrict__ tris, const float* __restrict__ uvs,
+                                                          int n, float4* __restrict__ tangents, double* __restrict__ box) {
+  VertexBox vb;
+  for (int i = blockIdx.x * kBuildBlock + threadIdx.x; i < n; i += gridDim.x * kBuildBlock) {
+    const float* o = tris + 9 * static_cast<size_t>(i);
+    vb.add(o);
+    tangents[i] = tangent_of(o, uvs + 6 * static_cast<size_t>(i));
+  }
+  vb.reduce(box);
 }
 
 int blocks_of(long long n, int b) { return static_cast<int>((n + b - 1) / b); }
@@ -1279,47 +1310,116 @@ __global__ void k_instance_matrices(DInstance* __restrict__ inst, int count) {
   d.mirror = det < 0 ? 1 : 0;
 }
 
-// One thread per triangle of instance blockIdx.y: world-space positions in
-// double, float32 v0 / e1 / e2 as the compile's Float32Array stores make them
-// (compile.ts:337-343), normals through the normal matrix normalised with
-// Math.hypot (or the face normal), uvs, material, flags, side; and the
-// largest coordinate for the epsilon.
-__global__ void k_flatten(const DInstance* __restrict__ inst, const DMeshRef* __restrict__ meshes,
-                          float* __restrict__ tris, float* __restrict__ nrm, float* __restrict__ uvs,
-                          uint32_t* __restrict__ mats, uint8_t* __restrict__ flags, uint8_t* __restrict__ sides,
-                          unsigned long long* __restrict__ max_coord) {
-  const DInstance& d = inst[blockIdx.y];
-  const DMeshRef mr = meshes[d.mesh];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Instances and meshes as the kernels below see them; base: the first
+// triangle of each instance, then the total.
+struct Instances {
+  const DInstance* inst;
+  const DMeshRef* meshes;
+  const int* base;
+  int count;
+};
+
+// Triangle i's instance: the last one that starts at or before it and is not
+// empty.
+__device__ __forceinline__ int instance_of(const Instances& in, int i) {
+  int lo = 0, hi = in.count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (in.base[mid] <= i) {
+      lo = mid;
+    } else {
+      hi = mid - 1;
+    }
+  }
+  return lo;
+}
+
+// World-space vertices of triangle k of an instance in double (addMesh,
+// compile.ts:212-306), its vertex indices, and float32 v0 / e1 / e2 as the
+// compile's Float32Array stores make them (compile.ts:337-343).
+__device__ __forceinline__ void world_triangle(const DInstance& d, const DMeshRef& mr, int k, int* ids, double* p,
+                                               float* t) {
+  for (int v = 0; v < 3; v++) ids[v] = 3 * k + v;
+  if (mr.idx) {
+    for (int v = 0; v < 3; v++) ids[v] = static_cast<int>(mr.idx[ids[v]]);
+  }
+  if (d.mirror) {  // a mirroring transform reverses the winding
+    const int x = ids[1];
+    ids[1] = ids[2];
+    ids[2] = x;
+  }
+  const double* w = d.world;
+  for (int v = 0; v < 3; v++) {
+    const float* q = mr.pos + 3 * static_cast<size_t>(ids[v]);
+    const double x = q[0], y = q[1], z = q[2];
+    p[3 * v] = w[0] * x + w[4] * y + w[8] * z + w[12];
+    p[3 * v + 1] = w[1] * x + w[5] * y + w[9] * z + w[13];
+    p[3 * v + 2] = w[2] * x + w[6] * y + w[10] * z + w[14];
+  }
+  for (int a = 0; a < 3; a++) {
+    t[a] = static_cast<float>(p[a]);
+    t[3 + a] = static_cast<float>(p[3 + a] - p[a]);
+    t[6 + a] = static_cast<float>(p[6 + a] - p[a]);
+  }
+}
+
+// Every instance's triangles straight into the build, the root's bounds, and
+// the largest coordinate for the epsilon. Nothing else of a triangle is kept:
+// k_finish_instances makes it again from the mesh, which stays in L2, for
+// fewer bytes than writing and gathering it would take.
+__global__ void __launch_bounds__(kBuildBlock) k_prepare_instances(Instances in, BuildState st,
+                                                                   unsigned long long* __restrict__ max_coord) {
+  __shared__ unsigned long long largest;
+  if (threadIdx.x == 0) largest = 0;
+  __syncthreads();
+  float m[12];
+  clear_box(m);
   double mc = 0;
-  if (k < mr.tri_count) {
-    const size_t o = static_cast<size_t>(d.tri_base) + k;
-    int ids[3] = {3 * k, 3 * k + 1, 3 * k + 2};
-    if (mr.idx) {
-      for (int v = 0; v < 3; v++) ids[v] = static_cast<int>(mr.idx[ids[v]]);
-    }
-    if (d.mirror) {  // a mirroring transform reverses the winding
-      const int t = ids[1];
-      ids[1] = ids[2];
-      ids[2] = t;
-    }
-    const double* w = d.world;
+  for (int i = blockIdx.x * kBuildBlock + threadIdx.x; i < st.n; i += gridDim.x * kBuildBlock) {
+    const int j = instance_of(in, i);
+    const DInstance& d = in.inst[j];
+    int ids[3];
     double p[9];
-    for (int v = 0; v < 3; v++) {
-      const float* q = mr.pos + 3 * static_cast<size_t>(ids[v]);
-      const double x = q[0], y = q[1], z = q[2];
-      p[3 * v] = w[0] * x + w[4] * y + w[8] * z + w[12];
-      p[3 * v + 1] = w[1] * x + w[5] * y + w[9] * z + w[13];
-      p[3 * v + 2] = w[2] * x + w[6] * y + w[10] * z + w[14];
-    }
-    float* t = tris + 9 * o;
-    for (int a = 0; a < 3; a++) {
-      t[a] = static_cast<float>(p[a]);
-      t[3 + a] = static_cast<float>(p[3 + a] - p[a]);
-      t[6 + a] = static_cast<float>(p[6 + a] - p[a]);
-    }
+    float t[9];
+    world_triangle(d, in.meshes[d.mesh], i - in.base[j], ids, p, t);
     for (int q = 0; q < 9; q++) mc = fmax(mc, fabs(p[q]));
-    float* nn = nrm + 9 * o;
+    put_prim(st.prims[0], i, t, m);
+  }
+  for (int off = 16; off > 0; off >>= 1) mc = fmax(mc, __shfl_xor_sync(0xffffffffu, mc, off));
+  if ((threadIdx.x & 31) == 0) atomicMax(&largest, static_cast<unsigned long long>(__double_as_longlong(mc)));
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(max_coord, largest);
+  put_root_bounds(st, m);
+}
+
+// The compiled arrays of instanced geometry in BVH order, for callers that
+// keep them (all or none).
+struct CompiledArrays {
+  float *triangles, *normals, *uvs, *tangents;
+  uint32_t* materials;
+  uint8_t *flags, *sides;
+};
+
+// Every triangle in BVH order, in the render layout (device_scene.cuh): rows of
+// vertices with the flag word (the last of a leaf marked from the leaf
+// bitmap), material, normals and uvs, tangent; and the vertex bounding box.
+// Normals go through the normal matrix and are normalised with Math.hypot, or
+// are the face normal. ALL: the compiled arrays too. What bounds it: DRAM, and
+// the double divisions of the normals.
+template <bool ALL>
+__global__ void __launch_bounds__(kBuildBlock) k_finish_instances(Instances in, BuildState st, PackedGeometry out,
+                                                                  CompiledArrays arrays, double* __restrict__ box) {
+  VertexBox vb;
+  for (int i = blockIdx.x * kBuildBlock + threadIdx.x; i < st.n; i += gridDim.x * kBuildBlock) {
+    const int s = static_cast<int>(st.order[i]);
+    const int j = instance_of(in, s);
+    const DInstance& d = in.inst[j];
+    const DMeshRef mr = in.meshes[d.mesh];
+    int ids[3];
+    double p[9];
+    float t[9];
+    world_triangle(d, mr, s - in.base[j], ids, p, t);
+    float n9[9], u6[6];
     if (mr.nrm && !d.flat) {
       for (int v = 0; v < 3; v++) {
         const float* q = mr.nrm + 3 * static_cast<size_t>(ids[v]);
@@ -1329,9 +1429,9 @@ __global__ void k_flatten(const DInstance* __restrict__ inst, const DMeshRef* __
         const double nz = d.nm[2] * x + d.nm[5] * y + d.nm[8] * z;
         double len = js_hypot3(nx, ny, nz);
         if (!(len != 0) || isnan(len)) len = 1;  // Math.hypot(...) || 1
-        nn[3 * v] = static_cast<float>(nx / len);
-        nn[3 * v + 1] = static_cast<float>(ny / len);
-        nn[3 * v + 2] = static_cast<float>(nz / len);
+        n9[3 * v] = static_cast<float>(nx / len);
+        n9[3 * v + 1] = static_cast<float>(ny / len);
+        n9[3 * v + 2] = static_cast<float>(nz / len);
       }
     } else {
       const double ex = p[3] - p[0], ey = p[4] - p[1], ez = p[5] - p[2];
@@ -1345,37 +1445,38 @@ __global__ void k_flatten(const DInstance* __restrict__ inst, const DMeshRef* __
         f3[2] = static_cast<float>(cz / len);
       }
       for (int v = 0; v < 3; v++)
-        for (int a = 0; a < 3; a++) nn[3 * v + a] = f3[a];
+        for (int a = 0; a < 3; a++) n9[3 * v + a] = f3[a];
     }
-    float* u = uvs + 6 * o;
     for (int v = 0; v < 3; v++) {
-      u[2 * v] = mr.uv ? mr.uv[2 * static_cast<size_t>(ids[v])] : 0.0f;
-      u[2 * v + 1] = mr.uv ? mr.uv[2 * static_cast<size_t>(ids[v]) + 1] : 0.0f;
+      u6[2 * v] = mr.uv ? mr.uv[2 * static_cast<size_t>(ids[v])] : 0.0f;
+      u6[2 * v + 1] = mr.uv ? mr.uv[2 * static_cast<size_t>(ids[v]) + 1] : 0.0f;
     }
-    mats[o] = d.material;
-    flags[o] = static_cast<uint8_t>(d.flags);
-    sides[o] = static_cast<uint8_t>(d.side);
+    vb.add(t);
+    const float4 tg = tangent_of(t, u6);
+    const int next = i + 1;
+    const bool last = next == st.n || ((st.leaf_bits[next >> 5] >> (next & 31)) & 1u) != 0;
+    const float word = __int_as_float(d.flags | (d.side << 8) | (last ? kLeafEnd : 0));
+    const size_t I = static_cast<size_t>(i);
+    for (int a = 0; a < 3; a++)
+      out.tris[3 * I + a] = make_float4(t[a], static_cast<float>(static_cast<double>(t[a]) + static_cast<double>(t[3 + a])),
+                                        static_cast<float>(static_cast<double>(t[a]) + static_cast<double>(t[6 + a])), word);
+    out.mats[i] = static_cast<int>(d.material);
+    out.attrs[4 * I] = make_float4(n9[0], n9[1], n9[2], n9[3]);
+    out.attrs[4 * I + 1] = make_float4(n9[4], n9[5], n9[6], n9[7]);
+    out.attrs[4 * I + 2] = make_float4(n9[8], u6[0], u6[1], u6[2]);
+    out.attrs[4 * I + 3] = make_float4(u6[3], u6[4], u6[5], 0.0f);
+    out.tangents[i] = tg;
+    if (ALL) {
+      for (int q = 0; q < 9; q++) arrays.triangles[9 * I + q] = t[q];
+      for (int q = 0; q < 9; q++) arrays.normals[9 * I + q] = n9[q];
+      for (int q = 0; q < 6; q++) arrays.uvs[6 * I + q] = u6[q];
+      reinterpret_cast<float4*>(arrays.tangents)[i] = tg;
+      arrays.materials[i] = d.material;
+      arrays.flags[i] = static_cast<uint8_t>(d.flags);
+      arrays.sides[i] = static_cast<uint8_t>(d.side);
+    }
   }
-  for (int off = 16; off > 0; off >>= 1) mc = fmax(mc, __shfl_xor_sync(0xffffffffu, mc, off));
-  if ((threadIdx.x & 31) == 0) atomicMax(max_coord, static_cast<unsigned long long>(__double_as_longlong(mc)));
-}
-
-// Float32 arrays into BVH order (compile.ts:364-377, the float path).
-__global__ void k_reorder_f32(const uint32_t* __restrict__ order, int n, const float* __restrict__ tris_in,
-                              const float* __restrict__ nrm, const float* __restrict__ uv,
-                              const uint32_t* __restrict__ mats, const uint8_t* __restrict__ flags,
-                              const uint8_t* __restrict__ sides, float* __restrict__ tris_out,
-                              float* __restrict__ nrm_out, float* __restrict__ uv_out, uint32_t* __restrict__ mats_out,
-                              uint8_t* __restrict__ flags_out, uint8_t* __restrict__ sides_out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const size_t s = order[i];
-  for (int k = 0; k < 9; k++) tris_out[9 * static_cast<size_t>(i) + k] = tris_in[9 * s + k];
-  for (int k = 0; k < 9; k++) nrm_out[9 * static_cast<size_t>(i) + k] = nrm[9 * s + k];
-  for (int k = 0; k < 6; k++) uv_out[6 * static_cast<size_t>(i) + k] = uv[6 * s + k];
-  mats_out[i] = mats[s];
-  flags_out[i] = flags[s];
-  sides_out[i] = sides[s];
+  vb.reduce(box);
 }
 
 }  // namespace
@@ -1405,7 +1506,7 @@ struct BuildBuffers {
   // instanced geometry
   DevArray<DInstance> inst;
   DevArray<DMeshRef> mesh_refs;
-  DevArray<float> flat_nrm, flat_uv;
+  DevArray<int> inst_base;
   std::vector<DevArray<float>> mesh_pos, mesh_nrm, mesh_uv;
   std::vector<DevArray<uint32_t>> mesh_idx;
   std::vector<int> mesh_tris;
@@ -1414,12 +1515,10 @@ struct BuildBuffers {
 SceneBuilder::SceneBuilder() : b_(new BuildBuffers()) {}
 SceneBuilder::~SceneBuilder() { delete b_; }
 
-int SceneBuilder::build_device(const float* d_tris, int n, float* d_bounds, int* d_nodes, uint32_t* d_order,
-                               cudaStream_t s, int bins) {
-  last_levels_ = 0;
-  if (n <= 0) return 0;
+// The state of a build of n triangles, its buffers made and cleared and its
+// root queued; the triangles are the caller's to put in (k_prepare*).
+static BuildState start_build(BuildBuffers& B, int n, uint32_t* d_order, int bins, cudaStream_t s) {
   if (bins < 2 || bins > kMaxBins) throw std::runtime_error("bin count out of range");
-  BuildBuffers& B = *b_;
   const size_t N = static_cast<size_t>(n);
   BuildState st{};
   st.n = n;
@@ -1456,14 +1555,23 @@ int SceneBuilder::build_device(const float* d_tris, int n, float* d_bounds, int*
   st.depth_bits = B.depth_bits.ensure(rows + kRankGroup);
   if (B.depth_bits.n != had) B.dirty_words = B.depth_bits.n;
   st.rank = B.rank.ensure(rows / kRankGroup + 2);
-  int* sums = B.scan_sums.ensure(kScanBlocks);
   st.order = d_order;
   check(cudaMemsetAsync(st.ctl, 0, sizeof(BuildCtl), s), "memset");
   check(cudaMemsetAsync(st.leaf_bits, 0, sizeof(unsigned) * (st.words + 1), s), "memset");
   check(cudaMemsetAsync(st.depth_bits, 0, sizeof(unsigned) * B.dirty_words, s), "memset");
   B.dirty_words = B.depth_bits.n;  // until this build's depth is known
   k_root<<<1, kBuildBlock, 0, s>>>(st);
-  k_prepare<<<std::min(blocks_of(n, kBuildBlock), 2 * kBuildGrid), kBuildBlock, 0, s>>>(d_tris, st);
+  return st;
+}
+
+// Splits the prepared triangles and numbers the nodes; returns their count
+// and, in *levels_out, the levels of the tree.
+static int run_build(BuildBuffers& B, const BuildState& st, float* d_bounds, int* d_nodes, int* levels_out,
+                     cudaStream_t s) {
+  const int n = st.n;
+  const size_t N = static_cast<size_t>(n);
+  const size_t max_nodes = N / (kSub + 1) + 1;
+  int* sums = B.scan_sums.ensure(kScanBlocks);
   const size_t smem = sizeof(SubWarp) * kSubWarps;
   check(cudaFuncSetAttribute(k_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
         "shared memory");
@@ -1484,8 +1592,7 @@ int SceneBuilder::build_device(const float* d_tris, int n, float* d_bounds, int*
       k_bin<<<grid, kBuildBlock, 0, s>>>(levels, st);
       k_part<<<grid, kBuildBlock, 0, s>>>(levels, st);
     }
-    k_subtrees<<<static_cast<int>(std::min<size_t>((max_subtrees + kSubWarps - 1) / kSubWarps, 2 * kBuildGrid)),
-                 32 * kSubWarps, smem, s>>>(st);
+    k_subtrees<<<std::min(blocks_of(n, kSubWarps), 2 * kBuildGrid), 32 * kSubWarps, smem, s>>>(st);
     k_rank_sums<<<kScanBlocks, kScanThreads, 0, s>>>(st, sums);
     k_rank_write<<<kScanBlocks, kScanThreads, 0, s>>>(st, sums);
     k_emit<<<blocks_of(n, 256), 256, 0, s>>>(st, d_bounds, d_nodes);
@@ -1498,8 +1605,21 @@ int SceneBuilder::build_device(const float* d_tris, int n, float* d_bounds, int*
     want = levels + 8;
   }
   B.dirty_words = static_cast<size_t>(ctl.inner_depth + 1) * st.words;
-  last_levels_ = ctl.slot_depth + 1;
+  *levels_out = ctl.slot_depth + 1;
   return 1 + 2 * ctl.inner_nodes;
+}
+
+namespace {
+int prepare_blocks(int n) { return std::min(blocks_of(n, kBuildBlock), 2 * kBuildGrid); }
+}  // namespace
+
+int SceneBuilder::build_device(const float* d_tris, int n, float* d_bounds, int* d_nodes, uint32_t* d_order,
+                               cudaStream_t s, int bins) {
+  last_levels_ = 0;
+  if (n <= 0) return 0;
+  const BuildState st = start_build(*b_, n, d_order, bins, s);
+  k_prepare<<<prepare_blocks(n), kBuildBlock, 0, s>>>(d_tris, st);
+  return run_build(*b_, st, d_bounds, d_nodes, &last_levels_, s);
 }
 
 void SceneBuilder::upload_meshes(int count, const MeshInput* meshes, cudaStream_t s) {
@@ -1555,7 +1675,7 @@ long long SceneBuilder::instance_triangles(int count, const InstanceInput* inst)
 }
 
 void SceneBuilder::compile_instances(int count, const InstanceInput* inst, int bins, cudaStream_t s,
-                                     DeviceGeometry* out, float* times_ms) {
+                                     const PackedGeometry& packed, bool arrays, DeviceGeometry* out, float* times_ms) {
   BuildBuffers& B = *b_;
   const long long total = instance_triangles(count, inst);
   if (total < 0) throw std::runtime_error("an instance names a mesh that was not uploaded");
@@ -1566,59 +1686,62 @@ void SceneBuilder::compile_instances(int count, const InstanceInput* inst, int b
   cudaEvent_t ev[4];
   for (auto& e : ev) check(cudaEventCreate(&e), "event");
   check(cudaEventRecord(ev[0], s), "event");
-  // Instance table: tri_base and words on the host, matrices on the device.
+  // Instance table: first triangles and words on the host, matrices on the device.
   std::vector<DInstance> h(std::max(count, 1));
-  long long base = 0;
-  int max_tris = 0;
+  std::vector<int> bases(count + 1, 0);
   for (int i = 0; i < count; i++) {
     DInstance d{};
     std::memcpy(d.world, inst[i].world, sizeof(d.world));
-    d.tri_base = base;
     d.mesh = inst[i].mesh;
     d.flags = inst[i].flags;
     d.side = inst[i].side;
     d.flat = inst[i].flat_shading;
     d.material = inst[i].material;
-    base += B.mesh_tris[d.mesh];
-    max_tris = std::max(max_tris, B.mesh_tris[d.mesh]);
+    bases[i + 1] = bases[i] + B.mesh_tris[d.mesh];
     h[i] = d;
   }
   DInstance* d_inst = B.inst.ensure(h.size());
+  int* d_base = B.inst_base.ensure(bases.size());
   check(cudaMemcpyAsync(d_inst, h.data(), sizeof(DInstance) * h.size(), cudaMemcpyHostToDevice, s), "upload");
-  k_instance_matrices<<<blocks_of(count, 128), 128, 0, s>>>(d_inst, count);
-  float* d_tris = B.tris.ensure(9 * N);
-  float* d_n = B.flat_nrm.ensure(9 * N);
-  float* d_uv = B.flat_uv.ensure(6 * N);
-  uint32_t* d_m = B.mats.ensure(N);
-  uint8_t* d_f = B.flags.ensure(N);
-  uint8_t* d_s = B.sides.ensure(N);
+  check(cudaMemcpyAsync(d_base, bases.data(), sizeof(int) * bases.size(), cudaMemcpyHostToDevice, s), "upload");
+  if (count > 0) k_instance_matrices<<<blocks_of(count, 128), 128, 0, s>>>(d_inst, count);
+  const Instances in{d_inst, B.mesh_refs.p, d_base, count};
   unsigned long long* d_mc = B.max_coord.ensure(1);
   check(cudaMemsetAsync(d_mc, 0, sizeof(unsigned long long), s), "memset");
-  if (count > 0 && max_tris > 0) {
-    const dim3 grid(blocks_of(max_tris, 256), count);
-    k_flatten<<<grid, 256, 0, s>>>(d_inst, B.mesh_refs.p, d_tris, d_n, d_uv, d_m, d_f, d_s, d_mc);
-  }
-  check(cudaGetLastError(), "flatten");
-  check(cudaEventRecord(ev[1], s), "event");
   float* d_bounds = B.bounds.ensure(6 * cap);
   int* d_nodes = B.nodes.ensure(3 * cap);
   uint32_t* d_order = B.order.ensure(N);
-  const int m = build_device(d_tris, n, d_bounds, d_nodes, d_order, s, bins);
+  last_levels_ = 0;
+  int m = 0;
+  BuildState st{};
+  if (n > 0) {
+    st = start_build(B, n, d_order, bins, s);
+    k_prepare_instances<<<prepare_blocks(n), kBuildBlock, 0, s>>>(in, st, d_mc);
+  }
+  check(cudaGetLastError(), "flatten");
+  check(cudaEventRecord(ev[1], s), "event");
+  if (n > 0) m = run_build(B, st, d_bounds, d_nodes, &last_levels_, s);
   check(cudaEventRecord(ev[2], s), "event");
-  float* t_out = B.tris_out.ensure(9 * N);
-  float* n_out = B.nrm_out.ensure(9 * N);
-  float* uv_out = B.uv_out.ensure(6 * N);
-  float* tg_out = B.tan_out.ensure(4 * N);
-  uint32_t* m_out = B.mats_out.ensure(N);
-  uint8_t* f_out = B.flags_out.ensure(N);
-  uint8_t* s_out = B.sides_out.ensure(N);
+  DeviceGeometry g{};
+  CompiledArrays ca{};
+  if (arrays) {
+    g.triangles = ca.triangles = B.tris_out.ensure(9 * N);
+    g.normals = ca.normals = B.nrm_out.ensure(9 * N);
+    g.uvs = ca.uvs = B.uv_out.ensure(6 * N);
+    g.tangents = ca.tangents = B.tan_out.ensure(4 * N);
+    g.materials = ca.materials = B.mats_out.ensure(N);
+    g.flags = ca.flags = B.flags_out.ensure(N);
+    g.sides = ca.sides = B.sides_out.ensure(N);
+  }
   double box_init[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
   double* d_box = B.box.ensure(6);
   check(cudaMemcpyAsync(d_box, box_init, sizeof(box_init), cudaMemcpyHostToDevice, s), "upload");
   if (n > 0) {
-    k_reorder_f32<<<blocks_of(n, 256), 256, 0, s>>>(d_order, n, d_tris, d_n, d_uv, d_m, d_f, d_s, t_out, n_out,
-                                                    uv_out, m_out, f_out, s_out);
-    k_tangents<<<blocks_of(n, 256), 256, 0, s>>>(t_out, uv_out, n, tg_out, d_box);
+    if (arrays) {
+      k_finish_instances<true><<<prepare_blocks(n), kBuildBlock, 0, s>>>(in, st, packed, ca, d_box);
+    } else {
+      k_finish_instances<false><<<prepare_blocks(n), kBuildBlock, 0, s>>>(in, st, packed, ca, d_box);
+    }
   }
   check(cudaGetLastError(), "compile");
   double box[6];
@@ -1636,18 +1759,10 @@ void SceneBuilder::compile_instances(int count, const InstanceInput* inst, int b
     for (int i = 0; i < 3; i++) cudaEventElapsedTime(&times_ms[i], ev[i], ev[i + 1]);
   }
   for (auto& e : ev) cudaEventDestroy(e);
-  DeviceGeometry g{};
   g.n = n;
   g.node_count = m;
   g.root_count = (m > 0 && root[1] > 0) ? root[1] : 0;
   g.epsilon = n > 0 ? std::max(diagonal * 1e-5, std::max(max_coordinate * 2e-6, 1e-7)) : std::max(1e-5, 1e-7);
-  g.triangles = t_out;
-  g.normals = n_out;
-  g.uvs = uv_out;
-  g.tangents = tg_out;
-  g.materials = m_out;
-  g.flags = f_out;
-  g.sides = s_out;
   g.bounds = d_bounds;
   g.nodes = d_nodes;
   g.order = d_order;
@@ -1661,7 +1776,7 @@ size_t SceneBuilder::device_bytes() const {
              B.uv.n * 8 + B.colors.n * 8 + B.tris.n * 4 + B.tris_out.n * 4 + B.nrm_out.n * 4 + B.uv_out.n * 4 +
              B.col_out.n * 4 + B.tan_out.n * 4 + B.bounds.n * 4 + B.nodes.n * 4 + B.mats.n * 4 + B.mats_out.n * 4 +
              B.order.n * 4 + B.flags.n + B.sides.n + B.flags_out.n + B.sides_out.n + B.has_color.n +
-             B.flat_nrm.n * 4 + B.flat_uv.n * 4 + B.inst.n * sizeof(DInstance) + B.ctl.n * sizeof(BuildCtl) +
+             B.inst.n * sizeof(DInstance) + B.inst_base.n * 4 + B.ctl.n * sizeof(BuildCtl) +
              (B.inner_a.n + B.inner_b.n + B.leaf_a.n + B.leaf_b.n) * 16 + (B.inner_t.n + B.leaf_t.n) * 4 +
              (B.leaf_bits.n + B.depth_bits.n + B.rank.n + B.scan_sums.n + B.seg_left.n + B.seg_cum.n) * 4 +
              B.subtrees.n * sizeof(Subtree);
@@ -1756,7 +1871,7 @@ void SceneBuilder::compile_host(int n, const double* p, const double* nrm, const
   double box_init[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
   double* d_box = B.box.ensure(6);
   up(d_box, box_init, sizeof(box_init));
-  k_tangents<<<blocks_of(n, 256), 256, 0, s>>>(t_out, uv_out, n, tg_out, d_box);
+  k_tangents<<<prepare_blocks(n), kBuildBlock, 0, s>>>(t_out, uv_out, n, reinterpret_cast<float4*>(tg_out), d_box);
   check(cudaGetLastError(), "compile");
   auto down = [&](void* h, const void* d, size_t bytes) {
     check(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s), "download");

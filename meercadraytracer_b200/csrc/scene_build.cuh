@@ -40,6 +40,15 @@ struct DeviceGeometry {
   const int* nodes;
 };
 
+// Triangles in the render layout (device_scene.cuh): 3 rows, a material, 4
+// attribute vectors and a tangent per triangle.
+struct PackedGeometry {
+  float4* tris;
+  int* mats;
+  float4* attrs;
+  float4* tangents;
+};
+
 class SceneBuilder {
  public:
   SceneBuilder();
@@ -74,9 +83,11 @@ class SceneBuilder {
   long long instance_triangles(int count, const InstanceInput* inst) const;
   // compileGeometry of the instances entirely on the device: the flatten of
   // addMesh (src/compile.ts:212-306), the BVH with `bins` bins, the reorder,
-  // tangents and epsilon. times_ms (3 floats, or null): flatten, build, finish.
-  void compile_instances(int count, const InstanceInput* inst, int bins, cudaStream_t s, DeviceGeometry* out,
-                         float* times_ms);
+  // tangents and epsilon. The triangles go to `packed` (room for
+  // instance_triangles); `arrays`: the compiled arrays of *out as well, which
+  // are null otherwise. times_ms (3 floats, or null): flatten, build, finish.
+  void compile_instances(int count, const InstanceInput* inst, int bins, cudaStream_t s, const PackedGeometry& packed,
+                         bool arrays, DeviceGeometry* out, float* times_ms);
   // Device memory the builder holds between builds.
   size_t device_bytes() const;
 

@@ -48,7 +48,6 @@
 namespace mcrt {
 
 constexpr int kSentinel = 0x7fffffff;  // empty stack / finished ray
-constexpr int kLeafEnd = 1 << 16;      // in a triangle's word: last triangle of its leaf
 constexpr int kRefill = 16;            // refill a warp's finished lanes once this many are idle
 // The same threshold for the render's own kernels, measured on the mid workload
 // (closest hits: 12, shadow rays: 24, of thresholds between 4 and 32).
