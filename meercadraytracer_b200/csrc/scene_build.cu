@@ -35,9 +35,10 @@ static_assert(kBins <= kMaxBins, "the default bin count must fit the bin arrays"
 constexpr int kMaxLeaf = 4;    // bvh.ts:4
 constexpr int kBuildDepth = 100;  // bvh.ts:5
 constexpr int kBuildBlock = 256;
-// A node of at most kTinyMax triangles is split by half a warp, one triangle
-// per lane: its bins are never materialised (see sub_split_tiny).
-constexpr int kTinyMax = 16;
+// A node of at most kTinyMax triangles is finished by one lane (lane_subtree):
+// 12 measured best of 6 to 32 (16.4 M triangles rebuilt and traced: 44.8 ms at
+// 6, 40.8 at 12, 42.0 at 16, 59.8 at 32).
+constexpr int kTinyMax = 12;
 constexpr int kWideMin = 1 << 15;  // see BuildCtl::slot_depth
 
 void check(cudaError_t e, const char* what) {
@@ -149,6 +150,8 @@ __host__ __device__ inline double js_hypot3(double a, double b, double c) {
 // is the split of exactly one inner node: both kinds of node are kept at such
 // a position until they are numbered.
 constexpr int kSub = 256;          // triangles of a subtree that one warp finishes
+constexpr int kSubWarps = 2;       // warps of a block that finishes subtrees
+constexpr int kSubTodo = 8;       // nodes of one that wait: each at least as large as all that came after it
 constexpr int kSegMax = 4096;      // most triangles of a level kernel's segment (a multiple of kBuildBlock)
 constexpr int kSegMin = 512;
 constexpr unsigned kRootTag = 0xffffffffu;
@@ -368,81 +371,91 @@ __global__ void __launch_bounds__(kBuildBlock) k_root(BuildState st) {
   if (threadIdx.x == 0) st.ctl->inner_depth = -1;
 }
 
-// The cheapest split of a node's bins (bvh.ts:110-134), on one warp, lane i
-// holding bin i: the right sweep's unions and counts are suffix scans, the
-// left sweep's prefix scans (min, max and sums are exact in any order, and the
-// areas and costs are the same expressions, so every candidate cost equals the
-// one-thread sweep's); the first minimum in (axis, split) order wins, as
-// there. The unions are taken on the float bin bounds and widened to double
-// for the areas: min and max commute with the exact float-to-double
-// conversion, so the values are the reference's, for half the shuffles. The
-// result is the same in every lane.
-struct Choice {
-  double cost;
-  int axis, split, nleft;  // axis < 0: no candidate
+// Unions of a node's bins from the left (0) and from the right (1), per axis:
+// [side][axis][k] covers bins [0, k] or [k, bins). Box bounds and counts, the
+// boxes as ordered integers.
+template <int MB>
+struct Sweeps {
+  int cnt[2][3][MB];
+  int box[2][3][MB][6];
 };
 
-__device__ Choice best_split(const int (*cnt)[kMaxBins], const int (*bbox)[kMaxBins][6], const bool* live, int bins) {
+// The cheapest split of a node: after bin `split` of `axis`; axis < 0: no
+// candidate.
+struct Choice {
+  double cost;
+  int axis, split, nleft;
+};
+
+__device__ __forceinline__ double box_area(const int* b) {
+  return area(unordered(b[0]), unordered(b[1]), unordered(b[2]), unordered(b[3]), unordered(b[4]), unordered(b[5]));
+}
+
+// The first minimum in (axis, split) order of the warp's candidates, each lane
+// offering one (cost INFINITY: none), the same in every lane. Costs are never
+// negative, so their bits order as integers do: three integer reductions
+// instead of five rounds of double shuffles.
+__device__ __forceinline__ Choice first_minimum(double cost, int axis, int split, int nleft) {
   const unsigned full = 0xffffffffu;
+  const unsigned hi = static_cast<unsigned>(__double2hiint(cost)), lo = static_cast<unsigned>(__double2loint(cost));
+  const unsigned h = __reduce_min_sync(full, hi);
+  const unsigned l = __reduce_min_sync(full, hi == h ? lo : ~0u);
+  const unsigned at = __reduce_min_sync(full, hi == h && lo == l ? static_cast<unsigned>((axis << 8) | split) : ~0u);
+  const double best = __hiloint2double(static_cast<int>(h), static_cast<int>(l));
+  if (!(best < INFINITY)) return Choice{INFINITY, -1, -1, 0};
+  const unsigned who = __ballot_sync(full, hi == h && lo == l && static_cast<unsigned>((axis << 8) | split) == at);
+  return Choice{best, static_cast<int>(at >> 8), static_cast<int>(at & 0xff), __shfl_sync(full, nleft, __ffs(who) - 1)};
+}
+
+// The cheapest split of a node's bins (bvh.ts:110-134), on one warp. Six lane
+// groups sweep the three axes from both sides at once, a lane per pair of box
+// bounds (and one for the counts), into shared memory; then each lane costs
+// the splits after its bins. Min, max and sums are exact in any order and the
+// areas and costs are the same expressions in double, so every candidate cost
+// is the one-thread sweep's, and the first minimum wins, as there. Scans by
+// shuffles of all seven values took three times the instructions.
+template <int MB>
+__device__ Choice best_split(const int (*cnt)[MB], const int (*bbox)[MB][6], Sweeps<MB>& w, const bool* live, int bins) {
   const int lane = threadIdx.x & 31;
-  Choice best{INFINITY, -1, -1, 0};
-  for (int a = 0; a < 3; a++) {
-    if (!live[a]) continue;
-    const bool in = lane < bins;
-    const int* o = bbox[a][lane < kMaxBins ? lane : 0];
-    const int c = in ? cnt[a][lane] : 0;
-    const float b0 = in ? unordered(o[0]) : INFINITY, b1 = in ? unordered(o[1]) : INFINITY;
-    const float b2 = in ? unordered(o[2]) : INFINITY, b3 = in ? unordered(o[3]) : -INFINITY;
-    const float b4 = in ? unordered(o[4]) : -INFINITY, b5 = in ? unordered(o[5]) : -INFINITY;
-    // Suffix: bins [lane, bins).
-    int rc = c;
-    float r0 = b0, r1 = b1, r2 = b2, r3 = b3, r4 = b4, r5 = b5;
-    // Prefix: bins [0, lane].
-    int lc = c;
-    float l0 = b0, l1 = b1, l2 = b2, l3 = b3, l4 = b4, l5 = b5;
-    for (int off = 1; off < bins; off <<= 1) {
-      const int oc = __shfl_down_sync(full, rc, off);
-      const float o0 = __shfl_down_sync(full, r0, off), o1 = __shfl_down_sync(full, r1, off);
-      const float o2 = __shfl_down_sync(full, r2, off), o3 = __shfl_down_sync(full, r3, off);
-      const float o4 = __shfl_down_sync(full, r4, off), o5 = __shfl_down_sync(full, r5, off);
-      if (lane + off < 32) {
-        rc += oc;
-        r0 = fminf(r0, o0); r1 = fminf(r1, o1); r2 = fminf(r2, o2);
-        r3 = fmaxf(r3, o3); r4 = fmaxf(r4, o4); r5 = fmaxf(r5, o5);
+  if (lane < 24) {
+    const int side = lane >= 12 ? 1 : 0, a = (lane - 12 * side) >> 2, q = lane & 3;
+    int k = side ? bins - 1 : 0;
+    const int step = side ? -1 : 1;
+    if (q < 3) {
+      int lo = ordered(INFINITY), hi = ordered(-INFINITY);
+#pragma unroll 4
+      for (int i = 0; i < bins; i++, k += step) {
+        lo = min(lo, bbox[a][k][q]);
+        hi = max(hi, bbox[a][k][3 + q]);
+        w.box[side][a][k][q] = lo;
+        w.box[side][a][k][3 + q] = hi;
       }
-      const int pc = __shfl_up_sync(full, lc, off);
-      const float p0 = __shfl_up_sync(full, l0, off), p1 = __shfl_up_sync(full, l1, off);
-      const float p2 = __shfl_up_sync(full, l2, off), p3 = __shfl_up_sync(full, l3, off);
-      const float p4 = __shfl_up_sync(full, l4, off), p5 = __shfl_up_sync(full, l5, off);
-      if (lane >= off) {
-        lc += pc;
-        l0 = fminf(l0, p0); l1 = fminf(l1, p1); l2 = fminf(l2, p2);
-        l3 = fmaxf(l3, p3); l4 = fmaxf(l4, p4); l5 = fmaxf(l5, p5);
+    } else {
+      int c = 0;
+#pragma unroll 4
+      for (int i = 0; i < bins; i++, k += step) {
+        c += cnt[a][k];
+        w.cnt[side][a][k] = c;
       }
     }
-    const double right_area = rc > 0 ? area(r0, r1, r2, r3, r4, r5) : 0;
-    // Split after bin `lane`: the left union with the right union from lane + 1.
-    const int rc2 = __shfl_down_sync(full, rc, 1);
-    const double ra2 = __shfl_down_sync(full, right_area, 1);
-    double cost = INFINITY;
-    if (lane < bins - 1 && lc != 0 && rc2 != 0) {
-      cost = lc * area(l0, l1, l2, l3, l4, l5) + rc2 * ra2;
-      if (isnan(cost)) cost = INFINITY;
-    }
-    int at = lane, atl = lc;
-    for (int off = 16; off > 0; off >>= 1) {
-      const double oc = __shfl_xor_sync(full, cost, off);
-      const int oi = __shfl_xor_sync(full, at, off);
-      const int ol = __shfl_xor_sync(full, atl, off);
-      if (oc < cost || (oc == cost && oi < at)) {
-        cost = oc;
-        at = oi;
-        atl = ol;
-      }
-    }
-    if (cost < best.cost) best = Choice{cost, a, at, atl};
   }
-  return best;
+  __syncwarp();
+  double best = INFINITY;
+  int axis = 0, split = 0, nleft = 0;
+  for (int c = lane; c < 3 * bins; c += 32) {
+    const int a = c >= 2 * bins ? 2 : (c >= bins ? 1 : 0), k = c - a * bins;
+    if (k >= bins - 1 || !live[a]) continue;
+    const int lc = w.cnt[0][a][k], rc = w.cnt[1][a][k + 1];
+    if (lc == 0 || rc == 0) continue;
+    const double cost = lc * box_area(w.box[0][a][k]) + rc * box_area(w.box[1][a][k + 1]);
+    if (cost < best) {  // false for a NaN
+      best = cost;
+      axis = a;
+      split = k;
+      nleft = lc;
+    }
+  }
+  return first_minimum(best, axis, split, nleft);
 }
 
 // The choice (bvh.ts:137-163): mode -1 a SAH leaf, 0 the binned split, 1 the
@@ -476,14 +489,17 @@ __device__ __forceinline__ void bin_prim(int* cnt, int* bb, const int* v) {
 }
 
 // One segment of a level (see above). What bounds it: shared-memory atomics,
-// seven per triangle and axis. A warp whose triangles all fall into one bin of
-// an axis (neighbours in the model, at the upper levels) reduces them first
-// and adds once.
-__global__ void __launch_bounds__(kBuildBlock) k_bin(int level, BuildState st) {
+// seven per triangle and axis, and the latency of a node's steps. A warp whose
+// triangles all fall into one bin of an axis (neighbours in the model, at the
+// upper levels) reduces them first and adds once; the next triangle is loaded
+// while one is binned. Four blocks per SM (64 registers): 16.4 M triangles
+// rebuilt and traced 40.1 ms, three blocks 40.7, two 41.3.
+__global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st) {
   using Scan = cub::BlockScan<int, kBuildBlock>;
   __shared__ typename Scan::TempStorage scan_tmp;
   __shared__ int cnt[3][kMaxBins];
   __shared__ int bbox[3][kMaxBins][6];
+  __shared__ Sweeps<kMaxBins> sweeps;
   __shared__ int s_flag, s_child[2], s_seg0[2], s_acc[2], s_mode, s_axis, s_bin, s_nleft;
   const unsigned full = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -498,23 +514,37 @@ __global__ void __launch_bounds__(kBuildBlock) k_bin(int level, BuildState st) {
       (&cnt[0][0])[i] = 0;
       for (int q = 0; q < 6; q++) (&bbox[0][0][0])[6 * i + q] = ordered(q < 3 ? INFINITY : -INFINITY);
     }
-    float box[12];
-    for (int i = 0; i < 12; i++) box[i] = unordered(nd.box[i]);
     double lo[3], scale[3];
     bool live[3];
-    binning(box + 6, box + 9, bins, lo, scale, live);
+    {
+      float cmin[3], cmax[3];
+      for (int i = 0; i < 3; i++) {
+        cmin[i] = unordered(nd.box[6 + i]);
+        cmax[i] = unordered(nd.box[9 + i]);
+      }
+      binning(cmin, cmax, bins, lo, scale, live);
+    }
     __syncthreads();
     const int first = nfirst + seg * st.seg, end = min(nfirst + ncount, first + st.seg);
+    float4 na = make_float4(INFINITY, INFINITY, INFINITY, -INFINITY);
+    float4 nb = make_float4(-INFINITY, -INFINITY, 0.0f, 0.0f);
+    float nc = 0.0f;
+    const int got = first + tid;
+    if (got < end) {
+      na = p.a[got];
+      nb = p.b[got];
+      nc = p.c[got].x;
+    }
     for (int base = first; base < end; base += kBuildBlock) {
-      const int k = base + tid;
+      const int k = base + tid, ahead = k + kBuildBlock;
       const bool valid = k < end;
-      float4 a4 = make_float4(INFINITY, INFINITY, INFINITY, -INFINITY);
-      float4 b4 = make_float4(-INFINITY, -INFINITY, 0.0f, 0.0f);
-      float cz = 0.0f;
-      if (valid) {
-        a4 = p.a[k];
-        b4 = p.b[k];
-        cz = p.c[k].x;
+      const float4 a4 = valid ? na : make_float4(INFINITY, INFINITY, INFINITY, -INFINITY);
+      const float4 b4 = valid ? nb : make_float4(-INFINITY, -INFINITY, 0.0f, 0.0f);
+      const float cz = nc;
+      if (ahead < end) {  // the next triangle is on its way while this one is binned
+        na = p.a[ahead];
+        nb = p.b[ahead];
+        nc = p.c[ahead].x;
       }
       const int v[6] = {ordered(a4.x), ordered(a4.y), ordered(a4.z), ordered(a4.w), ordered(b4.x), ordered(b4.y)};
       const float c3[3] = {b4.z, b4.w, cz};
@@ -576,8 +606,10 @@ __global__ void __launch_bounds__(kBuildBlock) k_bin(int level, BuildState st) {
       __syncthreads();
     }
     if (tid < 32) {
-      const Choice c = best_split(cnt, bbox, live, bins);
+      const Choice c = best_split<kMaxBins>(cnt, bbox, sweeps, live, bins);
       if (lane == 0) {
+        float box[6];
+        for (int i = 0; i < 6; i++) box[i] = unordered(nd.box[i]);
         int axis, nleft;
         const int mode = choose(c, box, ncount, axis, nleft);  // never a leaf: more than kSub triangles
         nd.mode = s_mode = mode;
@@ -735,244 +767,272 @@ __global__ void __launch_bounds__(kBuildBlock) k_part(int level, BuildState st) 
 
 // ---- subtrees
 
-// Shared memory of a warp that finishes a subtree.
-struct SubWarp {
-  float pr[9][kSub];      // box min xyz, max xyz, centroid xyz
-  unsigned leaf[kSub];    // by position: count | depth << 9 | parent's first << 16 | right << 24, 0 for none
-  int cnt[3][kMaxBins];
-  int bbox[3][kMaxBins][6];
-  uint2 todo[kSub / (kTinyMax + 1) + 2];       // nodes of more than kTinyMax triangles
-  uint2 tiny[kSub / (kMaxLeaf + 1) + 2];       // smaller ones
-  uint8_t ord[kSub];      // the triangles' order
+// A node of a subtree, positions within it. up: depth | parent's first << 8 |
+// right << 16 | root << 17.
+struct SubNode {
+  int first, count;
+  unsigned up;
+  float box[6];
 };
-constexpr int kSubWarps = 2;
 
-// A subtree's node: x = first | count << 16; y = depth | parent's first << 8 |
-// right << 16 | root << 17 (positions within the subtree).
-__device__ __forceinline__ uint2 sub_node(int first, int count, int depth, int pfirst, int side) {
-  return make_uint2(first | (count << 16), depth | (pfirst << 8) | (side << 16));
-}
-__device__ __forceinline__ unsigned sub_tag(const Subtree& t, uint2 e) {
-  if (e.y >> 17) return t.tag;
-  return 2u * static_cast<unsigned>(t.first + ((e.y >> 8) & 0xff)) + ((e.y >> 16) & 1u);
+// Shared memory of a warp that finishes a subtree, for at most MB bins.
+template <int MB>
+struct SubWarp {
+  float4 a[kSub];         // the triangles: box min xyz, max x
+  float4 b[kSub];         // box max yz, centroid xy
+  float c[kSub];          // centroid z
+  int cnt[3][MB];
+  int bbox[3][MB][6];
+  Sweeps<MB> sweeps;
+  SubNode todo[kSubTodo];          // nodes of more than kTinyMax triangles
+  uint2 tiny[kSub / (kMaxLeaf + 1) + 1];  // smaller ones: first | count << 16, SubNode::up
+  uint8_t ord[kSub], moved[kSub];  // the triangles' order; a partition under way
+};
+
+__device__ __forceinline__ unsigned sub_tag(const Subtree& t, unsigned up) {
+  if (up >> 17) return t.tag;
+  return 2u * static_cast<unsigned>(t.first + ((up >> 8) & 0xff)) + ((up >> 16) & 1u);
 }
 
-// After a split: a child is a leaf, or waits in one of the two lists.
-__device__ __forceinline__ void sub_child(SubWarp& w, int first, int count, int depth, int pfirst, int side,
-                                          int& ntodo, int& ntiny, bool write) {
-  const bool leaf = count <= kMaxLeaf || depth >= kBuildDepth;
-  if (leaf) {
-    if (write) w.leaf[first] = count | (depth << 9) | (pfirst << 16) | (side << 24);
-  } else if (count <= kTinyMax) {
-    if (write) w.tiny[ntiny] = sub_node(first, count, depth, pfirst, side);
-    ntiny++;
-  } else {
-    if (write) w.todo[ntodo] = sub_node(first, count, depth, pfirst, side);
-    ntodo++;
+__device__ __forceinline__ float centroid_of(float4 b, float c, int axis) { return axis == 2 ? c : (axis == 0 ? b.z : b.w); }
+
+// binning() from a warp's centroid bounds (ordered integers), each axis's
+// division on a lane of its own.
+__device__ __forceinline__ void warp_binning(const int* cmin, const int* cmax, int bins, double* lo, double* scale,
+                                             bool* live) {
+  const unsigned full = 0xffffffffu;
+  const int a = threadIdx.x & 3;
+  const float mn = unordered(a == 0 ? cmin[0] : (a == 1 ? cmin[1] : cmin[2]));
+  const float mx = unordered(a == 0 ? cmax[0] : (a == 1 ? cmax[1] : cmax[2]));
+  const double extent = static_cast<double>(mx) - static_cast<double>(mn);
+  const double sc = extent > 0 ? bins / extent : 0.0;
+  for (int q = 0; q < 3; q++) {
+    lo[q] = unordered(cmin[q]);
+    scale[q] = __shfl_sync(full, sc, q);
+    live[q] = unordered(cmax[q]) > unordered(cmin[q]);  // the difference of two floats is never rounded to 0
   }
 }
 
-// One node of more than kTinyMax triangles, by the whole warp: its bounds, its
-// bins in shared memory, the split and the partition.
-__device__ void sub_split(const BuildState& st, const Subtree& t, SubWarp& w, uint2 e, int& ntodo, int& ntiny) {
-  constexpr int kRounds = kSub / 32;
+// A node of more than kTinyMax triangles: its bins, their sweeps and the
+// partition. Returns the split's mode (-1: a SAH leaf) with axis and nleft; the
+// children's boxes are sweeps.box[0][axis][left_at] and [1][axis][left_at + 1].
+template <int MB>
+__device__ int sub_split(const BuildState& st, SubWarp<MB>& w, const SubNode& e, int& axis, int& nleft, int& left_at) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int f = e.x & 0xffff, n = e.x >> 16, depth = e.y & 0xff;
-  int id[kRounds];
-  float m[12];
-  clear_box(m);
-#pragma unroll
-  for (int r = 0; r < kRounds; r++) {
-    id[r] = -1;
-    if (32 * r + lane < n) {
-      id[r] = w.ord[f + 32 * r + lane];
-      for (int q = 0; q < 3; q++) {
-        m[q] = fminf(m[q], w.pr[q][id[r]]);
-        m[3 + q] = fmaxf(m[3 + q], w.pr[3 + q][id[r]]);
-        m[6 + q] = fminf(m[6 + q], w.pr[6 + q][id[r]]);
-        m[9 + q] = fmaxf(m[9 + q], w.pr[6 + q][id[r]]);
-      }
-    }
+  const int f = e.first, n = e.count, bins = st.bins;
+  float cmn[3] = {INFINITY, INFINITY, INFINITY}, cmx[3] = {-INFINITY, -INFINITY, -INFINITY};
+  for (int k = lane; k < n; k += 32) {
+    const int id = w.ord[f + k];
+    const float4 b = w.b[id];
+    const float c = w.c[id];
+    cmn[0] = fminf(cmn[0], b.z); cmn[1] = fminf(cmn[1], b.w); cmn[2] = fminf(cmn[2], c);
+    cmx[0] = fmaxf(cmx[0], b.z); cmx[1] = fmaxf(cmx[1], b.w); cmx[2] = fmaxf(cmx[2], c);
   }
-  float box[12];
-#pragma unroll
-  for (int i = 0; i < 12; i++) box[i] = unordered(warp_bound(m[i], is_max(i)));
-  for (int i = lane; i < 3 * kMaxBins; i += 32) {
+  int cmin[3], cmax[3];
+  for (int q = 0; q < 3; q++) {
+    cmin[q] = __reduce_min_sync(full, ordered(cmn[q]));
+    cmax[q] = __reduce_max_sync(full, ordered(cmx[q]));
+  }
+  double lo[3], scale[3];
+  bool live[3];
+  warp_binning(cmin, cmax, bins, lo, scale, live);
+  for (int i = lane; i < 3 * MB; i += 32) {
     (&w.cnt[0][0])[i] = 0;
     for (int q = 0; q < 6; q++) (&w.bbox[0][0][0])[6 * i + q] = ordered(q < 3 ? INFINITY : -INFINITY);
   }
-  double lo[3], scale[3];
-  bool live[3];
-  binning(box + 6, box + 9, st.bins, lo, scale, live);
   __syncwarp();
-#pragma unroll
-  for (int r = 0; r < kRounds; r++) {
-    if (id[r] < 0) continue;
-    int v[6];
-    for (int q = 0; q < 6; q++) v[q] = ordered(w.pr[q][id[r]]);
-    for (int a = 0; a < 3; a++) {
-      if (!live[a]) continue;
-      const int b = bin_of(w.pr[6 + a][id[r]], lo[a], scale[a], st.bins);
-      bin_prim(&w.cnt[a][b], w.bbox[a][b], v);
+  for (int k = lane; k < n; k += 32) {
+    const int id = w.ord[f + k];
+    const float4 a = w.a[id], b = w.b[id];
+    const float c = w.c[id];
+    const int v[6] = {ordered(a.x), ordered(a.y), ordered(a.z), ordered(a.w), ordered(b.x), ordered(b.y)};
+    for (int q = 0; q < 3; q++) {
+      if (!live[q]) continue;
+      const int x = bin_of(centroid_of(b, c, q), lo[q], scale[q], bins);
+      bin_prim(&w.cnt[q][x], w.bbox[q][x], v);
     }
   }
   __syncwarp();
-  const Choice c = best_split(w.cnt, w.bbox, live, st.bins);
-  int axis, nleft;
-  const int mode = choose(c, box, n, axis, nleft);  // never a leaf: more than 16 triangles
-  if (lane == 0) put_inner(st, t.first + f + nleft, box, t.first + f, depth, axis, sub_tag(t, e));
-  int lpos = f, rpos = f + nleft;
-#pragma unroll
-  for (int r = 0; r < kRounds; r++) {
-    if (32 * r >= n) break;
-    const bool valid = id[r] >= 0;
-    const bool left = valid && (mode == 0 ? bin_of(w.pr[6 + axis][id[r]], lo[axis], scale[axis], st.bins) <= c.split
-                                          : 32 * r + lane < nleft);
+  const Choice c = best_split<MB>(w.cnt, w.bbox, w.sweeps, live, bins);
+  const int mode = choose(c, e.box, n, axis, nleft);
+  if (mode < 0) return mode;
+  left_at = c.split;
+  const double l = axis == 0 ? lo[0] : (axis == 1 ? lo[1] : lo[2]);
+  const double sc = axis == 0 ? scale[0] : (axis == 1 ? scale[1] : scale[2]);
+  int lpos = 0, rpos = nleft;
+  for (int base = 0; base < n; base += 32) {
+    const int k = base + lane;
+    const bool valid = k < n;
+    const int id = valid ? w.ord[f + k] : 0;
+    const bool left = valid && (mode == 0 ? bin_of(centroid_of(w.b[id], w.c[id], axis), l, sc, bins) <= c.split : k < nleft);
     const unsigned b = __ballot_sync(full, left);
     const int pre = __popc(b & ((1u << lane) - 1u));
-    if (valid) w.ord[left ? lpos + pre : rpos + (lane - pre)] = static_cast<uint8_t>(id[r]);
+    if (valid) w.moved[left ? lpos + pre : rpos + (lane - pre)] = static_cast<uint8_t>(id);
     lpos += __popc(b);
-    rpos += min(32, n - 32 * r) - __popc(b);
+    rpos += min(32, n - base) - __popc(b);
   }
-  sub_child(w, f, nleft, depth + 1, f, 0, ntodo, ntiny, lane == 0);
-  sub_child(w, f + nleft, n - nleft, depth + 1, f, 1, ntodo, ntiny, lane == 0);
   __syncwarp();
+  for (int k = lane; k < n; k += 32) w.ord[f + k] = w.moved[k];
+  __syncwarp();
+  return mode;
 }
 
-// Two nodes of at most kTinyMax triangles, half a warp each, one triangle per
-// lane; `valid`: this half holds one. No bins: per axis the lanes sort their
-// triangles by bin (a bitonic network on bin * 16 + lane), then prefix and
-// suffix unions over the sorted order give, at the last triangle of each
-// occupied bin b, the left set {bins <= b} and the right set {bins > b} of the
-// split after b. Split positions between occupied bins have the same two sets
-// and so the same cost as the occupied bin before them, and positions before
-// the first or from the last occupied bin leave a side empty, so the first
-// minimum over these candidates in (axis, split) order is the binned sweep's:
-// the same costs from the same float unions, the same choice.
-__device__ void sub_split_tiny(const BuildState& st, const Subtree& t, SubWarp& w, uint2 e, bool valid, int& ntodo,
-                               int& ntiny, int& deep) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, i = lane & 15;
-  const int f = e.x & 0xffff, n = valid ? e.x >> 16 : 0, depth = e.y & 0xff;
-  const bool has = i < n;
-  const int id = has ? w.ord[f + i] : 0;
-  float p[9];
-#pragma unroll
-  for (int q = 0; q < 9; q++) p[q] = has ? w.pr[q][id] : (q >= 3 && q < 6 ? -INFINITY : INFINITY);
-  float m[12];
-#pragma unroll
-  for (int q = 0; q < 9; q++) m[q] = q >= 3 && q < 6 ? fmaxf(p[q], -INFINITY) : fminf(p[q], INFINITY);  // no NaN
-#pragma unroll
-  for (int q = 0; q < 3; q++) m[9 + q] = has ? fmaxf(p[6 + q], -INFINITY) : -INFINITY;
-  const unsigned half = lane < 16 ? 0x0000ffffu : 0xffff0000u;
-  float box[12];
-#pragma unroll
-  for (int q = 0; q < 12; q++)
-    box[q] = unordered(is_max(q) ? __reduce_max_sync(half, ordered(m[q])) : __reduce_min_sync(half, ordered(m[q])));
-  double lo[3], scale[3];
-  bool live[3];
-  binning(box + 6, box + 9, st.bins, lo, scale, live);
-  Choice best{INFINITY, -1, -1, 0};
-  for (int a = 0; a < 3; a++) {
-    // Sort the half's triangles by bin; lanes without one sort last.
-    const int bin = (has && live[a]) ? bin_of(p[6 + a], lo[a], scale[a], st.bins) : kMaxBins;
-    int key = (bin << 4) | i;
-#pragma unroll
-    for (int kk = 2; kk <= 16; kk <<= 1) {
-#pragma unroll
-      for (int jj = kk >> 1; jj > 0; jj >>= 1) {
-        const int other = __shfl_xor_sync(full, key, jj, 16);
-        const bool keep_min = ((i & jj) == 0) == ((i & kk) == 0);
-        key = keep_min ? min(key, other) : max(key, other);
-      }
-    }
-    const int src = key & 15, sb = key >> 4;
-    float l0 = __shfl_sync(full, p[0], src, 16), l1 = __shfl_sync(full, p[1], src, 16);
-    float l2 = __shfl_sync(full, p[2], src, 16), l3 = __shfl_sync(full, p[3], src, 16);
-    float l4 = __shfl_sync(full, p[4], src, 16), l5 = __shfl_sync(full, p[5], src, 16);
-    float r0 = l0, r1 = l1, r2 = l2, r3 = l3, r4 = l4, r5 = l5;
-#pragma unroll
-    for (int off = 1; off < 16; off <<= 1) {
-      const float o0 = __shfl_up_sync(full, l0, off, 16), o1 = __shfl_up_sync(full, l1, off, 16);
-      const float o2 = __shfl_up_sync(full, l2, off, 16), o3 = __shfl_up_sync(full, l3, off, 16);
-      const float o4 = __shfl_up_sync(full, l4, off, 16), o5 = __shfl_up_sync(full, l5, off, 16);
-      if (i >= off) {
-        l0 = fminf(l0, o0); l1 = fminf(l1, o1); l2 = fminf(l2, o2);
-        l3 = fmaxf(l3, o3); l4 = fmaxf(l4, o4); l5 = fmaxf(l5, o5);
-      }
-      const float p0 = __shfl_down_sync(full, r0, off, 16), p1 = __shfl_down_sync(full, r1, off, 16);
-      const float p2 = __shfl_down_sync(full, r2, off, 16), p3 = __shfl_down_sync(full, r3, off, 16);
-      const float p4 = __shfl_down_sync(full, r4, off, 16), p5 = __shfl_down_sync(full, r5, off, 16);
-      if (i + off < 16) {
-        r0 = fminf(r0, p0); r1 = fminf(r1, p1); r2 = fminf(r2, p2);
-        r3 = fmaxf(r3, p3); r4 = fmaxf(r4, p4); r5 = fmaxf(r5, p5);
-      }
-    }
-    // Split after bin sb (this lane the last of its bin): positions [0, i] left, (i, n) right.
-    const double right_here = i < n ? area(r0, r1, r2, r3, r4, r5) : 0;
-    const double right_area = __shfl_down_sync(full, right_here, 1, 16);
-    const int next_bin = __shfl_down_sync(full, sb, 1, 16);
-    double cost = INFINITY;
-    const int lc = i + 1, rc = n - i - 1;
-    if (live[a] && i < n - 1 && sb != next_bin) {
-      cost = lc * area(l0, l1, l2, l3, l4, l5) + rc * right_area;
-      if (isnan(cost)) cost = INFINITY;
-    }
-    int at = sb, atl = lc;
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1) {
-      const double oc = __shfl_xor_sync(full, cost, off, 16);
-      const int oi = __shfl_xor_sync(full, at, off, 16);
-      const int ol = __shfl_xor_sync(full, atl, off, 16);
-      if (oc < cost || (oc == cost && oi < at)) {
-        cost = oc;
-        at = oi;
-        atl = ol;
-      }
-    }
-    if (cost < best.cost) best = Choice{cost, a, at, atl};
+// A box that one lane grows.
+struct LaneBox {
+  float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  __device__ __forceinline__ void add(float4 p, float4 q) {
+    b[0] = fminf(b[0], p.x); b[1] = fminf(b[1], p.y); b[2] = fminf(b[2], p.z);
+    b[3] = fmaxf(b[3], p.w); b[4] = fmaxf(b[4], q.x); b[5] = fmaxf(b[5], q.y);
   }
-  int axis, nleft;
-  const int mode = choose(best, box, n, axis, nleft);
-  bool left = false;
-  if (has && mode >= 0) {
-    const float c = axis == 0 ? p[6] : (axis == 1 ? p[7] : p[8]);
-    const double l = axis == 0 ? lo[0] : (axis == 1 ? lo[1] : lo[2]);
-    const double sc = axis == 0 ? scale[0] : (axis == 1 ? scale[1] : scale[2]);
-    left = mode == 0 ? bin_of(c, l, sc, st.bins) <= best.split : i < nleft;
-  }
-  const unsigned b = __ballot_sync(full, left) >> (lane & 16);
-  const int pre = __popc(b & ((1u << i) - 1u));
-  if (has && mode >= 0) w.ord[f + (left ? pre : nleft + (i - pre))] = static_cast<uint8_t>(id);
-  if (valid && i == 0) {
+  __device__ __forceinline__ double size() const { return area(b[0], b[1], b[2], b[3], b[4], b[5]); }
+};
+
+// A node of at most kTinyMax triangles and everything below it, by one lane,
+// while the other lanes do theirs: a warp per such node leaves three quarters
+// of its lanes idle and pays every warp-wide step for a few triangles. No bins
+// either: per axis the lane sorts the triangles by bin, and sweeps them from
+// the right (areas kept) and from the left. At the last triangle of each
+// occupied bin b these give the left set {bins <= b} and the right set
+// {bins > b} of the split after b. Split positions between occupied bins have
+// the same two sets and so the same cost as the occupied bin before them, and
+// positions before the first or from the last occupied bin leave a side empty,
+// so the first minimum over these candidates in (axis, split) order is the
+// binned sweep's: the same costs from the same unions, the same choice.
+// `inner_deep`, `slot_deep`: as in BuildCtl.
+template <int MB>
+__device__ void lane_subtree(const BuildState& st, const Subtree& t, SubWarp<MB>& w, uint2 root, int& inner_deep,
+                             int& slot_deep) {
+  int key[kTinyMax];         // bin << 8 | triangle, in bin order
+  double right[kTinyMax];    // area of the triangles from here on
+  uint2 wait[2];             // the larger child waits: at most log2(12 / 5) of them
+  int waiting = 0;
+  uint2 e = root;
+  const int bins = st.bins;
+  for (;;) {
+    const int f = e.x & 0xff, n = e.x >> 16, depth = e.y & 0xff;
+    LaneBox box;
+    float cmn[3] = {INFINITY, INFINITY, INFINITY}, cmx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int k = 0; k < n; k++) {
+      const int id = w.ord[f + k];
+      const float4 a = w.a[id], b = w.b[id];
+      const float c = w.c[id];
+      box.add(a, b);
+      cmn[0] = fminf(cmn[0], b.z); cmn[1] = fminf(cmn[1], b.w); cmn[2] = fminf(cmn[2], c);
+      cmx[0] = fmaxf(cmx[0], b.z); cmx[1] = fmaxf(cmx[1], b.w); cmx[2] = fmaxf(cmx[2], c);
+    }
+    Choice best{INFINITY, -1, 0, 0};
+    double best_lo = 0, best_scale = 0;
+#pragma unroll 1
+    for (int q = 0; q < 3; q++) {
+      const double lo = q == 0 ? cmn[0] : (q == 1 ? cmn[1] : cmn[2]);
+      const double extent = static_cast<double>(q == 0 ? cmx[0] : (q == 1 ? cmx[1] : cmx[2])) - lo;
+      if (!(extent > 0)) continue;
+      const double scale = bins / extent;
+      for (int k = 0; k < n; k++) {
+        const int id = w.ord[f + k];
+        const int b = bin_of(centroid_of(w.b[id], w.c[id], q), lo, scale, bins);
+        int j = k;
+        for (; j > 0 && (key[j - 1] >> 8) > b; j--) key[j] = key[j - 1];
+        key[j] = (b << 8) | id;
+      }
+      LaneBox r;
+      for (int k = n - 1; k > 0; k--) {
+        const int id = key[k] & 0xff;
+        r.add(w.a[id], w.b[id]);
+        right[k] = r.size();
+      }
+      LaneBox l;
+      int at = key[0];
+      for (int k = 0; k < n - 1; k++) {
+        const int id = at & 0xff, b = at >> 8;
+        l.add(w.a[id], w.b[id]);
+        at = key[k + 1];
+        if (b == (at >> 8)) continue;
+        const double cost = (k + 1) * l.size() + (n - k - 1) * right[k + 1];
+        if (cost < best.cost) {  // false for a NaN
+          best = Choice{cost, q, b, k + 1};
+          best_lo = lo;
+          best_scale = scale;
+        }
+      }
+    }
+    int axis, nleft;
+    const int mode = choose(best, box.b, n, axis, nleft);
+    bool next = false;
     if (mode < 0) {
-      w.leaf[f] = n | (depth << 9) | (((e.y >> 8) & 0xff) << 16) | (((e.y >> 16) & 1u) << 24);
+      put_leaf(st, t.first + f, box.b, n, depth, sub_tag(t, e.y));
+      set_bit(st.leaf_bits, t.first + f);
+      slot_deep = max(slot_deep, depth);
     } else {
-      put_inner(st, t.first + f + nleft, box, t.first + f, depth, axis, sub_tag(t, e));
+      put_inner(st, t.first + f + nleft, box.b, t.first + f, depth, axis, sub_tag(t, e.y));
+      inner_deep = max(inner_deep, depth);
+      // The stable partition, and the children's boxes if they are leaves.
+      LaneBox kid[2];
+      int lpos = 0, rpos = nleft;
+      for (int k = 0; k < n; k++) key[k] = w.ord[f + k];
+      for (int k = 0; k < n; k++) {
+        const int id = key[k];
+        const float4 b = w.b[id];
+        const bool left = mode == 0 ? bin_of(centroid_of(b, w.c[id], axis), best_lo, best_scale, bins) <= best.split
+                                    : k < nleft;
+        if (left) {
+          kid[0].add(w.a[id], b);
+          w.ord[f + lpos++] = static_cast<uint8_t>(id);
+        } else {
+          kid[1].add(w.a[id], b);
+          w.ord[f + rpos++] = static_cast<uint8_t>(id);
+        }
+      }
+      const bool last = depth + 1 >= kBuildDepth;
+      uint2 keep = make_uint2(0, 0);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int kf = f + (q ? nleft : 0), kc = q ? n - nleft : nleft;
+        const unsigned up = static_cast<unsigned>(depth + 1) | (f << 8) | (q << 16);
+        if (last || kc <= kMaxLeaf) {
+          put_leaf(st, t.first + kf, kid[q].b, kc, depth + 1, sub_tag(t, up));
+          set_bit(st.leaf_bits, t.first + kf);
+        } else if (!next) {
+          keep = make_uint2(kf | (kc << 16), up);
+          next = true;
+        } else {
+          const uint2 other = make_uint2(kf | (kc << 16), up);
+          const bool bigger = kc > static_cast<int>(keep.x >> 16);
+          wait[waiting++] = bigger ? other : keep;
+          keep = bigger ? keep : other;
+        }
+      }
+      if (next) e = keep;
     }
+    if (next) continue;
+    if (waiting == 0) break;
+    e = wait[--waiting];
   }
-  // Both halves' children into the lists, in the same order in every lane.
-  for (int h = 0; h < 2; h++) {
-    const int hm = __shfl_sync(full, mode, 16 * h), hn = __shfl_sync(full, n, 16 * h);
-    const int hf = __shfl_sync(full, f, 16 * h), hl = __shfl_sync(full, nleft, 16 * h);
-    const int hd = __shfl_sync(full, depth, 16 * h);
-    if (hn == 0) continue;
-    deep = max(deep, hm >= 0 ? hd : -1);
-    if (hm < 0) continue;
-    sub_child(w, hf, hl, hd + 1, hf, 0, ntodo, ntiny, lane == 0);
-    sub_child(w, hf + hl, hn - hl, hd + 1, hf, 1, ntodo, ntiny, lane == 0);
+}
+
+// The bounds of triangles [first, first + count) of the order, in every lane.
+template <int MB>
+__device__ void sub_bounds(SubWarp<MB>& w, int first, int count, float* box) {
+  float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  for (int k = threadIdx.x & 31; k < count; k += 32) {
+    const int id = w.ord[first + k];
+    const float4 a = w.a[id], b = w.b[id];
+    m[0] = fminf(m[0], a.x); m[1] = fminf(m[1], a.y); m[2] = fminf(m[2], a.z);
+    m[3] = fmaxf(m[3], a.w); m[4] = fmaxf(m[4], b.x); m[5] = fmaxf(m[5], b.y);
   }
-  __syncwarp();
+  for (int q = 0; q < 6; q++) box[q] = unordered(warp_bound(m[q], is_max(q)));
 }
 
 // Finishes subtrees, one warp each, from a queue: a depth-first walk over its
-// larger nodes, then pairs of tiny ones, then its leaves and the order of its
-// triangles. What bounds it: issue slots (shuffles and shared-memory atomics);
-// nothing but the triangles in and the nodes out touches DRAM.
+// larger nodes, the smaller child first (so few nodes wait), then a lane per
+// tiny node, then the order of the triangles. What bounds it: issue slots and
+// shared-memory latency, at the warps that shared memory leaves room for; only
+// the triangles in and the nodes out touch DRAM.
+template <int MB>
 __global__ void __launch_bounds__(32 * kSubWarps) k_subtrees(BuildState st) {
   extern __shared__ __align__(16) unsigned char smem[];
-  SubWarp& w = reinterpret_cast<SubWarp*>(smem)[threadIdx.x >> 5];
+  SubWarp<MB>& w = reinterpret_cast<SubWarp<MB>*>(smem)[threadIdx.x >> 5];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int count = st.ctl->subtrees;
@@ -985,8 +1045,7 @@ __global__ void __launch_bounds__(32 * kSubWarps) k_subtrees(BuildState st) {
     const Subtree t = st.subtrees[s];
     const Prims p = st.prims[t.parity];
     const int n = t.count;
-    const bool leaf = n <= kMaxLeaf || t.depth >= kBuildDepth;
-    if (leaf) {  // at the depth limit of any size
+    if (n <= kMaxLeaf || t.depth >= kBuildDepth) {  // a leaf; at the depth limit of any size
       float m[12];
       clear_box(m);
       for (int k = lane; k < n; k += 32) {
@@ -1005,66 +1064,85 @@ __global__ void __launch_bounds__(32 * kSubWarps) k_subtrees(BuildState st) {
     }
     __syncwarp();
     for (int k = lane; k < n; k += 32) {
-      const float4 a4 = p.a[t.first + k], b4 = p.b[t.first + k];
-      const float2 c2 = p.c[t.first + k];
-      w.pr[0][k] = a4.x; w.pr[1][k] = a4.y; w.pr[2][k] = a4.z;
-      w.pr[3][k] = a4.w; w.pr[4][k] = b4.x; w.pr[5][k] = b4.y;
-      w.pr[6][k] = b4.z; w.pr[7][k] = b4.w; w.pr[8][k] = c2.x;
-      w.leaf[k] = 0;
+      w.a[k] = p.a[t.first + k];
+      w.b[k] = p.b[t.first + k];
+      w.c[k] = p.c[t.first + k].x;
       w.ord[k] = static_cast<uint8_t>(k);
     }
-    const uint2 root = make_uint2(n << 16, t.depth | (1u << 17));
-    int ntodo = 0, ntiny = 0;
-    if (n > kTinyMax) {
-      if (lane == 0) w.todo[0] = root;
-      ntodo = 1;
+    __syncwarp();
+    SubNode e{0, n, static_cast<unsigned>(t.depth) | (1u << 17), {}};
+    int waiting = 0, tiny = 0;
+    bool next = n > kTinyMax;
+    if (next) {
+      sub_bounds(w, 0, n, e.box);
     } else {
-      if (lane == 0) w.tiny[0] = root;
-      ntiny = 1;
+      if (lane == 0) w.tiny[0] = make_uint2(n << 16, e.up);
+      tiny = 1;
+    }
+    while (next) {
+      const int depth = static_cast<int>(e.up & 0xff);
+      int axis, nleft, left_at;
+      const int mode = sub_split(st, w, e, axis, nleft, left_at);
+      const bool last = depth + 1 >= kBuildDepth;
+      SubNode keep{};
+      next = false;
+      if (mode < 0) {
+        if (lane == 0) {
+          put_leaf(st, t.first + e.first, e.box, e.count, depth, sub_tag(t, e.up));
+          set_bit(st.leaf_bits, t.first + e.first);
+        }
+        slot_deep = max(slot_deep, depth);
+      } else {
+        if (lane == 0)
+          put_inner(st, t.first + e.first + nleft, e.box, t.first + e.first, depth, axis, sub_tag(t, e.up));
+        inner_deep = max(inner_deep, depth);
+      }
+#pragma unroll
+      for (int q = 0; q < 2 && mode >= 0; q++) {
+        SubNode kid{e.first + (q ? nleft : 0), q ? e.count - nleft : nleft,
+                    static_cast<unsigned>(depth + 1) | (e.first << 8) | (q << 16), {}};
+        const bool leaf = last || kid.count <= kMaxLeaf;
+        if (!leaf && kid.count <= kTinyMax) {
+          if (lane == 0) w.tiny[tiny] = make_uint2(kid.first | (kid.count << 16), kid.up);
+          tiny++;
+          continue;
+        }
+        if (mode == 0) {
+          for (int i = 0; i < 6; i++) kid.box[i] = unordered(w.sweeps.box[q][axis][left_at + q][i]);
+        } else {
+          sub_bounds(w, kid.first, kid.count, kid.box);
+        }
+        if (leaf) {
+          if (lane == 0) {
+            put_leaf(st, t.first + kid.first, kid.box, kid.count, depth + 1, sub_tag(t, kid.up));
+            set_bit(st.leaf_bits, t.first + kid.first);
+          }
+        } else if (!next) {
+          keep = kid;
+          next = true;
+        } else {
+          const bool bigger = kid.count > keep.count;
+          if (lane == 0) w.todo[waiting] = bigger ? kid : keep;
+          waiting++;
+          if (!bigger) keep = kid;
+        }
+      }
+      __syncwarp();  // the sweeps are read, the lists written
+      if (next) {
+        e = keep;
+      } else if (waiting > 0) {
+        e = w.todo[--waiting];
+        next = true;
+        __syncwarp();
+      }
     }
     __syncwarp();
-    while (ntodo > 0) {
-      const uint2 e = w.todo[--ntodo];
-      inner_deep = max(inner_deep, static_cast<int>(e.y & 0xff));
-      __syncwarp();
-      sub_split(st, t, w, e, ntodo, ntiny);
-    }
-    while (ntiny > 0) {
-      const int take = min(ntiny, 2);
-      ntiny -= take;
-      const bool valid = (lane >> 4) < take;
-      const uint2 e = valid ? w.tiny[ntiny + (lane >> 4)] : make_uint2(0, 0);
-      __syncwarp();
-      sub_split_tiny(st, t, w, e, valid, ntodo, ntiny, inner_deep);
-    }
-    for (int base = 0; base < n; base += 32) {
-      const int k = base + lane;
-      const unsigned info = k < n ? w.leaf[k] : 0u;
-      if (info) {
-        float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        const int c = info & 0x1ff, depth = (info >> 9) & 0x7f;
-        for (int q = 0; q < c; q++) {
-          const int id = w.ord[k + q];
-          for (int a = 0; a < 3; a++) {
-            m[a] = fminf(m[a], w.pr[a][id]);
-            m[3 + a] = fmaxf(m[3 + a], w.pr[3 + a][id]);
-          }
-        }
-        // The root itself can be a leaf (the SAH's choice): then it keeps its tag.
-        const unsigned tag = c == n ? t.tag : 2u * static_cast<unsigned>(t.first + ((info >> 16) & 0xff)) + (info >> 24);
-        put_leaf(st, t.first + k, m, c, depth, tag);
-        if (c > kMaxLeaf && depth < kBuildDepth) slot_deep = max(slot_deep, depth);
-      }
-      if (k < n) st.order[t.first + k] = __float_as_int(p.c[t.first + w.ord[k]].y);
-      const unsigned starts = __ballot_sync(full, info != 0u);
-      if (lane == 0) {
-        const int at = t.first + base, sh = at & 31;
-        if (starts << sh) atomicOr(st.leaf_bits + (at >> 5), starts << sh);
-        if (sh && (starts >> (32 - sh))) atomicOr(st.leaf_bits + (at >> 5) + 1, starts >> (32 - sh));
-      }
-    }
+    for (int k = lane; k < tiny; k += 32) lane_subtree(st, t, w, w.tiny[k], inner_deep, slot_deep);
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) st.order[t.first + k] = __float_as_int(p.c[t.first + w.ord[k]].y);
     __syncwarp();
   }
+  inner_deep = __reduce_max_sync(full, inner_deep);
   slot_deep = __reduce_max_sync(full, slot_deep);
   if (lane == 0) {
     if (inner_deep >= 0) atomicMax(&st.ctl->inner_depth, inner_deep);
@@ -1572,8 +1650,11 @@ static int run_build(BuildBuffers& B, const BuildState& st, float* d_bounds, int
   const size_t N = static_cast<size_t>(n);
   const size_t max_nodes = N / (kSub + 1) + 1;
   int* sums = B.scan_sums.ensure(kScanBlocks);
-  const size_t smem = sizeof(SubWarp) * kSubWarps;
-  check(cudaFuncSetAttribute(k_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+  // Bin arrays for 16 bins leave room for more warps than those for 32.
+  const bool few = st.bins <= 16;
+  const auto subtrees = few ? k_subtrees<16> : k_subtrees<kMaxBins>;
+  const size_t smem = (few ? sizeof(SubWarp<16>) : sizeof(SubWarp<kMaxBins>)) * kSubWarps;
+  check(cudaFuncSetAttribute(subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
         "shared memory");
   // The levels, a few more than a balanced tree has, and the rest of the
   // build behind them; whether that was all is read back once, at the end.
@@ -1592,7 +1673,7 @@ static int run_build(BuildBuffers& B, const BuildState& st, float* d_bounds, int
       k_bin<<<grid, kBuildBlock, 0, s>>>(levels, st);
       k_part<<<grid, kBuildBlock, 0, s>>>(levels, st);
     }
-    k_subtrees<<<std::min(blocks_of(n, kSubWarps), 2 * kBuildGrid), 32 * kSubWarps, smem, s>>>(st);
+    subtrees<<<std::min(blocks_of(n, kSubWarps), 2 * kBuildGrid), 32 * kSubWarps, smem, s>>>(st);
     k_rank_sums<<<kScanBlocks, kScanThreads, 0, s>>>(st, sums);
     k_rank_write<<<kScanBlocks, kScanThreads, 0, s>>>(st, sums);
     k_emit<<<blocks_of(n, 256), 256, 0, s>>>(st, d_bounds, d_nodes);
