@@ -39,6 +39,11 @@ constexpr int kBlock = 128;
 // ray with more distinct see-through hits sets kStatusShadowListOverflow.
 constexpr int kShadowSeen = 64;
 constexpr int kSortMin = 1 << 16;  // shorter queues are shaded in the order they are in
+// Queues of at most this many paths are taken to their ends by one launch
+// (k_tail). Between 2,048 and 16,384 whole renders measured within 3 % of one
+// another (a 64 x 64 tile 0.45 -> 0.24 ms from 4,096 on, a 633 x 471 draft of 7
+// passes 1.84 -> 1.76 at 8,192, 1.80 at 2,048).
+constexpr int kTailMax = 8192;
 constexpr int kMaxIterations = 1 << 16;  // bounce / pass-through iterations of one chunk
 
 // Appends to a queue counter with one atomic per coalesced group of threads.
@@ -320,23 +325,25 @@ MCRT_D bool light_at(const DLight& L, V3 p, V3& l, V3& radiance, float& distance
   return false;
 }
 
-// Where a shade step puts its output: continuing paths and shadow rays.
+// Where a shade step puts its output, continuing paths and shadow rays: the
+// wavefront's queues.
 struct StageQueues {
   int* next;
   unsigned int* next_count;
   float4* shadow;  // 3 float4 per shadow ray
   unsigned int* shadow_count;
+  MCRT_D void push_next(int pid) const { next[queue_append(next_count)] = pid; }
+  MCRT_D float4* push_shadow() const { return shadow + 3 * static_cast<size_t>(queue_append(shadow_count)); }
 };
 
+template <class QS>
 struct ShadowEmitter {
-  float4* queue;
-  unsigned int* counter;
+  QS& qs;
   int pid;
   unsigned long long mask;
   // Queues a shadow ray whose unshadowed contribution is `w`.
   MCRT_D void emit(V3 o, V3 d, float max_t, V3 w, int slot, bool cast_only) {
-    unsigned idx = queue_append(counter);
-    float4* e = queue + 3 * static_cast<size_t>(idx);
+    float4* e = qs.push_shadow();
     e[0] = make_float4(o.x, o.y, o.z, max_t);
     e[1] = make_float4(d.x, d.y, d.z, __int_as_float(pid));
     e[2] = make_float4(w.x, w.y, w.z, __int_as_float(slot | (cast_only ? 0x10000 : 0)));
@@ -347,7 +354,8 @@ struct ShadowEmitter {
 // Direct light of one light: the unshadowed contribution goes straight into
 // `out` when no shadow ray is needed (visibleLight, tracer.ts:515-526), or to
 // a shadow ray weighted by throughput and the environment combine factor.
-MCRT_D void direct_light(const FrameParams& fp, const DScene& sc, ShadowEmitter& em, const DLight& L, int li,
+template <class EM>
+MCRT_D void direct_light(const FrameParams& fp, const DScene& sc, EM& em, const DLight& L, int li,
                          bool receive, V3 p, V3 g, V3 l, float light_distance, V3 c, V3& out, V3 weight) {
   if (fp.shadows == 2 || (fp.shadows == 1 && (!L.cast_shadow || !receive))) {
     out = out + c;
@@ -361,7 +369,8 @@ MCRT_D void direct_light(const FrameParams& fp, const DScene& sc, ShadowEmitter&
 }
 
 // One iteration of samplePixel's loop for path `pid`.
-MCRT_D void shade_path(const DScene& sc, const FrameParams& fp, const PathState& ps, int pid, const StageQueues& qs) {
+template <class QS>
+MCRT_D void shade_path(const DScene& sc, const FrameParams& fp, const PathState& ps, int pid, QS& qs) {
   // The hit word and flags first: a miss (most camera rays of open scenes)
   // reads little more, so the rest of the path state is loaded after the test.
   const float4 h4 = ps.hit[pid];
@@ -437,7 +446,7 @@ MCRT_D void shade_path(const DScene& sc, const FrameParams& fp, const PathState&
   V3 Lr = V3{L4.x, L4.y, L4.z};
   float fog_factor = T4.w;
   float last_env_scale = L4.w;
-  ShadowEmitter em{qs.shadow, qs.shadow_count, pid, 0ull};
+  ShadowEmitter<QS> em{qs, pid, 0ull};
   const bool front = (word & 0x80000000u) != 0;
   const float inf = __int_as_float(0x7f800000);
 
@@ -492,7 +501,7 @@ MCRT_D void shade_path(const DScene& sc, const FrameParams& fp, const PathState&
       const float side = dot(g, d) > 0.0f ? sc.eps : -sc.eps;
       V3 no = p + g * side;
       ps.ray_o[pid] = make_float4(no.x, no.y, no.z, 0.0f);
-      qs.next[queue_append(qs.next_count)] = pid;
+      qs.push_next(pid);
     }
     ps.thr[pid] = make_float4(T.x, T.y, T.z, fog_factor);
     if (!seen) ps.rad[pid] = L4;  // read by resolve if the path ends here
@@ -793,7 +802,7 @@ MCRT_D void shade_path(const DScene& sc, const FrameParams& fp, const PathState&
           ps.ray_o[pid] = make_float4(no.x, no.y, no.z, 0.0f);
           ps.ray_d[pid] = make_float4(sdir.x, sdir.y, sdir.z, 0.0f);
           ps.med[pid] = make_float4(med.x, med.y, med.z, 0.0f);
-          qs.next[queue_append(qs.next_count)] = pid;
+          qs.push_next(pid);
         }
       }
     }
@@ -1005,6 +1014,175 @@ __global__ void __launch_bounds__(kBlock) k_resolve(DScene sc, FrameParams fp, P
                                                     const int* __restrict__ queue, int n, int capacity) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < n) resolve_path(sc, fp, ps, queue[q], capacity);
+}
+
+// -------------------------------------------------------------------- tail
+// A closest-hit or a shadow query, as one type, so that a warp walks both at
+// once. (The shadow query's ray and limit serve for both.)
+struct TailQuery {
+  ShadowQuery s;
+  bool shadow, culls;
+  int pid;
+  float u, v;
+  unsigned hit_word;
+  MCRT_D void load_closest(int path) {
+    shadow = false;
+    pid = path;
+    const float4 o = s.ps.ray_o[path], d = s.ps.ray_d[path];
+    s.r = make_trav_ray(V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z});
+    s.max_t = __int_as_float(0x7f800000);
+    culls = (s.ps.flags[path] & kFlagCull) != 0;
+    u = v = 0.0f;
+    hit_word = 0u;
+  }
+  MCRT_D void load_shadow(int entry) {
+    shadow = true;
+    s.load(entry);
+  }
+  MCRT_D const TravRay& ray() const { return s.r; }
+  MCRT_D float t_max() const { return s.max_t; }
+  MCRT_D int side(int word) const { return !shadow && culls ? tri_side(word) : 2; }
+  MCRT_D HitAction hit(int k, const TriHit& h, int word) {
+    if (shadow) return s.hit(k, h, word);
+    s.max_t = h.t;
+    u = h.u;
+    v = h.v;
+    hit_word = (h.front ? 0x80000000u : 0u) | static_cast<unsigned>(k + 1);
+    return kGoOn;
+  }
+  MCRT_D bool resume() { return s.resume(); }
+  MCRT_D void finish() {
+    if (shadow) {
+      s.finish();
+    } else {
+      s.ps.hit[pid] = make_float4(hit_word != 0u ? s.max_t : 0.0f, u, v, __uint_as_float(hit_word));
+    }
+  }
+};
+
+// A shade step's output of one path in k_tail: its shadow rays go to the
+// path's own entries.
+struct PathQueues {
+  float4* shadow;
+  int shadows;
+  bool goes_on;
+  MCRT_D void push_next(int) { goes_on = true; }
+  MCRT_D float4* push_shadow() { return shadow + 3 * static_cast<size_t>(shadows++); }
+};
+
+// Not inlined, so that its arithmetic is compiled for itself, as it is in the
+// wavefront's shading kernels: inlined into k_tail the compiler fused other
+// multiplies and adds, and last bits differed from the wavefront's.
+__device__ __noinline__ void tail_shade(const DScene& sc, const FrameParams& fp, const PathState& ps, int pid,
+                                        PathQueues& qs) {
+  shade_path(sc, fp, ps, pid, qs);
+}
+
+constexpr int kTailLanes = 8;  // lanes per path
+constexpr int kTailBlock = 64;
+
+// Takes few paths to their ends in one launch: eight lanes per path, of which
+// the first shades it and walks its next ray while the others walk the shadow
+// rays it cast. Bounce by bounce launches cost such paths a host
+// synchronisation, four launches and the latency of two walks each; here a
+// bounce is one walk's latency and a shading step's. What bounds it: those
+// latencies (dependent fetches). The stages are the wavefront's own functions
+// in the same order for each path: resolve after its shadow rays, shading
+// after its closest hit. `params(pid)`: a path's frame parameters; `fetch`:
+// the queue's work counter.
+template <class P>
+MCRT_D void finish_paths(const DScene& sc, const PathState& ps, P params, const int* __restrict__ queue, int n,
+                         int capacity, int slots, unsigned* fetch, unsigned long long* closest_total,
+                         unsigned long long* any_total, unsigned* status_out) {
+  constexpr unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, rank = lane & (kTailLanes - 1), leader = lane & ~(kTailLanes - 1);
+  // Groups of a warp that take paths: all four, or fewer while there are warps to spare.
+  const int warps = static_cast<int>(gridDim.x) * (kTailBlock / 32);
+  const int groups = n <= warps ? 1 : (n <= 2 * warps ? 2 : 4);
+  int below[kStackMax + 2];
+  float seen[kShadowSeen + 10];
+  TravStack st;
+  st.init(below);
+  unsigned status = 0;
+  TailQuery q{ShadowQuery{sc, ps, capacity, &status, seen}};
+  int pid = -1;      // the group's path (its leader's value)
+  int first = 0;     // its entries of the shadow queue, one per slot: those of its place among the n
+  int shadows = 0;   // shadow rays it waits for
+  bool goes_on = false, out_of_paths = leader / kTailLanes >= groups;
+  int iterations = 0;
+  unsigned long long closest = 0, any = 0;
+  for (;;) {
+    if (rank == 0 && pid < 0 && !out_of_paths) {
+      const unsigned i = atomicAdd(fetch, 1u);
+      if (i < static_cast<unsigned>(n)) {
+        pid = queue[i];
+        first = static_cast<int>(i) * slots;
+        goes_on = true;
+        iterations = 0;
+      } else {
+        out_of_paths = true;
+      }
+    }
+    if (!__any_sync(full, rank == 0 && pid >= 0)) break;
+    // Every lane of a group sees its path's state.
+    const int path = __shfl_sync(full, pid, leader);
+    const int waiting = __shfl_sync(full, shadows, leader);
+    const int entries = __shfl_sync(full, first, leader);
+    for (int base = 0; base == 0 || __any_sync(full, path >= 0 && base < waiting); base += kTailLanes - 1) {
+      WalkState w;
+      st.clear();
+      if (rank == 0) {
+        if (base == 0 && pid >= 0 && goes_on) {
+          q.load_closest(pid);
+          w.start(sc);
+          closest++;
+        }
+      } else if (path >= 0 && base + rank - 1 < waiting) {
+        q.load_shadow(entries + base + rank - 1);
+        w.start(sc);
+        any++;
+      }
+      while (__any_sync(full, w.has)) walk_step(sc, q, st, w, status);
+    }
+    __syncwarp();  // hits and slots are written
+    if (rank == 0 && pid >= 0) {
+      const FrameParams& fp = params(pid);
+      if (iterations > 0) resolve_path(sc, fp, ps, pid, capacity);  // the step before
+      shadows = 0;
+      if (goes_on) {
+        PathQueues qs{ps.shadow_queue + 3 * static_cast<size_t>(first), 0, false};
+        tail_shade(sc, fp, ps, pid, qs);
+        shadows = qs.shadows;
+        goes_on = qs.goes_on;
+        if (++iterations > kMaxIterations) {
+          status |= kStatusIterationLimit;
+          goes_on = false;
+          shadows = 0;
+        }
+        if (!goes_on && shadows == 0) resolve_path(sc, fp, ps, pid, capacity);
+      }
+      if (!goes_on && shadows == 0) pid = -1;
+    }
+    __syncwarp();  // shadow rays are written
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    closest += __shfl_xor_sync(full, closest, off);
+    any += __shfl_xor_sync(full, any, off);
+  }
+  if (lane == 0 && closest + any > 0) {
+    atomicAdd(closest_total, closest);
+    atomicAdd(any_total, any);
+  }
+  if (status) atomicOr(status_out, status);
+}
+
+__global__ void __launch_bounds__(kTailBlock) k_tail(const __grid_constant__ DScene sc,
+                                                     const __grid_constant__ FrameParams fp,
+                                                     const __grid_constant__ PathState ps,
+                                                     const int* __restrict__ queue, int n, int capacity, int slots,
+                                                     Counters* cnt) {
+  finish_paths(sc, ps, [&](int) -> const FrameParams& { return fp; }, queue, n, capacity, slots, &cnt->fetch,
+               &cnt->tail_closest, &cnt->tail_any, &cnt->status);
 }
 
 // -------------------------------------------------------------- accumulate
@@ -1381,6 +1559,7 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
     e = buffers.side_stream(&side, &fork, &join);
     overlap = e == cudaSuccess;
   }
+  bool tails = false;      // a tail launch counted rays on the device
   bool side_busy = false;  // side work queued since the main stream last joined it
   auto join_side = [&]() {
     if (side_busy) {
@@ -1406,6 +1585,20 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
       // loop this long means corrupt state, reported rather than spun on.
       if (++iterations > kMaxIterations) {
         e = cudaErrorLaunchTimeout;
+        break;
+      }
+      if (n <= kTailMax) {
+        // Few paths left (or few from the start): one launch takes them to
+        // their ends, with the side stream's work on them done first.
+        join_side();
+        cudaMemsetAsync(&cnt->fetch, 0, sizeof(unsigned int), stream);
+        tm.start();
+        const int limit = resident_limit(reinterpret_cast<const void*>(k_tail), kTailBlock);
+        const int blocks = std::min(limit, blocks_for(n, kTailBlock / 32));
+        k_tail<<<blocks, kTailBlock, 0, stream>>>(scene, f, ps, ps.queue[cur], n, cap, buffers.slots(), cnt);
+        tm.stop(st.ms_extend, st.n_extend);
+        st.launches++;
+        tails = true;
         break;
       }
       // The camera rays walk warp-coherent where a warp's 32 rays (passes of
@@ -1494,7 +1687,14 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
   if (e == cudaSuccess) {
     e = cudaMemcpyAsync(host, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess) st.status |= host->status;
+    if (e == cudaSuccess) {
+      st.status |= host->status;
+      if (tails) {
+        st.closest_rays += host->tail_closest;
+        st.any_rays += host->tail_any;
+      }
+      if (host->status & kStatusIterationLimit) e = cudaErrorLaunchTimeout;
+    }
   }
   return e;
 }
@@ -1573,12 +1773,29 @@ __global__ void __launch_bounds__(kBlock) k_batch_raygen(const BatchTables* __re
   }
 }
 
+// Takes a scene's last paths of the chunk to their ends once at most kTailMax
+// are queued; the other stages of the iteration then leave the queue alone and
+// k_batch_advance finds nothing queued behind it.
+__global__ void __launch_bounds__(kTailBlock) k_batch_tail(const __grid_constant__ DScene sc, int s, BatchTables* t,
+                                                           const __grid_constant__ PathState ps, int capacity,
+                                                           int slots, BatchCounters* bc) {
+  SceneQueues* sq = &t->scenes[s];
+  const int n = static_cast<int>(sq->count);
+  if (n == 0 || n > kTailMax) return;
+  PathState pq = ps;
+  pq.shadow_queue += 3ull * sq->base * static_cast<unsigned>(slots);
+  const FrameParams* __restrict__ params = t->fp;
+  finish_paths(sc, pq, [&](int pid) -> const FrameParams& { return params[ps.seg[pid]]; },
+               ps.queue[t->iteration & 1] + sq->base, n, capacity, slots, &sq->fetch, &bc->closest, &bc->any,
+               &bc->status);
+}
+
 template <int B>
 __global__ void __launch_bounds__(B, 1024 / B) k_batch_extend(DScene sc, int s, BatchTables* t, PathState ps,
                                                     BatchCounters* bc) {
   SceneQueues* sq = &t->scenes[s];
   const int n = static_cast<int>(sq->count);
-  if (n == 0) return;
+  if (n <= kTailMax) return;  // none, or k_batch_tail's
   unsigned status = 0;
   ExtendQuery q{sc, ps, ps.queue[t->iteration & 1] + sq->base, 0, {}, nullptr, 0};
   walk<kRefillClosest>(sc, q, n, &sq->fetch, status);
@@ -1588,6 +1805,7 @@ __global__ void __launch_bounds__(B, 1024 / B) k_batch_extend(DScene sc, int s, 
 __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSM) k_batch_shade(DScene sc, int s, BatchTables* t, PathState ps, int slots) {
   SceneQueues* sq = &t->scenes[s];
   const int n = static_cast<int>(sq->count);
+  if (n <= kTailMax) return;
   const int cur = t->iteration & 1;
   // In shading order once the queue is long enough to be sorted (k_batch_class_*).
   const int* qin = (n >= kSortMin ? ps.binned : ps.queue[cur]) + sq->base;
@@ -1632,6 +1850,7 @@ __global__ void __launch_bounds__(kBlock) k_batch_resolve(DScene sc, int s, Batc
                                                           int capacity) {
   SceneQueues* sq = &t->scenes[s];
   const int n = static_cast<int>(sq->count);
+  if (n <= kTailMax) return;
   const int* qin = ps.queue[t->iteration & 1] + sq->base;
   const FrameParams* __restrict__ params = t->fp;
   const int stride = gridDim.x * blockDim.x;
@@ -1700,8 +1919,10 @@ __global__ void k_batch_advance(BatchTables* t, int nscenes, BatchCounters* bc, 
   unsigned long long closest = 0, any = 0;
   for (int s = 0; s < nscenes; s++) {
     SceneQueues& q = t->scenes[s];
-    closest += q.count;
-    any += q.shadow_count;
+    if (q.count > kTailMax) {  // k_batch_tail counts its own
+      closest += q.count;
+      any += q.shadow_count;
+    }
     q.count = q.next_count;
     q.next_count = 0;
     q.shadow_count = 0;
@@ -1798,6 +2019,8 @@ cudaError_t batch_grids(BatchGrids* g, int variant, int capacity) {
   g->variant = (variant >= 0 && variant < kVariantCount) ? variant : 0;
   g->block = bv.block;
   g->raygen = resident_blocks(reinterpret_cast<const void*>(k_batch_raygen), kBlock);
+  g->tail = std::min(resident_blocks(reinterpret_cast<const void*>(k_batch_tail), kTailBlock),
+                     blocks_for(kTailMax, kTailBlock / 32));
   g->extend = resident_blocks(reinterpret_cast<const void*>(bv.extend), bv.block);
   // Shading launches many more blocks than fit at once (each taking a few
   // 128-path tiles): blocks that finish make room for fresh ones, as in the
@@ -1824,9 +2047,10 @@ cudaError_t launch_batch_iteration(const DScene* scenes, int nscenes, BatchTable
                                    int capacity, int slots, BatchCounters* counters, const BatchGrids& g, bool graph,
                                    cudaGraphConditionalHandle handle, cudaStream_t s, const SceneLanes* lanes) {
   const BatchVariant& bv = batch_variant(g.variant);
-  // One scene's stages, in order: closest hits, shading order, shading, shadow
-  // rays, resolve. Scenes touch disjoint queue ranges, bins and slots.
+  // One scene's stages, in order: the tail (which does the rest's work once few
+  // paths are left), closest hits, shading order, shading, shadow rays, resolve. Scenes touch disjoint queue ranges, bins and slots.
   auto chain = [&](int i, cudaStream_t q) {
+    k_batch_tail<<<g.tail, kTailBlock, 0, q>>>(scenes[i], i, t, ps, capacity, slots, counters);
     bv.extend<<<g.extend, bv.block, 0, q>>>(scenes[i], i, t, ps, counters);
     k_batch_class_count<<<g.sort, 256, 0, q>>>(scenes[i], i, t, ps);
     k_batch_class_scatter<<<g.sort, 256, 0, q>>>(scenes[i], i, t, ps);

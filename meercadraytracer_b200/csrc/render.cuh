@@ -74,6 +74,8 @@ struct Counters {
   unsigned int status;
   unsigned int fetch;         // next query a closest-hit traversal warp takes
   unsigned int fetch_shadow;  // the same for the any-hit (shadow) traversal
+  unsigned int pad;
+  unsigned long long tail_closest, tail_any;  // queries of tail launches, counted on the device
 };
 
 // Work and time of the kernels of one render, for benchmarks.
@@ -194,7 +196,7 @@ struct BatchCounters {
 
 // Grid sizes of the batched kernels on the current device, for a traversal variant.
 struct BatchGrids {
-  int raygen, extend, shade, shadow, resolve, accumulate, sort;
+  int raygen, tail, extend, shade, shadow, resolve, accumulate, sort;
   int variant, block;
 };
 

@@ -316,6 +316,94 @@ enum HitAction { kGoOn, kStop, kPause };
 // Root reference of the scene: node 0, or the single leaf at triangle 0.
 MCRT_D int root_ref(const DScene& sc) { return sc.root_count > 0 ? ~0 : 0; }
 
+// Where one lane's walk stands.
+struct WalkState {
+  int node = kSentinel;  // next node to visit (kSentinel: none)
+  int leaf = 0;          // postponed leaf (< 0), or 0
+  int left = 0;          // node visits and leaves the current query may still take
+  bool has = false;      // this lane holds an unfinished query
+  MCRT_D void start(const DScene& sc) {
+    has = true;
+    leaf = 0;
+    left = max_steps(sc);
+    node = sc.tri_count == 0 ? kSentinel : root_ref(sc);
+  }
+};
+
+// One round of every lane's walk: inner nodes until each holds a leaf, then
+// leaves; finishes the queries that end. All 32 lanes call it.
+template <class Q>
+MCRT_D void walk_step(const DScene& sc, Q& q, TravStack& st, WalkState& w, unsigned& status) {
+  // A lane may start at, or come back to, a leaf with none postponed.
+  {
+    const bool take = w.node < 0 && w.leaf == 0;
+    w.leaf = take ? w.node : w.leaf;
+    st.pop(w.node, take);
+  }
+  // Descend until every lane holds a leaf (or has finished).
+  while (static_cast<unsigned>(w.node) < static_cast<unsigned>(kSentinel)) {
+    if (--w.left < 0) break;
+    const NodeHit h = test_node(sc.nodes, w.node, q.ray(), q.t_max());
+    // Nearer child next, the other pushed. The far reference is
+    // derived from the near one by xor rather than by a second select
+    // on the same condition: nvcc 12.9 at -O1 and above merged such a
+    // select pair into one value, pushing the near child twice.
+    const int near_ref = (h.h0 && (!h.h1 || h.e0 <= h.e1)) ? h.left : h.right;
+    if (!st.push(h.left ^ h.right ^ near_ref, h.h0 && h.h1)) status |= kStatusStackOverflow;
+    w.node = near_ref;
+    st.pop(w.node, !(h.h0 || h.h1));
+    const bool take = w.node < 0 && w.leaf == 0;  // postpone the leaf, keep descending
+    w.leaf = take ? w.node : w.leaf;
+    st.pop(w.node, take);
+    if (!__any_sync(__activemask(), w.leaf == 0)) break;
+  }
+  // Test the postponed leaf, then any leaf reached right after it, each
+  // lane going on to its next triangle on its own.
+  bool stop = false, paused = false;
+  if (w.leaf < 0 && --w.left >= 0) {
+    const TriFrame f = make_frame(q.ray());
+    int k = ~w.leaf;
+    for (;;) {
+      const TriRows rows = load_rows(sc, f, k);
+      const bool end = leaf_end(rows.word()) || k + 1 >= sc.tri_count;
+      TriHit th;
+      if (intersect_triangle(f, rows, q.t_max(), q.side(rows.word()), th)) {
+        const HitAction a = q.hit(k, th, rows.word());
+        stop = a == kStop;
+        paused = a == kPause;
+        if (a != kGoOn) {
+          w.leaf = end ? 0 : ~(k + 1);  // the rest of the leaf, for a pause
+          w.left += end ? 0 : 1;        // which is no further step
+          break;
+        }
+      }
+      k++;
+      if (end) {
+        w.leaf = 0;
+        if (w.node >= 0) break;
+        w.leaf = w.node;
+        k = ~w.node;
+        st.pop(w.node, true);
+        if (--w.left < 0) break;
+      }
+    }
+  }
+  if (w.left < 0) {
+    status |= kStatusStepLimit;
+    stop = true;
+  }
+  if (paused) stop = !q.resume();
+  if (stop) {
+    w.node = kSentinel;
+    w.leaf = 0;
+  }
+  if (w.has && w.node == kSentinel && w.leaf == 0) {
+    q.finish();
+    w.has = false;
+    w.left = 0;
+  }
+}
+
 // Persistent while-while traversal of queries [0, n) for one warp, taking
 // work from *counter. Q supplies, per lane:
 //   void load(int index)      start query `index` (ray, limits, result state)
@@ -347,17 +435,12 @@ template <int REFILL = kRefill, class Q>
 MCRT_D void traverse_persistent(const DScene& sc, Q& q, int n, int lanes, unsigned* counter, TravStack& st,
                                 unsigned& status) {
   const unsigned lane = threadIdx.x & 31;
-  const bool empty = sc.tri_count == 0;
-  const int step_limit = max_steps(sc);
-  int node = kSentinel;  // next node to visit (kSentinel: none)
-  int leaf = 0;          // postponed leaf (< 0), or 0
-  int left = 0;          // node visits and leaves the current query may still take
-  bool has = false;      // this lane holds an unfinished query
+  WalkState w;
   bool exhausted = static_cast<int>(lane) >= lanes;
   const int refill = 32 - lanes + max(1, REFILL * lanes / 32);  // lanes without a query that call for a refill
   for (;;) {
     // Refill finished lanes with one atomic per warp.
-    const bool need = !has && !exhausted;
+    const bool need = !w.has && !exhausted;
     const unsigned mneed = __ballot_sync(0xffffffffu, need);
     if (mneed) {
       const int leader = __ffs(mneed) - 1;
@@ -368,87 +451,17 @@ MCRT_D void traverse_persistent(const DScene& sc, Q& q, int n, int lanes, unsign
         const unsigned idx = base + __popc(mneed & lanemask_lt());
         if (idx < static_cast<unsigned>(n)) {
           q.load(static_cast<int>(idx));
-          has = true;
           st.clear();
-          leaf = 0;
-          left = step_limit;
-          node = empty ? kSentinel : root_ref(sc);
+          w.start(sc);
         } else {
           exhausted = true;
         }
       }
     }
-    if (__all_sync(0xffffffffu, !has)) return;  // every lane is exhausted
+    if (__all_sync(0xffffffffu, !w.has)) return;  // every lane is exhausted
     do {
-      // A lane may start at, or come back to, a leaf with none postponed.
-      {
-        const bool take = node < 0 && leaf == 0;
-        leaf = take ? node : leaf;
-        st.pop(node, take);
-      }
-      // Descend until every lane holds a leaf (or has finished).
-      while (static_cast<unsigned>(node) < static_cast<unsigned>(kSentinel)) {
-        if (--left < 0) break;
-        const NodeHit h = test_node(sc.nodes, node, q.ray(), q.t_max());
-        // Nearer child next, the other pushed. The far reference is
-        // derived from the near one by xor rather than by a second select
-        // on the same condition: nvcc 12.9 at -O1 and above merged such a
-        // select pair into one value, pushing the near child twice.
-        const int near_ref = (h.h0 && (!h.h1 || h.e0 <= h.e1)) ? h.left : h.right;
-        if (!st.push(h.left ^ h.right ^ near_ref, h.h0 && h.h1)) status |= kStatusStackOverflow;
-        node = near_ref;
-        st.pop(node, !(h.h0 || h.h1));
-        const bool take = node < 0 && leaf == 0;  // postpone the leaf, keep descending
-        leaf = take ? node : leaf;
-        st.pop(node, take);
-        if (!__any_sync(__activemask(), leaf == 0)) break;
-      }
-      // Test the postponed leaf, then any leaf reached right after it, each
-      // lane going on to its next triangle on its own.
-      bool stop = false, paused = false;
-      if (leaf < 0 && --left >= 0) {
-        const TriFrame f = make_frame(q.ray());
-        int k = ~leaf;
-        for (;;) {
-          const TriRows rows = load_rows(sc, f, k);
-          const bool end = leaf_end(rows.word()) || k + 1 >= sc.tri_count;
-          TriHit th;
-          if (intersect_triangle(f, rows, q.t_max(), q.side(rows.word()), th)) {
-            const HitAction a = q.hit(k, th, rows.word());
-            stop = a == kStop;
-            paused = a == kPause;
-            if (a != kGoOn) {
-              leaf = end ? 0 : ~(k + 1);  // the rest of the leaf, for a pause
-              left += end ? 0 : 1;        // which is no further step
-              break;
-            }
-          }
-          k++;
-          if (end) {
-            leaf = 0;
-            if (node >= 0) break;
-            leaf = node;
-            k = ~node;
-            st.pop(node, true);
-            if (--left < 0) break;
-          }
-        }
-      }
-      if (left < 0) {
-        status |= kStatusStepLimit;
-        stop = true;
-      }
-      if (paused) stop = !q.resume();
-      if (stop) {
-        node = kSentinel;
-        leaf = 0;
-      }
-      if (has && node == kSentinel && leaf == 0) {
-        q.finish();
-        has = false;
-        left = 0;
-      }
-    } while (__popc(__ballot_sync(0xffffffffu, !has)) < refill && __any_sync(0xffffffffu, has));
+      walk_step(sc, q, st, w, status);
+    } while (__popc(__ballot_sync(0xffffffffu, !w.has)) < refill && __any_sync(0xffffffffu, w.has));
   }
 }
 
