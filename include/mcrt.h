@@ -16,6 +16,7 @@
 #ifndef MCRT_H
 #define MCRT_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #include "mcrt_types.h"
@@ -61,6 +62,12 @@ int32_t mcrt_version(void);
 
 /* Number of CUDA devices visible. */
 int32_t mcrt_device_count(int32_t* count);
+
+/* Pinned host memory, for results: every function that writes into host
+ * memory copies straight into it, without the runtime's staging, and batched
+ * images arrive while the host goes on. Any host memory may be used instead. */
+int32_t mcrt_host_alloc(size_t bytes, void** out);
+int32_t mcrt_host_free(void* p);
 
 /* new WorkerExecutor(...) / createTileHandler(), src/executors.ts:54-94,
  * src/protocol.ts:55: an executor on `device`. */

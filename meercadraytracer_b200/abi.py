@@ -165,6 +165,12 @@ class mcrt_instance(C.Structure):
     ]
 
 
+# mcrt_instance as a numpy record, for filling many at once.
+INSTANCE_DTYPE = np.dtype([("world", np.float64, 16), ("mesh", np.int32), ("material", np.uint32), ("flags", np.uint8),
+                           ("side", np.uint8), ("flat_shading", np.uint8), ("pad_", np.uint8, 5)])
+assert INSTANCE_DTYPE.itemsize == C.sizeof(mcrt_instance)
+
+
 class mcrt_build_info(C.Structure):
     _fields_ = [
         ("flatten_ms", C.c_double), ("build_ms", C.c_double), ("finish_ms", C.c_double), ("total_ms", C.c_double),

@@ -22,7 +22,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
 
-from . import abi
+from . import abi, pinned
 from ._lib import call, load
 from .executors import GpuExecutor
 from .types import CompiledCamera, CompiledScene, TraceSettings
@@ -62,6 +62,11 @@ class BatchRenderer:
         self._executors: Dict[int, Tuple[CompiledScene, GpuExecutor]] = {}
         self._buffers: Dict[int, Tuple[np.ndarray, Optional[np.ndarray], Optional[np.ndarray]]] = {}
         self._adopted: set = set()
+        # Buffers of requests that ended before their copies may have: kept for three more steps (two
+        # chunks are in flight at most, and each step finishes the oldest).
+        self._steps = 0
+        self._open: set = set()  # requests whose DONE event has not been seen
+        self._retired: List[Tuple[int, object]] = []
 
     # ----------------------------------------------------------- scenes
     def executor(self, scene: CompiledScene) -> GpuExecutor:
@@ -112,13 +117,14 @@ class BatchRenderer:
         rid = C.c_int64()
         call("mcrt_batch_submit", self._h, C.byref(c), C.byref(rid))
         self._buffers[rid.value] = buffers
+        self._open.add(rid.value)
         return rid.value
 
     def submit(self, r: RenderRequest) -> int:
         """Queues a request; returns its id. Its images are result(id) / preview(id) / progress(id)."""
-        image = np.zeros(r.width * r.height * 4, np.uint8)
-        preview = np.zeros(r.width * r.height * 4, np.uint8) if r.preview_block > 1 else None
-        progress = np.zeros(r.width * r.height * 4, np.uint8) if r.progress else None
+        image = pinned.zeros(r.width * r.height * 4, np.uint8)
+        preview = pinned.zeros(r.width * r.height * 4, np.uint8) if r.preview_block > 1 else None
+        progress = pinned.zeros(r.width * r.height * 4, np.uint8) if r.progress else None
         return self._submit_c(self._c_request(r, image, preview, progress), (image, preview, progress))
 
     def submit_to(self, executor: GpuExecutor, versions: Tuple[int, int], camera: CompiledCamera,
@@ -126,9 +132,9 @@ class BatchRenderer:
                   srgb: bool = True, progress: bool = False) -> int:
         """As submit, for a scene that `executor` already holds under `versions` (geometry, shading),
         as SceneSync.sync leaves it."""
-        image = np.zeros(width * height * 4, np.uint8)
-        preview = np.zeros(width * height * 4, np.uint8) if preview_block > 1 else None
-        prog = np.zeros(width * height * 4, np.uint8) if progress else None
+        image = pinned.zeros(width * height * 4, np.uint8)
+        preview = pinned.zeros(width * height * 4, np.uint8) if preview_block > 1 else None
+        prog = pinned.zeros(width * height * 4, np.uint8) if progress else None
         c = self._c_fields(executor, versions, camera, settings, width, height, samples, preview_block, srgb, image,
                            preview, prog)
         return self._submit_c(c, (image, preview, prog))
@@ -141,8 +147,15 @@ class BatchRenderer:
         events = (abi.mcrt_batch_event * max(1, max_events))()
         n = C.c_int32()
         idle = C.c_int32()
+        self._steps += 1
         call("mcrt_batch_step", self._h, events, int(max_events), C.byref(n), C.byref(idle))
-        return [(events[i].id, events[i].kind, events[i].samples) for i in range(n.value)], bool(idle.value)
+        if self._retired:
+            self._retired = [] if idle.value else [r for r in self._retired if r[0] > self._steps]
+        out = [(events[i].id, events[i].kind, events[i].samples) for i in range(n.value)]
+        for rid, kind, _ in out:
+            if kind == EVENT_DONE:
+                self._open.discard(rid)
+        return out, bool(idle.value)
 
     def result(self, rid: int) -> np.ndarray:
         return self._buffers[rid][0]
@@ -156,15 +169,23 @@ class BatchRenderer:
 
     def forget(self, rid: int) -> None:
         """Drops the host buffers of a finished or cancelled request."""
-        self._buffers.pop(rid, None)
+        buffers = self._buffers.pop(rid, None)
+        if rid in self._open:
+            self._open.discard(rid)
+            if buffers is not None:
+                self._retired.append((self._steps + 3, buffers))
 
     def render(self, requests: Sequence[RenderRequest]) -> List[np.ndarray]:
         """Renders every request to completion in one batch (mcrt_batch_render)."""
-        images = [np.zeros(r.width * r.height * 4, np.uint8) for r in requests]
+        images = [pinned.empty(r.width * r.height * 4, np.uint8) for r in requests]
         arr = (abi.mcrt_request * max(1, len(requests)))()
         for i, r in enumerate(requests):
             arr[i] = self._c_request(r, images[i], None)
-        call("mcrt_batch_render", self._h, int(len(requests)), arr)
+        try:
+            call("mcrt_batch_render", self._h, int(len(requests)), arr)
+        except Exception:
+            self._retired.append((self._steps + 3, images))  # a failed call may leave chunks in flight
+            raise
         return images
 
     def set_chunk(self, paths: int) -> None:
@@ -181,8 +202,9 @@ class BatchRenderer:
 
     def dispose(self) -> None:
         if self._h is not None:
-            call("mcrt_batch_destroy", self._h)
+            call("mcrt_batch_destroy", self._h)  # waits for what is in flight
             self._h = None
+        self._retired = []
         for _, ex in self._executors.values():
             if id(ex) not in self._adopted:
                 ex.dispose()

@@ -1254,7 +1254,9 @@ __global__ void k_tile_output(const float4* __restrict__ samples, FrameParams fp
   out[i] = samples[b];
 }
 
-// Closest hits of arbitrary rays (origin, -, direction, -): debugging and parity.
+constexpr int kFewBlock = 64;
+
+// Closest hits of arbitrary rays (origin, -, direction, -).
 struct RayQuery {
   const DScene& sc;
   const float4* rays;
@@ -1290,6 +1292,26 @@ __global__ void __launch_bounds__(kBlock) k_trace_rays(DScene sc, const float4* 
   if (status) atomicOr(fetch + 1, status);
 }
 
+// Few rays (at most kFewRays), read from and answered into host memory that
+// the device sees, so that a call is one launch and one wait: no counters to
+// clear, no copies. One ray per warp while there are warps for it.
+template <class Q>
+MCRT_D void trace_few(const DScene& sc, Q& q, int n, unsigned* status_out) {
+  const int lanes = query_lanes(n), lane = threadIdx.x & 31;
+  const int i = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane;
+  int below[kStackMax + 2];
+  TravStack st;
+  st.init(below);
+  unsigned status = 0;
+  WalkState w;
+  if (lane < lanes && i < n) {
+    q.load(i);
+    w.start(sc);
+  }
+  while (__any_sync(0xffffffffu, w.has)) walk_step(sc, q, st, w, status);
+  if (status) atomicOr_system(status_out, status);
+}
+
 // Number of hits along each ray (intersectAny with a counting visitor).
 struct CountQuery {
   const DScene& sc;
@@ -1322,6 +1344,18 @@ __global__ void __launch_bounds__(kBlock) k_count_hits(DScene sc, const float4* 
   CountQuery q{sc, rays, counts, 0, 0, 0.0f, {}};
   walk<kRefill>(sc, q, n, fetch, status);
   if (status) atomicOr(fetch + 1, status);
+}
+
+__global__ void __launch_bounds__(kFewBlock) k_trace_few(DScene sc, const float4* __restrict__ rays, int n, int cull,
+                                                         int4* __restrict__ hits, unsigned* status) {
+  RayQuery q{sc, rays, cull, hits, 0, {}};
+  trace_few(sc, q, n, status);
+}
+
+__global__ void __launch_bounds__(kFewBlock) k_count_few(DScene sc, const float4* __restrict__ rays, int n,
+                                                         int* __restrict__ counts, unsigned* status) {
+  CountQuery q{sc, rays, counts, 0, 0, 0.0f, {}};
+  trace_few(sc, q, n, status);
 }
 
 // ------------------------------------------------------------------- host
@@ -1679,12 +1713,13 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
     }
   }
   join_side();
-  if (side) {
-    const cudaError_t es = cudaStreamSynchronize(side);
-    if (e == cudaSuccess) e = es;
+  if (e != cudaSuccess) {  // nothing of a failed render stays in flight
+    if (side) cudaStreamSynchronize(side);
+    cudaStreamSynchronize(stream);
+    return e;
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-  if (e == cudaSuccess) {
+  {
+    // The side stream's work is behind the main one's by now: one wait for all.
     e = cudaMemcpyAsync(host, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e == cudaSuccess) {
@@ -1740,6 +1775,21 @@ cudaError_t launch_count_hits(const DScene& scene, const float4* rays, int count
   if (count <= 0) return cudaSuccess;
   cudaMemsetAsync(fetch, 0, sizeof(unsigned), s);
   k_count_hits<<<walk_blocks(k_count_hits, count), kBlock, 0, s>>>(scene, rays, count, counts, fetch);
+  return cudaGetLastError();
+}
+
+// Few rays, host memory (pinned, read and written by the kernel): a warp each.
+cudaError_t launch_trace_few(const DScene& scene, const float4* rays, int count, int cull, int4* hits,
+                             unsigned* status, cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  k_trace_few<<<blocks_for(count, kFewBlock / 32), kFewBlock, 0, s>>>(scene, rays, count, cull, hits, status);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_count_few(const DScene& scene, const float4* rays, int count, int* counts, unsigned* status,
+                             cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  k_count_few<<<blocks_for(count, kFewBlock / 32), kFewBlock, 0, s>>>(scene, rays, count, counts, status);
   return cudaGetLastError();
 }
 

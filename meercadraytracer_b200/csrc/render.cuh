@@ -255,5 +255,12 @@ cudaError_t launch_trace_rays(const DScene& scene, const float4* rays, int count
                               unsigned* fetch, cudaStream_t s);
 cudaError_t launch_count_hits(const DScene& scene, const float4* rays, int count, int* counts, unsigned* fetch,
                               cudaStream_t s);
+// The same for at most kFewRays rays, all arrays in pinned host memory and
+// *status zeroed by the caller: one launch, no counters.
+constexpr int kFewRays = 4096;
+cudaError_t launch_trace_few(const DScene& scene, const float4* rays, int count, int cull, int4* hits,
+                             unsigned* status, cudaStream_t s);
+cudaError_t launch_count_few(const DScene& scene, const float4* rays, int count, int* counts, unsigned* status,
+                             cudaStream_t s);
 
 }  // namespace mcrt

@@ -27,7 +27,7 @@ from typing import Any, Dict, List, Optional, Sequence, Set, Tuple
 
 import numpy as np
 
-from . import abi
+from . import abi, pinned
 from ._lib import NOALLOC_MAX_RAYS, McrtError, call, load, mcrt_stats
 from .types import (
     CompiledBvh,
@@ -137,7 +137,7 @@ class GpuExecutor:
 
     def _render_tile(self, m: Dict[str, Any]) -> np.ndarray:
         tile: Tile = m["tile"]
-        out = np.zeros(tile.width * tile.height * 4, np.float32)
+        out = pinned.zeros(tile.width * tile.height * 4, np.float32)
         cam = abi.to_c_camera(m["camera"])
         st = abi.to_c_settings(m["settings"])
         t = abi.to_c_tile(tile)
@@ -190,7 +190,7 @@ class GpuExecutor:
                  settings: TraceSettings, samples: int = 16, srgb: bool = True) -> np.ndarray:
         """raytraceCompiled (src/raytrace.ts:69-82) on the device: RGBA8 bytes."""
         gv, sv = self.load_scene(scene)
-        out = np.zeros(width * height * 4, np.uint8)
+        out = pinned.empty(width * height * 4, np.uint8)
         cam, st = abi.to_c_camera(camera), abi.to_c_settings(settings)
         with self._lock:
             call("mcrt_raytrace", self._h, gv, sv, C.byref(cam), C.byref(st), int(width), int(height), int(samples),
@@ -218,7 +218,7 @@ class GpuExecutor:
                 call("mcrt_raytrace_device", self._h, gv, sv, C.byref(cam), C.byref(st), int(width), int(height),
                      int(samples), int(bool(srgb)), C.c_void_p(device_ptr))
                 return None
-            out = np.zeros(width * height * 4, np.uint8)
+            out = pinned.empty(width * height * 4, np.uint8)
             call("mcrt_raytrace", self._h, gv, sv, C.byref(cam), C.byref(st), int(width), int(height), int(samples),
                  int(bool(srgb)), abi.ptr(out, C.c_uint8))
             return out
@@ -261,10 +261,10 @@ class GpuExecutor:
         """intersectClosest for rays [n, 8] (origin, -, direction, -) on the resident geometry."""
         rays = np.ascontiguousarray(rays, np.float32)
         n = rays.shape[0]
-        tri = np.zeros(n, np.int32)
-        t = np.zeros(n, np.float32)
-        u = np.zeros(n, np.float32)
-        front = np.zeros(n, np.int32)
+        tri = pinned.empty(n, np.int32)
+        t = pinned.empty(n, np.float32)
+        u = pinned.empty(n, np.float32)
+        front = pinned.empty(n, np.int32)
         with self._lock:
             call("mcrt_intersect_closest", self._h, int(geometry_version), n, abi.ptr(rays, C.c_float), int(cull),
                  abi.ptr(tri, C.c_int32), abi.ptr(t, C.c_float), abi.ptr(u, C.c_float), abi.ptr(front, C.c_int32))
@@ -291,7 +291,7 @@ class GpuExecutor:
     def intersect_any_count(self, geometry_version: int, rays: np.ndarray) -> np.ndarray:
         rays = np.ascontiguousarray(rays, np.float32)
         n = rays.shape[0]
-        counts = np.zeros(n, np.int32)
+        counts = pinned.empty(n, np.int32)
         with self._lock:
             call("mcrt_intersect_any_count", self._h, int(geometry_version), n, abi.ptr(rays, C.c_float),
                  abi.ptr(counts, C.c_int32))
@@ -302,15 +302,15 @@ class GpuExecutor:
         """buildBvh (src/bvh.ts:16-178) on the GPU."""
         tris = np.ascontiguousarray(triangles, np.float32)
         cap = max(1, 2 * count - 1)
-        bounds = np.zeros(cap * 6, np.float32)
-        nodes = np.zeros(cap * 3, np.int32)
-        order = np.zeros(max(1, count), np.uint32)
+        bounds = pinned.empty(cap * 6, np.float32)
+        nodes = pinned.empty(cap * 3, np.int32)
+        order = pinned.empty(max(1, count), np.uint32)
         m = C.c_int32()
         with self._lock:
             call("mcrt_build_bvh", self._h, abi.ptr(tris, C.c_float), int(count), abi.ptr(bounds, C.c_float),
                  abi.ptr(nodes, C.c_int32), abi.ptr(order, C.c_uint32), C.byref(m))
         k = int(m.value)
-        return CompiledBvh(bounds[: k * 6].copy(), nodes[: k * 3].copy(), k), order[:count].copy()
+        return CompiledBvh(bounds[: k * 6], nodes[: k * 3], k), order[:count]
 
     def compile_sink(self, sink: Any) -> CompiledGeometry:
         """compileGeometry after the flatten (src/compile.ts:359-403) on the GPU."""
@@ -369,12 +369,15 @@ class GpuExecutor:
         is resident (geometry version returned in the info); with `download` the compiled arrays
         come back as a CompiledGeometry too."""
         arr = (abi.mcrt_instance * max(1, len(instances)))()
-        for i, (world, mesh, material, flags, side, flat) in enumerate(instances):
-            w = np.asarray(world, np.float64).reshape(16)
-            for k in range(16):
-                arr[i].world[k] = float(w[k])
-            arr[i].mesh, arr[i].material = int(mesh), int(material)
-            arr[i].flags, arr[i].side, arr[i].flat_shading = int(flags), int(side), int(bool(flat))
+        if len(instances):
+            # The same memory as a numpy record array: one assignment per column.
+            a = np.frombuffer(arr, abi.INSTANCE_DTYPE)
+            worlds, meshes, materials, flags, sides, flats = zip(*instances)
+            a["world"] = np.stack([np.asarray(w, np.float64).reshape(16) for w in worlds])
+            # Narrowed as C does: the low bits of whatever integer is given.
+            for name, column in (("mesh", meshes), ("material", materials), ("flags", flags), ("side", sides)):
+                a[name] = np.array([int(v) for v in column], np.int64).astype(a.dtype[name])
+            a["flat_shading"] = [int(bool(v)) for v in flats]
         self._versions += 1
         version = self._versions
         info = abi.mcrt_build_info()

@@ -1,0 +1,100 @@
+"""Result arrays in pinned host memory.
+
+The device copies straight into pinned memory; into ordinary memory the
+runtime copies through a buffer of its own, one array at a time, while the
+caller waits, and a large new array's pages fault in on the way. `empty` gives
+numpy arrays on blocks of a pool: a block returns when its last array (or view
+of it) is gone, so a program that drops each frame's image reuses one block.
+The pool holds at most LIMIT bytes, in use or not; beyond that, and for small
+arrays, `empty` is numpy's own.
+
+A block is handed out again as soon as its arrays are gone, so whoever queues a
+copy into one keeps the array until that copy is done.
+"""
+from __future__ import annotations
+
+import ctypes as C
+import operator
+import threading
+import weakref
+from typing import Any, Dict, List
+
+import numpy as np
+
+from ._lib import McrtError, call
+
+SMALL = 1 << 16
+LIMIT = 256 << 20
+
+
+class _Pool:
+    def __init__(self) -> None:
+        self._lock = threading.RLock()  # give() may run inside take(): a collection can free arrays there
+        self._free: Dict[int, List[int]] = {}
+        self._held = 0  # bytes of all blocks, in use or free
+
+    @staticmethod
+    def block_size(nbytes: int) -> int:
+        """The size class of nbytes: quarters of powers of two."""
+        step = 1 << max(12, nbytes.bit_length() - 3)
+        return -(-nbytes // step) * step
+
+    def take(self, size: int) -> int:
+        """Address of a block of `size` bytes, or 0 when the pool's limit leaves no room."""
+        with self._lock:
+            blocks = self._free.get(size)
+            if blocks:
+                return blocks.pop()
+            drop = []
+            for other in sorted(self._free, reverse=True):  # make room from other sizes' free blocks
+                while self._held + size > LIMIT and self._free[other]:
+                    drop.append(self._free[other].pop())
+                    self._held -= other
+            if self._held + size > LIMIT:
+                size = 0
+            else:
+                self._held += size
+        for p in drop:
+            call("mcrt_host_free", C.c_void_p(p))
+        if size == 0:
+            return 0
+        p = C.c_void_p()
+        try:
+            call("mcrt_host_alloc", size, C.byref(p))
+        except McrtError:
+            with self._lock:
+                self._held -= size
+            return 0
+        return int(p.value or 0)
+
+    def give(self, address: int, size: int) -> None:
+        with self._lock:
+            self._free.setdefault(size, []).append(address)
+
+    def empty(self, count: int, dtype: Any) -> np.ndarray:
+        count, dtype = operator.index(count), np.dtype(dtype)
+        nbytes = count * dtype.itemsize
+        if nbytes < SMALL:
+            return np.empty(count, dtype)
+        size = self.block_size(nbytes)
+        address = self.take(size) if size <= LIMIT else 0
+        if not address:
+            return np.empty(count, dtype)
+        block = (C.c_uint8 * size).from_address(address)
+        # At interpreter exit the driver takes the memory back with the process.
+        weakref.finalize(block, self.give, address, size).atexit = False
+        return np.frombuffer(block, dtype, count)
+
+
+_pool = _Pool()
+
+
+def empty(count: int, dtype: Any) -> np.ndarray:
+    """An uninitialised one-dimensional array, in pinned memory where that is worth it."""
+    return _pool.empty(count, dtype)
+
+
+def zeros(count: int, dtype: Any) -> np.ndarray:
+    a = _pool.empty(count, dtype)
+    a.fill(0)
+    return a

@@ -47,7 +47,8 @@ def test_oracle_agrees_on_the_repeated_rays(setup):
             assert abs(h.t - hits["t"][i]) <= 1e-5 * h.t
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 591, 593, 4735, 4737, 9473, 18945, 37889, 75777, 151553])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 591, 593, 1024, 4095, 4096, 4097, 4735, 4737, 9473, 16383, 16384, 16385, 18945, 37889,
+                               75777, 151553])
 def test_answers_do_not_depend_on_the_number_of_rays(setup, n):
     ex, version, _, rays = setup
     base = ex.intersect_closest(version, rays)
