@@ -18,6 +18,7 @@ constexpr uint32_t kFlagToneMap = 2u;    // toneMapped, tracer.ts:103
 constexpr uint32_t kFlagCull = 4u;       // cull, tracer.ts:109
 constexpr uint32_t kFlagDone = 8u;       // the path loop ended; finalize after this bounce's shadows
 constexpr uint32_t kFlagDirect = 16u;    // the sample was written directly (a background)
+constexpr uint32_t kCameraFlags = kFlagToneMap | kFlagCull;  // of a camera ray
 MCRT_HD uint32_t flag_passes(uint32_t f) { return (f >> 8) & 0xffu; }
 MCRT_HD uint32_t flag_bounce(uint32_t f) { return (f >> 16) & 0xffu; }
 MCRT_HD int flag_last_env(uint32_t f) { return static_cast<int>(f >> 24) - 1; }
@@ -74,7 +75,7 @@ struct Counters {
   unsigned int status;
   unsigned int fetch;         // next query a closest-hit traversal warp takes
   unsigned int fetch_shadow;  // the same for the any-hit (shadow) traversal
-  unsigned int pad;
+  unsigned int placed;        // entries of the shading order last made
   unsigned long long tail_closest, tail_any;  // queries of tail launches, counted on the device
 };
 
