@@ -188,7 +188,7 @@ MCRT_D int material_class(const DScene& sc, int m) {
 
 // ------------------------------------------------------------------ extend
 // Closest hit of each queued path's ray (intersectClosest, bvh.ts:202-282),
-// persistent: warps take rays from cnt->fetch until the queue is drained.
+// persistent: warps take rays from a work counter until the queue is drained.
 // With `hist` (shared memory, kShadeClasses counters) each finished query
 // also stores its hit's shading class by queue position (ps.cls) and counts
 // it, the first half of the shading-order sort.
@@ -282,14 +282,20 @@ struct ClassHistogram {
 // B threads per block.
 // 1024 / B blocks per SM: 64 registers, no spills (56 with 20 bytes of spills
 // measured 1-2 % slower on incoherent rays, 72 no faster).
+// n < 0: launched before the host knows how many paths the bounce before
+// continued (Wavefront::run); a queue that k_tail takes is left alone.
 template <int B>
 __global__ void __launch_bounds__(B, 1024 / B) k_extend(DScene sc, PathState ps, const int* __restrict__ queue, int n,
-                                              Counters* cnt, unsigned int* bins, CameraRays camera) {
+                                              Counters* cnt, int bounce, bool sort, CameraRays camera) {
+  if (n < 0) {
+    n = static_cast<int>(cnt->bounce[(bounce & 1) ^ 1].next_count);
+    if (n <= kTailMax) return;
+  }
   __shared__ unsigned int hist[kShadeClasses];
-  ClassHistogram ch{bins, hist};
+  ClassHistogram ch{sort && n >= kSortMin ? ps.bins : nullptr, hist};
   unsigned status = 0;
   ExtendQuery q{sc, ps, queue, 0, {}, ch.begin(), 0, camera};
-  walk<kRefillClosest>(sc, q, n, &cnt->fetch, status);
+  walk<kRefillClosest>(sc, q, n, &cnt->bounce[bounce & 1].fetch, status);
   if (status) atomicOr(&cnt->status, status);
   ch.end();
 }
@@ -300,13 +306,13 @@ __global__ void __launch_bounds__(B, 1024 / B) k_extend(DScene sc, PathState ps,
 // on the 1080p frame than 64.
 template <int B>
 __global__ void __launch_bounds__(B, 1152 / B) k_extend_packet(DScene sc, FrameParams fp, PathState ps, int n,
-                                                     Counters* cnt, unsigned int* bins, CameraRays camera) {
+                                                     Counters* cnt, int bounce, bool sort, CameraRays camera) {
   __shared__ int2 stack[(B / 32) * kStackMax];
   __shared__ unsigned int hist[kShadeClasses];
-  ClassHistogram ch{bins, hist};
+  ClassHistogram ch{sort ? ps.bins : nullptr, hist};
   unsigned status = 0;
   CameraQuery q{ExtendQuery{sc, ps, nullptr, 0, {}, ch.begin(), 0, camera}, fp, {}, 0};
-  traverse_packet(sc, q, n, &cnt->fetch, stack + (threadIdx.x >> 5) * kStackMax, status);
+  traverse_packet(sc, q, n, &cnt->bounce[bounce & 1].fetch, stack + (threadIdx.x >> 5) * kStackMax, status);
   if (status) atomicOr(&cnt->status, status);
   ch.end();
 }
@@ -897,16 +903,36 @@ MCRT_D void shade_path(const DScene& sc, const FrameParams& fp, const PathState&
 // 8, 10.6 at 10 and 11.4 at 12.
 constexpr int kShadeBlocksPerSM = 8;
 constexpr long long kShadeGridFactor = 16;  // batched shading grid, in resident grids
+// Most blocks of the plain path's shading, in resident grids. Its first bounce
+// is launched for all paths and shades the hits, so a block per 128 paths can
+// leave most of them empty (0.1 ms for 190 k); with fewer blocks, each taking
+// several tiles, warps stay in the shading code from tile to tile. The mid
+// scene's 1080p frame, 262 k tiles a chunk of which 30-40 % hold hits: shading
+// 5.70 ms with a block per tile, 5.27 with at most 64 resident grids, 5.71 with
+// 16, 5.91 with 4. (Resolving takes 1.66 ms with a block per tile, 1.25 with 2 to
+// 16 resident grids.)
+constexpr int kShadeGrids = 64;
 
 __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSM) k_shade(DScene sc, FrameParams fp, PathState ps,
                                                   const int* __restrict__ qin, int n, int* __restrict__ qout,
-                                                  Counters* cnt, bool camera) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int pid = qin[q];  // with the count, not behind it
-  if (camera && q >= static_cast<int>(cnt->placed)) return;
-  const StageQueues qs{qout, &cnt->next_count, ps.shadow_queue, &cnt->shadow_count};
-  shade_path(sc, fp, ps, pid, qs, camera);
+                                                  Counters* cnt, int bounce, bool camera) {
+  BounceCounters& bc = cnt->bounce[bounce & 1];
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    // The next bounce's counters and class bins: nothing uses them any more
+    // once shading begins, nor yet.
+    if (threadIdx.x == 0) cnt->bounce[(bounce & 1) ^ 1] = BounceCounters{};
+    ps.bins[threadIdx.x] = 0;
+  }
+  const StageQueues qs{qout, &bc.next_count, ps.shadow_queue, &bc.shadow_count};
+  const int stride = gridDim.x * blockDim.x;
+#pragma unroll 1
+  for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+    const int q = base + threadIdx.x;
+    const int pid = q < n ? qin[q] : 0;  // with the count, not behind it
+    if (camera) n = min(n, static_cast<int>(bc.placed));
+    if (q < n) shade_path(sc, fp, ps, pid, qs, camera);
+    __syncwarp();
+  }
 }
 
 // ------------------------------------------------------------------ shadow
@@ -1057,13 +1083,17 @@ struct QueuedShadows : ShadowQuery {
 
 // 1024 / B blocks per SM: 64 registers; the see-through lookups between the
 // walk's loops spill 44 bytes (72 registers: no spills, no faster; 56: 1-2 %
-// slower).
+// slower). n < 0: as many as shading cast.
 template <int B>
-__global__ void __launch_bounds__(B, 1024 / B) k_shadow(DScene sc, PathState ps, int n, int capacity, Counters* cnt) {
+__global__ void __launch_bounds__(B, 1024 / B) k_shadow(DScene sc, PathState ps, int n, int capacity, Counters* cnt,
+                                              int bounce) {
+  BounceCounters& bc = cnt->bounce[bounce & 1];
+  if (n < 0) n = static_cast<int>(bc.shadow_count);
+  if (n == 0) return;
   unsigned status = 0;
   float seen[kShadowSeen + 10];
   QueuedShadows q{{sc, ps, capacity, &status, seen}, n - 1};
-  walk<kRefillShadow>(sc, q, n, &cnt->fetch_shadow, status);
+  walk<kRefillShadow>(sc, q, n, &bc.fetch_shadow, status);
   if (status) atomicOr(&cnt->status, status);
 }
 
@@ -1099,9 +1129,14 @@ MCRT_D void resolve_path(const DScene& sc, const FrameParams& fp, const PathStat
 }
 
 __global__ void __launch_bounds__(kBlock) k_resolve(DScene sc, FrameParams fp, PathState ps,
-                                                    const int* __restrict__ queue, int n, int capacity) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) resolve_path(sc, fp, ps, queue[q], capacity);
+                                                    const int* __restrict__ queue, int n, int capacity,
+                                                    const unsigned int* placed) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
+    const int pid = queue[q];  // with the count, not behind it
+    if (placed) n = min(n, static_cast<int>(*placed));
+    if (q < n) resolve_path(sc, fp, ps, pid, capacity);
+  }
 }
 
 // -------------------------------------------------------------------- tail
@@ -1268,8 +1303,9 @@ __global__ void __launch_bounds__(kTailBlock) k_tail(const __grid_constant__ DSc
                                                      const __grid_constant__ FrameParams fp,
                                                      const __grid_constant__ PathState ps,
                                                      const int* __restrict__ queue, int n, int capacity, int slots,
-                                                     Counters* cnt) {
-  finish_paths(sc, ps, [&](int) -> const FrameParams& { return fp; }, queue, n, capacity, slots, &cnt->fetch,
+                                                     Counters* cnt, int bounce) {
+  finish_paths(sc, ps, [&](int) -> const FrameParams& { return fp; }, queue, n, capacity, slots,
+               &cnt->bounce[bounce & 1].fetch,
                &cnt->tail_closest, &cnt->tail_any, &cnt->status);
 }
 
@@ -1449,19 +1485,19 @@ __global__ void __launch_bounds__(kFewBlock) k_count_few(DScene sc, const float4
 // ------------------------------------------------------------------- host
 PathBuffers::~PathBuffers() {
   release();
-  if (fork_) cudaEventDestroy(fork_);
-  if (join_) cudaEventDestroy(join_);
-  if (side_) cudaStreamDestroy(side_);
+  if (side_.shaded) cudaEventDestroy(side_.shaded);
+  if (side_.resolved) cudaEventDestroy(side_.resolved);
+  if (side_.shadows) cudaStreamDestroy(side_.shadows);
+  if (side_.counts) cudaStreamDestroy(side_.counts);
 }
 
-cudaError_t PathBuffers::side_stream(cudaStream_t* side, cudaEvent_t* fork, cudaEvent_t* join) {
+cudaError_t PathBuffers::side_streams(Side* side) {
   cudaError_t e = cudaSuccess;
-  if (!side_) e = cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking);
-  if (e == cudaSuccess && !fork_) e = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming);
-  if (e == cudaSuccess && !join_) e = cudaEventCreateWithFlags(&join_, cudaEventDisableTiming);
+  for (cudaStream_t* s : {&side_.shadows, &side_.counts})
+    if (e == cudaSuccess && !*s) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+  for (cudaEvent_t* v : {&side_.shaded, &side_.resolved})
+    if (e == cudaSuccess && !*v) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
   *side = side_;
-  *fork = fork_;
-  *join = join_;
   return e;
 }
 
@@ -1614,8 +1650,8 @@ int walk_blocks(K kernel, long long n, int block = kBlock) {
 // shared-memory short stack, is kept for the callers that name pairs by it:
 // the walk's stack is in local memory, so pairs of one block size share their
 // kernels.
-using ExtendFn = void (*)(DScene, PathState, const int*, int, Counters*, unsigned int*, CameraRays);
-using ShadowFn = void (*)(DScene, PathState, int, int, Counters*);
+using ExtendFn = void (*)(DScene, PathState, const int*, int, Counters*, int, bool, CameraRays);
+using ShadowFn = void (*)(DScene, PathState, int, int, Counters*, int);
 
 struct PlainVariant {
   int block, stack;
@@ -1690,20 +1726,25 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
   // the main one: neither touches what the other reads or writes, and each
   // fills the other's tail of idle SMs. Shading k + 1 waits for the side
   // stream (it rewrites the shadow queue, the slots and the path queue that
-  // resolve reads). Timed renders keep one stream, so every kernel's events
-  // bracket it alone.
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
+  // resolve reads). Both are queued right behind shading k, by counts that only
+  // the device knows yet; the host reads the counts on a third stream while
+  // they run, and queues what depends on them (sort, shading, or the end) well
+  // before they finish. With a wait for the counts before either was queued,
+  // and four small clears a bounce, the GPU idled 20-25 us a bounce: a 320 x
+  // 240 still of 16 passes 1.07 -> 1.00 ms, a 633 x 471 draft of 7 1.51 -> 1.47,
+  // a 720p frame of 4 over 500 k triangles 6.10 -> 5.80.
+  // Timed renders keep one stream, so every kernel's events bracket it alone.
+  PathBuffers::Side side;
   bool overlap = !timed;
   if (overlap && e == cudaSuccess) {
-    e = buffers.side_stream(&side, &fork, &join);
+    e = buffers.side_streams(&side);
     overlap = e == cudaSuccess;
   }
   bool tails = false;      // a tail launch counted rays on the device
   bool side_busy = false;  // side work queued since the main stream last joined it
   auto join_side = [&]() {
     if (side_busy) {
-      cudaStreamWaitEvent(stream, join, 0);
+      cudaStreamWaitEvent(stream, side.resolved, 0);
       side_busy = false;
     }
   };
@@ -1713,20 +1754,45 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
     FrameParams f = fp;
     f.pass0 = fp.pass0 + first;
     f.npass = np;
-    tm.start();
-    const bool sorted_start = sort_shading && n >= kSortMin;
+    // The camera rays walk warp-coherent where a warp's 32 rays (passes of
+    // 32 / npass pixels of a row) span at most 1/360 of the image height:
+    // measured on the mid scene at 64 passes, the coherent walk was 1-3 %
+    // faster per frame from 640x360 to 2560x1440 and a third slower per
+    // launch at 320x180. (Their shadow rays lose with it at every size: lanes
+    // blocked early idle until the warp's last ray ends, where the per-lane
+    // walk refills them.)
     const int warp_pixels = 32 / std::max(1, std::min(f.npass, 32));
     const bool coherent = packet_first && n > kTailMax && warp_pixels * 360 <= f.height;
-    if (!coherent) k_raygen<<<blocks_for(n, kBlock), kBlock, 0, stream>>>(f, ps, n, !sorted_start);
-    tm.stop(st.ms_raygen, st.n_raygen);
-    st.launches++;
+    const CameraRays camera = sort_shading && n >= kSortMin ? camera_rays(scene, f) : CameraRays{};
+    cudaMemsetAsync(cnt->bounce, 0, sizeof(cnt->bounce), stream);
+    if (camera.on) cudaMemsetAsync(ps.bins, 0, 2 * kShadeClasses * sizeof(unsigned int), stream);
+    if (!coherent) {
+      tm.start();
+      k_raygen<<<blocks_for(n, kBlock), kBlock, 0, stream>>>(f, ps, n, !camera.on);
+      tm.stop(st.ms_raygen, st.n_raygen);
+      st.launches++;
+    }
     st.samples += n;
     int cur = 0;
-    int iterations = 0;
-    while (n > 0) {
+    int bounce = 1;
+    // Bounce `b`'s closest hits; count < 0: as many as the bounce before continued.
+    auto extend = [&](int b, const int* queue, int count, int most) {
+      const bool lead = b == 1;
+      tm.start();
+      if (lead && coherent) {
+        k_extend_packet<kBlock><<<persistent_blocks(k_extend_packet<kBlock>, most), kBlock, 0, stream>>>(
+            scene, f, ps, most, cnt, b, camera.on, camera);
+      } else {
+        tv.extend<<<walk_blocks(tv.extend, most, tv.block), tv.block, 0, stream>>>(
+            scene, ps, queue, count, cnt, b, sort_shading, lead ? camera : CameraRays{});
+      }
+      tm.stop(st.ms_extend, st.n_extend);
+    };
+    if (n > kTailMax) extend(bounce, ps.queue[cur], n, n);
+    for (; n > 0; bounce++) {
       // Paths end by bounce count, pass-through count or Russian roulette; a
       // loop this long means corrupt state, reported rather than spun on.
-      if (++iterations > kMaxIterations) {
+      if (bounce > kMaxIterations) {
         e = cudaErrorLaunchTimeout;
         break;
       }
@@ -1734,90 +1800,79 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
         // Few paths left (or few from the start): one launch takes them to
         // their ends, with the side stream's work on them done first.
         join_side();
-        cudaMemsetAsync(&cnt->fetch, 0, sizeof(unsigned int), stream);
         tm.start();
         const int limit = resident_limit(reinterpret_cast<const void*>(k_tail), kTailBlock);
         const int blocks = std::min(limit, blocks_for(n, kTailBlock / 32));
-        k_tail<<<blocks, kTailBlock, 0, stream>>>(scene, f, ps, ps.queue[cur], n, cap, buffers.slots(), cnt);
+        k_tail<<<blocks, kTailBlock, 0, stream>>>(scene, f, ps, ps.queue[cur], n, cap, buffers.slots(), cnt, bounce);
         tm.stop(st.ms_extend, st.n_extend);
         st.launches++;
         tails = true;
         break;
       }
-      // The camera rays walk warp-coherent where a warp's 32 rays (passes of
-      // 32 / npass pixels of a row) span at most 1/360 of the image height:
-      // measured on the mid scene at 64 passes, the coherent walk was 1-3 %
-      // faster per frame from 640x360 to 2560x1440 and a third slower per
-      // launch at 320x180. (Their shadow rays lose with it at every size: lanes
-      // blocked early idle until the warp's last ray ends, where the per-lane
-      // walk refills them.)
-      // A queue long enough to shade in hit-class order has its classes
-      // counted by the closest-hit kernel itself (ExtendQuery with a
-      // histogram); the scatter then puts the queue in that order.
-      const bool sort = sort_shading && n >= kSortMin;
-      unsigned int* class_bins = sort ? ps.bins : nullptr;
-      const CameraRays camera = iterations == 1 && sort ? camera_rays(scene, f) : CameraRays{};
-      if (sort) cudaMemsetAsync(ps.bins, 0, 2 * kShadeClasses * sizeof(unsigned int), stream);
-      cudaMemsetAsync(&cnt->fetch, 0, sizeof(unsigned int), stream);
-      tm.start();
-      if (coherent && iterations == 1) {
-        k_extend_packet<kBlock><<<persistent_blocks(k_extend_packet<kBlock>, n), kBlock, 0, stream>>>(
-            scene, f, ps, n, cnt, class_bins, camera);
-      } else {
-        tv.extend<<<walk_blocks(tv.extend, n, tv.block), tv.block, 0, stream>>>(scene, ps, ps.queue[cur], n,
-                                                                                      cnt, class_bins, camera);
-      }
-      tm.stop(st.ms_extend, st.n_extend);
+      // The closest hits of this bounce are under way. A queue long enough to
+      // shade in hit-class order has its classes counted by them (ExtendQuery
+      // with a histogram); the scatter then puts the queue in that order.
+      BounceCounters* bc = &cnt->bounce[bounce & 1];
+      const bool lead = bounce == 1 && camera.on;
       st.closest_rays += n;
+      st.launches++;
       const int* shade_queue = ps.queue[cur];
-      if (sort) {
+      if (sort_shading && n >= kSortMin) {
         // The camera rays' order goes where their queue would be: resolving
         // reads it too, beside the next bounce's sort.
-        shade_queue = camera.on ? ps.queue[cur] : ps.binned;
-        k_class_scatter<<<blocks_for(n, 256), 256, 0, stream>>>(ps, camera.on ? nullptr : ps.queue[cur], n, ps.bins,
-                                                                const_cast<int*>(shade_queue), camera.ends ? 1 : 0,
-                                                                &cnt->placed);
-        st.launches += 1;
+        shade_queue = lead ? ps.queue[cur] : ps.binned;
+        k_class_scatter<<<blocks_for(n, 256), 256, 0, stream>>>(ps, lead ? nullptr : ps.queue[cur], n, ps.bins,
+                                                                const_cast<int*>(shade_queue),
+                                                                lead && camera.ends ? 1 : 0, &bc->placed);
+        st.launches++;
       }
       join_side();
-      cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned int), stream);
+      const int shade_blocks = std::min(
+          blocks_for(n, kBlock), kShadeGrids * resident_limit(reinterpret_cast<const void*>(k_shade), kBlock));
+      const int resolve_blocks =
+          std::min(blocks_for(n, kBlock), 2 * resident_limit(reinterpret_cast<const void*>(k_resolve), kBlock));
       tm.start();
-      k_shade<<<blocks_for(n, kBlock), kBlock, 0, stream>>>(scene, f, ps, shade_queue, n, ps.queue[cur ^ 1], cnt,
-                                                            camera.on);
+      k_shade<<<shade_blocks, kBlock, 0, stream>>>(scene, f, ps, shade_queue, n, ps.queue[cur ^ 1], cnt,
+                                                            bounce, lead);
       tm.stop(st.ms_shade, st.n_shade);
-      cudaMemcpyAsync(host, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream);
-      e = cudaStreamSynchronize(stream);
-      if (e != cudaSuccess) break;
-      const int n_next = static_cast<int>(host->next_count);
-      const int n_shadow = static_cast<int>(host->shadow_count);
-      st.status |= host->status;
-      if (camera.on) n = static_cast<int>(host->placed);
-      cudaStream_t sh = stream;
-      if (overlap) {
-        cudaEventRecord(fork, stream);
-        cudaStreamWaitEvent(side, fork, 0);
-        sh = side;
-      }
-      if (n_shadow > 0) {
-        cudaMemsetAsync(&cnt->fetch_shadow, 0, sizeof(unsigned int), sh);
+      st.launches++;
+      // Bounce k's shadow rays and resolve, k + 1's closest hits, and the counts.
+      auto shadow = [&](int count, int most, cudaStream_t s) {
         tm.start();
-        tv.shadow<<<walk_blocks(tv.shadow, n_shadow, tv.block), tv.block, 0, sh>>>(scene, ps, n_shadow, cap,
-                                                                                         cnt);
+        tv.shadow<<<walk_blocks(tv.shadow, most, tv.block), tv.block, 0, s>>>(scene, ps, count, cap, cnt, bounce);
         tm.stop(st.ms_shadow, st.n_shadow);
-        st.any_rays += n_shadow;
         st.launches++;
-      }
-      if (n > 0) {
+      };
+      auto resolve = [&](cudaStream_t s) {
         tm.start();
-        k_resolve<<<blocks_for(n, kBlock), kBlock, 0, sh>>>(scene, f, ps, ps.queue[cur], n, cap);
+        k_resolve<<<resolve_blocks, kBlock, 0, s>>>(scene, f, ps, ps.queue[cur], n, cap,
+                                                           lead ? &bc->placed : nullptr);
         tm.stop(st.ms_resolve, st.n_resolve);
         st.launches++;
-      }
+      };
+      const cudaStream_t copier = overlap ? side.counts : stream;
       if (overlap) {
-        cudaEventRecord(join, side);
+        cudaEventRecord(side.shaded, stream);
+        extend(bounce + 1, ps.queue[cur ^ 1], -1, n);
+        cudaStreamWaitEvent(side.shadows, side.shaded, 0);
+        shadow(-1, n, side.shadows);
+        resolve(side.shadows);
+        cudaEventRecord(side.resolved, side.shadows);
         side_busy = true;
+        cudaStreamWaitEvent(side.counts, side.shaded, 0);
       }
-      st.launches += 2;
+      cudaMemcpyAsync(host, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, copier);
+      e = cudaStreamSynchronize(copier);
+      if (e != cudaSuccess) break;
+      const int n_next = static_cast<int>(host->bounce[bounce & 1].next_count);
+      const int n_shadow = static_cast<int>(host->bounce[bounce & 1].shadow_count);
+      st.status |= host->status;
+      st.any_rays += n_shadow;
+      if (!overlap) {
+        if (n_shadow > 0) shadow(n_shadow, n_shadow, stream);
+        resolve(stream);
+        if (n_next > kTailMax) extend(bounce + 1, ps.queue[cur ^ 1], n_next, n_next);
+      }
       n = n_next;
       cur ^= 1;
     }
@@ -1831,7 +1886,8 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
   }
   join_side();
   if (e != cudaSuccess) {  // nothing of a failed render stays in flight
-    if (side) cudaStreamSynchronize(side);
+    if (side.shadows) cudaStreamSynchronize(side.shadows);
+    if (side.counts) cudaStreamSynchronize(side.counts);
     cudaStreamSynchronize(stream);
     return e;
   }
@@ -1859,11 +1915,11 @@ cudaError_t primary_hits(const DScene& scene, FrameParams fp, PathBuffers& buffe
   fp.capacity = buffers.capacity();
   fp.slot_count = buffers.slots();
   k_raygen<<<blocks_for(n, kBlock), kBlock, 0, stream>>>(fp, ps, n, true);
-  cudaMemsetAsync(&buffers.counters()->fetch, 0, sizeof(unsigned int), stream);
+  Counters* cnt = buffers.counters();
+  cudaMemsetAsync(cnt->bounce, 0, sizeof(cnt->bounce), stream);
   const PlainVariant& tv = plain_variant(0);
   tv.extend<<<walk_blocks(tv.extend, n, tv.block), tv.block, 0, stream>>>(scene, ps, ps.queue[0], n,
-                                                                                  buffers.counters(), nullptr,
-                                                                                  CameraRays{});
+                                                                                  cnt, 0, false, CameraRays{});
   return cudaGetLastError();
 }
 

@@ -69,13 +69,20 @@ struct PathState {
   int* seg;              // batched renders: the segment each path belongs to
 };
 
-struct Counters {
-  unsigned int next_count;
-  unsigned int shadow_count;
-  unsigned int status;
+// One bounce's counters. Bounce i of a chunk uses pair member i & 1: its walk
+// reads how many paths bounce i - 1 continued from the other one.
+struct BounceCounters {
+  unsigned int next_count;    // paths that go on to the next bounce
+  unsigned int shadow_count;  // shadow rays cast
+  unsigned int placed;        // entries of the shading order
   unsigned int fetch;         // next query a closest-hit traversal warp takes
   unsigned int fetch_shadow;  // the same for the any-hit (shadow) traversal
-  unsigned int placed;        // entries of the shading order last made
+};
+
+struct Counters {
+  BounceCounters bounce[2];
+  unsigned int status;
+  unsigned int pad;
   unsigned long long tail_closest, tail_any;  // queries of tail launches, counted on the device
 };
 
@@ -102,14 +109,18 @@ class PathBuffers {
   size_t bytes() const { return bytes_; }
   Counters* counters() const { return counters_; }
   Counters* host_counters() const { return host_counters_; }
-  // A second stream and two events (made on first use, kept until destruction)
-  // for running a bounce's shadow rays beside the next bounce's closest hits.
-  cudaError_t side_stream(cudaStream_t* side, cudaEvent_t* fork, cudaEvent_t* join);
+  // Two more streams and their events (made on first use, kept until
+  // destruction): one for running a bounce's shadow rays beside the next
+  // bounce's closest hits, one for reading back its counters meanwhile.
+  struct Side {
+    cudaStream_t shadows = nullptr, counts = nullptr;
+    cudaEvent_t shaded = nullptr, resolved = nullptr;
+  };
+  cudaError_t side_streams(Side* side);
 
  private:
   void release();
-  cudaStream_t side_ = nullptr;
-  cudaEvent_t fork_ = nullptr, join_ = nullptr;
+  Side side_;
   PathState st_{};
   Counters* counters_ = nullptr;
   Counters* host_counters_ = nullptr;
