@@ -60,7 +60,7 @@ MCRT_D unsigned int queue_append(unsigned int* counter) {
 // once REFILL lanes are idle.
 template <int REFILL, class Q>
 MCRT_D void walk(const DScene& sc, Q& q, int n, unsigned* counter, unsigned& status) {
-  int below[kStackMax + 2];
+  int below[kStackMax + 3];
   TravStack st;
   st.init(below);
   traverse_persistent<REFILL>(sc, q, n, query_lanes(n), counter, st, status);
@@ -1222,7 +1222,7 @@ MCRT_D void finish_paths(const DScene& sc, const PathState& ps, P params, const 
   // Groups of a warp that take paths: all four, or fewer while there are warps to spare.
   const int warps = static_cast<int>(gridDim.x) * (kTailBlock / 32);
   const int groups = n <= warps ? 1 : (n <= 2 * warps ? 2 : 4);
-  int below[kStackMax + 2];
+  int below[kStackMax + 3];
   float seen[kShadowSeen + 10];
   TravStack st;
   st.init(below);
@@ -1423,7 +1423,7 @@ template <class Q>
 MCRT_D void trace_few(const DScene& sc, Q& q, int n, unsigned* status_out) {
   const int lanes = query_lanes(n), lane = threadIdx.x & 31;
   const int i = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane;
-  int below[kStackMax + 2];
+  int below[kStackMax + 3];
   TravStack st;
   st.init(below);
   unsigned status = 0;
