@@ -371,6 +371,14 @@ __global__ void __launch_bounds__(kBuildBlock) k_root(BuildState st) {
   if (threadIdx.x == 0) st.ctl->inner_depth = -1;
 }
 
+// A bin: its box as ordered integers, and its count. Seven words apart, the
+// rows of 32 bins lie in different banks word by word (six apart, in pairs).
+using BinRow = int[7];
+
+__device__ __forceinline__ int empty_bin_word(int word) {
+  return word == 6 ? 0 : ordered(word < 3 ? INFINITY : -INFINITY);
+}
+
 // Unions of a node's bins from the left (0) and from the right (1), per axis:
 // [side][axis][k] covers bins [0, k] or [k, bins). Box bounds and counts, the
 // boxes as ordered integers.
@@ -415,7 +423,7 @@ __device__ __forceinline__ Choice first_minimum(double cost, int axis, int split
 // is the one-thread sweep's, and the first minimum wins, as there. Scans by
 // shuffles of all seven values took three times the instructions.
 template <int MB>
-__device__ Choice best_split(const int (*cnt)[MB], const int (*bbox)[MB][6], Sweeps<MB>& w, const bool* live, int bins) {
+__device__ Choice best_split(const BinRow (*row)[MB], Sweeps<MB>& w, const bool* live, int bins) {
   const int lane = threadIdx.x & 31;
   if (lane < 24) {
     const int side = lane >= 12 ? 1 : 0, a = (lane - 12 * side) >> 2, q = lane & 3;
@@ -425,8 +433,8 @@ __device__ Choice best_split(const int (*cnt)[MB], const int (*bbox)[MB][6], Swe
       int lo = ordered(INFINITY), hi = ordered(-INFINITY);
 #pragma unroll 4
       for (int i = 0; i < bins; i++, k += step) {
-        lo = min(lo, bbox[a][k][q]);
-        hi = max(hi, bbox[a][k][3 + q]);
+        lo = min(lo, row[a][k][q]);
+        hi = max(hi, row[a][k][3 + q]);
         w.box[side][a][k][q] = lo;
         w.box[side][a][k][3 + q] = hi;
       }
@@ -434,7 +442,7 @@ __device__ Choice best_split(const int (*cnt)[MB], const int (*bbox)[MB][6], Swe
       int c = 0;
 #pragma unroll 4
       for (int i = 0; i < bins; i++, k += step) {
-        c += cnt[a][k];
+        c += row[a][k][6];
         w.cnt[side][a][k] = c;
       }
     }
@@ -482,23 +490,46 @@ __device__ __forceinline__ void binning(const float* cmin, const float* cmax, in
   }
 }
 
-__device__ __forceinline__ void bin_prim(int* cnt, int* bb, const int* v) {
-  atomicAdd(cnt, 1);
-  atomicMin(bb, v[0]); atomicMin(bb + 1, v[1]); atomicMin(bb + 2, v[2]);
-  atomicMax(bb + 3, v[3]); atomicMax(bb + 4, v[4]); atomicMax(bb + 5, v[5]);
+__device__ __forceinline__ void bin_prim(int* row, const int* v) {
+  atomicAdd(row + 6, 1);
+  atomicMin(row, v[0]); atomicMin(row + 1, v[1]); atomicMin(row + 2, v[2]);
+  atomicMax(row + 3, v[3]); atomicMax(row + 4, v[4]); atomicMax(row + 5, v[5]);
 }
 
-// One segment of a level (see above). What bounds it: shared-memory atomics,
-// seven per triangle and axis, and the latency of a node's steps. A warp whose
+// The same where a bin takes many triangles: a bound is read first, without
+// conflicts, and added to only if it grows. A bound read too early is smaller
+// than it is by now, which costs an addition and changes nothing. (Not for a
+// subtree's bins, of eight triangles at most on average: 16.4 M triangles
+// rebuilt and traced 34.0 ms without, 34.6 with.)
+__device__ __forceinline__ void bin_prim_checked(int* row, const int* v) {
+  atomicAdd(row + 6, 1);
+  const volatile int* now = row;
+  int r[6];
+  for (int q = 0; q < 6; q++) r[q] = now[q];
+  for (int q = 0; q < 3; q++) {
+    if (v[q] < r[q]) atomicMin(row + q, v[q]);
+    if (v[3 + q] > r[3 + q]) atomicMax(row + 3 + q, v[3 + q]);
+  }
+}
+
+// One segment of a level (see above). What bounds it: the latency of a node's
+// steps at the lower levels, of loads and shared memory at the upper ones (0.21
+// ms a level for 16.4 M triangles; reading them takes 0.09). A warp whose
 // triangles all fall into one bin of an axis (neighbours in the model, at the
-// upper levels) reduces them first and adds once; the next triangle is loaded
-// while one is binned. Four blocks per SM (64 registers): 16.4 M triangles
-// rebuilt and traced 40.1 ms, three blocks 40.7, two 41.3.
-__global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st) {
-  using Scan = cub::BlockScan<int, kBuildBlock>;
+// upper levels) reduces them first and adds once; elsewhere a triangle adds to
+// the bounds that it grows, few of a segment's (bin_prim_checked); the next
+// triangle is loaded while one is binned. Adding to all six bounds of each bin,
+// in rows of six words, was bound by the additions' conflicts: all levels
+// together 7.4 -> 4.95 ms. 64 registers: 16.4 M triangles rebuilt and traced
+// 40.1 ms, with 85 registers 40.7, with 128 41.3.
+// B: 64 or 128 threads once a level has segments for every SM many times over
+// (run_build): most of a small node's time is one warp's, the split's, and more
+// and smaller blocks keep more nodes under way.
+template <int B>
+__global__ void __launch_bounds__(B, 1024 / B) k_bin(int level, BuildState st) {
+  using Scan = cub::BlockScan<int, B>;
   __shared__ typename Scan::TempStorage scan_tmp;
-  __shared__ int cnt[3][kMaxBins];
-  __shared__ int bbox[3][kMaxBins][6];
+  __shared__ BinRow row[3][kMaxBins];
   __shared__ Sweeps<kMaxBins> sweeps;
   __shared__ int s_flag, s_child[2], s_seg0[2], s_acc[2], s_mode, s_axis, s_bin, s_nleft;
   const unsigned full = 0xffffffffu;
@@ -510,10 +541,7 @@ __global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st
     const int j = st.segs[level & 1][s];
     Node& nd = st.nodes[level & 1][j];
     const int nfirst = nd.first, ncount = nd.count, nseg = nd.nseg, seg = s - nd.seg0, depth = nd.depth;
-    for (int i = tid; i < 3 * kMaxBins; i += kBuildBlock) {
-      (&cnt[0][0])[i] = 0;
-      for (int q = 0; q < 6; q++) (&bbox[0][0][0])[6 * i + q] = ordered(q < 3 ? INFINITY : -INFINITY);
-    }
+    for (int i = tid; i < 3 * kMaxBins * 7; i += B) (&row[0][0][0])[i] = empty_bin_word(i % 7);
     double lo[3], scale[3];
     bool live[3];
     {
@@ -535,8 +563,8 @@ __global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st
       nb = p.b[got];
       nc = p.c[got].x;
     }
-    for (int base = first; base < end; base += kBuildBlock) {
-      const int k = base + tid, ahead = k + kBuildBlock;
+    for (int base = first; base < end; base += B) {
+      const int k = base + tid, ahead = k + B;
       const bool valid = k < end;
       const float4 a4 = valid ? na : make_float4(INFINITY, INFINITY, INFINITY, -INFINITY);
       const float4 b4 = valid ? nb : make_float4(-INFINITY, -INFINITY, 0.0f, 0.0f);
@@ -563,11 +591,11 @@ __global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st
             reduced = true;
           }
           if (lane == 0) {
-            bin_prim(&cnt[a][b0], bbox[a][b0], w);
-            if (here > 1) atomicAdd(&cnt[a][b0], here - 1);
+            bin_prim(row[a][b0], w);
+            if (here > 1) atomicAdd(&row[a][b0][6], here - 1);
           }
         } else if (valid) {
-          bin_prim(&cnt[a][b], bbox[a][b], v);
+          bin_prim_checked(row[a][b], v);
         }
       }
     }
@@ -575,22 +603,21 @@ __global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st
     if (nseg > 1) {
       // This segment's cumulative counts, and its bins folded into the node's.
       Acc& acc = st.acc[level & 1][nd.acc];
-      if (tid < 96) {
-        const int a = tid >> 5;
-        int c = cnt[a][lane];
+      for (int a = tid >> 5; a < 3; a += B / 32) {
+        int c = row[a][lane][6];
         for (int off = 1; off < 32; off <<= 1) {
           const int o = __shfl_up_sync(full, c, off);
           if (lane >= off) c += o;
         }
         st.seg_cum[(static_cast<size_t>(s) * 3 + a) * kMaxBins + lane] = c;
       }
-      for (int i = tid; i < 3 * bins; i += kBuildBlock) {
+      for (int i = tid; i < 3 * bins; i += B) {
         const int a = i / bins, b = i - a * bins;
-        if (!live[a] || cnt[a][b] == 0) continue;
-        atomicAdd(&acc.cnt[a][b], cnt[a][b]);
+        if (!live[a] || row[a][b][6] == 0) continue;
+        atomicAdd(&acc.cnt[a][b], row[a][b][6]);
         for (int q = 0; q < 3; q++) {
-          atomicMin(&acc.bb[a][b][q], bbox[a][b][q]);
-          atomicMax(&acc.bb[a][b][3 + q], bbox[a][b][3 + q]);
+          atomicMin(&acc.bb[a][b][q], row[a][b][q]);
+          atomicMax(&acc.bb[a][b][3 + q], row[a][b][3 + q]);
         }
       }
       __threadfence();
@@ -599,14 +626,14 @@ __global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st
       __syncthreads();
       if (!s_flag) continue;
       __threadfence();
-      for (int i = tid; i < 3 * kMaxBins; i += kBuildBlock) {
-        (&cnt[0][0])[i] = __ldcg(&acc.cnt[0][0] + i);
-        for (int q = 0; q < 6; q++) (&bbox[0][0][0])[6 * i + q] = __ldcg(&acc.bb[0][0][0] + 6 * i + q);
+      for (int i = tid; i < 3 * kMaxBins; i += B) {
+        (&row[0][0])[i][6] = __ldcg(&acc.cnt[0][0] + i);
+        for (int q = 0; q < 6; q++) (&row[0][0])[i][q] = __ldcg(&acc.bb[0][0][0] + 6 * i + q);
       }
       __syncthreads();
     }
     if (tid < 32) {
-      const Choice c = best_split<kMaxBins>(cnt, bbox, sweeps, live, bins);
+      const Choice c = best_split<kMaxBins>(row, sweeps, live, bins);
       if (lane == 0) {
         float box[6];
         for (int i = 0; i < 6; i++) box[i] = unordered(nd.box[i]);
@@ -654,7 +681,7 @@ __global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st
     // Triangles going left before each of the node's segments.
     const int seg0 = s - seg;
     int running = 0;
-    for (int base = 0; base < nseg; base += kBuildBlock) {
+    for (int base = 0; base < nseg; base += B) {
       const int i = base + tid;
       int left = 0;
       if (i < nseg && nseg > 1) {
@@ -671,10 +698,12 @@ __global__ void __launch_bounds__(kBuildBlock, 4) k_bin(int level, BuildState st
 }
 
 // The stable partition of one segment (bvh.ts:145-171): each warp takes an
-// eighth of it, counts its lefts, and moves its triangles to the places its
+// equal share of it (at most 32 rounds: kSegMax / B), counts its lefts, and moves its triangles to the places its
 // predecessors leave. What bounds it: DRAM (40 bytes read and written).
-__global__ void __launch_bounds__(kBuildBlock) k_part(int level, BuildState st) {
-  constexpr int kWarps = kBuildBlock / 32;
+template <int B>
+__global__ void __launch_bounds__(B) k_part(int level, BuildState st) {
+  static_assert(kSegMax / B <= 32, "a warp's rounds are its lanes");
+  constexpr int kWarps = B / 32;
   __shared__ int s_lefts[kWarps];
   __shared__ int s_box[2][12];
   const unsigned full = 0xffffffffu;
@@ -689,7 +718,7 @@ __global__ void __launch_bounds__(kBuildBlock) k_part(int level, BuildState st) 
     const int child[2] = {nd.child[0], nd.child[1]};
     const int first = nfirst + seg * st.seg, end = min(nfirst + nd.count, first + st.seg);
     if (tid < 24) (&s_box[0][0])[tid] = ordered(is_max(tid % 12) ? -INFINITY : INFINITY);
-    const int rounds = (end - first + kBuildBlock - 1) / kBuildBlock;  // an equal share for every warp
+    const int rounds = (end - first + B - 1) / B;  // an equal share for every warp
     const int from = first + warp * 32 * rounds;
     unsigned mine = 0;  // lane r: the warp's round r, lanes going left
     for (int r = 0; r < rounds; r++) {
@@ -781,8 +810,7 @@ struct SubWarp {
   float4 a[kSub];         // the triangles: box min xyz, max x
   float4 b[kSub];         // box max yz, centroid xy
   float c[kSub];          // centroid z
-  int cnt[3][MB];
-  int bbox[3][MB][6];
+  BinRow row[3][MB];
   Sweeps<MB> sweeps;
   SubNode todo[kSubTodo];          // nodes of more than kTinyMax triangles
   uint2 tiny[kSub / (kMaxLeaf + 1) + 1];  // smaller ones: first | count << 16, SubNode::up
@@ -838,8 +866,7 @@ __device__ int sub_split(const BuildState& st, SubWarp<MB>& w, const SubNode& e,
   bool live[3];
   warp_binning(cmin, cmax, bins, lo, scale, live);
   for (int i = lane; i < 3 * MB; i += 32) {
-    (&w.cnt[0][0])[i] = 0;
-    for (int q = 0; q < 6; q++) (&w.bbox[0][0][0])[6 * i + q] = ordered(q < 3 ? INFINITY : -INFINITY);
+    for (int q = 0; q < 7; q++) (&w.row[0][0])[i][q] = empty_bin_word(q);
   }
   __syncwarp();
   for (int k = lane; k < n; k += 32) {
@@ -850,11 +877,11 @@ __device__ int sub_split(const BuildState& st, SubWarp<MB>& w, const SubNode& e,
     for (int q = 0; q < 3; q++) {
       if (!live[q]) continue;
       const int x = bin_of(centroid_of(b, c, q), lo[q], scale[q], bins);
-      bin_prim(&w.cnt[q][x], w.bbox[q][x], v);
+      bin_prim(w.row[q][x], v);
     }
   }
   __syncwarp();
-  const Choice c = best_split<MB>(w.cnt, w.bbox, w.sweeps, live, bins);
+  const Choice c = best_split<MB>(w.row, w.sweeps, live, bins);
   const int mode = choose(c, e.box, n, axis, nleft);
   if (mode < 0) return mode;
   left_at = c.split;
@@ -1669,9 +1696,22 @@ static int run_build(BuildBuffers& B, const BuildState& st, float* d_bounds, int
     for (; levels < want; levels++) {
       const long long most = static_cast<long long>(N / st.seg) +
                              std::min<long long>(max_nodes, levels < 30 ? 1ll << levels : max_nodes);
-      const int grid = static_cast<int>(std::min<long long>(most, 2 * kBuildGrid));
-      k_bin<<<grid, kBuildBlock, 0, s>>>(levels, st);
-      k_part<<<grid, kBuildBlock, 0, s>>>(levels, st);
+      // Segments this level has if the tree is balanced, and blocks to suit:
+      // smaller ones from four and eight segments per SM. 16.4 M triangles
+      // rebuilt and traced 33.8 -> 32.6 ms, 1.3 M 3.82 -> 3.70 (3.81 from 8 and
+      // 16 per SM, 3.79 all from 4); with 64 threads at every level, 100 k
+      // triangles' hierarchy 0.96 -> 1.01 ms.
+      const long long segs = std::max<long long>(
+          n / st.seg, std::min<long long>(max_nodes, levels < 30 ? 1ll << levels : max_nodes));
+      const int bin_block = segs >= 8 * 148 ? 64 : (segs >= 4 * 148 ? 128 : 256);
+      const int part_block = segs >= 4 * 148 ? 128 : 256;
+      const auto bin = bin_block == 64 ? k_bin<64> : (bin_block == 128 ? k_bin<128> : k_bin<256>);
+      const auto part = part_block == 128 ? k_part<128> : k_part<256>;
+      const auto grid = [&](int block) {
+        return static_cast<int>(std::min<long long>(most, 2 * kBuildGrid * (kBuildBlock / block)));
+      };
+      bin<<<grid(bin_block), bin_block, 0, s>>>(levels, st);
+      part<<<grid(part_block), part_block, 0, s>>>(levels, st);
     }
     subtrees<<<std::min(blocks_of(n, kSubWarps), 2 * kBuildGrid), 32 * kSubWarps, smem, s>>>(st);
     k_rank_sums<<<kScanBlocks, kScanThreads, 0, s>>>(st, sums);
