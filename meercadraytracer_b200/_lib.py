@@ -133,7 +133,8 @@ def call(name: str, *args) -> None:
 
 
 def traversal_variants() -> list:
-    """The (threads per block, short-stack entries) pairs the traversal kernels were compiled for."""
+    """The pairs that name the traversal kernels: threads per block, and a second number that no longer
+    changes the kernel (the walk's stack is in local memory)."""
     n = C.c_int32()
     call("mcrt_traversal_variants", 0, None, None, C.byref(n))
     blocks = (C.c_int32 * max(1, n.value))()

@@ -3,9 +3,9 @@
 Three things are picked by timing short runs of the real workload on the
 device, not by rules of thumb:
 
-  * the traversal kernels' variant: threads per block and shared-memory
-    short-stack entries per thread (the closest-hit and shadow kernels are
-    compiled for several pairs, _lib.traversal_variants());
+  * the traversal kernels' variant: threads per block (the closest-hit and
+    shadow kernels are named by several pairs, _lib.traversal_variants(), of
+    which the second number no longer changes the kernel);
   * the path pool (queue size): paths in flight per launch series;
   * for the serving loop, the chunk size: the most paths one chunk may hold so
     that a chunk takes about `target_ms` on the slowest scene, which bounds

@@ -192,7 +192,7 @@ class BatchRenderer:
         call("mcrt_batch_set_chunk", self._h, int(paths))
 
     def set_traversal(self, block: int, stack: int) -> None:
-        """Traversal kernels by threads per block and short-stack depth (_lib.traversal_variants())."""
+        """Traversal kernels by a pair of _lib.traversal_variants(): threads per block decide."""
         call("mcrt_batch_set_traversal", self._h, int(block), int(stack))
 
     def stats(self) -> Dict[str, float]:

@@ -205,7 +205,7 @@ struct mcrt_executor {
   std::unordered_map<int, std::unique_ptr<TextureGpu>> textures;
   PathBuffers paths;
   int capacity = 1 << 25;  // paths in flight: 32M, about 17 GB of path state with 5 lights
-  int variant = 0;         // traversal kernels' (block, short stack) variant
+  int variant = 0;         // traversal kernels' variant (plain_variant)
   int step_limit = 0;      // > 0: a query's step budget (mcrt_set_step_limit)
   bool timed = false;
   RenderStats stats;

@@ -35,9 +35,11 @@
 // local memory. Against scalar tests on component-major nodes with a
 // shared-memory short stack inside the query's struct: bounce rays of a
 // 1280x720 frame of 500,000 random triangles 5.17 -> 3.98 ms, its shadow rays
-// 3.27 -> 2.34 ms; shadow rays of the 1.3 M-triangle 1080p frame at 64 passes
-// 17.4 -> 13.0 ms, its closest hits 18.7 -> 16.2 ms. Every test is the same
-// operations in the same rounding, so hits are those of before bit for bit.
+// 3.27 -> 2.34 ms (3.83 and 1.95 with the changes noted at walk_step and at
+// the shadow queue); shadow rays of the 1.3 M-triangle 1080p frame at 64 passes
+// 17.4 -> 13.0 ms (12.3), its closest hits 18.7 -> 16.2 ms (15.8 without the
+// making of the camera rays). Every test is the same operations in the same
+// rounding, so hits are those of before bit for bit.
 //
 // Child references: >= 0 an inner node index; < 0 a leaf whose first triangle
 // is ~ref. The last triangle of every leaf carries kLeafEnd in its flag word.

@@ -440,7 +440,7 @@ class GpuExecutor:
         call("mcrt_set_capacity", self._h, int(paths))
 
     def set_traversal(self, block: int, stack: int) -> None:
-        """Traversal kernels by threads per block and short-stack depth (_lib.traversal_variants())."""
+        """Traversal kernels by a pair of _lib.traversal_variants(): threads per block decide."""
         call("mcrt_set_traversal", self._h, int(block), int(stack))
 
     def set_step_limit(self, steps: int) -> None:
