@@ -42,3 +42,16 @@ def test_keeping_after_dropping_is_bounded(monkeypatch):
         gc.collect()
     kept = [pool.empty(1 << 20, np.uint8) for _ in range(50)]
     assert pinned_count(kept) == len(pool.blocks) <= 2 + pinned.FRESH
+
+
+@pytest.mark.parametrize("images", [1, 3, 12])
+def test_first_results_kept_and_later_ones_dropped(monkeypatch, images):
+    pool = HostPool(monkeypatch)
+    first = [pool.empty(1 << 20, np.uint8) for _ in range(images)]
+    for calls in range(8):
+        batch = [pool.empty(1 << 20, np.uint8) for _ in range(images)]
+        have = pinned_count(batch)
+        del batch
+        gc.collect()
+    assert have == images and pinned_count(first) == min(images, pinned.FRESH)
+    assert len(pool.blocks) == images + pinned_count(first)
