@@ -339,10 +339,13 @@ int32_t mcrt_batch_set_chunk(mcrt_batch* batch, int32_t paths);
 int32_t mcrt_batch_set_traversal(mcrt_batch* batch, int32_t block, int32_t stack);
 /* Queues a request; *id identifies it in events. */
 int32_t mcrt_batch_submit(mcrt_batch* batch, const mcrt_request* request, int64_t* id);
-/* Stops a request (a camera move restarts it as a new request). */
+/* Stops a request (a camera move restarts it as a new request). Its images
+ * are not written any more. */
 int32_t mcrt_batch_cancel(mcrt_batch* batch, int64_t id);
 /* Launches the next chunk, waits for the previous one and returns up to
- * max_events events; *idle is 1 when nothing is queued or in flight. */
+ * max_events events; *idle is 1 when nothing is queued or in flight. Requests'
+ * images are written during the call only: they stay as they are, whatever
+ * kind of memory they are in, until the next one. */
 int32_t mcrt_batch_step(mcrt_batch* batch, mcrt_batch_event* events, int32_t max_events, int32_t* n_events,
                         int32_t* idle);
 /* Submits `count` requests and runs until all are done. When nothing else is

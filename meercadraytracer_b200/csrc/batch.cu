@@ -546,12 +546,15 @@ cudaError_t BatchEngine::launch(Chunk& c) {
       if (e == cudaSuccess && !counters_host_[k]->more) break;
     }
   }
+  // The chunk before this one: its images go to the host while this one is
+  // traced, and before they are rewritten below.
+  if (e == cudaSuccess && inflight_.size() > 1) e = copy_out(inflight_.front());
   // Accumulation in chunk order: after the previous chunk's (the other half
   // may still be tracing it), and after any copy to the host of an image this
   // chunk rewrites.
   bool wait_copy = false;
   for (const SegmentPlan& s : c.segs) wait_copy = wait_copy || s.r->copying > 0;
-  if (e == cudaSuccess && wait_copy && copy_pending_) e = cudaStreamWaitEvent(st, last_copy_, 0);
+  if (e == cudaSuccess && wait_copy) e = cudaStreamWaitEvent(st, last_copy_, 0);
   if (e == cudaSuccess && accumulated_pending_) e = cudaStreamWaitEvent(st, accumulated_, 0);
   if (e == cudaSuccess) e = launch_batch_accumulate(tables_dev_[k], ps, grids_, st);
   if (e == cudaSuccess) e = cudaEventRecord(accumulated_, st);
@@ -559,34 +562,44 @@ cudaError_t BatchEngine::launch(Chunk& c) {
   if (e == cudaSuccess) e = cudaEventRecord(c.done, st);
   if (e != cudaSuccess) return e;
   totals_.chunks++;
-  // Images a request's client is waiting for: its preview, the image after
-  // each completed pass (when asked for), and the final image.
-  c.copies = false;
   c.passes_done.assign(c.segs.size(), 0);
   for (size_t j = 0; j < c.segs.size(); j++) {
     const SegmentPlan& s = c.segs[j];
+    if (!s.preview && s.pix0 + s.npix == s.r->pixels()) c.passes_done[j] = s.pass0 + s.passes;
+  }
+  return e;
+}
+
+// A request's preview, the image after each completed pass (when asked for),
+// and the final image.
+cudaError_t BatchEngine::copy_out(Chunk& c) {
+  if (c.copied_out) return cudaSuccess;
+  c.copied_out = true;
+  cudaError_t e = cudaSuccess;
+  for (size_t j = 0; j < c.segs.size() && e == cudaSuccess; j++) {
+    const SegmentPlan& s = c.segs[j];
     Request& r = *s.r;
-    const bool pass_end = !s.preview && s.pix0 + s.npix == r.pixels();
-    const bool last = pass_end && s.pass0 + s.passes == r.d.samples;
-    if (pass_end) c.passes_done[j] = s.pass0 + s.passes;
-    uint8_t* dst = s.preview ? r.host_preview : (last ? r.host_image : (pass_end ? r.host_progress : nullptr));
+    if (r.cancelled) continue;
+    const bool last = c.passes_done[j] == r.d.samples;
+    uint8_t* dst = s.preview ? r.host_preview : (last ? r.host_image : (c.passes_done[j] > 0 ? r.host_progress : nullptr));
     if (!dst) continue;
-    if (!c.copies) e = cudaStreamWaitEvent(copy_stream_, c.done, 0);
-    c.copies = true;
+    if (c.copies.empty()) e = cudaStreamWaitEvent(copy_stream_, c.done, 0);
+    c.copies.push_back(&r);
     r.copying++;
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(dst, r.image, static_cast<size_t>(r.pixels()) * 4, cudaMemcpyDeviceToHost, copy_stream_);
   }
-  if (e == cudaSuccess && c.copies) e = cudaEventRecord(c.copied, copy_stream_);
-  if (e == cudaSuccess && c.copies) e = cudaEventRecord(last_copy_, copy_stream_);
-  if (c.copies) copy_pending_ = true;
+  if (e == cudaSuccess && !c.copies.empty()) e = cudaEventRecord(c.copied, copy_stream_);
+  if (e == cudaSuccess && !c.copies.empty()) e = cudaEventRecord(last_copy_, copy_stream_);
   return e;
 }
 
 cudaError_t BatchEngine::finish(Chunk& c, std::vector<BatchEvent>& events) {
-  cudaError_t e = cudaEventSynchronize(c.done);
-  if (e == cudaSuccess && c.copies) e = cudaEventSynchronize(c.copied);
+  cudaError_t e = copy_out(c);
+  if (e == cudaSuccess) e = cudaEventSynchronize(c.done);
+  if (e == cudaSuccess && !c.copies.empty()) e = cudaEventSynchronize(c.copied);
   if (e != cudaSuccess) return e;
+  for (Request* r : c.copies) r->copying--;
   // Device time once: the part of this chunk after the chunk finished
   // before it (the two halves overlap).
   float ms = 0;
@@ -606,10 +619,6 @@ cudaError_t BatchEngine::finish(Chunk& c, std::vector<BatchEvent>& events) {
     const SegmentPlan& s = c.segs[j];
     Request& r = *s.r;
     r.inflight--;
-    const bool copied = s.preview ? r.host_preview != nullptr
-                                  : (c.passes_done[j] > 0 && (c.passes_done[j] == r.d.samples ? r.host_image != nullptr
-                                                                                               : r.host_progress != nullptr));
-    if (copied) r.copying--;
     if (r.cancelled) continue;
     if (s.preview) {
       events.push_back(BatchEvent{r.id, kEventPreview, 0});
@@ -620,7 +629,6 @@ cudaError_t BatchEngine::finish(Chunk& c, std::vector<BatchEvent>& events) {
       events.push_back(BatchEvent{r.id, kEventProgress, c.passes_done[j]});
     }
   }
-  if (inflight_.size() <= 1) copy_pending_ = false;  // this chunk's copies were the last enqueued
   for (auto it = requests_.begin(); it != requests_.end();) {
     Request& r = **it;
     if ((r.finished || r.cancelled) && r.inflight == 0) {

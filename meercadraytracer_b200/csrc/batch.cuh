@@ -86,10 +86,12 @@ class BatchEngine {
   // completes a pass short of the last.
   long long submit(const BatchRequestDesc& d, uint8_t* host_image, uint8_t* host_preview,
                    uint8_t* host_progress = nullptr);
-  // Stops a request; its buffers return to the arena once no chunk uses them.
+  // Stops a request; its buffers return to the arena once no chunk uses them,
+  // and its host images are not written any more.
   bool cancel(long long id);
   // Launches the next chunk (if any request has work), then waits for the
-  // chunk before it and appends the events it completed. *idle: nothing is
+  // chunk before it and its images' copies to the host, and appends the events
+  // it completed; no copy to the host is under way when it returns. *idle: nothing is
   // queued, active or in flight. *progressed (if given): a chunk was launched
   // or finished; a step that does neither while not idle is a scheduling
   // fault, which callers report instead of stepping again.
@@ -142,7 +144,7 @@ class BatchEngine {
     int group = 0;            // passes of that group while it is split by pixel range
     int branch = -1;          // half of the pool a whole-batch render gives it (render_whole)
     int inflight = 0;         // chunks in flight that hold a segment of this request
-    int copying = 0;          // chunks in flight copying this request's image to the host
+    int copying = 0;          // copies of this request's image to the host that are queued
     long long pixels() const { return static_cast<long long>(d.fp.width) * d.fp.height; }
   };
   struct SegmentPlan {
@@ -154,10 +156,11 @@ class BatchEngine {
     int slot;  // half of the pool, stream, tables and graph
     std::vector<SegmentPlan> segs;
     cudaEvent_t start = nullptr, done = nullptr, copied = nullptr;
-    bool copies = false;
     // Per segment: the pass count its image holds when the chunk ends, if
     // the chunk completes a pass of the request (else 0).
     std::vector<int> passes_done;
+    bool copied_out = false;            // copy_out has run
+    std::vector<Request*> copies;       // requests whose images it copies
   };
 
   PathState slot_state(int slot) const;
@@ -169,6 +172,11 @@ class BatchEngine {
   // The chunk's tables as its kernels read them (host copy).
   void fill_tables(const Chunk& c, BatchTables* T);
   cudaError_t launch(Chunk& c);
+  // Queues the copies of the images that clients wait for from the oldest
+  // chunk in flight. Within the step that finishes the chunk and waits for
+  // them, so that no step leaves a copy under way: what an event names stays
+  // as it is until the next step, in pinned memory too.
+  cudaError_t copy_out(Chunk& c);
   cudaError_t finish(Chunk& c, std::vector<BatchEvent>& events);
   void release(Request& r);
 
@@ -210,7 +218,6 @@ class BatchEngine {
   // Copy-stream event of the last chunk that copied images to the host: a
   // chunk's accumulation waits for it before rewriting an image being copied.
   cudaEvent_t last_copy_ = nullptr;
-  bool copy_pending_ = false;
   // Recorded after each chunk's accumulation; the next chunk's waits for it.
   cudaEvent_t accumulated_ = nullptr;
   bool accumulated_pending_ = false;
