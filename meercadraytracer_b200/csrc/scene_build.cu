@@ -267,7 +267,11 @@ __device__ __forceinline__ int warp_bound(float v, bool max) {
 }
 
 // A triangle's box and centroid (bvh.ts:22-33) into place i, and into the
-// thread's bounds.
+// thread's bounds. A bound that is NaN (a vertex that is) is left out of every
+// union, as the reference's comparisons leave it out: it is kept as the value
+// that changes none, since min and max over ordered integers would take a NaN
+// for the largest, and each split that keeps it would be lost. The centroid
+// stays NaN and goes to the last bin.
 __device__ __forceinline__ void put_prim(const Prims& p, int i, const float* o, float* m) {
   double lo[3], hi[3];
   for (int a = 0; a < 3; a++) {
@@ -275,9 +279,9 @@ __device__ __forceinline__ void put_prim(const Prims& p, int i, const float* o, 
     lo[a] = fmin(v0, fmin(v1, v2));
     hi[a] = fmax(v0, fmax(v1, v2));
   }
-  const float4 a4 = make_float4(static_cast<float>(lo[0]), static_cast<float>(lo[1]), static_cast<float>(lo[2]),
-                                static_cast<float>(hi[0]));
-  const float4 b4 = make_float4(static_cast<float>(hi[1]), static_cast<float>(hi[2]),
+  const float4 a4 = make_float4(fminf(static_cast<float>(lo[0]), INFINITY), fminf(static_cast<float>(lo[1]), INFINITY),
+                                fminf(static_cast<float>(lo[2]), INFINITY), fmaxf(static_cast<float>(hi[0]), -INFINITY));
+  const float4 b4 = make_float4(fmaxf(static_cast<float>(hi[1]), -INFINITY), fmaxf(static_cast<float>(hi[2]), -INFINITY),
                                 static_cast<float>((lo[0] + hi[0]) * 0.5), static_cast<float>((lo[1] + hi[1]) * 0.5));
   const float cz = static_cast<float>((lo[2] + hi[2]) * 0.5);
   p.a[i] = a4;
@@ -400,16 +404,20 @@ __device__ __forceinline__ double box_area(const int* b) {
 }
 
 // The first minimum in (axis, split) order of the warp's candidates, each lane
-// offering one (cost INFINITY: none), the same in every lane. Costs are never
-// negative, so their bits order as integers do: three integer reductions
-// instead of five rounds of double shuffles.
+// offering one (cost INFINITY: none), the same in every lane. Costs are ordered
+// by their bits, flipped so that they compare as unsigned integers do (a set
+// whose box is empty on one axis, its vertices being NaN there, has a cost of
+// -INFINITY): three integer reductions instead of five rounds of double shuffles.
 __device__ __forceinline__ Choice first_minimum(double cost, int axis, int split, int nleft) {
-  const unsigned full = 0xffffffffu;
-  const unsigned hi = static_cast<unsigned>(__double2hiint(cost)), lo = static_cast<unsigned>(__double2loint(cost));
+  const unsigned full = 0xffffffffu, sign = 0x80000000u;
+  const unsigned flip = static_cast<unsigned>(__double2hiint(cost) >> 31);
+  const unsigned hi = static_cast<unsigned>(__double2hiint(cost)) ^ (flip | sign);
+  const unsigned lo = static_cast<unsigned>(__double2loint(cost)) ^ flip;
   const unsigned h = __reduce_min_sync(full, hi);
   const unsigned l = __reduce_min_sync(full, hi == h ? lo : ~0u);
   const unsigned at = __reduce_min_sync(full, hi == h && lo == l ? static_cast<unsigned>((axis << 8) | split) : ~0u);
-  const double best = __hiloint2double(static_cast<int>(h), static_cast<int>(l));
+  const unsigned back = h & sign ? 0u : ~0u;
+  const double best = __hiloint2double(static_cast<int>(h ^ (back | sign)), static_cast<int>(l ^ back));
   if (!(best < INFINITY)) return Choice{INFINITY, -1, -1, 0};
   const unsigned who = __ballot_sync(full, hi == h && lo == l && static_cast<unsigned>((axis << 8) | split) == at);
   return Choice{best, static_cast<int>(at >> 8), static_cast<int>(at & 0xff), __shfl_sync(full, nleft, __ffs(who) - 1)};
