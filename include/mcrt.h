@@ -342,6 +342,10 @@ int32_t mcrt_batch_submit(mcrt_batch* batch, const mcrt_request* request, int64_
 /* Stops a request (a camera move restarts it as a new request). Its images
  * are not written any more. */
 int32_t mcrt_batch_cancel(mcrt_batch* batch, int64_t id);
+/* *holds: 1 while a request is queued or on the device, finished or cancelled
+ * requests not counted once nothing of them is in flight. Until then its
+ * executor's scene stays as it is, and its images too unless it is cancelled. */
+int32_t mcrt_batch_holds(mcrt_batch* batch, int64_t id, int32_t* holds);
 /* Launches the next chunk, waits for the previous one and returns up to
  * max_events events; *idle is 1 when nothing is queued or in flight. Requests'
  * images are written during the call only: they stay as they are, whatever
@@ -354,7 +358,7 @@ int32_t mcrt_batch_step(mcrt_batch* batch, mcrt_batch_event* events, int32_t max
  * launch (every chunk planned ahead, the requests split between the two
  * halves of the pool, each half's chunks run in a device-driven loop);
  * otherwise chunk by chunk as mcrt_batch_step runs them. Images are the
- * same either way. */
+ * same either way. A call that fails cancels its requests. */
 int32_t mcrt_batch_render(mcrt_batch* batch, int32_t count, const mcrt_request* requests);
 int32_t mcrt_batch_get_stats(mcrt_batch* batch, mcrt_batch_stats* out);
 

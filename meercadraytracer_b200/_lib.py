@@ -84,6 +84,7 @@ SIGNATURES = {
     "mcrt_batch_set_chunk": (_i32, [_vp, _i32]),
     "mcrt_batch_submit": (_i32, [_vp, _vp, _P(C.c_int64)]),
     "mcrt_batch_cancel": (_i32, [_vp, C.c_int64]),
+    "mcrt_batch_holds": (_i32, [_vp, C.c_int64, _P(_i32)]),
     "mcrt_batch_step": (_i32, [_vp, _vp, _i32, _P(_i32), _P(_i32)]),
     "mcrt_batch_render": (_i32, [_vp, _i32, _vp]),
     "mcrt_batch_get_stats": (_i32, [_vp, _vp]),

@@ -62,10 +62,7 @@ class BatchRenderer:
         self._executors: Dict[int, Tuple[CompiledScene, GpuExecutor]] = {}
         self._buffers: Dict[int, Tuple[np.ndarray, Optional[np.ndarray], Optional[np.ndarray]]] = {}
         self._adopted: set = set()
-        # Buffers of requests that ended before their copies may have: kept for three more steps (two
-        # chunks are in flight at most, and each step finishes the oldest).
-        self._steps = 0
-        self._open: set = set()  # requests whose DONE event has not been seen
+        # Buffers of forgotten requests that the engine still holds, which may write them yet.
         self._retired: List[Tuple[int, object]] = []
 
     # ----------------------------------------------------------- scenes
@@ -117,7 +114,6 @@ class BatchRenderer:
         rid = C.c_int64()
         call("mcrt_batch_submit", self._h, C.byref(c), C.byref(rid))
         self._buffers[rid.value] = buffers
-        self._open.add(rid.value)
         return rid.value
 
     def submit(self, r: RenderRequest) -> int:
@@ -147,15 +143,22 @@ class BatchRenderer:
         events = (abi.mcrt_batch_event * max(1, max_events))()
         n = C.c_int32()
         idle = C.c_int32()
-        self._steps += 1
-        call("mcrt_batch_step", self._h, events, int(max_events), C.byref(n), C.byref(idle))
+        try:
+            call("mcrt_batch_step", self._h, events, int(max_events), C.byref(n), C.byref(idle))
+        finally:
+            self._release()
+        return [(events[i].id, events[i].kind, events[i].samples) for i in range(n.value)], bool(idle.value)
+
+    def _holds(self, rid: int) -> bool:
+        if self._h is None:
+            return False
+        holds = C.c_int32()
+        call("mcrt_batch_holds", self._h, int(rid), C.byref(holds))
+        return bool(holds.value)
+
+    def _release(self) -> None:
         if self._retired:
-            self._retired = [] if idle.value else [r for r in self._retired if r[0] > self._steps]
-        out = [(events[i].id, events[i].kind, events[i].samples) for i in range(n.value)]
-        for rid, kind, _ in out:
-            if kind == EVENT_DONE:
-                self._open.discard(rid)
-        return out, bool(idle.value)
+            self._retired = [r for r in self._retired if self._holds(r[0])]
 
     def result(self, rid: int) -> np.ndarray:
         return self._buffers[rid][0]
@@ -170,10 +173,8 @@ class BatchRenderer:
     def forget(self, rid: int) -> None:
         """Drops the host buffers of a finished or cancelled request."""
         buffers = self._buffers.pop(rid, None)
-        if rid in self._open:
-            self._open.discard(rid)
-            if buffers is not None:
-                self._retired.append((self._steps + 3, buffers))
+        if buffers is not None and self._holds(rid):
+            self._retired.append((rid, buffers))
 
     def render(self, requests: Sequence[RenderRequest]) -> List[np.ndarray]:
         """Renders every request to completion in one batch (mcrt_batch_render)."""
@@ -183,9 +184,8 @@ class BatchRenderer:
             arr[i] = self._c_request(r, images[i], None)
         try:
             call("mcrt_batch_render", self._h, int(len(requests)), arr)
-        except Exception:
-            self._retired.append((self._steps + 3, images))  # a failed call may leave chunks in flight
-            raise
+        finally:
+            self._release()
         return images
 
     def set_chunk(self, paths: int) -> None:

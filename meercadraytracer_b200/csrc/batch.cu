@@ -372,6 +372,12 @@ bool BatchEngine::cancel(long long id) {
   return false;
 }
 
+bool BatchEngine::holds(long long id) const {
+  for (const auto& r : requests_)
+    if (r->id == id) return true;
+  return false;
+}
+
 void BatchEngine::release(Request& r) {
   if (r.sum) arena_.free(r.sum);
   r.sum = nullptr;
@@ -641,6 +647,23 @@ cudaError_t BatchEngine::finish(Chunk& c, std::vector<BatchEvent>& events) {
   return cudaSuccess;
 }
 
+cudaError_t BatchEngine::finish_oldest(std::vector<BatchEvent>& events) {
+  const cudaError_t e = finish(inflight_.front(), events);
+  Chunk& done = inflight_.front();
+  if (done.start) cudaEventDestroy(done.start);
+  if (held_done_) cudaEventDestroy(held_done_);
+  held_done_ = done.done;  // the next chunk's device time counts from here
+  if (done.copied) cudaEventDestroy(done.copied);
+  inflight_.pop_front();
+  return e;
+}
+
+cudaError_t BatchEngine::drain(std::vector<BatchEvent>& events) {
+  cudaError_t e = cudaSetDevice(device_);
+  while (e == cudaSuccess && !inflight_.empty()) e = finish_oldest(events);
+  return e;
+}
+
 cudaError_t BatchEngine::step(std::vector<BatchEvent>& events, bool* idle, bool* progressed) {
   cudaError_t e = cudaSetDevice(device_);
   if (e != cudaSuccess) return e;
@@ -660,13 +683,7 @@ cudaError_t BatchEngine::step(std::vector<BatchEvent>& events, bool* idle, bool*
     }
   }
   if (!inflight_.empty() && (inflight_.size() == 2 || !launched)) {
-    e = finish(inflight_.front(), events);
-    Chunk& done = inflight_.front();
-    if (done.start) cudaEventDestroy(done.start);
-    if (held_done_) cudaEventDestroy(held_done_);
-    held_done_ = done.done;  // the next chunk's device time counts from here
-    if (done.copied) cudaEventDestroy(done.copied);
-    inflight_.pop_front();
+    e = finish_oldest(events);
     if (e != cudaSuccess) return e;
   }
   bool pending = false;

@@ -89,6 +89,8 @@ class BatchEngine {
   // Stops a request; its buffers return to the arena once no chunk uses them,
   // and its host images are not written any more.
   bool cancel(long long id);
+  // The request is queued, or a chunk in flight holds a segment of it.
+  bool holds(long long id) const;
   // Launches the next chunk (if any request has work), then waits for the
   // chunk before it and its images' copies to the host, and appends the events
   // it completed; no copy to the host is under way when it returns. *idle: nothing is
@@ -96,6 +98,8 @@ class BatchEngine {
   // or finished; a step that does neither while not idle is a scheduling
   // fault, which callers report instead of stepping again.
   cudaError_t step(std::vector<BatchEvent>& events, bool* idle, bool* progressed = nullptr);
+  // Waits for the chunks in flight, as step() does, and launches nothing.
+  cudaError_t drain(std::vector<BatchEvent>& events);
   // Renders every queued request to completion as one graph launch: the
   // requests are split between the two halves of the pool, each half's
   // chunks are planned ahead and uploaded at once, and each half runs its
@@ -178,6 +182,7 @@ class BatchEngine {
   // as it is until the next step, in pinned memory too.
   cudaError_t copy_out(Chunk& c);
   cudaError_t finish(Chunk& c, std::vector<BatchEvent>& events);
+  cudaError_t finish_oldest(std::vector<BatchEvent>& events);
   void release(Request& r);
 
   int device_ = 0;

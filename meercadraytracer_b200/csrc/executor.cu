@@ -1530,38 +1530,55 @@ int32_t mcrt_batch_step(mcrt_batch* b, mcrt_batch_event* events, int32_t max_eve
   });
 }
 
+int32_t mcrt_batch_holds(mcrt_batch* b, int64_t id, int32_t* holds) {
+  return guard([&] {
+    if (!b || !holds) fail(MCRT_ERR_INVALID, "batch or output is NULL");
+    *holds = b->engine.holds(id) ? 1 : 0;
+  });
+}
+
 int32_t mcrt_batch_render(mcrt_batch* b, int32_t count, const mcrt_request* requests) {
   return guard([&] {
     checked_batch(b);
     if (count < 0 || (count > 0 && !requests)) fail(MCRT_ERR_INVALID, "bad request list");
-    for (int i = 0; i < count; i++) submit_request(b, requests + i);
-    // The whole batch as one graph launch when no request needs host work
-    // between chunks (BatchEngine::render_whole); otherwise, or for what is
-    // left, chunk by chunk.
-    {
-      check_slots(b);
+    std::vector<int64_t> ids;
+    try {
+      for (int i = 0; i < count; i++) ids.push_back(submit_request(b, requests + i));
+      // The whole batch as one graph launch when no request needs host work
+      // between chunks (BatchEngine::render_whole); otherwise, or for what is
+      // left, chunk by chunk.
+      {
+        check_slots(b);
+        std::vector<BatchEvent> ev;
+        const unsigned earlier = b->engine.totals().status;
+        bool rendered = false;
+        cuda_check(b->engine.render_whole(ev, &rendered), "whole-batch render");
+        if (b->engine.totals().status & kStatusIterationLimit)
+          fail(MCRT_ERR_CUDA, "a batched chunk did not finish within its iteration limit");
+        check_walk(b->engine.totals().status & ~earlier);
+      }
+      // Every step launches or finishes a chunk until the engine is idle, so
+      // this loop ends; a step that does neither is a scheduling fault and fails
+      // the call rather than spinning.
+      bool idle = false;
+      while (!idle) {
+        check_slots(b);
+        std::vector<BatchEvent> ev;
+        const unsigned earlier = b->engine.totals().status;
+        bool progressed = false;
+        cuda_check(b->engine.step(ev, &idle, &progressed), "batch step");
+        if (!idle && !progressed) fail(MCRT_ERR_LIMIT, "the batch engine could not schedule a pending request");
+        if (b->engine.totals().status & kStatusIterationLimit)
+          fail(MCRT_ERR_CUDA, "a batched chunk did not finish within its iteration limit");
+        check_walk(b->engine.totals().status & ~earlier);
+      }
+    } catch (...) {
+      // The caller's memory and scenes are its own again once the call returns.
+      for (const int64_t id : ids) b->engine.cancel(id);
       std::vector<BatchEvent> ev;
-      const unsigned earlier = b->engine.totals().status;
-      bool rendered = false;
-      cuda_check(b->engine.render_whole(ev, &rendered), "whole-batch render");
-      if (b->engine.totals().status & kStatusIterationLimit)
-        fail(MCRT_ERR_CUDA, "a batched chunk did not finish within its iteration limit");
-      check_walk(b->engine.totals().status & ~earlier);
-    }
-    // Every step launches or finishes a chunk until the engine is idle, so
-    // this loop ends; a step that does neither is a scheduling fault and fails
-    // the call rather than spinning.
-    bool idle = false;
-    while (!idle) {
-      check_slots(b);
-      std::vector<BatchEvent> ev;
-      const unsigned earlier = b->engine.totals().status;
-      bool progressed = false;
-      cuda_check(b->engine.step(ev, &idle, &progressed), "batch step");
-      if (!idle && !progressed) fail(MCRT_ERR_LIMIT, "the batch engine could not schedule a pending request");
-      if (b->engine.totals().status & kStatusIterationLimit)
-        fail(MCRT_ERR_CUDA, "a batched chunk did not finish within its iteration limit");
-      check_walk(b->engine.totals().status & ~earlier);
+      b->engine.drain(ev);
+      for (const BatchEvent& e : ev) b->pending.push_back(e);
+      throw;
     }
   });
 }

@@ -67,10 +67,6 @@ class RenderServer:
         self.scenes: Dict[str, Tuple[GpuExecutor, Tuple[int, int], CompiledScene]] = {}
         self.requests: Dict[int, ServedRequest] = {}
         self.live: Dict[int, int] = {}  # client -> its live request id
-        # Cancelled requests whose host buffers may still receive a copy from a chunk in
-        # flight: kept for two more engine steps (at most two chunks are in flight, and
-        # each step finishes the oldest).
-        self._retiring: Dict[int, int] = {}
         self.clock: Callable[[], float] = time.perf_counter
 
     def add_scene(self, name: str, scene: CompiledScene) -> None:
@@ -91,7 +87,7 @@ class RenderServer:
             r = self.requests.get(old)
             if r is not None and r.done is None:
                 r.cancelled = now
-            self._retiring[old] = 2
+            self.batch.forget(old)
         ex, versions, _ = self.scenes[scene]
         rid = self.batch.submit_to(ex, versions, camera, settings, width, height, samples, preview_block, srgb,
                                    progress=self.progress_images)
@@ -119,11 +115,6 @@ class RenderServer:
                     del self.live[r.client]
                 if self.keep_images:
                     r.image = self.batch.result(rid)
-                self.batch.forget(rid)
-        for rid in list(self._retiring):
-            self._retiring[rid] -= 1
-            if self._retiring[rid] <= 0:
-                del self._retiring[rid]
                 self.batch.forget(rid)
         return events, idle
 
@@ -217,7 +208,7 @@ def simulate_clients(server: RenderServer, clients: Sequence[Client], settings: 
         for c in list(server.live):
             rid = server.live.pop(c)
             server.batch.cancel(rid)
-            server._retiring[rid] = 2
+            server.batch.forget(rid)
         for _ in range(1 << 22):
             _, idle = server.poll()
             if idle:
