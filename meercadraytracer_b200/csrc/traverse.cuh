@@ -410,12 +410,14 @@ MCRT_D void walk_step(const DScene& sc, Q& q, TravStack& st, WalkState& w, unsig
       }
     }
   }
-  if (w.left < 0 && (w.node != kSentinel || w.leaf != 0)) {
-    status |= kStatusStepLimit;
-    stop = true;
-  }
   if (paused) stop = !q.resume();
   if (stop) {
+    w.node = kSentinel;
+    w.leaf = 0;
+  }
+  // Out of steps with something left to visit (a query that its last step ended is none).
+  if (w.left < 0 && (w.node != kSentinel || w.leaf != 0)) {
+    status |= kStatusStepLimit;
     w.node = kSentinel;
     w.leaf = 0;
   }
