@@ -43,6 +43,8 @@ typedef struct mcrt_stats {
   uint64_t samples;       /* paths started */
   uint64_t launches;      /* kernels launched */
   double ms_total;        /* device time of whole render calls */
+  /* With mcrt_set_timing, by stage (camera rays that are made in the first
+     closest-hit kernel count as its work): */
   double ms_raygen, ms_extend, ms_shade, ms_shadow, ms_resolve, ms_accumulate;
   uint64_t n_raygen, n_extend, n_shade, n_shadow, n_resolve, n_accumulate;
   uint64_t path_bytes;    /* HBM held for path state */
@@ -244,7 +246,9 @@ int32_t mcrt_compile_instances(mcrt_executor* executor, int32_t version, int32_t
                                mcrt_compiled_out* out);
 
 /* Kernel timing with CUDA events on the executor's stream (adds a sync per
- * kernel; for profiling only). */
+ * kernel; for profiling only). Stages run one after another, each bounce's as
+ * kernels of their own, however few its paths are; the image's copy to the host
+ * is in none of the times. */
 int32_t mcrt_set_timing(mcrt_executor* executor, int32_t enabled);
 
 /* Path-state capacity (paths in flight per launch); the autotuner sets it. */

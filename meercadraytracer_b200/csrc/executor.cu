@@ -339,8 +339,8 @@ struct ChunkCtx {
   uint8_t* image;
   float4* sum;
   float* tile_out;
-  // Queued behind the last chunk, so that the frame's one wait covers it: the
-  // result's way to the host, if any.
+  // Queued behind the last chunk, so that the frame's one wait covers it (unless
+  // its stages are timed): the result's way to the host, if any.
   void* host = nullptr;
   const void* result = nullptr;
   size_t result_bytes = 0;
@@ -394,7 +394,7 @@ void run_frame(mcrt_executor* ex, FrameParams fp, int total, int passes, ChunkCt
     fp.pix0 = p0;
     fp.npix = std::min(span, total - p0);
     ctx.fp = fp;
-    ctx.last_span = p0 + span >= total;
+    ctx.last_span = !ex->timed && p0 + span >= total;
     Wavefront wf;
     wf.variant = ex->variant;
     e = wf.run(scene, fp, passes, ex->paths, ex->stream, &ex->stats, ex->timed, chunk, &ctx);
@@ -402,7 +402,10 @@ void run_frame(mcrt_executor* ex, FrameParams fp, int total, int passes, ChunkCt
   const unsigned walk = ex->stats.status;
   ex->stats.status |= earlier;
   cuda_check(e, "render");
-  if (!ctx.finished) cuda_check(cudaErrorUnknown, "render");  // every frame ends with a chunk
+  if (!ctx.finished) {
+    cuda_check(finish_frame(&ctx), "render");
+    cuda_check(cudaStreamSynchronize(ex->stream), "render");
+  }
   float ms = 0;
   cudaEventElapsedTime(&ms, ex->ev0, ex->ev1);
   ex->ms_total += ms;

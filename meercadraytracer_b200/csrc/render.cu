@@ -1733,13 +1733,15 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
   // and four small clears a bounce, the GPU idled 20-25 us a bounce: a 320 x
   // 240 still of 16 passes 1.07 -> 1.00 ms, a 633 x 471 draft of 7 1.51 -> 1.47,
   // a 720p frame of 4 over 500 k triangles 6.10 -> 5.80.
-  // Timed renders keep one stream, so every kernel's events bracket it alone.
+  // Timed renders keep one stream, so every kernel's events bracket it alone,
+  // and every stage of every bounce is a kernel of its own: no k_tail.
   PathBuffers::Side side;
   bool overlap = !timed;
   if (overlap && e == cudaSuccess) {
     e = buffers.side_streams(&side);
     overlap = e == cudaSuccess;
   }
+  const int tail_max = timed ? 0 : kTailMax;
   bool tails = false;      // a tail launch counted rays on the device
   bool side_busy = false;  // side work queued since the main stream last joined it
   auto join_side = [&]() {
@@ -1762,7 +1764,7 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
     // blocked early idle until the warp's last ray ends, where the per-lane
     // walk refills them.)
     const int warp_pixels = 32 / std::max(1, std::min(f.npass, 32));
-    const bool coherent = packet_first && n > kTailMax && warp_pixels * 360 <= f.height;
+    const bool coherent = packet_first && n > tail_max && warp_pixels * 360 <= f.height;
     const CameraRays camera = sort_shading && n >= kSortMin ? camera_rays(scene, f) : CameraRays{};
     cudaMemsetAsync(cnt->bounce, 0, sizeof(cnt->bounce), stream);
     if (camera.on) cudaMemsetAsync(ps.bins, 0, 2 * kShadeClasses * sizeof(unsigned int), stream);
@@ -1788,7 +1790,7 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
       }
       tm.stop(st.ms_extend, st.n_extend);
     };
-    if (n > kTailMax) extend(bounce, ps.queue[cur], n, n);
+    if (n > tail_max) extend(bounce, ps.queue[cur], n, n);
     for (; n > 0; bounce++) {
       // Paths end by bounce count, pass-through count or Russian roulette; a
       // loop this long means corrupt state, reported rather than spun on.
@@ -1796,15 +1798,13 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
         e = cudaErrorLaunchTimeout;
         break;
       }
-      if (n <= kTailMax) {
+      if (n <= tail_max) {
         // Few paths left (or few from the start): one launch takes them to
         // their ends, with the side stream's work on them done first.
         join_side();
-        tm.start();
         const int limit = resident_limit(reinterpret_cast<const void*>(k_tail), kTailBlock);
         const int blocks = std::min(limit, blocks_for(n, kTailBlock / 32));
         k_tail<<<blocks, kTailBlock, 0, stream>>>(scene, f, ps, ps.queue[cur], n, cap, buffers.slots(), cnt, bounce);
-        tm.stop(st.ms_extend, st.n_extend);
         st.launches++;
         tails = true;
         break;
@@ -1871,7 +1871,7 @@ cudaError_t Wavefront::run(const DScene& scene, FrameParams fp, int passes, Path
       if (!overlap) {
         if (n_shadow > 0) shadow(n_shadow, n_shadow, stream);
         resolve(stream);
-        if (n_next > kTailMax) extend(bounce + 1, ps.queue[cur ^ 1], n_next, n_next);
+        if (n_next > tail_max) extend(bounce + 1, ps.queue[cur ^ 1], n_next, n_next);
       }
       n = n_next;
       cur ^= 1;
