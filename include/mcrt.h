@@ -165,6 +165,12 @@ int32_t mcrt_intersect_any_count(mcrt_executor* executor, int32_t geometry_versi
 int32_t mcrt_build_bvh(mcrt_executor* executor, const float* triangles, int32_t count, float* bounds,
                        int32_t* nodes, uint32_t* order, int32_t* node_count);
 
+/* The same in two calls, for arrays of the hierarchy's own size: the build,
+ * whose result stays on the device until the executor's next build or compile,
+ * and its download (`bounds` and `nodes` hold *node_count nodes). */
+int32_t mcrt_bvh_build(mcrt_executor* executor, const float* triangles, int32_t count, int32_t* node_count);
+int32_t mcrt_bvh_read(mcrt_executor* executor, float* bounds, int32_t* nodes, uint32_t* order);
+
 /* compileGeometry after the flatten, src/compile.ts:359-403, on the GPU:
  * float32 rounding of world-space triangles, BVH, reorder into BVH order,
  * tangents (writeTangent, src/compile.ts:406-432) and epsilon. Inputs and

@@ -89,6 +89,8 @@ SIGNATURES = {
     "mcrt_batch_render": (_i32, [_vp, _i32, _vp]),
     "mcrt_batch_get_stats": (_i32, [_vp, _vp]),
     "mcrt_build_bvh": (_i32, [_vp, _P(_f), _i32, _P(_f), _P(_i32), _P(_u32), _P(_i32)]),
+    "mcrt_bvh_build": (_i32, [_vp, _P(_f), _i32, _P(_i32)]),
+    "mcrt_bvh_read": (_i32, [_vp, _P(_f), _P(_i32), _P(_u32)]),
     "mcrt_compile_geometry": (_i32, [_vp, _i32, _P(_d), _P(_d), _P(_d), _P(_d), _P(_u8), _P(_u32), _P(_u8), _P(_u8),
                                      _P(_f), _P(_f), _P(_f), _P(_f), _P(_f), _P(_u32), _P(_u8), _P(_u8), _P(_f),
                                      _P(_i32), _P(_u32), _P(_i32), _P(_d), _P(_i32)]),

@@ -1140,7 +1140,24 @@ int32_t mcrt_build_bvh(mcrt_executor* ex, const float* triangles, int32_t count,
     checked(ex);
     if (count < 0 || (count > 0 && (!triangles || !bounds || !nodes || !order)) || !node_count)
       fail(MCRT_ERR_INVALID, "bad BVH build arguments");
-    *node_count = ex->builder.build_bvh_host(triangles, count, bounds, nodes, order, ex->stream);
+    *node_count = ex->builder.build_bvh_host(triangles, count, ex->stream);
+    ex->builder.read_bvh(bounds, nodes, order, ex->stream);
+  });
+}
+
+int32_t mcrt_bvh_build(mcrt_executor* ex, const float* triangles, int32_t count, int32_t* node_count) {
+  return guard([&] {
+    checked(ex);
+    if (count < 0 || (count > 0 && !triangles) || !node_count) fail(MCRT_ERR_INVALID, "bad BVH build arguments");
+    *node_count = ex->builder.build_bvh_host(triangles, count, ex->stream);
+  });
+}
+
+int32_t mcrt_bvh_read(mcrt_executor* ex, float* bounds, int32_t* nodes, uint32_t* order) {
+  return guard([&] {
+    checked(ex);
+    if (!bounds || !nodes || !order) fail(MCRT_ERR_INVALID, "bad BVH read arguments");
+    if (!ex->builder.read_bvh(bounds, nodes, order, ex->stream)) fail(MCRT_ERR_INVALID, "no BVH was built");
   });
 }
 

@@ -1808,6 +1808,7 @@ long long SceneBuilder::instance_triangles(int count, const InstanceInput* inst)
 void SceneBuilder::compile_instances(int count, const InstanceInput* inst, int bins, cudaStream_t s,
                                      const PackedGeometry& packed, bool arrays, DeviceGeometry* out, float* times_ms) {
   BuildBuffers& B = *b_;
+  bvh_count_ = -1;
   const long long total = instance_triangles(count, inst);
   if (total < 0) throw std::runtime_error("an instance names a mesh that was not uploaded");
   if (total > (1ll << 30)) throw std::runtime_error("too many triangles");
@@ -1922,22 +1923,35 @@ size_t SceneBuilder::device_bytes() const {
   return t;
 }
 
-int SceneBuilder::build_bvh_host(const float* tris, int n, float* bounds, int* nodes, uint32_t* order,
-                                 cudaStream_t s) {
-  if (n <= 0) return 0;
-  BuildBuffers& B = *b_;
-  const size_t cap = std::max(1, 2 * n - 1);
-  float* d_tris = B.tris.ensure(9 * static_cast<size_t>(n));
-  float* d_bounds = B.bounds.ensure(6 * cap);
-  int* d_nodes = B.nodes.ensure(3 * cap);
-  uint32_t* d_order = B.order.ensure(n);
-  check(cudaMemcpyAsync(d_tris, tris, sizeof(float) * 9 * n, cudaMemcpyHostToDevice, s), "upload");
-  const int m = build_device(d_tris, n, d_bounds, d_nodes, d_order, s);
-  check(cudaMemcpyAsync(bounds, d_bounds, sizeof(float) * 6 * m, cudaMemcpyDeviceToHost, s), "download");
-  check(cudaMemcpyAsync(nodes, d_nodes, sizeof(int) * 3 * m, cudaMemcpyDeviceToHost, s), "download");
-  check(cudaMemcpyAsync(order, d_order, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s), "download");
-  check(cudaStreamSynchronize(s), "download");
+int SceneBuilder::build_bvh_host(const float* tris, int n, cudaStream_t s) {
+  bvh_count_ = -1;
+  int m = 0;
+  if (n > 0) {
+    BuildBuffers& B = *b_;
+    const size_t N = static_cast<size_t>(n);
+    const size_t cap = std::max<size_t>(1, 2 * N - 1);
+    float* d_tris = B.tris.ensure(9 * N);
+    float* d_bounds = B.bounds.ensure(6 * cap);
+    int* d_nodes = B.nodes.ensure(3 * cap);
+    uint32_t* d_order = B.order.ensure(N);
+    check(cudaMemcpyAsync(d_tris, tris, sizeof(float) * 9 * N, cudaMemcpyHostToDevice, s), "upload");
+    m = build_device(d_tris, n, d_bounds, d_nodes, d_order, s);
+  }
+  bvh_count_ = std::max(n, 0);
+  bvh_nodes_ = m;
   return m;
+}
+
+bool SceneBuilder::read_bvh(float* bounds, int* nodes, uint32_t* order, cudaStream_t s) {
+  if (bvh_count_ < 0) return false;
+  if (bvh_count_ == 0) return true;
+  BuildBuffers& B = *b_;
+  const size_t m = static_cast<size_t>(bvh_nodes_);
+  check(cudaMemcpyAsync(bounds, B.bounds.p, sizeof(float) * 6 * m, cudaMemcpyDeviceToHost, s), "download");
+  check(cudaMemcpyAsync(nodes, B.nodes.p, sizeof(int) * 3 * m, cudaMemcpyDeviceToHost, s), "download");
+  check(cudaMemcpyAsync(order, B.order.p, sizeof(uint32_t) * bvh_count_, cudaMemcpyDeviceToHost, s), "download");
+  check(cudaStreamSynchronize(s), "download");
+  return true;
 }
 
 void SceneBuilder::compile_host(int n, const double* p, const double* nrm, const double* uv, const double* colors,
@@ -1946,6 +1960,7 @@ void SceneBuilder::compile_host(int n, const double* p, const double* nrm, const
                                 float* tangents_out, float* colors_out, uint32_t* materials_out, uint8_t* flags_out,
                                 uint8_t* sides_out, float* bounds_out, int* nodes_out, uint32_t* order_out,
                                 int* node_count_out, double* epsilon_out, int* any_colors, cudaStream_t s) {
+  bvh_count_ = -1;
   int any = 0;
   for (int i = 0; i < n && has_color && colors; i++) any |= has_color[i] ? 1 : 0;
   *any_colors = any;

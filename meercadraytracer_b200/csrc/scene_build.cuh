@@ -63,8 +63,12 @@ class SceneBuilder {
   int build_device(const float* d_tris, int n, float* d_bounds, int* d_nodes, uint32_t* d_order, cudaStream_t s,
                    int bins = 16);
 
-  // buildBvh from and to host arrays.
-  int build_bvh_host(const float* tris, int n, float* bounds, int* nodes, uint32_t* order, cudaStream_t s);
+  // buildBvh from host arrays; the hierarchy stays on the device, until the
+  // next build of any kind, for read_bvh. Returns the node count.
+  int build_bvh_host(const float* tris, int n, cudaStream_t s);
+  // The nodes and triangle order of build_bvh_host's hierarchy; false if there
+  // is none.
+  bool read_bvh(float* bounds, int* nodes, uint32_t* order, cudaStream_t s);
 
   // compileGeometry after the flatten, from and to host arrays.
   void compile_host(int n, const double* p, const double* nrm, const double* uv, const double* colors,
@@ -94,6 +98,7 @@ class SceneBuilder {
  private:
   BuildBuffers* b_;
   int last_levels_ = 0;
+  int bvh_count_ = -1, bvh_nodes_ = 0;  // triangles and nodes of the hierarchy that read_bvh reads
 };
 
 }  // namespace mcrt

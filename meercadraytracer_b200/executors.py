@@ -301,16 +301,18 @@ class GpuExecutor:
     def build_bvh(self, triangles: np.ndarray, count: int) -> Tuple[CompiledBvh, np.ndarray]:
         """buildBvh (src/bvh.ts:16-178) on the GPU."""
         tris = np.ascontiguousarray(triangles, np.float32)
-        cap = max(1, 2 * count - 1)
-        bounds = pinned.empty(cap * 6, np.float32)
-        nodes = pinned.empty(cap * 3, np.int32)
-        order = pinned.empty(max(1, count), np.uint32)
         m = C.c_int32()
         with self._lock:
-            call("mcrt_build_bvh", self._h, abi.ptr(tris, C.c_float), int(count), abi.ptr(bounds, C.c_float),
-                 abi.ptr(nodes, C.c_int32), abi.ptr(order, C.c_uint32), C.byref(m))
-        k = int(m.value)
-        return CompiledBvh(bounds[: k * 6], nodes[: k * 3], k), order[:count]
+            # In two steps, so that a kept hierarchy holds the memory of its nodes, not of the most there could be.
+            call("mcrt_bvh_build", self._h, abi.ptr(tris, C.c_float), int(count), C.byref(m))
+            k = int(m.value)
+            bounds = pinned.empty(k * 6, np.float32)
+            nodes = pinned.empty(k * 3, np.int32)
+            order = pinned.empty(int(count), np.uint32)
+            if k:
+                call("mcrt_bvh_read", self._h, abi.ptr(bounds, C.c_float), abi.ptr(nodes, C.c_int32),
+                     abi.ptr(order, C.c_uint32))
+        return CompiledBvh(bounds, nodes, k), order
 
     def compile_sink(self, sink: Any) -> CompiledGeometry:
         """compileGeometry after the flatten (src/compile.ts:359-403) on the GPU."""
