@@ -594,7 +594,9 @@ int32_t mcrt_host_alloc(size_t bytes, void** out) {
   return guard([&] {
     if (!out) fail(MCRT_ERR_INVALID, "out is NULL");
     *out = nullptr;
-    cuda_check(cudaHostAlloc(out, std::max<size_t>(bytes, 1), cudaHostAllocPortable), "pinned host memory");
+    const cudaError_t e = cudaHostAlloc(out, std::max<size_t>(bytes, 1), cudaHostAllocPortable);
+    if (e != cudaSuccess) cudaGetLastError();  // callers go on without: the next launch's check must not find it
+    cuda_check(e, "pinned host memory");
   });
 }
 
