@@ -69,6 +69,10 @@ int32_t mcrt_device_count(int32_t* count);
  * memory copies straight into it, without the runtime's staging, and batched
  * images arrive while the host goes on. Any host memory may be used instead. */
 int32_t mcrt_host_alloc(size_t bytes, void** out);
+/* The same from `device`, which is made current as every call on an executor
+ * makes its own: a thread that has not used a device yet would make a context
+ * on device 0 otherwise. */
+int32_t mcrt_host_alloc_on(int32_t device, size_t bytes, void** out);
 int32_t mcrt_host_free(void* p);
 
 /* new WorkerExecutor(...) / createTileHandler(), src/executors.ts:54-94,

@@ -59,6 +59,7 @@ SIGNATURES = {
     "mcrt_version": (_i32, []),
     "mcrt_device_count": (_i32, [_P(_i32)]),
     "mcrt_host_alloc": (_i32, [C.c_size_t, _P(_vp)]),
+    "mcrt_host_alloc_on": (_i32, [_i32, C.c_size_t, _P(_vp)]),
     "mcrt_host_free": (_i32, [_vp]),
     "mcrt_executor_create": (_i32, [_i32, _P(_vp)]),
     "mcrt_executor_destroy": (_i32, [_vp]),

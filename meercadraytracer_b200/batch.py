@@ -118,9 +118,9 @@ class BatchRenderer:
 
     def submit(self, r: RenderRequest) -> int:
         """Queues a request; returns its id. Its images are result(id) / preview(id) / progress(id)."""
-        image = pinned.zeros(r.width * r.height * 4, np.uint8)
-        preview = pinned.zeros(r.width * r.height * 4, np.uint8) if r.preview_block > 1 else None
-        progress = pinned.zeros(r.width * r.height * 4, np.uint8) if r.progress else None
+        image = pinned.zeros(r.width * r.height * 4, np.uint8, self.device)
+        preview = pinned.zeros(r.width * r.height * 4, np.uint8, self.device) if r.preview_block > 1 else None
+        progress = pinned.zeros(r.width * r.height * 4, np.uint8, self.device) if r.progress else None
         return self._submit_c(self._c_request(r, image, preview, progress), (image, preview, progress))
 
     def submit_to(self, executor: GpuExecutor, versions: Tuple[int, int], camera: CompiledCamera,
@@ -128,9 +128,9 @@ class BatchRenderer:
                   srgb: bool = True, progress: bool = False) -> int:
         """As submit, for a scene that `executor` already holds under `versions` (geometry, shading),
         as SceneSync.sync leaves it."""
-        image = pinned.zeros(width * height * 4, np.uint8)
-        preview = pinned.zeros(width * height * 4, np.uint8) if preview_block > 1 else None
-        prog = pinned.zeros(width * height * 4, np.uint8) if progress else None
+        image = pinned.zeros(width * height * 4, np.uint8, self.device)
+        preview = pinned.zeros(width * height * 4, np.uint8, self.device) if preview_block > 1 else None
+        prog = pinned.zeros(width * height * 4, np.uint8, self.device) if progress else None
         c = self._c_fields(executor, versions, camera, settings, width, height, samples, preview_block, srgb, image,
                            preview, prog)
         return self._submit_c(c, (image, preview, prog))
@@ -178,7 +178,7 @@ class BatchRenderer:
 
     def render(self, requests: Sequence[RenderRequest]) -> List[np.ndarray]:
         """Renders every request to completion in one batch (mcrt_batch_render)."""
-        images = [pinned.empty(r.width * r.height * 4, np.uint8) for r in requests]
+        images = [pinned.empty(r.width * r.height * 4, np.uint8, self.device) for r in requests]
         arr = (abi.mcrt_request * max(1, len(requests)))()
         for i, r in enumerate(requests):
             arr[i] = self._c_request(r, images[i], None)

@@ -600,6 +600,11 @@ int32_t mcrt_host_alloc(size_t bytes, void** out) {
   });
 }
 
+int32_t mcrt_host_alloc_on(int32_t device, size_t bytes, void** out) {
+  const int32_t r = guard([&] { cuda_check(cudaSetDevice(device), "cudaSetDevice"); });
+  return r == MCRT_OK ? mcrt_host_alloc(bytes, out) : r;
+}
+
 int32_t mcrt_host_free(void* p) {
   return guard([&] {
     if (p) cuda_check(cudaFreeHost(p), "pinned host memory");

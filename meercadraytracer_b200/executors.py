@@ -137,7 +137,7 @@ class GpuExecutor:
 
     def _render_tile(self, m: Dict[str, Any]) -> np.ndarray:
         tile: Tile = m["tile"]
-        out = pinned.zeros(tile.width * tile.height * 4, np.float32)
+        out = pinned.zeros(tile.width * tile.height * 4, np.float32, self.device)
         cam = abi.to_c_camera(m["camera"])
         st = abi.to_c_settings(m["settings"])
         t = abi.to_c_tile(tile)
@@ -190,7 +190,7 @@ class GpuExecutor:
                  settings: TraceSettings, samples: int = 16, srgb: bool = True) -> np.ndarray:
         """raytraceCompiled (src/raytrace.ts:69-82) on the device: RGBA8 bytes."""
         gv, sv = self.load_scene(scene)
-        out = pinned.empty(width * height * 4, np.uint8)
+        out = pinned.empty(width * height * 4, np.uint8, self.device)
         cam, st = abi.to_c_camera(camera), abi.to_c_settings(settings)
         with self._lock:
             call("mcrt_raytrace", self._h, gv, sv, C.byref(cam), C.byref(st), int(width), int(height), int(samples),
@@ -218,7 +218,7 @@ class GpuExecutor:
                 call("mcrt_raytrace_device", self._h, gv, sv, C.byref(cam), C.byref(st), int(width), int(height),
                      int(samples), int(bool(srgb)), C.c_void_p(device_ptr))
                 return None
-            out = pinned.empty(width * height * 4, np.uint8)
+            out = pinned.empty(width * height * 4, np.uint8, self.device)
             call("mcrt_raytrace", self._h, gv, sv, C.byref(cam), C.byref(st), int(width), int(height), int(samples),
                  int(bool(srgb)), abi.ptr(out, C.c_uint8))
             return out
@@ -261,10 +261,10 @@ class GpuExecutor:
         """intersectClosest for rays [n, 8] (origin, -, direction, -) on the resident geometry."""
         rays = np.ascontiguousarray(rays, np.float32)
         n = rays.shape[0]
-        tri = pinned.empty(n, np.int32)
-        t = pinned.empty(n, np.float32)
-        u = pinned.empty(n, np.float32)
-        front = pinned.empty(n, np.int32)
+        tri = pinned.empty(n, np.int32, self.device)
+        t = pinned.empty(n, np.float32, self.device)
+        u = pinned.empty(n, np.float32, self.device)
+        front = pinned.empty(n, np.int32, self.device)
         with self._lock:
             call("mcrt_intersect_closest", self._h, int(geometry_version), n, abi.ptr(rays, C.c_float), int(cull),
                  abi.ptr(tri, C.c_int32), abi.ptr(t, C.c_float), abi.ptr(u, C.c_float), abi.ptr(front, C.c_int32))
@@ -291,7 +291,7 @@ class GpuExecutor:
     def intersect_any_count(self, geometry_version: int, rays: np.ndarray) -> np.ndarray:
         rays = np.ascontiguousarray(rays, np.float32)
         n = rays.shape[0]
-        counts = pinned.empty(n, np.int32)
+        counts = pinned.empty(n, np.int32, self.device)
         with self._lock:
             call("mcrt_intersect_any_count", self._h, int(geometry_version), n, abi.ptr(rays, C.c_float),
                  abi.ptr(counts, C.c_int32))
@@ -306,9 +306,9 @@ class GpuExecutor:
             # In two steps, so that a kept hierarchy holds the memory of its nodes, not of the most there could be.
             call("mcrt_bvh_build", self._h, abi.ptr(tris, C.c_float), int(count), C.byref(m))
             k = int(m.value)
-            bounds = pinned.empty(k * 6, np.float32)
-            nodes = pinned.empty(k * 3, np.int32)
-            order = pinned.empty(int(count), np.uint32)
+            bounds = pinned.empty(k * 6, np.float32, self.device)
+            nodes = pinned.empty(k * 3, np.int32, self.device)
+            order = pinned.empty(int(count), np.uint32, self.device)
             if k:
                 call("mcrt_bvh_read", self._h, abi.ptr(bounds, C.c_float), abi.ptr(nodes, C.c_int32),
                      abi.ptr(order, C.c_uint32))

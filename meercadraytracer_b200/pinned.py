@@ -25,7 +25,7 @@ import ctypes as C
 import operator
 import threading
 import weakref
-from typing import Any, Dict, List
+from typing import Any, Dict, List, Optional
 
 import numpy as np
 
@@ -50,8 +50,9 @@ class _Pool:
         step = 1 << max(12, nbytes.bit_length() - 3)
         return -(-nbytes // step) * step
 
-    def take(self, size: int) -> int:
-        """Address of a block of `size` bytes, or 0 when the limit leaves no room or too few were dropped."""
+    def take(self, size: int, device: Optional[int] = None) -> int:
+        """Address of a block of `size` bytes, or 0 when the limit leaves no room or too few were dropped.
+        A new one is allocated from `device`; any device may copy into it."""
         with self._lock:
             blocks = self._free.get(size)
             if blocks:
@@ -76,7 +77,10 @@ class _Pool:
             return 0
         p = C.c_void_p()
         try:
-            call("mcrt_host_alloc", size, C.byref(p))
+            if device is None:
+                call("mcrt_host_alloc", size, C.byref(p))
+            else:
+                call("mcrt_host_alloc_on", int(device), size, C.byref(p))
         except McrtError:
             with self._lock:
                 self._held -= size
@@ -93,7 +97,7 @@ class _Pool:
         with self._lock:
             self._fresh[size] = min(self._fresh.get(size, FRESH) + 1, FRESH + self._blocks.get(size, 0))
 
-    def empty(self, count: int, dtype: Any) -> np.ndarray:
+    def empty(self, count: int, dtype: Any, device: Optional[int] = None) -> np.ndarray:
         count, dtype = operator.index(count), np.dtype(dtype)
         nbytes = count * dtype.itemsize
         if nbytes < SMALL:
@@ -101,7 +105,7 @@ class _Pool:
         size = self.block_size(nbytes)
         if size > LIMIT:
             return np.empty(count, dtype)
-        address = self.take(size)
+        address = self.take(size, device)
         if not address:
             plain = np.empty(count, dtype)
             weakref.finalize(plain, self.dropped, size).atexit = False
@@ -115,12 +119,12 @@ class _Pool:
 _pool = _Pool()
 
 
-def empty(count: int, dtype: Any) -> np.ndarray:
-    """An uninitialised one-dimensional array, in pinned memory where that is worth it."""
-    return _pool.empty(count, dtype)
+def empty(count: int, dtype: Any, device: Optional[int] = None) -> np.ndarray:
+    """An uninitialised one-dimensional array, in pinned memory where that is worth it, for results of `device`."""
+    return _pool.empty(count, dtype, device)
 
 
-def zeros(count: int, dtype: Any) -> np.ndarray:
-    a = _pool.empty(count, dtype)
+def zeros(count: int, dtype: Any, device: Optional[int] = None) -> np.ndarray:
+    a = _pool.empty(count, dtype, device)
     a.fill(0)
     return a
