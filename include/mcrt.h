@@ -67,7 +67,8 @@ int32_t mcrt_device_count(int32_t* count);
 
 /* Pinned host memory, for results: every function that writes into host
  * memory copies straight into it, without the runtime's staging, and batched
- * images arrive while the host goes on. Any host memory may be used instead. */
+ * images arrive while the host goes on. Any host memory may be used instead.
+ * It is zeroed and page aligned, and any thread may free it. */
 int32_t mcrt_host_alloc(size_t bytes, void** out);
 /* The same from `device`, which is made current as every call on an executor
  * makes its own: a thread that has not used a device yet would make a context

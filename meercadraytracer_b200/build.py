@@ -27,9 +27,10 @@ SOURCES = {
     "render.cu": [],
     "executor.cu": [],
     "batch.cu": [],
+    "host_memory.cu": [],
     "scene_build.cu": ["--fmad=false"],
 }
-HEADERS = ["mcrt_math.cuh", "device_scene.cuh", "traverse.cuh", "render.cuh", "scene_build.cuh", "batch.cuh", "dfg_lut.h"]
+HEADERS = ["mcrt_math.cuh", "device_scene.cuh", "traverse.cuh", "render.cuh", "scene_build.cuh", "batch.cuh", "host_memory.cuh", "dfg_lut.h"]
 
 
 def nvcc() -> str:

@@ -22,6 +22,7 @@
 
 #include "batch.cuh"
 #include "dfg_lut.h"
+#include "host_memory.cuh"
 #include "mcrt.h"
 #include "render.cuh"
 #include "scene_build.cuh"
@@ -594,9 +595,7 @@ int32_t mcrt_host_alloc(size_t bytes, void** out) {
   return guard([&] {
     if (!out) fail(MCRT_ERR_INVALID, "out is NULL");
     *out = nullptr;
-    const cudaError_t e = cudaHostAlloc(out, std::max<size_t>(bytes, 1), cudaHostAllocPortable);
-    if (e != cudaSuccess) cudaGetLastError();  // callers go on without: the next launch's check must not find it
-    cuda_check(e, "pinned host memory");
+    cuda_check(host_alloc(bytes, out), "pinned host memory");
   });
 }
 
@@ -607,7 +606,7 @@ int32_t mcrt_host_alloc_on(int32_t device, size_t bytes, void** out) {
 
 int32_t mcrt_host_free(void* p) {
   return guard([&] {
-    if (p) cuda_check(cudaFreeHost(p), "pinned host memory");
+    if (p && !host_free(p)) fail(MCRT_ERR_INVALID, "not memory of mcrt_host_alloc, or freed before");
   });
 }
 

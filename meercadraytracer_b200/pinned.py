@@ -8,13 +8,14 @@ of it) is gone, so a program that drops each frame's image reuses one block.
 The pool holds at most LIMIT bytes, in use or not; beyond that, and for small
 arrays, `empty` is numpy's own.
 
-Allocating a block costs more than it saves once (0.4 ms a MB: a 1080p image
-into a new block 5.2 ms, into ordinary memory 3.6, into a block used before
-1.5), so new blocks are for programs whose results come back: a size has FRESH
-new blocks to begin with, and earns one more with each result of that size that
-is dropped, whichever memory it was in, at most FRESH more than it has. A program that keeps its results gets ordinary
-memory after that: twelve images kept from each batch 25 ms a batch with a new
-block for each, 12.8 with this.
+A new block costs its pages (host_memory.cu): a 1080p image into a new block
+3.3 ms, into ordinary memory 4.0, into a block used before 1.5; of results below
+a megabyte some pay 0.3 to 1 ms for a slab that others are cut from. So new
+blocks are for programs whose results come back: a size has FRESH new blocks to
+begin with, and earns one more with each result of that size that is dropped,
+whichever memory it was in, at most FRESH more than it has. A program that keeps
+its results gets ordinary memory after that: the pool's room is for those that
+return.
 
 A block is handed out again as soon as its arrays are gone, so whoever queues a
 copy into one keeps the array until that copy is done.
