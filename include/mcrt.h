@@ -75,6 +75,12 @@ int32_t mcrt_host_alloc(size_t bytes, void** out);
  * on device 0 otherwise. */
 int32_t mcrt_host_alloc_on(int32_t device, size_t bytes, void** out);
 int32_t mcrt_host_free(void* p);
+/* Room for `bytes` of it, all blocks together, made ahead: allocations then ask
+ * nothing of the driver, which may let a thread that serves renders wait. The
+ * largest reservation counts; the room goes back with the last
+ * mcrt_host_unreserve and its last block. */
+int32_t mcrt_host_reserve(int32_t device, size_t bytes);
+int32_t mcrt_host_unreserve(void);
 
 /* new WorkerExecutor(...) / createTileHandler(), src/executors.ts:54-94,
  * src/protocol.ts:55: an executor on `device`. */

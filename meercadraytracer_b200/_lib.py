@@ -61,6 +61,8 @@ SIGNATURES = {
     "mcrt_host_alloc": (_i32, [C.c_size_t, _P(_vp)]),
     "mcrt_host_alloc_on": (_i32, [_i32, C.c_size_t, _P(_vp)]),
     "mcrt_host_free": (_i32, [_vp]),
+    "mcrt_host_reserve": (_i32, [_i32, C.c_size_t]),
+    "mcrt_host_unreserve": (_i32, []),
     "mcrt_executor_create": (_i32, [_i32, _P(_vp)]),
     "mcrt_executor_destroy": (_i32, [_vp]),
     "mcrt_send_geometry": (_i32, [_vp, _i32, _P(abi.mcrt_geometry)]),

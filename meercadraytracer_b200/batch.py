@@ -23,7 +23,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import numpy as np
 
 from . import abi, pinned
-from ._lib import call, load
+from ._lib import McrtError, call, load
 from .executors import GpuExecutor
 from .types import CompiledCamera, CompiledScene, TraceSettings
 
@@ -47,6 +47,10 @@ class RenderRequest:
     progress: bool = False  # copy the image to the host after every completed pass (scheduled pass by pass)
 
 
+# The most pinned memory a batch makes ahead for its requests' images: 25 ms once.
+RESERVE = 128 << 20
+
+
 class BatchRenderer:
     """A batch engine on one device with the scenes it has seen kept resident."""
 
@@ -59,6 +63,14 @@ class BatchRenderer:
         self._h = handle
         self.device = device
         self.capacity = int(capacity)
+        # Requests' images are allocated while chunks run; their memory is not. A request of P pixels
+        # takes 20 P bytes of the budget and has up to three images of 4 P.
+        self._reserved = False
+        try:
+            call("mcrt_host_reserve", int(device), min(RESERVE, int(memory_budget) // 16))
+            self._reserved = True
+        except McrtError:
+            pass  # new blocks as they are needed, or ordinary memory
         self._executors: Dict[int, Tuple[CompiledScene, GpuExecutor]] = {}
         self._buffers: Dict[int, Tuple[np.ndarray, Optional[np.ndarray], Optional[np.ndarray]]] = {}
         self._adopted: set = set()
@@ -205,6 +217,9 @@ class BatchRenderer:
             call("mcrt_batch_destroy", self._h)  # waits for what is in flight
             self._h = None
         self._retired = []
+        if self._reserved:
+            self._reserved = False
+            call("mcrt_host_unreserve")
         for _, ex in self._executors.values():
             if id(ex) not in self._adopted:
                 ex.dispose()

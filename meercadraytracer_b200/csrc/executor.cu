@@ -610,6 +610,17 @@ int32_t mcrt_host_free(void* p) {
   });
 }
 
+int32_t mcrt_host_reserve(int32_t device, size_t bytes) {
+  return guard([&] {
+    cuda_check(cudaSetDevice(device), "cudaSetDevice");
+    cuda_check(host_reserve(bytes), "pinned host memory");
+  });
+}
+
+int32_t mcrt_host_unreserve(void) {
+  return guard([&] { host_unreserve(); });
+}
+
 int32_t mcrt_executor_create(int32_t device, mcrt_executor** out) {
   return guard([&] {
     if (!out) fail(MCRT_ERR_INVALID, "out is NULL");

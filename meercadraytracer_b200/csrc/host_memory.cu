@@ -9,6 +9,11 @@
 // (15.6). A small block costs 0.3 ms for the locking alone, 64 KB or 1 MB alike
 // (0.95 and 1.6 from the runtime), so small blocks are cut from slabs.
 //
+// Either can take far longer, since the driver serves one memory call at a time
+// for all processes on the machine: 20-110 ms now and then, once half a second,
+// which a served client saw as the wait for its preview. So programs that
+// allocate while chunks run reserve room ahead (host_reserve).
+//
 // And it is the process's own memory: a forked child has a copy of what was in
 // it, where it shares the runtime's with the parent's later results.
 #include "host_memory.cuh"
@@ -21,6 +26,7 @@
 #include <memory>
 #include <mutex>
 #include <thread>
+#include <vector>
 
 namespace mcrt {
 namespace {
@@ -37,6 +43,7 @@ struct Mapping {
   int device = 0;                 // whose context locked it
   std::map<size_t, size_t> free;  // a slab's free ranges: offset -> length
   size_t used = 0;
+  bool reserved = false;
 };
 
 struct Block {
@@ -48,6 +55,8 @@ struct HostMemory {
   std::mutex mu;
   std::map<char*, std::unique_ptr<Mapping>> mappings;
   std::map<char*, Block> blocks;  // handed out
+  size_t reserved = 0;            // bytes of the reserved mappings
+  int reservations = 0;
 };
 
 // Never destroyed: blocks may come back while the process ends.
@@ -148,14 +157,12 @@ cudaError_t host_alloc(size_t bytes, void** out) {
   const bool slab = bytes <= kSlabBlock;
   std::unique_ptr<Mapping> made;
   std::unique_lock<std::mutex> lock(h.mu);
-  if (slab) {
-    for (auto& m : h.mappings) {
-      char* p = cut(*m.second, bytes);
-      if (!p) continue;
-      h.blocks[p] = Block{m.second.get(), bytes};
-      *out = p;
-      return cudaSuccess;
-    }
+  for (auto& m : h.mappings) {
+    char* p = cut(*m.second, bytes);
+    if (!p) continue;
+    h.blocks[p] = Block{m.second.get(), bytes};
+    *out = p;
+    return cudaSuccess;
   }
   lock.unlock();  // the driver is not waited for under the lock
   const cudaError_t e = map_pinned(slab ? kSlab : bytes, &made);
@@ -180,7 +187,7 @@ bool host_free(void* pointer) {
     const Block b = it->second;
     uncut(*b.in, it->first, b.bytes);
     h.blocks.erase(it);
-    if (b.in->used == 0) {  // the last block of its mapping
+    if (b.in->used == 0 && !b.in->reserved) {  // the last block of its mapping
       const auto m = h.mappings.find(b.in->base);
       gone = std::move(m->second);
       h.mappings.erase(m);
@@ -188,6 +195,52 @@ bool host_free(void* pointer) {
   }
   if (gone) unmap_pinned(*gone);
   return true;
+}
+
+cudaError_t host_reserve(size_t bytes) {
+  if (bytes > SIZE_MAX / 2) return cudaErrorMemoryAllocation;
+  bytes = (std::max<size_t>(bytes, 1) + kPage - 1) / kPage * kPage;
+  HostMemory& h = memory();
+  std::unique_lock<std::mutex> lock(h.mu);
+  const size_t have = h.reserved;
+  h.reservations++;
+  if (have >= bytes) return cudaSuccess;
+  h.reserved = bytes;  // another thread's reservation counts on it meanwhile
+  lock.unlock();
+  std::unique_ptr<Mapping> made;
+  const cudaError_t e = map_pinned(bytes - have, &made);
+  lock.lock();
+  if (e != cudaSuccess) {
+    h.reserved -= bytes - have;
+    h.reservations--;
+    return e;
+  }
+  made->free[0] = made->bytes;
+  made->reserved = true;
+  char* base = made->base;
+  h.mappings[base] = std::move(made);
+  return cudaSuccess;
+}
+
+void host_unreserve() {
+  HostMemory& h = memory();
+  std::vector<std::unique_ptr<Mapping>> gone;
+  {
+    std::lock_guard<std::mutex> lock(h.mu);
+    if (h.reservations == 0 || --h.reservations > 0) return;
+    h.reserved = 0;
+    for (auto it = h.mappings.begin(); it != h.mappings.end();) {
+      Mapping& m = *it->second;
+      m.reserved = false;
+      if (m.used == 0) {
+        gone.push_back(std::move(it->second));
+        it = h.mappings.erase(it);
+      } else {
+        ++it;
+      }
+    }
+  }
+  for (const auto& m : gone) unmap_pinned(*m);
 }
 
 }  // namespace mcrt

@@ -14,4 +14,10 @@ cudaError_t host_alloc(size_t bytes, void** out);
 // if `p` is not from host_alloc.
 bool host_free(void* p);
 
+// Makes room for at least `bytes` of blocks ahead, with the current device, so
+// that host_alloc needs nothing of the driver until it is used up. Kept until
+// as many host_unreserve calls have been made, and its blocks are back.
+cudaError_t host_reserve(size_t bytes);
+void host_unreserve();
+
 }  // namespace mcrt
