@@ -61,6 +61,7 @@ class BatchRenderer:
         call("mcrt_batch_create", int(device), int(capacity), int(memory_budget), int(bool(use_graph)),
              C.byref(handle))
         self._h = handle
+        pinned.attach()
         self.device = device
         self.capacity = int(capacity)
         # Requests' images are allocated while chunks run; their memory is not. A request of P pixels
@@ -216,6 +217,7 @@ class BatchRenderer:
         if self._h is not None:
             call("mcrt_batch_destroy", self._h)  # waits for what is in flight
             self._h = None
+            pinned.detach()
         self._retired = []
         if self._reserved:
             self._reserved = False

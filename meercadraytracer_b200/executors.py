@@ -70,6 +70,7 @@ class GpuExecutor:
         handle = C.c_void_p()
         call("mcrt_executor_create", int(device), C.byref(handle))
         self._h = handle
+        pinned.attach()
         self.device = device
         self.textures: Set[int] = set()  # texture ids this executor holds (TileExecutor.textures)
         self._pending_pixels: Dict[int, np.ndarray] = {}
@@ -155,6 +156,7 @@ class GpuExecutor:
         self._worker.shutdown(wait=True)
         call("mcrt_executor_destroy", self._h)
         self._h = None
+        pinned.detach()
 
     def __del__(self):  # pragma: no cover - best effort
         try:

@@ -6,7 +6,8 @@ caller waits, and a large new array's pages fault in on the way. `empty` gives
 numpy arrays on blocks of a pool: a block returns when its last array (or view
 of it) is gone, so a program that drops each frame's image reuses one block.
 The pool holds at most LIMIT bytes, in use or not; beyond that, and for small
-arrays, `empty` is numpy's own.
+arrays, `empty` is numpy's own. It gives its memory back when the last executor
+and batch are disposed.
 
 A new block costs its pages (host_memory.cu): a 1080p image into a new block
 3.3 ms, into ordinary memory 4.0, into a block used before 1.5; of results below
@@ -44,6 +45,30 @@ class _Pool:
         self._held = 0  # bytes of all blocks, in use or free
         self._blocks: Dict[int, int] = {}  # blocks of each size, in use or free
         self._fresh: Dict[int, int] = {}  # new blocks each size may still have
+        self.users = 0  # executors and batches
+        self._closed = False  # the last of them is gone
+
+    def attach(self) -> None:
+        """An executor or a batch begins to ask for results."""
+        with self._lock:
+            self.users += 1
+            self._closed = False
+
+    def detach(self) -> None:
+        """It is disposed: with the last one the free blocks go back, and those in use as they are dropped."""
+        with self._lock:
+            self.users -= 1
+            if self.users > 0:
+                return
+            self._closed = True
+            gone = [(size, p) for size, free in self._free.items() for p in free]
+            self._free.clear()
+            self._fresh.clear()
+            for size, _ in gone:
+                self._held -= size
+                self._blocks[size] -= 1
+        for _, p in gone:
+            call("mcrt_host_free", C.c_void_p(p))
 
     @staticmethod
     def block_size(nbytes: int) -> int:
@@ -91,8 +116,13 @@ class _Pool:
 
     def give(self, address: int, size: int) -> None:
         with self._lock:
-            self._free.setdefault(size, []).append(address)
-            self.dropped(size)
+            if not self._closed:
+                self._free.setdefault(size, []).append(address)
+                self.dropped(size)
+                return
+            self._held -= size
+            self._blocks[size] -= 1
+        call("mcrt_host_free", C.c_void_p(address))
 
     def dropped(self, size: int) -> None:
         with self._lock:
@@ -118,6 +148,15 @@ class _Pool:
 
 
 _pool = _Pool()
+
+
+def attach() -> None:
+    """Before an executor's or a batch's first result; detach() once it is disposed."""
+    _pool.attach()
+
+
+def detach() -> None:
+    _pool.detach()
 
 
 def empty(count: int, dtype: Any, device: Optional[int] = None) -> np.ndarray:
