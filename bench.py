@@ -606,6 +606,8 @@ def run_large(device: int, count: int, frames: int, bins: int = 32, tune: bool =
                 from meercadraytracer_b200._lib import traversal_variants
 
                 for b_, s_ in traversal_variants():
+                    if any(k_.startswith(f"{b_}x") for k_ in variant_ms):
+                        continue  # pairs of one block size name the same kernels
                     ex.set_traversal(b_, s_)
                     ex.reset_stats()
                     ex.raytrace_resident((info["version"], sv), cam, L.width, L.height, st, spp, srgb,

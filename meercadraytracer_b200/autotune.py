@@ -87,6 +87,17 @@ def _store(cache_path: Optional[str], key: str, value: Dict[str, Any]) -> None:
     os.replace(tmp, cache_path)
 
 
+def _time_variants(variants: Sequence[Tuple[int, int]], use: Callable[[int, int], None],
+                   timed: Callable[[], float]) -> Dict[Tuple[int, int], float]:
+    """The time of each variant, measured once per kernel: pairs of one block size name the same one."""
+    by_block: Dict[int, float] = {}
+    for b, s in variants:
+        if b not in by_block:
+            use(b, s)
+            by_block[b] = timed()
+    return {(b, s): by_block[b] for b, s in variants}
+
+
 def _best(timings: Dict[Any, float]) -> Any:
     return min(timings, key=lambda k: timings[k])
 
@@ -123,10 +134,7 @@ def tune_plain(executor: Any, scene: CompiledScene, camera: CompiledCamera, sett
     variants = list(variants or traversal_variants())
     executor.set_capacity(max(capacities))
     executor.raytrace(scene, camera, width, height, settings, 1, True)  # warm-up: scene resident, buffers sized
-    tv: Dict[Tuple[int, int], float] = {}
-    for b, s in variants:
-        executor.set_traversal(b, s)
-        tv[(b, s)] = timed()
+    tv = _time_variants(variants, executor.set_traversal, timed)
     block, stack = _best(tv)
     executor.set_traversal(block, stack)
     tc: Dict[int, float] = {}
@@ -164,10 +172,7 @@ def tune_batch(renderer: Any, requests: Sequence[Any], chunks: Optional[Sequence
 
     variants = list(variants or traversal_variants())
     renderer.render(requests[:1])  # warm-up: graph, scenes resident
-    tv: Dict[Tuple[int, int], float] = {}
-    for b, s in variants:
-        renderer.set_traversal(b, s)
-        tv[(b, s)] = timed()
+    tv = _time_variants(variants, renderer.set_traversal, timed)
     block, stack = _best(tv)
     renderer.set_traversal(block, stack)
     half = capacity // 2  # two chunks share the pool
