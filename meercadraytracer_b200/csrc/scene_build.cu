@@ -39,7 +39,8 @@ constexpr int kBuildBlock = 256;
 // 12 measured best of 6 to 32 (16.4 M triangles rebuilt and traced: 44.8 ms at
 // 6, 40.8 at 12, 42.0 at 16, 59.8 at 32).
 constexpr int kTinyMax = 12;
-constexpr int kWideMin = 1 << 15;  // see BuildCtl::slot_depth
+// Of nodes of at least kWideMin triangles small children count as a level (BuildCtl::slot_depth).
+constexpr int kWideMin = 1 << 15;
 
 void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
@@ -206,7 +207,10 @@ struct BuildCtl {
   LevelCtl level[kLevels + 1];
   int subtrees, next_subtree;
   int inner_depth;   // deepest inner node, -1 for none
-  int slot_depth;    // deepest node that is not a leaf its parent's split already decided
+  // The depth that the reported level count goes by: of the deepest node that
+  // is split, or is a leaf only by its cost, or is a small child of a node of
+  // kWideMin triangles. The build itself does not use it.
+  int slot_depth;
   int inner_nodes;   // set by k_rank_write
 };
 
@@ -671,7 +675,6 @@ __global__ void __launch_bounds__(B, 1024 / B) k_bin(int level, BuildState st) {
             const int t = atomicAdd(&st.ctl->subtrees, 1);
             st.subtrees[t] = Subtree{nfirst + (q ? nleft : 0), kids[q], depth + 1,
                                      2u * static_cast<unsigned>(nfirst) + q, (level + 1) & 1};
-            // A wide node's small children were nodes of the next level.
             if (ncount >= kWideMin) deepest = depth + 1;
           }
           nd.child[q] = s_child[q];

@@ -34,14 +34,14 @@ def test_a_slow_reader_sees_the_image_its_event_names(small, passes, use_graph):
     from meercadraytracer_b200.executors import GpuExecutor
 
     compiled, cam, st = small
-    # Dropped results earn pinned blocks: until the request's three images get them.
-    for _ in range(20):
-        blocks = [pinned.empty(W * H * 4, np.uint8) for _ in range(3 + 2 * pinned.FRESH)]
-        del blocks
     ex = GpuExecutor(0)
     renderer = BatchRenderer(0, capacity=2 * passes * W * H, memory_budget=64 << 20, use_graph=use_graph)
     try:
-        want = {n: ex.raytrace(compiled, cam, W, H, st, n, True) for n in range(passes, SAMPLES + 1, passes)}
+        want = {n: ex.raytrace(compiled, cam, W, H, st, n, True).copy() for n in range(passes, SAMPLES + 1, passes)}
+        # Dropped results earn pinned blocks: until the request's three images get them.
+        for _ in range(20):
+            blocks = [pinned.empty(W * H * 4, np.uint8) for _ in range(3 + 2 * pinned.FRESH)]
+            del blocks
         rid = renderer.submit(RenderRequest(compiled, cam, W, H, st, SAMPLES, 4, progress=True))
         assert renderer.progress(rid).base is not None  # pinned
         seen, previews = [], 0
