@@ -376,14 +376,16 @@ class GpuExecutor:
         if len(instances):
             # The same memory as a numpy record array: one assignment per column.
             a = np.frombuffer(arr, abi.INSTANCE_DTYPE)
-            # Each row by itself: one of another length is refused, wherever it stands.
-            rows = [(world, mesh, material, flag, side, flat) for world, mesh, material, flag, side, flat in instances]
-            worlds, meshes, materials, flags, sides, flats = zip(*rows)
+            # strict: a row of another length is refused, wherever it stands.
+            worlds, meshes, materials, flags, sides, flats = zip(*instances, strict=True)
             a["world"] = np.stack([np.asarray(w, np.float64).reshape(16) for w in worlds])
             # Narrowed as C does: the low bits of whatever integer is given.
-            low = (1 << 64) - 1
             for name, column in (("mesh", meshes), ("material", materials), ("flags", flags), ("side", sides)):
-                a[name] = np.array([int(v) & low for v in column], np.uint64).astype(a.dtype[name])
+                values = [int(v) for v in column]
+                try:
+                    a[name] = np.array(values, np.int64).astype(a.dtype[name])
+                except OverflowError:
+                    a[name] = np.array([v & 0xffffffff for v in values], np.uint64).astype(a.dtype[name])
             a["flat_shading"] = [int(bool(v)) for v in flats]
         self._versions += 1
         version = self._versions
