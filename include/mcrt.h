@@ -9,7 +9,8 @@
  * addon (or any FFI) binds these functions one to one.
  *
  * Conventions: every function returns MCRT_OK (0) or an error code, and
- * mcrt_last_error() then returns the message (per thread). Host pointers are
+ * mcrt_last_error() then returns the message (per thread); what the output
+ * arrays of a call that failed hold is unspecified. Host pointers are
  * borrowed for the duration of the call. Calls on one executor must not run
  * concurrently; separate executors are independent.
  */
@@ -68,7 +69,7 @@ int32_t mcrt_device_count(int32_t* count);
 /* Pinned host memory, for results: every function that writes into host
  * memory copies straight into it, without the runtime's staging, and batched
  * images arrive while the host goes on. Any host memory may be used instead.
- * It is zeroed and page aligned, and any thread may free it. */
+ * It is page aligned, and any thread may free it. */
 int32_t mcrt_host_alloc(size_t bytes, void** out);
 /* The same from `device`, which is made current as every call on an executor
  * makes its own: a thread that has not used a device yet would make a context

@@ -7,8 +7,8 @@
 
 namespace mcrt {
 
-// `bytes` of zeroed host memory that every device copies into directly, page
-// aligned, made with the current device. Any thread.
+// `bytes` of host memory that every device copies into directly, page aligned,
+// made with the current device. Any thread.
 cudaError_t host_alloc(size_t bytes, void** out);
 // Gives it back. Any thread; the caller's current device stays as it is. False
 // if `p` is not from host_alloc.
