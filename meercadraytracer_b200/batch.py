@@ -47,7 +47,7 @@ class RenderRequest:
     progress: bool = False  # copy the image to the host after every completed pass (scheduled pass by pass)
 
 
-# The most pinned memory a batch makes ahead for its requests' images: 25 ms once.
+# The most pinned memory a batch makes ahead for its requests' images: 20 ms once.
 RESERVE = 128 << 20
 
 

@@ -568,6 +568,7 @@ cudaError_t BatchEngine::launch(Chunk& c) {
   if (e == cudaSuccess) e = cudaEventRecord(c.done, st);
   if (e != cudaSuccess) return e;
   totals_.chunks++;
+  c.launched = true;
   c.passes_done.assign(c.segs.size(), 0);
   for (size_t j = 0; j < c.segs.size(); j++) {
     const SegmentPlan& s = c.segs[j];
@@ -601,6 +602,16 @@ cudaError_t BatchEngine::copy_out(Chunk& c) {
 }
 
 cudaError_t BatchEngine::finish(Chunk& c, std::vector<BatchEvent>& events) {
+  if (!c.launched) {
+    // Its launch failed: there is no image to deliver, so its requests end.
+    const cudaError_t stopped = cudaStreamSynchronize(stream_[c.slot]);
+    for (const SegmentPlan& s : c.segs) {
+      s.r->inflight--;
+      s.r->cancelled = true;
+    }
+    retire();
+    return stopped;
+  }
   cudaError_t e = copy_out(c);
   if (e == cudaSuccess) e = cudaEventSynchronize(c.done);
   if (e == cudaSuccess && !c.copies.empty()) e = cudaEventSynchronize(c.copied);
@@ -635,6 +646,12 @@ cudaError_t BatchEngine::finish(Chunk& c, std::vector<BatchEvent>& events) {
       events.push_back(BatchEvent{r.id, kEventProgress, c.passes_done[j]});
     }
   }
+  retire();
+  return cudaSuccess;
+}
+
+// Requests that have ended and are in no chunk return their buffers.
+void BatchEngine::retire() {
   for (auto it = requests_.begin(); it != requests_.end();) {
     Request& r = **it;
     if ((r.finished || r.cancelled) && r.inflight == 0) {
@@ -644,15 +661,18 @@ cudaError_t BatchEngine::finish(Chunk& c, std::vector<BatchEvent>& events) {
       ++it;
     }
   }
-  return cudaSuccess;
 }
 
 cudaError_t BatchEngine::finish_oldest(std::vector<BatchEvent>& events) {
   const cudaError_t e = finish(inflight_.front(), events);
   Chunk& done = inflight_.front();
   if (done.start) cudaEventDestroy(done.start);
-  if (held_done_) cudaEventDestroy(held_done_);
-  held_done_ = done.done;  // the next chunk's device time counts from here
+  if (done.launched) {
+    if (held_done_) cudaEventDestroy(held_done_);
+    held_done_ = done.done;  // the next chunk's device time counts from here
+  } else if (done.done) {
+    cudaEventDestroy(done.done);
+  }
   if (done.copied) cudaEventDestroy(done.copied);
   inflight_.pop_front();
   return e;
@@ -810,15 +830,7 @@ cudaError_t BatchEngine::render_whole(std::vector<BatchEvent>& events, bool* ren
     r->inflight = 0;
     r->branch = -1;
   }
-  for (auto it = requests_.begin(); it != requests_.end();) {
-    Request& r = **it;
-    if ((r.finished || r.cancelled) && r.inflight == 0) {
-      release(r);
-      it = requests_.erase(it);
-    } else {
-      ++it;
-    }
-  }
+  retire();
   *rendered = true;
   return cudaSuccess;
 }

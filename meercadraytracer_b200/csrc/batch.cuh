@@ -163,6 +163,7 @@ class BatchEngine {
     // Per segment: the pass count its image holds when the chunk ends, if
     // the chunk completes a pass of the request (else 0).
     std::vector<int> passes_done;
+    bool launched = false;              // all of it is queued
     bool copied_out = false;            // copy_out has run
     std::vector<Request*> copies;       // requests whose images it copies
   };
@@ -184,6 +185,7 @@ class BatchEngine {
   cudaError_t finish(Chunk& c, std::vector<BatchEvent>& events);
   cudaError_t finish_oldest(std::vector<BatchEvent>& events);
   void release(Request& r);
+  void retire();
 
   int device_ = 0;
   int capacity_ = 0, half_ = 0, chunk_paths_ = 0;
