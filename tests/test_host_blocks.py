@@ -1,6 +1,8 @@
 """mcrt_host_alloc: blocks of every size apart from one another, from any thread, and a forked child's own copy."""
 import ctypes as C
+import gc
 import os
+import signal
 import threading
 
 import numpy as np
@@ -94,11 +96,17 @@ def test_a_forked_child_keeps_its_image(gpu):
     assert image.base is not None  # pinned
     want, at = image.copy(), image.ctypes.data
     ready, go = os.pipe(), os.pipe()
-    child = os.fork()
-    if child == 0:  # memory only: no CUDA call in here
-        os.write(ready[1], b"x")
-        os.read(go[0], 1)
-        os._exit(0 if np.array_equal(image, want) else 1)
+    gc.collect()
+    gc.disable()  # no finalizer, and so no CUDA call, runs in the child
+    try:
+        child = os.fork()
+        if child == 0:  # memory only
+            signal.alarm(60)
+            os.write(ready[1], b"x")
+            os.read(go[0], 1)
+            os._exit(0 if np.array_equal(image, want) else 1)
+    finally:
+        gc.enable()
     os.read(ready[0], 1)
     del image
     later = gpu.raytrace(compiled, cam, 320, 240, trace_settings({"seed": 2}), 1, True)
